@@ -276,6 +276,82 @@ int fcfcg_axis_ftab(fcfcg_axis *a, int allow_log) {
   return FCFCG_OK;
 }
 
+/*
+ * Edge table: cells a fixed fraction of an octave wide (16 to 4096 per
+ * octave), each with the one edge that lies in it or within half its width
+ * of it, as a float, and the column below that edge (0 below the first edge,
+ * k + 1 in bin k).  A value of the cell has no other edge within half a
+ * cell, so with a window below that the bin and its certainty follow from
+ * the one comparison.  A cell with several edges near holds a NaN, which
+ * every comparison fails: ambiguous.  The cells run from below the lowest
+ * positive edge to above top; the finest spacing that leaves no NaN cell is
+ * not exceeded, nor ETAB_MAX cells.
+ */
+#define ETAB_MAX 4096
+static float etab_value(long c, int lg) {
+  const uint32_t u = (uint32_t) c << lg;
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+}
+static long etab_cell(double v, int lg) {
+  const float f = (float) v;
+  uint32_t u;
+  memcpy(&u, &f, 4);
+  return (long) (u >> lg);
+}
+
+int fcfcg_axis_etab(fcfcg_axis *a, double top, int root) {
+  const int n = a->nbin;
+  double *e = malloc(sizeof(double) * (n + 1));
+  if (!e) return FCFCG_ERR_MEMORY;
+  for (int k = 0; k <= n; k++) e[k] = root ? sqrt(a->edge[k]) : a->edge[k];
+  const double first = e[0] > 0 ? e[0] : e[1];
+  free(a->etab);
+  a->etab = NULL;
+  for (int lg = 23 - 4; lg >= 23 - 12; lg--) {
+    const long lo = etab_cell(first * 0.8, lg) - 1,
+               hi = etab_cell(top * 1.05, lg) + 2;
+    const long m = hi - lo;
+    if (a->etab && m > ETAB_MAX) break;
+    float *t = malloc(sizeof(float) * 2 * (m + 2));
+    if (!t) {
+      free(e);
+      return FCFCG_ERR_MEMORY;
+    }
+    int multi = 0, k = 0;      /* k: the first edge above the cell's margin */
+    for (long c = 0; c < m; c++) {
+      const double x0 = etab_value(lo + c, lg), x1 = etab_value(lo + c + 1, lg);
+      const double w = 0.5 * (x1 - x0);
+      while (k <= n && e[k] < x0 - w) k++;
+      int near = 0;
+      while (k + near <= n && e[k + near] <= x1 + w) near++;
+      float edge = INFINITY;
+      if (near == 1) edge = (float) e[k];
+      if (near > 1) {
+        edge = NAN;
+        multi = 1;
+      }
+      t[2 * c] = edge;
+      t[2 * c + 1] = 12582912.f + (float) k;   /* k edges below: column k */
+    }
+    /* values below the cells: none of the edges is near, or (where the
+     * windows exceed the cells) ambiguous */
+    t[2 * m] = INFINITY;
+    t[2 * m + 1] = 12582912.f + (e[0] > 0 ? 0.f : 1.f);
+    t[2 * m + 2] = NAN;
+    t[2 * m + 3] = 12582912.f;
+    free(a->etab);
+    a->etab = t;
+    a->netab = (int) m;
+    a->elg = lg;
+    a->eoff = lo;
+    if (!multi) break;
+  }
+  free(e);
+  return FCFCG_OK;
+}
+
 /* allow_log: the kernels can use a bit-pattern FP32 table for this axis
  * (the s or s_perp axis in a box) */
 static int axis_finish(fcfcg_axis *a, const double *edge, int n, int hybrid,
@@ -300,6 +376,7 @@ static void axis_free(fcfcg_axis *a) {
   free(a->rtab);
   free(a->ftab);
   free(a->fedge);
+  free(a->etab);
   memset(a, 0, sizeof *a);
 }
 
@@ -470,6 +547,15 @@ int fcfcg_bins_setup(const fcfcg_binning *cfg, fcfcg_bins *b, char *err,
     FAIL(rc, "failed to create the separation lookup table");
   if (spi && (rc = axis_finish(&b->p, box ? pb : p2, np, hybrid, 0)))
     FAIL(rc, "failed to create the pi lookup table");
+  {
+    /* values up to the outer range: s^2, or for surveys s_perp^2 and pi of
+     * every pair within sqrt(s_perp_max^2 + pi_max^2) */
+    const double r2 = b->s.vmax + (spi && !box ? b->p.vmax : 0);
+    if ((rc = fcfcg_axis_etab(&b->s, r2, 0)))
+      FAIL(rc, "failed to create the separation edge table");
+    if (spi && (rc = fcfcg_axis_etab(&b->p, box ? b->p.vmax : sqrt(r2), !box)))
+      FAIL(rc, "failed to create the pi edge table");
+  }
   free(sb);
   free(s2);
   free(pb);

@@ -4,7 +4,7 @@
  * allocation-free FP64 counter.  The FP32 counting kernel is count32.cuh,
  * instantiated by the count32_*.cu files.
  */
-#include "count_common.cuh"
+#include "tile32.cuh"
 
 /*
  * FP64 counting kernel: the same traversal, every pair binned by the
@@ -126,13 +126,6 @@ __global__ void k_recheck(const fcfcg_launch L) {
 
 /* ------------------------------------------------------------------------ */
 
-static kfun_t pick32(int geom, int bin, int wt, int batch, int adj) {
-  if (adj) return fcfcg_pick32_adj(geom, bin);
-  if (batch) return geom == FCFCG_GEOM_BOX ? fcfcg_pick32_batch(bin, wt) : 0;
-  return geom == FCFCG_GEOM_BOX ? fcfcg_pick32_box(bin, wt)
-                                : fcfcg_pick32_survey(bin, wt);
-}
-
 static kfun_t pick64(int geom, int wt, int adj) {
   if (adj)
     return geom == FCFCG_GEOM_BOX ? (kfun_t) k_count64<FCFCG_GEOM_BOX, 1, 1>
@@ -164,6 +157,30 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
              &per_sm, (const void *) f, threads, smem)))
       return (int) e;
   } else {
+    if (!L->adjoint) {
+      int bin = L->bintype;
+      if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
+      if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
+      if (bin == FCFCG_BIN_SPI && L->tplin) bin = BIN_SPILIN;
+      f = L->geometry == FCFCG_GEOM_SURVEY
+              ? fcfcg_pick32_survey(bin, L->withwt)
+              : (L->mocks ? fcfcg_pick32_batch(bin, L->withwt)
+                          : fcfcg_pick32_box(bin, L->withwt));
+      if (!f) return (int) cudaErrorInvalidValue;
+      const size_t sm = fcfcg_k_tile32_tab(L) +
+          fcfcg_k_tile32_stage(L->withwt) +
+          fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
+      if ((e = cudaFuncSetAttribute((const void *) f,
+               cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm)) ||
+          (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+               &per_sm, (const void *) f, CT32_THREADS, sm)))
+        return (int) e;
+      if (per_sm < 1) return (int) cudaErrorInvalidConfiguration;
+      if (smem_used) *smem_used = sm;
+      if (qwarp_used) *qwarp_used = L->qwarp ? L->qwarp : QWARP_MAX;
+      f<<<nsm * per_sm, CT32_THREADS, sm, (cudaStream_t) stream>>>(Lq);
+      return (int) cudaGetLastError();
+    }
     /* a bit-pattern s table selects the kernel's log variant */
     int bin = !L->fslog ? L->bintype
         : (L->bintype == FCFCG_BIN_SPI ? BIN_SPIL
@@ -171,7 +188,7 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
     /* linear s bins: the s bin from s itself */
     if (L->slin && L->bintype == FCFCG_BIN_ISO) bin = BIN_ISOLIN;
     if (L->slin && L->bintype == FCFCG_BIN_SMU) bin = BIN_SMULIN;
-    f = pick32(L->geometry, bin, L->withwt, L->mocks != NULL, L->adjoint);
+    f = fcfcg_pick32_adj(L->geometry, bin);
     if (!f) return (int) cudaErrorInvalidValue;
     size_t tab = fcfcg_k_count32_tab_bytes(L->nfs, L->nfp, L->nsb, L->npb);
     size_t fixed = tab + (L->hist_smem ? (size_t) L->ntot * (L->withwt ? 8 : 4)
@@ -220,6 +237,18 @@ extern "C" size_t fcfcg_k_count32_tab_bytes(int nfs, int nfp, int nsb,
   size_t n = (((size_t) (nfs + nfp) * 2 + 3) & ~(size_t) 3);
   n += sizeof(float) * ((size_t) nsb + 1 + (npb ? (size_t) npb + 1 : 0));
   return (n + 15) & ~(size_t) 15;
+}
+
+extern "C" size_t fcfcg_k_tile32_tab(const fcfcg_launch *L) {
+  return ((size_t) (L->nse + L->npe) * 8 + 15) & ~(size_t) 15;
+}
+
+extern "C" size_t fcfcg_k_tile32_stage(int withwt) {
+  return (size_t) (CT32_THREADS / 32) * tile_warp_bytes(withwt);
+}
+
+extern "C" size_t fcfcg_k_tile32_hist(int hlen, int withwt) {
+  return ((size_t) hlen + 32) * (withwt ? 8 : 4);
 }
 
 /* Shared memory the FP32 kernel needs beyond its histogram, with the

@@ -1,5 +1,6 @@
 /*
- * count32.cuh -- the FP32 pair-counting kernel (instantiated by count32_*.cu).
+ * count32.cuh -- the FP32 kernel of the adjoint (instantiated by
+ * count32_adj.cu); the counts' is tile32.cuh.
  *
  * Work decomposition (replaces FCFC's dual k-d tree, src/fcfc/2pt_box/
  * dual_tree.c:245-373, and its OpenMP/MPI node-pair scheduler,

@@ -23,14 +23,17 @@
 #define BIN_SMUL 5
 #define BIN_ISOLIN 6
 #define BIN_SMULIN 7
-#define IS_SPI(B) ((B) == FCFCG_BIN_SPI || (B) == BIN_SPIL)
+/* tile kernel: (s_perp, pi) with linear pi bins */
+#define BIN_SPILIN 8
+#define IS_SPI(B) ((B) == FCFCG_BIN_SPI || (B) == BIN_SPIL || (B) == BIN_SPILIN)
+#define LINP(B) ((B) == BIN_SPILIN)
 #define IS_ISO(B) ((B) == FCFCG_BIN_ISO || (B) == BIN_ISOL || (B) == BIN_ISOLIN)
 #define IS_SMU(B) ((B) == FCFCG_BIN_SMU || (B) == BIN_SMUL || (B) == BIN_SMULIN)
 #define LOGTAB(B) ((B) >= BIN_SPIL && (B) <= BIN_SMUL)
 /* linear s bins: the s bin is floor((s - a) / d), no table */
 #define LINS(B) ((B) == BIN_ISOLIN || (B) == BIN_SMULIN)
 /* survey (s_perp, pi): the scan applies the line-of-sight prefilter */
-#define LOSCUT(G, B) ((G) == FCFCG_GEOM_SURVEY && (B) == FCFCG_BIN_SPI)
+#define LOSCUT(G, B) ((G) == FCFCG_GEOM_SURVEY && IS_SPI(B))
 
 #define CT_THREADS 256
 #define FULLMASK 0xffffffffu

@@ -31,6 +31,9 @@ typedef struct {
   uint32_t *sid, *cell_of;
   uint32_t *cstart;
   size_t ccap;
+  float *blk;                      /* blocks of the sorted copy */
+  uint32_t *bcell, *bstart;
+  size_t blkcap;
   int grid_valid;
   int gsig_n[3];
   double gsig_cw[3], gsig_lo[3];
@@ -53,6 +56,7 @@ struct fcfcg_ctx {
   uint16_t *d_fs, *d_fp, *d_rs, *d_rp;
   float *d_fse, *d_fpe;
   double *d_s2edge, *d_pedge;
+  float *d_se, *d_pe;             /* edge tables of the tile kernel */
   int *d_sten;
   float *d_stenD;
   unsigned long long *d_cnt, *d_wt, *d_stats, *d_bbox;
@@ -187,7 +191,8 @@ static int upload(fcfcg_ctx *c, void **dst, const void *src, size_t bytes) {
 
 static void slot_free(slot_t *s) {
   void *p[] = {s->x, s->y, s->z, s->s, s->w, s->l4, s->wq, s->sx, s->sy,
-               s->sz, s->ss, s->sw, s->sid, s->cell_of, s->cstart};
+               s->sz, s->ss, s->sw, s->sid, s->cell_of, s->cstart, s->blk,
+               s->bcell, s->bstart};
   for (size_t i = 0; i < sizeof p / sizeof p[0]; i++)
     if (p[i]) cudaFree(p[i]);
   memset(s, 0, sizeof *s);
@@ -201,7 +206,7 @@ void fcfcg_destroy(fcfcg_ctx *c) {
     for (int i = 0; i <= FCFCG_MAX_SLOT; i++) slot_free(c->slot + i);
     void *p[] = {c->cfill, c->fstart, c->scan_tmp, c->cchunk, c->chunks, c->d_fse,
                  c->d_fpe, c->d_fs,
-                 c->d_fp, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
+                 c->d_se, c->d_pe, c->d_fp, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
                  c->d_sten, c->d_stenD, c->d_cnt, c->d_wt, c->d_stats,
                  c->d_bbox, c->d_wd, c->d_gfix, c->d_head, c->d_queue, c->d_cnvt,
                  c->d_mock, c->d_mbase, c->d_bout, c->d_bstat, c->d_grad,
@@ -272,7 +277,13 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
     rc = upload(c, (void **) &c->d_fse, b->s.fedge, sizeof(float) * (b->s.nbin + 1));
     if (rc) return rc;
   }
+  rc = upload(c, (void **) &c->d_se, b->s.etab,
+              sizeof(float) * 2 * (b->s.netab + 2));
+  if (rc) return rc;
   if (b->bintype == FCFCG_BIN_SPI) {
+    rc = upload(c, (void **) &c->d_pe, b->p.etab,
+                sizeof(float) * 2 * (b->p.netab + 2));
+    if (rc) return rc;
     rc = upload(c, (void **) &c->d_rp, b->p.rtab, sizeof(uint16_t) * b->p.nrtab);
     if (rc) return rc;
     rc = upload(c, (void **) &c->d_pedge, b->p.edge,
@@ -697,8 +708,22 @@ static void grid_reach(const fcfcg_ctx *c, grid_t *g) {
   g->reach3 = r3;
 }
 
+/* Width of the tile kernel's k = 1 cells in units of the reach: at least
+ * the reach, wider where a cell would hold fewer than CELL_POINTS points,
+ * so that its blocks of 32 are full; at most CELL_WIDEN (wider cells widen
+ * the FP32 windows). */
+#define CELL_POINTS 256.0
+#define CELL_WIDEN 4.0
+static double cell_widen(double density, const double reach[3]) {
+  const double m = density * reach[0] * reach[1] * reach[2];
+  const double f = cbrt(CELL_POINTS / (m > 1e-30 ? m : 1e-30));
+  return f < 1 ? 1 : (f > CELL_WIDEN ? CELL_WIDEN : f);
+}
+
+/* tile: the grid of the tile kernel (k = 1 unless set or tuned; widen: its
+ * cells may be wider than the reach), else of the chunk kernels. */
 static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
-    const slot_t *B) {
+    const slot_t *B, int tile, int widen) {
   const fcfcg_bins *b = &c->bins;
   const int box = (b->geometry == FCFCG_GEOM_BOX);
   grid_reach(c, g);
@@ -733,8 +758,12 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
   int k = c->kcell;
   if (!k) k = (c->tuned_k && c->tuned_key == g->key)
                   ? c->tuned_k
-                  : pick_k(density, r3, box ? 24.0 : (spi ? 30.0 : 130.0));
+                  : (tile ? 1
+                          : pick_k(density, r3,
+                                   box ? 24.0 : (spi ? 30.0 : 130.0)));
   g->k = k;
+  const double f = (tile && widen && k == 1)
+                       ? cell_widen(density, g->reach) : 1;
   const double maxcells = 16.0 * 1024 * 1024;
   double scale = 1;
   for (;;) {
@@ -742,7 +771,7 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
     for (int d = 0; d < 3; d++) {
       /* cells a little wider than reach / k, so that k layers of neighbours
        * cover every separation below the reach */
-      double cwt = g->reach[d] / k * scale * (1 + 1e-6);
+      double cwt = g->reach[d] / k * f * scale * (1 + 1e-6);
       int n = (int) floor(ext[d] / cwt);
       if (n < 1) n = 1;
       if (n > 4096) n = 4096;
@@ -893,6 +922,7 @@ static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
                  s->cell_of};
     for (size_t i = 0; i < sizeof p / sizeof p[0]; i++)
       if (p[i]) cudaFree(p[i]);
+    s->l4 = NULL;
     CK(cudaMalloc((void **) &s->l4, sizeof(float) * 4 * m));
     CK(cudaMalloc((void **) &s->wq, sizeof(int) * 2 * m));
     CK(cudaMalloc((void **) &s->sx, sizeof(double) * m));
@@ -907,15 +937,30 @@ static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   if (s->ccap < nc + 1) {
     c->bufgen++;
     if (s->cstart) cudaFree(s->cstart);
-    s->cstart = NULL;
+    if (s->bstart) cudaFree(s->bstart);
+    s->cstart = s->bstart = NULL;
     CK(cudaMalloc((void **) &s->cstart, sizeof(uint32_t) * (nc + 1)));
+    CK(cudaMalloc((void **) &s->bstart, sizeof(uint32_t) * (nc + 1)));
     s->ccap = nc + 1;
   }
-  const size_t nf = nc << fcfcg_grid_sub_bits(nc, n);
+  const size_t mb = fcfcg_max_blocks(n, nc);
+  if (s->blkcap < mb) {
+    c->bufgen++;
+    if (s->blk) cudaFree(s->blk);
+    if (s->bcell) cudaFree(s->bcell);
+    s->blk = NULL;
+    s->bcell = NULL;
+    s->blkcap = 0;
+    CK(cudaMalloc((void **) &s->blk, sizeof(float) * 8 * mb));
+    CK(cudaMalloc((void **) &s->bcell, sizeof(uint32_t) * 2 * mb));
+    s->blkcap = mb;
+  }
+  const size_t nf = nc << fcfcg_grid_curve_bits(nc, n);
   GROW(c->cfill, c->cfill_cap, sizeof(uint32_t) * (nf + 1));
   GROW(c->fstart, c->fstart_cap, sizeof(uint32_t) * (nf + 1));
   size_t st = fcfcg_scan_tmp_len(nf + 1) + 16;
   GROW(c->scan_tmp, c->scan_cap, sizeof(uint32_t) * st);
+  GROW(c->cchunk, c->cchunk_cap, sizeof(uint32_t) * 2 * (nc + 1));
   return FCFCG_OK;
 }
 
@@ -923,7 +968,7 @@ static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
 static int slot_sort(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   const size_t nc = (size_t) g->n[0] * g->n[1] * g->n[2];
   const size_t n = s->n;
-  const int sb = fcfcg_grid_sub_bits(nc, n);
+  const int sb = fcfcg_grid_curve_bits(nc, n);
   size_t st = fcfcg_scan_tmp_len((nc << sb) + 1) + 16;
   const int survey = (c->bins.geometry == FCFCG_GEOM_SURVEY);
   CKK(fcfcg_k_grid(c->stream, n, s->x, s->y, s->z, survey ? s->s : NULL,
@@ -932,7 +977,28 @@ static int slot_sort(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
                    st, s->l4, s->wq, s->sx, s->sy, s->sz,
                    survey ? s->ss : NULL, s->sw, s->sid));
   c->launches += n ? 6 : 4;
+  CKK(fcfcg_k_blocks(c->stream, s->cstart, (uint32_t) nc, n, c->cchunk,
+                     c->scan_tmp, s->l4, s->bstart, s->blk, s->bcell, NULL,
+                     0));
+  c->launches += 5;
   return FCFCG_OK;
+}
+
+
+/* Are the s bins linear as FCFC's integer table sees them: rescaled edges
+ * a + k d, integers, a >= 0, d >= 1? */
+static int linear_edges(const fcfcg_bins *b, double *a, double *d) {
+  if (b->bintype == FCFCG_BIN_SPI || b->s.tabtype != FCFCG_TAB_INT ||
+      b->s.nbin < 1)
+    return 0;
+  for (int k = 0; k <= b->s.nbin; k++) {
+    const double e = sqrt(b->s.edge[k]);
+    if (!(e == floor(e) && e * e == b->s.edge[k] && e < 1e6)) return 0;
+    if (k == 0) *a = e;
+    else if (k == 1) *d = e - *a;
+    else if (e != *a + k * *d) return 0;
+  }
+  return *d >= 1;
 }
 
 /* Lower end of cell c of a bit-pattern table (FP32 bits c << sh). */
@@ -941,6 +1007,221 @@ static double ftab_cell_value(long c, int sh) {
   float f;
   memcpy(&f, &u, 4);
   return (double) f;
+}
+
+/* Are the edges of an axis (their square roots with root) a + k d, to within
+ * LIN_TOL d? */
+#define LIN_TOL 1e-9
+static int even_edges(const fcfcg_axis *x, int root, double *a, double *d) {
+  const int n = x->nbin;
+  const double e0 = root ? sqrt(x->edge[0]) : x->edge[0],
+               en = root ? sqrt(x->edge[n]) : x->edge[n];
+  *a = e0;
+  *d = (en - e0) / n;
+  for (int k = 0; k <= n; k++) {
+    const double e = root ? sqrt(x->edge[k]) : x->edge[k];
+    if (!(fabs(e - (e0 + k * *d)) <= LIN_TOL * *d)) return 0;
+  }
+  return 1;
+}
+
+/* The cells of an axis' edge table in use, given the window at a value (w0 +
+ * w1 v): from *skip on, where it is below 0.45 of a cell; *last: the entry
+ * for the values below.  0 if the windows fit nowhere useful. */
+static int etab_use(const fcfcg_axis *x, double w0, double w1, double vmax,
+    int *n, int *lg, int *off, int *skip, int *last) {
+  int c0 = 0;
+  double v0 = 0;
+  for (long c = x->netab - 1; c >= 0; c--) {
+    const double x0 = ftab_cell_value(x->eoff + c, x->elg),
+                 x1 = ftab_cell_value(x->eoff + c + 1, x->elg);
+    if (!(w0 + w1 * x1 < 0.45 * (x1 - x0))) {
+      c0 = (int) c + 1;
+      v0 = x1;
+      break;
+    }
+  }
+  *skip = c0;
+  *n = x->netab - c0 + 1;
+  *lg = x->elg;
+  *off = (int) x->eoff + c0;
+  *last = x->netab + (c0 ? 1 : 0);
+  return v0 <= 0.25 * vmax;
+}
+
+/*
+ * The tile kernel's windows (tile32.cuh pair_bin), in the notation of
+ * fp32_bounds below: dc bounds the error of a separation component, E(s^2)
+ * = K2a s^2 + K1 s + K0a that of s^2.  rs = rsqrt.approx.ftz(s^2) is within
+ * e = 2^-22.9 (PTX ISA) of 1 / s.
+ *
+ * Linear s bins: with s0 = (hcol0 - 1/2) d - a, x = fl(fma(s^2, rs, s0))
+ * and t = x fl(1 / d): the column rn(t) and t's distance from it come from
+ * FMAs that round the exact product once (the column exactly; the distance,
+ * |f| <= 1/2, to u / 2).  s^2 rs is within e of s:
+ *   W = [(e (1 + 2 e) + K2a (1 + e)) smax + (K1 + K0a / st) (1 + e) +
+ *       u (smax + |s0|)] / d + u |s0| / d + u (columns + 1) + 2 u + LIN_TOL
+ * (x's rounding; s0's; 1 / d's; the edges').  Below st (mu bins only) every
+ * pair is ambiguous by its mu window; without mu a separation's error is <=
+ * sqrt(3) dc < K1 for any s.  st = max(80 dc, sqrt(40 K0a)) keeps E / s^2 <=
+ * 1/16.
+ *
+ * mu: x = fl(fl(|dz| rs) + q0), q0 = -1 / (2 nmu) (survey: fl(d.m), fl(mm
+ * s^2)), t = x nmu.  Relative terms of q: box rs, the product and the sum,
+ * e + 2 u (and u nmu |q0| = u / 2 for q0's rounding); survey 8 u.  Eq = Q1 /
+ * s + Q2 nmu + Q0 (Q2's term at q = nmu), with nmu K0a / (2 s^2) <= nmu K0a
+ * / (2 st) / s in Q1, and Q1 >= 0.51 st so that s < st is ambiguous.  The
+ * window test forms 1/2 - Eq in one FMA and the distance from the column in
+ * another: u each.
+ *
+ * pi, box: |dz| within dc.  Survey: pi = fl(|d.m| rsqrt(mm)), |m| >= 2 R:
+ *   |pi - pi_ref| <= Wp = 1.25 [sqrt(3) dc + 3 v sabs / R + R (2 dmr + 3 u +
+ *       e + 3 u + v sabs / R^2)]
+ * (d.m within 3 u |d| |m|, its direction, mm, the root and the product; the
+ * reference's s1 - s2 and S + t).  Linear bins: t = fl(pi + p0) fl(1 / d) as
+ * for s.
+ *
+ * Tables: the window of s^2 (box s_perp^2) is E; of a survey's s_perp^2 =
+ * fl(s^2 - pi^2), E + 2 s Wp(s) + u s^2.  E's term in s is replaced by its
+ * tangent at half the range, s <= s^2 / R + R / 4, so that the window is
+ * tl_ea s^2 + tl_eb; the edge's rounding and the difference's add 2 u v.
+ */
+static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
+    double K2a, double hw, double dmax, double R, double dmr, double sabs,
+    fcfcg_launch *L) {
+  const fcfcg_bins *b = &c->bins;
+  const int box = (b->geometry == FCFCG_GEOM_BOX);
+  const int spi = (b->bintype == FCFCG_BIN_SPI);
+  const double u = ldexp(1.0, -24), v = ldexp(1.0, -53);
+  const double er = pow(2.0, -22.9), s3 = sqrt(3.0);
+  const double nmu = b->nmu;
+  double a = 0, d = 0;
+  L->tlin = L->tplin = 0;
+  /* boxes' distance: the blocks' points, D, their difference and the
+   * extents, each rounded to u of at most hw, dmax or R */
+  L->box_eps = (float) (16 * u * (2 * hw + dmax + R));
+  L->near2 = (float) (1.52 * R * 1.52 * R);
+  const double st = fmax(80 * dc, sqrt(40 * K0a));
+  int rows = 1;
+  L->hrow0 = 0;
+  L->hrows = spi ? b->np : b->nmu;
+  if (b->bintype == FCFCG_BIN_SMU) {
+    const double q1 = fmax(1.25 * nmu * ((box ? dc : s3 * dc) + 0.5 * K1 +
+                                         0.5 * K0a / st +
+                                         (box ? 0 : 3 * v * sabs / R)),
+                           0.51 * st);
+    const double q2 = 1.25 * (0.5 * K2a + 2 * v + 2 * u +
+                              (box ? er + 3 * u : 8 * u + v * sabs / (R * R)));
+    const double q0 = (box ? 0 : 1.25 * nmu * (3 * u + 2 * dmr)) + 1e-7 + 4 * u;
+    const double qc = 0.5 - (q2 * nmu + q0);
+    if (qc < 0.05) return -1;
+    L->tl_q0 = (float) (-0.5 / nmu);
+    L->tl_q1 = nextafterf((float) q1, INFINITY);
+    L->tl_qc = nextafterf((float) qc, 0.f);
+    rows = b->nmu;
+  }
+  /* The windows W below carry a factor 1.1 over the derived bound.  A value
+   * more than TIGHT W beyond the last edge, or before the first, is outside
+   * for sure; within it, it is ambiguous (TIGHT < 1), so that the pairs of
+   * an outer limit at TIGHT W are either in a bin or ambiguous. */
+  const double TIGHT = 0.955;
+  L->tl_slo = L->tl_plo = -1.f;
+  L->tl_shi = FLT_MAX;
+  /* the error of a survey's pi grows as wp1 s + wp0 */
+  const double wp0 = 1.25 * (box ? dc : s3 * dc + 3 * v * sabs / R);
+  const double wp1 = box ? 0 : 1.25 * (2 * dmr + 6 * u + er + v * sabs / (R * R));
+  if (spi) {
+    const double pmax = box ? b->p.vmax : sqrt(b->p.vmax);
+    const double pmin = box ? b->p.vmin : sqrt(b->p.vmin);
+    const double Wp = wp0 + wp1 * R;
+    double Wv = 1.1 * (Wp + 2 * u * pmax);      /* window of pi */
+    int ok = even_edges(&b->p, !box, &a, &d);
+    if (ok) {
+      const int r0 = (int) ceil(a / d - LIN_TOL);
+      const double p0 = (r0 - 0.5) * d - a;
+      rows = r0 + b->np + 1;
+      const double W = 1.1 * ((Wp + u * (pmax + 2 * fabs(p0))) / d +
+                              u * (rows + 1) + 2 * u + LIN_TOL);
+      if (W > 0.45 || rows > 2 * b->np + 16) {
+        ok = 0;
+      } else {
+        L->tplin = 1;
+        L->hrow0 = r0;
+        L->tl_p0 = (float) p0;
+        L->tl_pinv = (float) (1.0 / d);
+        L->tl_hp = nextafterf((float) (0.5 - W), 0.f);
+        Wv = W * d;
+      }
+    }
+    if (!ok) {
+      rows = b->np + 2;
+      L->hrow0 = 1;
+      L->tl_hp = nextafterf((float) Wv, INFINITY);
+      if (b->p.nbin > FCFCG_FTAB_MAXBIN ||
+          !etab_use(&b->p, Wv, 0, pmax, &L->npe, &L->pe_lg, &L->pe_off,
+                    &L->pe_skip, &L->pe_last))
+        return -1;
+      L->pe = c->d_pe;
+    }
+    L->p_lim = (float) (pmax + TIGHT * Wv);
+    if (!b->p.min0) L->tl_plo = (float) (pmin - TIGHT * Wv);
+  } else {
+    const int ok = even_edges(&b->s, 1, &a, &d);
+    const int col0 = ok ? (int) ceil(a / d - LIN_TOL) : 0;
+    const int cols = col0 + b->ns + 1;
+    const double s0 = (col0 - 0.5) * d - a;
+    const double smax = a + d * b->s.nbin;
+    const double W = ok ? 1.1 * (((er * (1 + 2 * er) + K2a * (1 + er)) * smax +
+                                  (K1 + K0a / st) * (1 + er) +
+                                  u * (smax + 2 * fabs(s0))) / d +
+                                 u * (cols + 1) + 2 * u + LIN_TOL)
+                        : 1;
+    if (ok && W <= 0.45 && cols <= 2 * b->ns + 16) {
+      L->tlin = 1;
+      L->hcols = cols;
+      L->hcol0 = col0;
+      L->tl_inv = (float) (1.0 / d);
+      L->tl_s0 = (float) s0;
+      L->tl_h = nextafterf((float) (0.5 - W), 0.f);
+      const double hi = smax + TIGHT * W * d, lo = a - TIGHT * W * d;
+      L->s_lim = (float) (hi * hi);
+      if (lo > 0) L->tl_slo = (float) (lo * lo);
+    }
+  }
+  if (!L->tlin) {
+    const double r2 = b->s.vmax + (spi && !box ? b->p.vmax : 0);
+    const double r = sqrt(r2);
+    double e2 = K2a + 2 * u, e1 = K1, e0 = K0a;
+    if (spi && !box) {
+      e2 += 2 * wp1 + u;
+      e1 += 2 * wp0;
+    }
+    e2 += e1 / r;
+    e0 += e1 * r / 4;
+    L->tl_ea = nextafterf((float) (1.1 * e2), INFINITY);
+    L->tl_eb = nextafterf((float) (1.1 * e0), INFINITY);
+    const double Em = 1.01 * ((double) L->tl_ea * r2 + (double) L->tl_eb);
+    const double w1 = (spi && !box) ? 0 : (double) L->tl_ea,
+                 w0 = (spi && !box) ? Em : (double) L->tl_eb;
+    if (b->s.nbin > FCFCG_FTAB_MAXBIN || !(Em < 0.02 * b->s.vmax) ||
+        !etab_use(&b->s, w0, w1, b->s.vmax, &L->nse, &L->se_lg, &L->se_off,
+                  &L->se_skip, &L->se_last))
+      return -1;
+    L->se = c->d_se;
+    L->hcols = b->ns + 2;
+    L->hcol0 = 1;
+    /* (a survey's window of s_perp^2 is at least its constant part) */
+    const double wv = TIGHT * (double) L->tl_eb;
+    const double hi = b->s.vmax + TIGHT * ((spi && !box)
+        ? (double) L->tl_eb : (double) L->tl_ea * b->s.vmax + (double) L->tl_eb);
+    if (spi && !box) L->tl_shi = (float) hi;
+    else L->s_lim = (float) hi;
+    if (!b->s.min0) L->tl_slo = (float) (b->s.vmin - wv);
+  }
+  const double hl = (double) L->hcols * rows;
+  if (hl > 1e9) return -1;
+  L->hlen = (int) hl;
+  return 0;
 }
 
 /* Rounding bounds of the FP32 path; returns 0 when the FP32 windows stay
@@ -1019,7 +1300,7 @@ static double ftab_cell_value(long c, int sh) {
  * rechecked.
  */
 static int fp32_bounds(const fcfcg_ctx *c, const grid_t *g, double dmax,
-    const slot_t *A, const slot_t *B, fcfcg_launch *L) {
+    const slot_t *A, const slot_t *B, int tile, fcfcg_launch *L) {
   const fcfcg_bins *b = &c->bins;
   const int box = (b->geometry == FCFCG_GEOM_BOX);
   const double u = ldexp(1.0, -24), v = ldexp(1.0, -53);
@@ -1080,18 +1361,9 @@ static int fp32_bounds(const fcfcg_ctx *c, const grid_t *g, double dmax,
    *   evaluation.
    */
   L->slin = 0;
-  if (b->bintype != FCFCG_BIN_SPI && b->s.tabtype == FCFCG_TAB_INT &&
-      b->s.nbin >= 1) {
-    int ok = 1;
+  {
     double a = 0, d = 0;
-    for (int k = 0; k <= b->s.nbin && ok; k++) {
-      const double e = sqrt(b->s.edge[k]);
-      if (!(e == floor(e) && e * e == b->s.edge[k] && e < 1e6)) ok = 0;
-      else if (k == 0) a = e;
-      else if (k == 1) d = e - a;
-      else if (e != a + k * d) ok = 0;
-    }
-    if (ok && d >= 1) {
+    if (linear_edges(b, &a, &d)) {
       const double eta = ldexp(1.0, -22) + ldexp(1.0, -24);
       const double uu = ldexp(1.0, -24);
       const double A = 1.01 * (eta * (1 + 2 * eta) + (double) L->K2 * (1 + eta)
@@ -1152,6 +1424,8 @@ static int fp32_bounds(const fcfcg_ctx *c, const grid_t *g, double dmax,
     L->s_lim = (float) (smax2 + Es + 1e-6 * (1 + smax2));
   }
   L->Emax = (float) (Es * 1.01);
+  if (tile)
+    return tile_bounds(c, dc, K1, K0a, K2a, hw, dmax, R, dmr, sabs, L);
   if (b->s.nbin > FCFCG_FTAB_MAXBIN || !b->s.ftab) return -1;
   if (b->bintype == FCFCG_BIN_SPI &&
       (b->p.nbin > FCFCG_FTAB_MAXBIN || !b->p.ftab))
@@ -1222,6 +1496,9 @@ static void launch_cat(fcfcg_dcat *D, const slot_t *S) {
   D->w = S->sw;
   D->id = S->sid;
   D->cstart = S->cstart;
+  D->blk = S->blk;
+  D->bstart = S->bstart;
+  D->bcell = S->bcell;
   D->wexp = S->wexp;
 }
 
@@ -1330,11 +1607,24 @@ typedef struct {
   int hwa, hwb;
   int isauto, withwt, prec;
   grid_t g;
+  int tile;                      /* the tile kernel counts */
   int nsten, nin;                /* stencil entries, those within range */
   uint32_t ncell;
   size_t st;                     /* scan scratch length of the chunk list */
   fcfcg_launch L;                /* stencil pointers: set by the caller */
 } count_plan;
+
+/* log2 of the parts the tiles of a block are dealt to, so that a small
+ * catalogue still gives every warp of the GPU a few items: 8 items per
+ * warp (32 warps per SM), at most 16 parts (a part repeats the box tests of
+ * its block's neighbours). */
+static int tile_parts(size_t n, size_t ncell, int nsm) {
+  const double blocks = (double) n / 32 + 0.5 * (double) (n < ncell ? n : ncell);
+  const double want = 8.0 * 32 * nsm;
+  int p = 0;
+  while (p < 4 && blocks * (double) (1 << p) < want) p++;
+  return p;
+}
 
 #define STAT_WORDS 5   /* candidates, in range, rechecked, inline, chunks */
 
@@ -1353,11 +1643,37 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   P->isauto = isauto;
   P->withwt = withwt;
   grid_t *g = &P->g;
-  if ((rc = grid_setup(c, g, A, B))) return rc;
-  double dmax = 0;
-  if ((rc = stencil_build(c, g, isauto, sten, stD, &P->nsten, &dmax, NULL,
-                         &P->nin)))
-    return rc;
+  fcfcg_launch *L = &P->L;
+  /* The tile kernel's coarse grid; cells no wider than the reach, then the
+   * chunk kernels' finer cells where the FP32 windows do not fit; then the
+   * all-FP64 kernel on the latter. */
+  int prec = precision;
+  const int tile = (precision == FCFCG_PREC_FP32_RECHECK && !adj);
+  size_t tabbytes = 0, stage = 0;
+  for (int att = tile ? 0 : 2; ; att++) {
+    if ((rc = grid_setup(c, g, A, B, att < 2, att == 0))) return rc;
+    double dmax = 0;
+    if ((rc = stencil_build(c, g, isauto, sten, stD, &P->nsten, &dmax, NULL,
+                            &P->nin)))
+      return rc;
+    memset(L, 0, sizeof *L);
+    if (prec == FCFCG_PREC_FP64) break;
+    if (!fp32_bounds(c, g, dmax, A, B, tile, L)) {
+      if (!tile) launch_fp32_tables(c, L);
+      tabbytes = tile ? fcfcg_k_tile32_tab(L)
+                      : fcfcg_k_count32_tab_bytes(L->nfs, L->nfp, L->nsb,
+                                                  L->npb);
+      stage = tile ? fcfcg_k_tile32_stage(withwt)
+                   : fcfcg_k_count32_stage(P->nsten, withwt + (adj ? 1 : 0));
+      if (tabbytes + stage <= 200 * 1024) break;
+    }
+    if (att >= 2) {
+      prec = FCFCG_PREC_FP64;
+      tabbytes = stage = 0;
+      break;
+    }
+  }
+  P->tile = (tile && prec == FCFCG_PREC_FP32_RECHECK);
   if ((rc = slot_reserve(c, A, g))) return rc;
   if (B != A && (rc = slot_reserve(c, B, g))) return rc;
   P->ncell = (uint32_t) ((size_t) g->n[0] * g->n[1] * g->n[2]);
@@ -1365,9 +1681,10 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
        sizeof(uint32_t) * 2 * ((size_t) P->ncell + 1));
   P->st = fcfcg_scan_tmp_len(P->ncell + 1) + 16;
   GROW(c->scan_tmp, c->scan_cap, sizeof(uint32_t) * P->st);
-  size_t maxchunk = A->n / FCFCG_CHUNK + P->ncell + 1;
-  GROW(c->chunks, c->chunk_cap, sizeof(uint32_t) * 4 * maxchunk);
-  fcfcg_launch *L = &P->L;
+  if (!P->tile) {
+    size_t maxchunk = A->n / FCFCG_CHUNK + P->ncell + 1;
+    GROW(c->chunks, c->chunk_cap, sizeof(uint32_t) * 4 * maxchunk);
+  }
   L->geometry = b->geometry;
   L->bintype = b->bintype;
   L->isauto = isauto;
@@ -1385,29 +1702,20 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   L->tzero = -1;
   for (int t = 0; t < P->nsten; t++)
     if (!sten[4 * t] && !sten[4 * t + 1] && !sten[4 * t + 2]) L->tzero = t;
-  L->chunks = c->chunks;
+  L->chunks = P->tile ? NULL : c->chunks;
   L->chunk_head = c->d_head;
-  /* k_chunks leaves the number of chunks after the ncell + 1 counts and
-   * ncell offsets in cchunk */
-  L->nchunk_dev = c->cchunk + ((size_t) P->ncell + 1) + P->ncell;
+  /* the number of blocks, or of chunks: k_chunks leaves it after the ncell
+   * + 1 counts and ncell offsets in cchunk */
+  L->nblk_dev = A->bstart + P->ncell;
+  L->nchunk_dev = P->tile ? L->nblk_dev
+                          : c->cchunk + ((size_t) P->ncell + 1) + P->ncell;
   launch_cat(&L->A, A);
   launch_cat(&L->B, B);
   launch_bins(c, L);
-  int prec = precision;
-  if (prec == FCFCG_PREC_FP32_RECHECK && fp32_bounds(c, g, dmax, A, B, L))
-    prec = FCFCG_PREC_FP64;
-  if (prec == FCFCG_PREC_FP32_RECHECK) launch_fp32_tables(c, L);
-  size_t tabbytes = (prec == FCFCG_PREC_FP32_RECHECK)
-      ? fcfcg_k_count32_tab_bytes(L->nfs, L->nfp, L->nsb, L->npb) : 0;
-  size_t hbytes = (size_t) b->ntot * (withwt ? 8 : 4);
-  size_t stage = (prec == FCFCG_PREC_FP32_RECHECK)
-      ? fcfcg_k_count32_stage(P->nsten, withwt + (adj ? 1 : 0)) : 0;
-  if (tabbytes + stage > 200 * 1024) {
-    prec = FCFCG_PREC_FP64;
-    tabbytes = 0;
-    stage = 0;
-  }
+  const size_t hbytes = P->tile ? fcfcg_k_tile32_hist(L->hlen, withwt)
+                                : (size_t) b->ntot * (withwt ? 8 : 4);
   L->hist_smem = (tabbytes + stage + hbytes <= 200 * 1024);
+  L->pshift = tile_parts(A->n, P->ncell, c->nsm);
   L->hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
   L->qwarp = c->qwarp_force ? c->qwarp_force
       : ((c->tuned_q && c->tuned_q_key == g->key && c->tuned_q_wt == withwt)
@@ -1430,11 +1738,13 @@ static int count_launch(fcfcg_ctx *c, const count_plan *P, int sort_a,
   if (sort_b && P->B != P->A && (rc = slot_sort(c, P->B, &P->g))) return rc;
   /* work chunks: 64 points per CTA in the FP32 kernel, 32 per warp in the
    * FP64 kernel */
-  const uint32_t clen = (P->prec == FCFCG_PREC_FP32_RECHECK) ? FCFCG_CHUNK32
-                                                             : FCFCG_CHUNK;
-  CKK(fcfcg_k_chunks(c->stream, P->A->cstart, P->ncell, clen, c->cchunk,
-                     c->scan_tmp, P->st, c->chunks, NULL, NULL, 0));
-  c->launches += 5;
+  if (!P->tile) {
+    const uint32_t clen = (P->prec == FCFCG_PREC_FP32_RECHECK)
+                              ? FCFCG_CHUNK32 : FCFCG_CHUNK;
+    CKK(fcfcg_k_chunks(c->stream, P->A->cstart, P->ncell, clen, c->cchunk,
+                       c->scan_tmp, P->st, c->chunks, NULL, NULL, 0));
+    c->launches += 5;
+  }
   if (timed) CK(cudaEventRecord(c->ev[1], c->stream));
   CK(cudaMemsetAsync(c->d_cnt, 0, sizeof(unsigned long long) * b->ntot,
                      c->stream));
@@ -1870,6 +2180,14 @@ int fcfcg_graph_run(fcfcg_graph *G) {
   }
   for (int s = 0; s < FCFCG_MAX_SLOT; s++)
     if (G->has_last[s]) slot_mark(c->slot + s, G->last + s);
+  /* an item overflowed the recheck queue: a larger one for the next runs
+   * (which capture again) */
+  unsigned long long need = 0;
+  for (int i = 0; i < G->n; i++) {
+    const unsigned long long *st = stage_of(G, i) + 2 * (size_t) c->bins.ntot;
+    if (!G->empty[i] && st[3] && st[2] > need) need = st[2];
+  }
+  if (need) queue_grow(c, need + need / 4);
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev[0], c->ev[4]);
   c->stats.ms_total = ms;
@@ -1961,7 +2279,7 @@ int fcfcg_autotune(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
     /* the key of this catalogue pair, as the grid set-up computes it */
     grid_t g;
     memset(&g, 0, sizeof g);
-    grid_setup(c, &g, c->slot + sa, c->slot + sb);
+    grid_setup(c, &g, c->slot + sa, c->slot + sb, 1, 1);
     key = g.key;
     c->tuned_k = bk;
     c->tuned_key = key;
@@ -2267,8 +2585,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   const double density = nsum / (vol > 0 ? vol : 1);
   const int key = tune_key(density, gr.reach) + 1000;   /* batch keys */
   int k = c->kcell;
-  if (!k) k = (c->tuned_k && c->tuned_key == key) ? c->tuned_k
-                                                  : pick_k(density, gr.reach3, 24.0);
+  if (!k) k = (c->tuned_k && c->tuned_key == key) ? c->tuned_k : 1;
   BGROW(c->d_mbase, c->d_mbase_cap, sizeof(uint32_t) * (na + 1));
   if (c->h_mock_cap < (size_t) na) {
     free(c->h_mock);
@@ -2284,71 +2601,99 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
     free(wexp);
     BFAIL(FCFCG_ERR_MEMORY);
   }
-  grid_t gmin = gr, gmax = gr;
-  for (int d = 0; d < 3; d++) {
-    gmin.cw[d] = 1e300;
-    gmax.cw[d] = 0;
-  }
+  fcfcg_launch L;
+  grid_t gmin, gmax;
+  int nsten = 0, nin = 0, prec = FCFCG_PREC_FP32_RECHECK;
   size_t cells = 0;
-  double xabs = 0;
-  for (int a = 0; a < na; a++) {
-    const fcfcg_job *J = jobs + acc[a];
-    fcfcg_mock *M = c->h_mock + a;
-    memset(M, 0, sizeof *M);
-    hbase[a] = (uint32_t) cells;
-    if (J->status) continue;     /* no cells: never visited */
-    size_t nc = 1;
+  S->s2abs = 0;
+  S->wexp = 0;
+  /* as count_plan_make: wide cells, cells of the reach, finer cells while
+   * the FP32 windows do not fit; else FP64 */
+  for (int att = 0; ; att++) {
+    const int ka = att < 2 ? k : (c->kcell ? k : pick_k(density, gr.reach3, 24.0));
+    const double f = (att == 0 && ka == 1) ? cell_widen(density, gr.reach) : 1;
+    gmin = gmax = gr;
     for (int d = 0; d < 3; d++) {
-      const double L = J->box[d] * b->rescale;
-      const double cwt = gr.reach[d] / k * (1 + 1e-6);
-      int n = (int) floor(L / cwt);
-      if (n < 1) n = 1;
-      if (n > 4096) n = 4096;
-      M->ncell[d] = n;
-      M->cw[d] = L / n;
-      M->box[d] = L;
-      nc *= (size_t) n;
-      gmin.cw[d] = fmin(gmin.cw[d], M->cw[d]);
-      gmax.cw[d] = fmax(gmax.cw[d], M->cw[d]);
-      xabs = fmax(xabs, L);
+      gmin.cw[d] = 1e300;
+      gmax.cw[d] = 0;
     }
-    M->cell_base = (uint32_t) cells;
-    P[a].live = 1;
-    P[a].cell_base = M->cell_base;
-    for (int d = 0; d < 3; d++) {
-      P[a].ncell[d] = M->ncell[d];
-      P[a].cw[d] = M->cw[d];
+    cells = 0;
+    double xabs = 0;
+    for (int a = 0; a < na; a++) {
+      const fcfcg_job *J = jobs + acc[a];
+      fcfcg_mock *M = c->h_mock + a;
+      memset(M, 0, sizeof *M);
+      hbase[a] = (uint32_t) cells;
+      if (J->status) continue;     /* no cells: never visited */
+      size_t nc = 1;
+      for (int d = 0; d < 3; d++) {
+        const double Ld = J->box[d] * b->rescale;
+        const double cwt = gr.reach[d] / ka * f * (1 + 1e-6);
+        int n = (int) floor(Ld / cwt);
+        if (n < 1) n = 1;
+        if (n > 4096) n = 4096;
+        M->ncell[d] = n;
+        M->cw[d] = Ld / n;
+        M->box[d] = Ld;
+        nc *= (size_t) n;
+        gmin.cw[d] = fmin(gmin.cw[d], M->cw[d]);
+        gmax.cw[d] = fmax(gmax.cw[d], M->cw[d]);
+        xabs = fmax(xabs, Ld);
+      }
+      M->cell_base = (uint32_t) cells;
+      P[a].live = 1;
+      P[a].cell_base = M->cell_base;
+      for (int d = 0; d < 3; d++) {
+        P[a].ncell[d] = M->ncell[d];
+        P[a].cw[d] = M->cw[d];
+        P[a].inv[d] = 1.0 / M->cw[d];
+      }
+      cells += nc;
+      if (cells > 0x7FFFFFF0u) {
+        free(wexp);
+        free(hbase);
+        set_err(c, "batch grid too large");
+        BFAIL(FCFCG_ERR_UNSUPPORTED);
+      }
     }
-    cells += nc;
-    if (cells > 0x7FFFFFF0u) {
+    hbase[na] = (uint32_t) cells;
+    /* 4. one stencil for all: built for the narrowest cells (a superset of
+     * every catalogue's own); bounds for the widest */
+    double dmin = 0;
+    gmin.k = gmax.k = k;
+    if (gmin.cw[0] > 1e299) {        /* every catalogue failed its checks */
       free(wexp);
       free(hbase);
-      set_err(c, "batch grid too large");
-      BFAIL(FCFCG_ERR_UNSUPPORTED);
+      goto out;
+    }
+    if ((rc = stencil_build(c, &gmin, 1, c->sten, c->stD, &nsten, &dmin,
+                            gmax.cw, &nin))) {
+      free(wexp);
+      free(hbase);
+      goto out;
+    }
+    double dmax = 0;
+    for (int t = 0; t < nsten; t++)
+      for (int d = 0; d < 3; d++)
+        dmax = fmax(dmax, fabs((double) c->sten[4 * t + d]) * gmax.cw[d]);
+    S->xabs = xabs;
+    memset(&L, 0, sizeof L);
+    if (!fp32_bounds(c, &gmax, dmax, S, S, 1, &L) &&
+        fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt) <= 200 * 1024)
+      break;
+    if (att >= 2) {
+      prec = FCFCG_PREC_FP64;
+      break;
     }
   }
-  hbase[na] = (uint32_t) cells;
-  /* 4. one stencil for all: built for the narrowest cells (a superset of
-   * every catalogue's own); bounds for the widest */
-  int nsten = 0;
-  double dmin = 0;
-  gmin.k = gmax.k = k;
-  if (gmin.cw[0] > 1e299) {        /* every catalogue failed its checks */
+  if (prec != FCFCG_PREC_FP32_RECHECK) {
+    /* FP32 windows too wide for these boxes: count them in FP64 */
     free(wexp);
     free(hbase);
-    goto out;
+    free(acc);
+    free(base);
+    return batch_fp64(c, jobs, njobs, withwt, on_device);
   }
-  int nin = 0;
-  if ((rc = stencil_build(c, &gmin, 1, c->sten, c->stD, &nsten, &dmin,
-                          gmax.cw, &nin))) {
-    free(wexp);
-    free(hbase);
-    goto out;
-  }
-  double dmax = 0;
-  for (int t = 0; t < nsten; t++)
-    for (int d = 0; d < 3; d++)
-      dmax = fmax(dmax, fabs((double) c->sten[4 * t + d]) * gmax.cw[d]);
   /* 5. cell sort of every catalogue into the shared sorted arrays */
   const size_t m = N;
   if (S->scap < m) {
@@ -2376,10 +2721,13 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   }
   if (S->ccap < cells + 1) {
     if (S->cstart) cudaFree(S->cstart);
-    S->cstart = NULL;
+    if (S->bstart) cudaFree(S->bstart);
+    S->cstart = S->bstart = NULL;
     S->ccap = 0;
     cudaError_t e = cudaMalloc((void **) &S->cstart,
                                sizeof(uint32_t) * (cells + 1));
+    if (!e) e = cudaMalloc((void **) &S->bstart,
+                           sizeof(uint32_t) * (cells + 1));
     if (e) {
       free(wexp);
       free(hbase);
@@ -2387,9 +2735,25 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
     }
     S->ccap = cells + 1;
   }
+  const size_t mb = fcfcg_max_blocks(N, cells);
+  if (S->blkcap < mb) {
+    if (S->blk) cudaFree(S->blk);
+    if (S->bcell) cudaFree(S->bcell);
+    S->blk = NULL;
+    S->bcell = NULL;
+    S->blkcap = 0;
+    cudaError_t e = cudaMalloc((void **) &S->blk, sizeof(float) * 8 * mb);
+    if (!e) e = cudaMalloc((void **) &S->bcell, sizeof(uint32_t) * 2 * mb);
+    if (e) {
+      free(wexp);
+      free(hbase);
+      BCK(e);
+    }
+    S->blkcap = mb;
+  }
   /* fine counters: cells x sub-cells (the points of a cell grouped by
    * sub-cell in the sorted arrays) */
-  const int sb = fcfcg_grid_sub_bits(cells, N);
+  const int sb = fcfcg_grid_curve_bits(cells, N);
   const size_t nf = cells << sb;
   BGROW(c->cfill, c->cfill_cap, sizeof(uint32_t) * (nf + 1));
   BGROW(c->fstart, c->fstart_cap, sizeof(uint32_t) * (nf + 1));
@@ -2429,8 +2793,6 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   BCK(cudaStreamSynchronize(c->stream));
   free(hbase);
   /* 7. launch parameters */
-  fcfcg_launch L;
-  memset(&L, 0, sizeof L);
   L.geometry = FCFCG_GEOM_BOX;
   L.bintype = b->bintype;
   L.isauto = 1;
@@ -2439,32 +2801,17 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
     L.ncell[d] = 1;
     L.box[d] = b->box[d];
   }
-  S->xabs = xabs;
-  S->s2abs = 0;
-  S->wexp = 0;
   launch_cat(&L.A, S);
   launch_cat(&L.B, S);
   launch_bins(c, &L);
   L.mocks = (const fcfcg_mock *) c->d_mock;
   L.nmock = na;
-  int prec = FCFCG_PREC_FP32_RECHECK;
-  if (fp32_bounds(c, &gmax, dmax, S, S, &L)) prec = FCFCG_PREC_FP64;
-  size_t tabbytes = 0, stage = 0;
-  if (prec == FCFCG_PREC_FP32_RECHECK) {
-    launch_fp32_tables(c, &L);
-    tabbytes = fcfcg_k_count32_tab_bytes(L.nfs, L.nfp, L.nsb, L.npb);
-    stage = fcfcg_k_count32_stage(nsten, withwt);
-    if (tabbytes + stage > 200 * 1024) prec = FCFCG_PREC_FP64;
-  }
-  if (prec != FCFCG_PREC_FP32_RECHECK) {
-    /* FP32 windows too wide for these boxes: count them in FP64 */
-    free(wexp);
-    free(acc);
-    free(base);
-    return batch_fp64(c, jobs, njobs, withwt, on_device);
-  }
-  const size_t hbytes = (size_t) b->ntot * (withwt ? 8 : 4);
-  L.hist_smem = (tabbytes + stage + hbytes <= 200 * 1024);
+  L.mbase = c->d_mbase;
+  const size_t hbytes = fcfcg_k_tile32_hist(L.hlen, withwt);
+  L.hist_smem = (fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt) +
+                     hbytes <= 200 * 1024);
+  L.pshift = tile_parts(N, cells, c->nsm);
+  L.nblk_dev = S->bstart + cells;
   L.hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
   L.nsten = nsten;
   L.nin = nin;
@@ -2484,19 +2831,13 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   }
   L.sten = c->d_sten;
   L.stenD = c->d_stenD;
-  /* 8. work chunks of every catalogue, in catalogue order */
+  /* 8. blocks of every catalogue, in catalogue order */
   BGROW(c->cchunk, c->cchunk_cap, sizeof(uint32_t) * 2 * (cells + 1));
-  const size_t maxchunk = N / FCFCG_CHUNK + cells + 1;
-  BGROW(c->chunks, c->chunk_cap, sizeof(uint32_t) * 4 * maxchunk);
-  uint32_t nchunk = 0;
-  BCKK(fcfcg_k_chunks(c->stream, S->cstart, (uint32_t) cells, FCFCG_CHUNK32,
-                      c->cchunk, c->scan_tmp, stl, c->chunks, &nchunk,
+  BCKK(fcfcg_k_blocks(c->stream, S->cstart, (uint32_t) cells, N, c->cchunk,
+                      c->scan_tmp, S->l4, S->bstart, S->blk, S->bcell,
                       c->d_mbase, na));
   c->launches += 5;
   BCK(cudaEventRecord(c->ev[1], c->stream));
-  BCK(cudaStreamSynchronize(c->stream));
-  L.nchunk = nchunk;
-  L.chunks = c->chunks;
   L.chunk_head = c->d_head;
   BCK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * 4,
                       c->stream));
@@ -2525,9 +2866,12 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
       free(wexp);
       BFAIL(FCFCG_ERR_MEMORY);
     }
+    uint32_t nblk = 0;
     cudaError_t e = cudaMemcpyAsync(hres, c->d_bout,
                                     sizeof(unsigned long long) * per * na,
                                     cudaMemcpyDeviceToHost, c->stream);
+    if (!e) e = cudaMemcpyAsync(&nblk, L.nblk_dev, sizeof nblk,
+                                cudaMemcpyDeviceToHost, c->stream);
     if (!e) e = cudaMemcpyAsync(hstats, c->d_stats, sizeof hstats,
                                 cudaMemcpyDeviceToHost, c->stream);
     if (!e) e = cudaStreamSynchronize(c->stream);
@@ -2568,7 +2912,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
     o->ms_total = ms;
     o->cells_per_smax = k;
     o->nstencil = nsten;
-    o->nchunks = nchunk;
+    o->nchunks = nblk;
     o->precision_used = prec;
     o->warp_queue = prec == FCFCG_PREC_FP32_RECHECK ? (int) c->last_qwarp : 0;
     o->launches = c->launches;

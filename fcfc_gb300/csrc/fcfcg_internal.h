@@ -49,6 +49,12 @@ typedef struct {
   float *fedge;          /* nbin + 1 edges rounded to FP32 (host) */
   double vmin, vmax;     /* edge[0], edge[nbin] */
   int min0;              /* edge[0] == 0: no lower range check (smin0) */
+  /* edge table of the tile kernel (host): netab cells of the value's FP32
+   * bits >> elg, from cell eoff on, (edge, 1.5 2^23 + column) each, then two
+   * entries for the values below: no edge near, and ambiguous */
+  float *etab;
+  int netab, elg;
+  long eoff;
 } fcfcg_axis;
 
 typedef struct {
@@ -70,6 +76,9 @@ void fcfcg_bins_release(fcfcg_bins *b);
 /* Build the FP32 window table of an axis (ftab / foff / nftab); allow_log:
  * a bit-pattern table may replace a uniform one with multi-edge cells. */
 int fcfcg_axis_ftab(fcfcg_axis *a, int allow_log);
+/* Build the tile kernel's edge table of an axis for values up to top;
+ * root: of the square roots of the edges (pi of a survey). */
+int fcfcg_axis_etab(fcfcg_axis *a, double top, int root);
 /* Accessors of the opaque context used by the post-processing code. */
 const fcfcg_bins *fcfcg_ctx_bins(const fcfcg_ctx *c);
 const double *fcfcg_ctx_box_raw(const fcfcg_ctx *c);
@@ -85,6 +94,12 @@ typedef struct {
   const double *x, *y, *z, *s, *w;   /* rescaled FP64, |x|^2, weight */
   const uint32_t *id;    /* input index */
   const uint32_t *cstart;/* ncell + 1 */
+  /* blocks of at most 32 points of a cell: two float4 each, (box centre,
+   * bits of the first sorted index) and (half extents, bits of the count);
+   * bstart: the cells' first blocks (ncell + 1); bcell: (cell, catalogue of
+   * a batch) per block */
+  const float *blk;
+  const uint32_t *bstart, *bcell;
   int wexp;              /* weights scaled by 2^-wexp */
 } fcfcg_dcat;
 
@@ -115,6 +130,13 @@ typedef struct {
   const uint32_t *nchunk_dev;
   const uint32_t *chunks;
   uint32_t *chunk_head;
+  /* tile kernel: the number of A blocks (device), log2 of the parts a
+   * block's tiles are dealt to, slack of the block box distance, and for a
+   * batch the catalogues' first cells (nmock + 1) */
+  const uint32_t *nblk_dev;
+  int pshift;
+  float box_eps;
+  const uint32_t *mbase;
   fcfcg_dcat A, B;
   /* bins */
   int ns, nmu, np;
@@ -140,6 +162,27 @@ typedef struct {
    * that is a boundary */
   int slin, lin_k0;
   float lin_inv, lin_off, lin_A, lin_B;
+  /* the tile kernel's linear bins: column rn((s + tl_s0) tl_inv), an edge
+   * within the window at a distance >= tl_h from the column's middle; mu:
+   * rn((mu + tl_q0) nmu) and >= tl_qc - tl_q1 / s; |x_b|^2 below near2: the line of sight is
+   * tested per pair.  Shared histogram: hcols columns per row, bin (0, 0) at
+   * column hcol0, row hrow0; hrows rows of bins; hlen in all */
+  int tlin, tplin;             /* linear s bins; linear pi bins */
+  float tl_inv, tl_s0, tl_h, tl_q0, tl_q1, tl_qc, near2;
+  /* linear pi bins: row rn((pi + tl_p0) tl_pinv), window at tl_hp (pi by
+   * table: its window); tables: the window of s^2 or s_perp^2 is tl_ea s^2 +
+   * tl_eb */
+  float tl_p0, tl_pinv, tl_hp, tl_ea, tl_eb;
+  /* s^2 or s_perp^2, and pi, of an unambiguous pair outside the bins: below
+   * tl_slo, tl_plo, or (survey s_perp^2) from tl_shi on */
+  float tl_slo, tl_shi, tl_plo;
+  /* edge tables (float2 per cell: the edge, 1.5 2^23 + the column below it):
+   * cell = FP32 bits >> lg, from off on; in use from the skip-th, the last
+   * entry being entry *_last, for all values below */
+  const float *se, *pe;
+  int nse, npe, se_lg, pe_lg, se_off, pe_off, se_skip, pe_skip, se_last,
+      pe_last;
+  int hcols, hcol0, hrow0, hrows, hlen;
   float P0, P1, P2;            /* E(pi) (box) or E(pi^2) (survey) */
   float Q0, Q1, Q2;            /* E(q), q = nmu mu: Q1 / s + Q2 q + Q0 */
   float m2min;                 /* survey: |m|^2 below (next to the observer):
@@ -199,9 +242,11 @@ int fcfcg_k_prep(void *stream, size_t n, const double *x, const double *y,
     unsigned long long *wmax_bits, double *partial, double *wsum);
 size_t fcfcg_prep_partials(void);
 /* Sub-cell bits of a grid of ncell cells holding npoint points: 6 (4 x 4
- * x 4 sub-cells in Morton order within a cell), 3 (2 x 2 x 2) or 0; the
- * sort then uses (ncell << sb) fine counters. */
+ * x 4 sub-cells), 3 (2 x 2 x 2) or 0; the sort then uses (ncell << sb) fine
+ * counters.  curve: those of the sort along a Hilbert curve, also 9, 12 and
+ * 15 where cells hold many points. */
 int fcfcg_grid_sub_bits(size_t ncell, size_t npoint);
+int fcfcg_grid_curve_bits(size_t ncell, size_t npoint);
 /* Counting sort into the grid, cells in order and, within a cell, by
  * sub-cell (sb bits); cstart[0..nc] the cells' first sorted points.
  * Scratch: cell_of (n), fstart and cfill ((nc << sb) + 1 each), scan_tmp
@@ -219,6 +264,14 @@ int fcfcg_k_chunks(void *stream, const uint32_t *cstart, uint32_t ncell,
     uint32_t clen, uint32_t *cchunk, uint32_t *scan_tmp, size_t scan_tmp_len,
     uint32_t *chunks, uint32_t *nchunk_out, const uint32_t *mock_cell_base,
     int nmock);
+/* Blocks of at most 32 points of the cells of a sorted catalogue (see
+ * fcfcg_dcat): bstart (ncell + 1 entries), blk and bcell (at most n / 32 +
+ * min(n, ncell) blocks); count: ncell scratch words; mbase as above. */
+size_t fcfcg_max_blocks(size_t n, size_t ncell);
+int fcfcg_k_blocks(void *stream, const uint32_t *cstart, uint32_t ncell,
+    size_t n, uint32_t *count, uint32_t *scan_tmp, const float *l4,
+    uint32_t *bstart, float *blk, uint32_t *bcell, const uint32_t *mbase,
+    int nmock);
 /* One catalogue of a batch for the preparation kernels: its inputs (device
  * or GPU-readable host memory), its place o in the batch slot, its first
  * tile (tiles of fcfcg_batch_tile() points, numbered across the batch) and,
@@ -230,7 +283,7 @@ typedef struct {
   int live, wexp;
   int ncell[3];
   uint32_t cell_base;
-  double cw[3];
+  double cw[3], inv[3];  /* cell widths and their reciprocals */
 } fcfcg_prep_cat;
 
 size_t fcfcg_batch_tile(void);
@@ -260,6 +313,12 @@ int fcfcg_k_unsort(void *stream, size_t n, const uint32_t *sid,
     const double *in, double *out);
 int fcfcg_scan(void *stream, const uint32_t *in, size_t n, uint32_t *out,
     uint32_t *tmp);
+/* Shared memory of the tile kernel: its tables, and besides them and its
+ * histogram. */
+size_t fcfcg_k_tile32_tab(const fcfcg_launch *L);
+size_t fcfcg_k_tile32_stage(int withwt);
+/* And its histogram's, with a spare word per lane. */
+size_t fcfcg_k_tile32_hist(int hlen, int withwt);
 /* withwt: 0 unweighted, 1 weighted, 2 adjoint */
 size_t fcfcg_k_count32_stage(int nsten, int withwt);
 size_t fcfcg_k_count32_tab_bytes(int nfs, int nfp, int nsb, int npb);

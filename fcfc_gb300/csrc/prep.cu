@@ -253,47 +253,91 @@ static int scan_u32(cudaStream_t s, const uint32_t *in, size_t n,
 
 /*
  * The fine index of a point: its global cell (cells of one grid numbered
- * from cell_base), shifted left by sb, and with sb = 3 or 6 its sub-cell
- * (2 or 4 per axis) in Morton order.  Sorting by the fine index keeps each
- * cell's points contiguous and, within the cell, groups them by sub-cell,
- * so that runs of 32 or 64 consecutive points (the count kernel's
- * neighbour blocks and chunks) are compact.  The cell of an axis is
- * floor((v - lo) / cw) clamped to [0, n).
+ * from cell_base), shifted left by sb = 3 r, and its sub-cell (2^r per axis)
+ * along a Hilbert curve.  Sorting by the fine index keeps each cell's points
+ * contiguous and orders them so that runs of consecutive points (the count
+ * kernels' blocks) are compact.  A point's place along an axis is the
+ * integer part of (v - lo) 2^r / cw, clamped: with the reciprocal's rounding
+ * a point within an ulp of a cell's face may go to either side, which the
+ * count kernels' cell margins cover.
  */
-__device__ __forceinline__ uint32_t fine_of_point(double a, double b,
-    double d, int nx, int ny, int nz, double cwx, double cwy, double cwz,
-    double lox, double loy, double loz, uint32_t cell_base, int sb) {
-  const double v[3] = {a, b, d}, lo[3] = {lox, loy, loz},
-               cw[3] = {cwx, cwy, cwz};
-  const int n[3] = {nx, ny, nz};
-  const int r = sb / 3;                   /* bits per axis */
-  int c[3];
-  uint32_t m = 0;
+struct FineGrid {
+  int n[3];
+  double inv[3], lo[3];      /* 2^r / cell width */
+  uint32_t base;
+  int r;
+};
+
+static FineGrid fine_grid(const int n[3], const double cw[3],
+    const double lo[3], int sb) {
+  FineGrid g;
+  g.r = sb / 3;
   for (int k = 0; k < 3; k++) {
-    const double q = (v[k] - lo[k]) / cw[k];
-    const double t = floor(q);
-    c[k] = (t < 0) ? 0 : (t >= n[k] ? n[k] - 1 : (int) t);
-    if (r) {
-      const int lim = (1 << r) - 1;
-      int s = (int) floor((q - (double) c[k]) * (double) (1 << r));
-      s = s < 0 ? 0 : (s > lim ? lim : s);
-      for (int bit = 0; bit < r; bit++)
-        m |= (uint32_t) ((s >> bit) & 1) << (3 * bit + k);
+    g.n[k] = n[k];
+    g.inv[k] = (double) (1 << g.r) / cw[k];
+    g.lo[k] = lo[k];
+  }
+  g.base = 0;
+  return g;
+}
+
+/* Index of a sub-cell along the Hilbert curve of 2^r sub-cells per axis,
+ * by J. Skilling's transposition (AIP Conf. Proc. 707, 381, 2004): the axes
+ * are rotated and reflected from the highest bit down, Gray-decoded, and
+ * their bits interleaved. */
+__device__ __forceinline__ uint32_t hilbert3(uint32_t x, uint32_t y,
+    uint32_t z, int r) {
+  uint32_t X[3] = {x, y, z};
+  for (uint32_t Q = 1u << (r - 1); Q > 1; Q >>= 1) {
+    const uint32_t P = Q - 1;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      if (X[i] & Q) {
+        X[0] ^= P;
+      } else {
+        const uint32_t t = (X[0] ^ X[i]) & P;
+        X[0] ^= t;
+        X[i] ^= t;
+      }
     }
   }
-  const uint32_t cell = cell_base + ((uint32_t) c[2] * ny + c[1]) * nx + c[0];
-  return (cell << sb) | m;
+  X[1] ^= X[0];
+  X[2] ^= X[1];
+  uint32_t t = 0;
+  for (uint32_t Q = 1u << (r - 1); Q > 1; Q >>= 1)
+    if (X[2] & Q) t ^= Q - 1;
+  uint32_t h = 0;
+  for (int b = r - 1; b >= 0; b--)
+#pragma unroll
+    for (int i = 0; i < 3; i++) h = (h << 1) | (((X[i] ^ t) >> b) & 1u);
+  return h;
+}
+
+__device__ __forceinline__ uint32_t fine_of_point(const FineGrid &g,
+    double a, double b, double d) {
+  const double v[3] = {a, b, d};
+  int c[3];
+  uint32_t s[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    int X = __double2int_rd((v[k] - g.lo[k]) * g.inv[k]);
+    const int top = (g.n[k] << g.r) - 1;
+    X = X < 0 ? 0 : (X > top ? top : X);
+    c[k] = X >> g.r;
+    s[k] = (uint32_t) X & ((1u << g.r) - 1u);
+  }
+  const uint32_t cell = g.base +
+      ((uint32_t) c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
+  return g.r ? (cell << (3 * g.r)) | hilbert3(s[0], s[1], s[2], g.r) : cell;
 }
 
 __global__ void k_cell(size_t n, const double *__restrict__ x,
-    const double *__restrict__ y, const double *__restrict__ z, int nx,
-    int ny, int nz, double cwx, double cwy, double cwz, double lox,
-    double loy, double loz, uint32_t cell_base, int sb,
-    uint32_t *__restrict__ cell_of, uint32_t *__restrict__ count) {
+    const double *__restrict__ y, const double *__restrict__ z,
+    const FineGrid g, uint32_t *__restrict__ cell_of,
+    uint32_t *__restrict__ count) {
   for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n;
        i += (size_t) gridDim.x * blockDim.x) {
-    uint32_t c = fine_of_point(x[i], y[i], z[i], nx, ny, nz, cwx, cwy, cwz,
-                               lox, loy, loz, cell_base, sb);
+    const uint32_t c = fine_of_point(g, x[i], y[i], z[i]);
     cell_of[i] = c;
     atomicAdd(count + c, 1u);
   }
@@ -373,6 +417,16 @@ extern "C" int fcfcg_grid_sub_bits(size_t ncell, size_t npoint) {
   return 0;
 }
 
+extern "C" int fcfcg_grid_curve_bits(size_t ncell, size_t npoint) {
+  /* in coarse cells the finest of 32, 16 or 8 sub-cells per axis with at
+   * most 2 fine counters per point, so that clearing and scanning them stays
+   * below the cost of moving the points (a sub-cell then holds a few points,
+   * well below a block of 32); else 4, 2 or none */
+  for (int sb = 15; sb > 6; sb -= 3)
+    if (ncell << sb <= npoint * 2 && (ncell << sb) < 0xFFFFFFF0u) return sb;
+  return fcfcg_grid_sub_bits(ncell, npoint);
+}
+
 extern "C" int fcfcg_k_grid(void *stream, size_t n, const double *x,
     const double *y, const double *z, const double *s, const double *w,
     int has_w, int wexp, const int ncell[3], const double cw[3],
@@ -388,8 +442,7 @@ extern "C" int fcfcg_k_grid(void *stream, size_t n, const double *x,
   if (e) return (int) e;
   if (n) {
     k_cell<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0, st>>>(
-        n, x, y, z, ncell[0], ncell[1], ncell[2], cw[0], cw[1], cw[2], lo[0],
-        lo[1], lo[2], 0u, sb, cell_of, cfill);
+        n, x, y, z, fine_grid(ncell, cw, lo, sb), cell_of, cfill);
     if ((e = cudaGetLastError())) return (int) e;
   }
   int r = scan_u32(st, cfill, nf, fstart, scan_tmp);
@@ -564,12 +617,16 @@ __global__ void __launch_bounds__(PREP_THREADS) k_cell_batch(
   const size_t o = C->o, n = C->n;
   const size_t i0 = (size_t) (t - C->tile0) * BATCH_TILE;
   const size_t i1 = (i0 + BATCH_TILE < n) ? i0 + BATCH_TILE : n;
-  const int nx = C->ncell[0], ny = C->ncell[1], nz = C->ncell[2];
-  const double cwx = C->cw[0], cwy = C->cw[1], cwz = C->cw[2];
-  const uint32_t base = C->cell_base;
+  FineGrid g;
+  for (int k = 0; k < 3; k++) {
+    g.n[k] = C->ncell[k];
+    g.inv[k] = C->inv[k] * (double) (1 << (sb / 3));
+    g.lo[k] = 0.0;
+  }
+  g.base = C->cell_base;
+  g.r = sb / 3;
   for (size_t i = o + i0 + threadIdx.x; i < o + i1; i += PREP_THREADS) {
-    const uint32_t c = fine_of_point(x[i], y[i], z[i], nx, ny, nz, cwx, cwy,
-                                     cwz, 0.0, 0.0, 0.0, base, sb);
+    const uint32_t c = fine_of_point(g, x[i], y[i], z[i]);
     cell_of[i] = c;
     atomicAdd(count + c, 1u);
   }
@@ -690,6 +747,97 @@ extern "C" int fcfcg_k_chunks(void *stream, const uint32_t *cstart,
                              cudaMemcpyDeviceToHost, st)))
       return (int) e;
   return 0;
+}
+
+/* ------------------------------------------------------------------------ */
+/* Blocks of at most 32 points. */
+
+__global__ void k_block_count(const uint32_t *__restrict__ cstart,
+    uint32_t ncell, uint32_t *__restrict__ count) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
+       c += gridDim.x * blockDim.x)
+    count[c] = (cstart[c + 1] - cstart[c] + 31u) / 32u;
+}
+
+/* A warp per block: the points of a cell are cut as evenly as possible, and
+ * the block's box is that of its FP32 offsets from the cell centre (half
+ * extents rounded up). */
+__global__ void __launch_bounds__(PREP_THREADS) k_blocks(
+    const uint32_t *__restrict__ cstart, uint32_t ncell,
+    const uint32_t *__restrict__ bstart, const float4 *__restrict__ l4,
+    float4 *__restrict__ blk, uint2 *__restrict__ bcell,
+    const uint32_t *__restrict__ mbase, int nmock) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nblk = __ldg(bstart + ncell);
+  const uint32_t nw = gridDim.x * (PREP_THREADS / 32);
+  for (uint32_t b = blockIdx.x * (PREP_THREADS / 32) + (threadIdx.x >> 5);
+       b < nblk; b += nw) {
+    uint32_t lo = 0, hi = ncell;    /* last lo with bstart[lo] <= b */
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (__ldg(bstart + mid) <= b) lo = mid;
+      else hi = mid;
+    }
+    const uint32_t a = __ldg(cstart + lo), n = __ldg(cstart + lo + 1) - a;
+    const uint32_t q = b - __ldg(bstart + lo), nq = (n + 31u) / 32u;
+    const uint32_t i0 = (uint32_t) (((unsigned long long) n * q) / nq),
+                   i1 = (uint32_t) (((unsigned long long) n * (q + 1)) / nq);
+    const uint32_t m = i1 - i0;
+    const float4 v = __ldg(l4 + a + i0 + (lane < (int) m ? lane : 0));
+    float mn[3] = {v.x, v.y, v.z}, mx[3] = {v.x, v.y, v.z};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+        mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+      }
+    if (lane == 0) {
+      float c[3], e[3];
+      for (int k = 0; k < 3; k++) {
+        c[k] = 0.5f * mn[k] + 0.5f * mx[k];
+        e[k] = __fmul_ru(fmaxf(__fsub_ru(mx[k], c[k]), __fsub_ru(c[k], mn[k])),
+                         1.000001f);
+      }
+      blk[2 * (size_t) b] = make_float4(c[0], c[1], c[2],
+                                        __uint_as_float(a + i0));
+      blk[2 * (size_t) b + 1] = make_float4(e[0], e[1], e[2],
+                                            __uint_as_float(m));
+      uint32_t mk = 0;
+      if (mbase) {
+        int l = 0, h = nmock;       /* last l with mbase[l] <= the cell */
+        while (h - l > 1) {
+          const int mid = (l + h) >> 1;
+          if (__ldg(mbase + mid) <= lo) l = mid;
+          else h = mid;
+        }
+        mk = (uint32_t) l;
+      }
+      bcell[b] = make_uint2(lo, mk);
+    }
+  }
+}
+
+extern "C" size_t fcfcg_max_blocks(size_t n, size_t ncell) {
+  return n / 32 + (n < ncell ? n : ncell) + 1;
+}
+
+extern "C" int fcfcg_k_blocks(void *stream, const uint32_t *cstart,
+    uint32_t ncell, size_t n, uint32_t *count, uint32_t *scan_tmp,
+    const float *l4, uint32_t *bstart, float *blk, uint32_t *bcell,
+    const uint32_t *mbase, int nmock) {
+  cudaStream_t st = (cudaStream_t) stream;
+  k_block_count<<<grid_for(ncell, PREP_THREADS), PREP_THREADS, 0, st>>>(
+      cstart, ncell, count);
+  cudaError_t e = cudaGetLastError();
+  if (e) return (int) e;
+  int r = scan_u32(st, count, ncell, bstart, scan_tmp);
+  if (r) return r;
+  k_blocks<<<grid_for(fcfcg_max_blocks(n, ncell) * 32, PREP_THREADS),
+             PREP_THREADS, 0, st>>>(cstart, ncell, bstart,
+                                    (const float4 *) l4, (float4 *) blk,
+                                    (uint2 *) bcell, mbase, nmock);
+  return (int) cudaGetLastError();
 }
 
 /* Occupancy of a coarse grid over a catalogue's bounding box: one bit per

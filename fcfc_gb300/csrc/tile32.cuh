@@ -1,0 +1,1016 @@
+/*
+ * tile32.cuh -- the FP32 pair-counting kernel (instantiated by count32_*.cu).
+ *
+ * Work decomposition (replaces FCFC's dual k-d tree, src/fcfc/2pt_box/
+ * dual_tree.c:245-373, and its OpenMP/MPI node-pair scheduler,
+ * count_func.c:7431-7722):
+ *   - points are sorted into a coarse cell grid (cells about as wide as the
+ *     largest separation that counts) and, inside a cell, along a Hilbert
+ *     curve; a cell's points are cut into blocks of at most 32, each with
+ *     its bounding box (prep.cu:k_blocks);
+ *   - the unit of work is a tile: the points of one block (A, in shared
+ *     memory) against those of another (B, one per lane).  A persistent
+ *     warp takes a block A from a global counter, tests the boxes of 32
+ *     blocks B of the cell stencil at a time, one per lane, and visits the
+ *     tiles that can hold a pair;
+ *   - auto counts use half of the stencil, blocks from A's own on in A's
+ *     cell, and i < j within a block.
+ *
+ * Warps share only the CTA's histogram: there is no barrier and no list in
+ * the main loop (a batch has one per run of blocks of a catalogue).
+ *
+ * Per pair (FP32 path): separations on coordinates relative to the cell
+ * centres, four points of A per step with packed FP32, the bin from the
+ * separation itself (linear bins) or from a table of edges in shared
+ * memory, and a rounding bound: a pair whose s^2, mu, s_perp^2 or pi lies
+ * within the bound of a bin edge is queued and re-binned by the FP64 formula
+ * of the reference (metric_common.c of src/fcfc/2pt_box and src/fcfc/2pt),
+ * so integer counts equal the FP64 build.
+ *
+ * What bounds it: instruction issue and the FMA pipe (issue slots 78 % used,
+ * FMA pipe 50 %, ALU 56 % on an unweighted (s, mu) box).  1.5 warp
+ * instructions per in-range pair: 8 per pair slot for the distance test
+ * (1.9 slots per in-range pair) and 22 for binning the slots whose step is
+ * not empty (67 % of them).  A kernel that tested candidates first, queued
+ * them and binned them compacted took 2.7.  Counts of one launch, before and
+ * after: (s, mu) box of 2e6 points weighted 32.2 -> 23.8 ms, (s_perp, pi)
+ * with log bins 5.5 -> 3.4, log s bins of 4e5 points 3.5 -> 1.3, 256 mocks
+ * 607 -> 362 ms, survey (s, mu) RR + DR of 4e6 randoms 407 -> 310.
+ *
+ * Histograms live in shared memory (u32 counts, or int64 fixed-point weight
+ * products) and are merged into global 64/128-bit integer accumulators, so
+ * the results do not depend on the order of the additions.
+ */
+#ifndef FCFCG_TILE32_CUH
+#define FCFCG_TILE32_CUH
+#include "count_common.cuh"
+
+/* 1 / sqrt(x): relative error <= 2^-22.9 (PTX ISA); 0 gives +inf. */
+__device__ __forceinline__ float rsq_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+/* Shared memory of a warp: its block A, four points' coordinates at a time;
+ * 32 stencil entries; and its counters.  What the inner loop does not use is
+ * kept here: its registers decide the CTAs per SM. */
+struct TileWarp {
+  ulonglong2 p[8][3];      /* points 4k .. 4k + 3: x, y, z of each */
+  float4 sd[32];           /* stencil entry: -offset * width, image code */
+  uint2 si[32];            /* its first block and their number */
+  unsigned long long cnt[4];   /* as fcfcg_launch.stats */
+};
+/* with weights: (round(w 2^30), remainder, w) of each point of A */
+struct TileWarpW {
+  TileWarp t;
+  float4 aw[32];
+};
+
+__host__ __device__ __forceinline__ size_t tile_warp_bytes(int wt) {
+  return wt ? sizeof(TileWarpW) : sizeof(TileWarp);
+}
+
+/* Two FP32 values in a 64-bit register, for the packed instructions: each
+ * rounds its two components as the scalar ones do, in one issue slot (the
+ * FMA pipe takes two cycles). */
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f2 dup2(float a) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+/* Add 1 to a 32-bit shared bin at a shared-space byte address where ok, and
+ * to the lane's spare word elsewhere: a predicated shared atomic compiles to
+ * a branch around it (3.3 branch instructions each).  (No memory clobber:
+ * the bins are read only behind barriers and through atomics, and a clobber
+ * has the launch parameters loaded again after each pair.) */
+__device__ __forceinline__ void red_inc(uint32_t addr, uint32_t spare,
+    bool ok) {
+  asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(ok ? addr : spare));
+}
+
+/* The same for a pair within the outer range (c) with no edge in its windows
+ * (|f| < h, |fq| < hq); one with an edge sets bit BIT of rest.  The tests
+ * chain through predicates. */
+template <int BIT>
+__device__ __forceinline__ void red_pair(uint32_t addr, uint32_t spare,
+    bool in, float f, float h, float fq, float hq, uint32_t &rest) {
+  asm volatile("{.reg .pred c, g, a, b; .reg .f32 t; .reg .u32 x;\n\t"
+               "setp.ne.u32 c, %2, 0;\n\t"
+               "abs.f32 t, %3; setp.lt.and.f32 g|a, t, %4, c;\n\t"
+               "abs.f32 t, %5; setp.lt.and.f32 g|b, t, %6, g;\n\t"
+               "@a or.b32 %0, %0, %7;\n\t"
+               "@b or.b32 %0, %0, %7;\n\t"
+               "selp.u32 x, %1, %8, g;\n\t"
+               "red.shared.add.u32 [x], 1;}"
+               : "+r"(rest) : "r"(addr), "r"((uint32_t) in), "f"(f), "f"(h),
+                 "f"(fq), "f"(hq), "n"(BIT), "r"(spare));
+}
+template <int BIT>
+__device__ __forceinline__ void red_pair(uint32_t addr, uint32_t spare,
+    bool in, float f, float h, uint32_t &rest) {
+  asm volatile("{.reg .pred c, g, a; .reg .f32 t; .reg .u32 x;\n\t"
+               "setp.ne.u32 c, %2, 0;\n\t"
+               "abs.f32 t, %3; setp.lt.and.f32 g|a, t, %4, c;\n\t"
+               "@a or.b32 %0, %0, %5;\n\t"
+               "selp.u32 x, %1, %6, g;\n\t"
+               "red.shared.add.u32 [x], 1;}"
+               : "+r"(rest) : "r"(addr), "r"((uint32_t) in), "f"(f), "f"(h),
+                 "n"(BIT), "r"(spare));
+}
+
+/* Launch parameters of the inner loop, held in registers: as operands of
+ * the constant bank two in one instruction cost a load each time. */
+__device__ __forceinline__ float pin(float a) {
+  asm volatile("" : "+f"(a));
+  return a;
+}
+__device__ __forceinline__ uint32_t pin(uint32_t a) {
+  asm volatile("" : "+r"(a));
+  return a;
+}
+struct LinConst {
+  float slim;              /* the outer range */
+  float inv, s0, hs;       /* linear s bins */
+  float q0, nmu, q1, qc;   /* mu */
+  float p0, pinv, hp;      /* linear pi bins */
+  float ea, eb;            /* window of a table's value: ea s^2 + eb */
+  float hc;                /* columns of a row */
+  uint32_t ha, spare;
+};
+
+/* An axis by table: cells of the value's FP32 bits >> lg from off on, the
+ * last of n taking all below; (edge, 1.5 2^23 + column below the edge). */
+struct EdgeTab {
+  const float2 *t;
+  int lg, off;
+  uint32_t last;
+};
+
+#define TMAGIC 12582912.f                  /* 1.5 2^23 */
+#define TMAGIC_BITS 0x4B400000u
+
+/* Shared bin x (hcols columns per row, the first bin at row hrow0, column
+ * hcol0) to the global bin, or -1 out of range. */
+__device__ __forceinline__ int tile_gbin(const fcfcg_launch &L, uint32_t x) {
+  const int s = (int) (x % (uint32_t) L.hcols) - L.hcol0;
+  const int q = (int) (x / (uint32_t) L.hcols) - L.hrow0;
+  if (s < 0 || s >= L.ns || q < 0 || q >= L.hrows) return -1;
+  return s + q * L.ns;
+}
+
+/* fix_prod with the rounding constant and the cross term added before the
+ * one shift: (p + 2^8 + 2^9 c) >> 9 = ((p + 2^8) >> 9) + c, the same integer
+ * in fewer operations. */
+__device__ __forceinline__ long long tile_prod(int ia, float ra, float fa,
+    int ib, float rb, float fb) {
+  const float c = __fadd_rn(__fmul_rn(fa, rb), __fmul_rn(ra, fb));
+  const float t = __fmaf_rn(c, 2251799813685248.0f /* 2^51 */, TMAGIC);
+  const long long p = (long long) ia * (long long) ib +
+      (256ll - ((long long) TMAGIC_BITS << 9));
+  return (p + (long long) __float_as_int(t) * 512ll) >> 9;
+}
+
+/* Weighted sums in shared memory: two 32-bit words per bin (the high words
+ * hlen + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed;
+ * the carry out of lo is read from the returned value, and 2^30 of hi (2^62)
+ * moves to the global 128-bit accumulator when hi crosses +-2^30. */
+__device__ __forceinline__ uint32_t add_lo(uint32_t addr, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.shared.add.u32 %0, [%1], %2;"
+               : "=r"(old) : "r"(addr), "r"(v));
+  return old;
+}
+__device__ __forceinline__ int add_hi(uint32_t addr, int v) {
+  int old;
+  asm volatile("atom.shared.add.s32 %0, [%1], %2;"
+               : "=r"(old) : "r"(addr), "r"(v));
+  return old;
+}
+/* After hi went from oh to nh: move 2^62 if this add crossed +-2^30 (an add
+ * is below 2^20 in magnitude, so the top two bits of oh and nh differ). */
+__device__ __forceinline__ void hi_moved(const fcfcg_launch &L, uint32_t mock,
+    uint32_t addr, uint32_t ah, uint32_t hb, int oh, int nh) {
+  const int d = (nh >= HI_LIMIT && oh < HI_LIMIT) ? HI_LIMIT
+      : ((nh <= -HI_LIMIT && oh > -HI_LIMIT) ? -HI_LIMIT : 0);
+  if (!d) return;
+  asm volatile("red.shared.add.s32 [%0], %1;" :: "r"(ah), "r"(-d));
+  const int b = tile_gbin(L, (addr - hb) >> 2);
+  if (b >= 0)
+    add128((L.mocks ? L.mocks[mock].gwt : L.gwt) + 2 * b,
+           (long long) d << 32);
+}
+/* Two weighted pairs: their atomics overlap. */
+__device__ __forceinline__ void tile_add_w2(const fcfcg_launch &L,
+    uint32_t mock, uint32_t hb, uint32_t a0, uint32_t a1, long long v0,
+    long long v1) {
+  const uint32_t ho = 4u * (uint32_t) ((L.hist_smem ? L.hlen : 0) + 32);
+  const uint32_t l0 = add_lo(a0, (uint32_t) v0), l1 = add_lo(a1, (uint32_t) v1);
+  const int h0 = (int) (v0 >> 32) + ((l0 + (uint32_t) v0) < l0 ? 1 : 0),
+            h1 = (int) (v1 >> 32) + ((l1 + (uint32_t) v1) < l1 ? 1 : 0);
+  const int o0 = add_hi(a0 + ho, h0), o1 = add_hi(a1 + ho, h1);
+  const int n0 = o0 + h0, n1 = o1 + h1;
+  if ((((o0 ^ n0) | (o1 ^ n1)) & (int) 0xC0000000) && L.hist_smem) {
+    hi_moved(L, mock, a0, a0 + ho, hb, o0, n0);
+    hi_moved(L, mock, a1, a1 + ho, hb, o1, n1);
+  }
+}
+
+/* State of a warp's tile. */
+struct Tile {
+  int m;                    /* points of A */
+  int ilim;                 /* this lane's pairs: A points below ilim */
+  uint32_t first;           /* first sorted index of A */
+  uint32_t bj;              /* this lane's sorted index */
+  uint32_t code, mock;      /* image code of the cell pair, catalogue */
+  float bx, by, bz;         /* this lane's point, from A's cell centre */
+  float vx, vy, vz;         /* survey: 2 b + 2 c_A */
+  float ux, uy, uz, lh, lP; /* survey (s_perp, pi): line-of-sight cut */
+  int wi;                   /* this lane's weight */
+  float wr, wf;
+};
+
+/* Column of a value in a table, as 1.5 2^23 + column: the cell's, plus one
+ * from the cell's edge on; the edge's distance goes to dist.  A cell with
+ * several edges near it holds a NaN: the distance then exceeds no window. */
+__device__ __forceinline__ float tab_col(const EdgeTab &E, float v,
+    float &dist) {
+  const uint32_t i = (__float_as_uint(v) >> E.lg) - (uint32_t) E.off;
+  const float2 e = E.t[i < E.last ? i : E.last];
+  const float d = __fsub_rn(v, e.x);
+  dist = fabsf(d);
+  return d >= 0.f ? __fadd_rn(e.y, 1.f) : e.y;
+}
+
+/*
+ * The bins of two pairs.
+ *
+ * Linear bins: t = (s + s0) inv rounds to the bin's column rn(t) by adding
+ * 1.5 2^23 (no conversion instruction), and an edge lies within the window W
+ * of t when |t - rn(t)| >= 1/2 - W; W is taken at the top of the range.  mu
+ * likewise with t = (mu + q0) nmu, its window's term in q at q = nmu, so
+ * that one FMA remains; linear pi bins likewise.  Other bins: the edge table
+ * (tab_col) of s^2, s_perp^2 or pi (survey: pi^2), the window a linear bound
+ * ea s^2 + eb.
+ *
+ * v: 1.5 2^23 + the shared bin (row hcols + column, exact), so that its low
+ * bits are the bin.  No edge lies within the windows when |f| < h and |g| <
+ * k (k = 1, g = 0 without a second axis).
+ */
+struct PairBin {
+  f2 v, f, h, g, k;
+  f2 col, nq;              /* 1.5 2^23 + column; - row */
+  f2 s;                    /* s^2 or s_perp^2 */
+  float2 pi;
+};
+template <int GEOM, int BIN>
+__device__ __forceinline__ PairBin pair_bin(const LinConst &C,
+    const EdgeTab &ES, const EdgeTab &EP, f2 s2p, f2 dzp, f2 dmp, f2 mmp) {
+  constexpr bool SURVEY = GEOM == FCFCG_GEOM_SURVEY;
+  PairBin p;
+  const f2 mag = dup2(TMAGIC), neg = dup2(-1.f);
+  const float2 s2 = unpack2(s2p);
+  f2 rs = 0;
+  if (LINS(BIN) || IS_SMU(BIN)) rs = pack2(rsq_ftz(s2.x), rsq_ftz(s2.y));
+  /* rows: mu or pi */
+  f2 nq = 0;                        /* - the row */
+  f2 sv = s2p;                      /* the s axis' value */
+  if (IS_SMU(BIN)) {
+    f2 x;
+    if (SURVEY) {
+      const float2 m = unpack2(mul2(mmp, s2p)), d = unpack2(dmp);
+      x = pack2(fabsf(d.x) * rsq_ftz(m.x), fabsf(d.y) * rsq_ftz(m.y));
+    } else {
+      const float2 d = unpack2(dzp), q = unpack2(rs);
+      x = pack2(fabsf(d.x) * q.x, fabsf(d.y) * q.y);
+    }
+    const f2 q = add2(x, dup2(C.q0)), nmu = dup2(C.nmu);
+    nq = fma2(fma2(q, nmu, mag), neg, mag);
+    p.g = fma2(q, nmu, nq);
+    p.k = fma2(dup2(C.q1), rs, dup2(C.qc));
+  } else if (IS_SPI(BIN)) {
+    float2 &pi = p.pi;
+    if (SURVEY) {
+      /* pi = |d.m| / |m|, s_perp^2 = s^2 - pi^2 */
+      const float2 m = unpack2(mmp), d = unpack2(dmp);
+      pi = make_float2(fabsf(d.x) * rsq_ftz(m.x), fabsf(d.y) * rsq_ftz(m.y));
+      const f2 pp = pack2(pi.x, pi.y);
+      sv = fma2(mul2(pp, neg), pp, s2p);
+    } else {
+      const float2 d = unpack2(dzp);
+      pi = make_float2(fabsf(d.x), fabsf(d.y));
+    }
+    if (LINP(BIN)) {
+      const f2 q = add2(pack2(pi.x, pi.y), dup2(C.p0)), inv = dup2(C.pinv);
+      nq = fma2(fma2(q, inv, mag), neg, mag);
+      p.g = fma2(q, inv, nq);
+      p.k = dup2(C.hp);
+    } else {
+      float dx, dy;
+      const float rx = tab_col(EP, pi.x, dx), ry = tab_col(EP, pi.y, dy);
+      nq = fma2(pack2(rx, ry), neg, mag);
+      p.g = dup2(C.hp);
+      p.k = pack2(dx, dy);
+    }
+  } else {
+    p.g = 0;
+    p.k = dup2(1.f);
+  }
+  /* columns: s or s_perp */
+  f2 col;
+  if (LINS(BIN)) {
+    const f2 s = fma2(s2p, rs, dup2(C.s0)), inv = dup2(C.inv);
+    col = fma2(s, inv, mag);
+    p.f = fma2(s, inv, fma2(col, neg, mag));
+    p.h = dup2(C.hs);
+  } else {
+    const float2 v = unpack2(sv);
+    float dx, dy;
+    const float cx = tab_col(ES, v.x, dx), cy = tab_col(ES, v.y, dy);
+    col = pack2(cx, cy);
+    p.f = fma2(s2p, dup2(C.ea), dup2(C.eb));
+    p.h = pack2(dx, dy);
+  }
+  p.v = IS_ISO(BIN) ? col : fma2(nq, dup2(-C.hc), col);
+  p.col = col;
+  p.s = sv;
+  p.nq = nq;
+  return p;
+}
+
+__device__ __forceinline__ LinConst lin_const(const fcfcg_launch &L) {
+  LinConst C;
+  C.slim = L.s_lim;
+  C.inv = L.tl_inv;
+  C.s0 = L.tl_s0;
+  C.hs = L.tl_h;
+  C.q0 = L.tl_q0;
+  C.nmu = L.fnmu;
+  C.q1 = -L.tl_q1;
+  C.qc = L.tl_qc;
+  C.p0 = L.tl_p0;
+  C.pinv = L.tl_pinv;
+  C.hp = L.tl_hp;
+  C.ea = L.tl_ea;
+  C.eb = L.tl_eb;
+  C.hc = (float) L.hcols;
+  C.ha = C.spare = 0;
+  return C;
+}
+
+/*
+ * The tile's pairs that could not be binned in FP32 (bit i of mask: A point
+ * i of this lane): those with an edge within the rounding bound go to the
+ * FP64 recheck queue -- the warp reserves their places with one atomic --
+ * and those beyond the queue's capacity are binned here by the FP64
+ * formula.  Every ambiguous pair takes a ticket from the 64-bit fill
+ * counter, queued or not, so the counter cannot wrap and hand out slots
+ * twice.  Without a shared histogram every pair in range arrives here, and
+ * the unambiguous ones are counted in global memory.
+ */
+template <int GEOM, int BIN, int WT>
+__device__ __noinline__ void tile_rest(const fcfcg_launch &L, const Tile T,
+    TileWarpW *S, uint32_t mask, const EdgeTab ES, const EdgeTab EP) {
+  const int lane = threadIdx.x & 31;
+  const fcfcg_mock *M = L.mocks ? L.mocks + T.mock : NULL;
+  uint32_t n_in = 0, n_inl = 0;
+  if (!L.hist_smem) {
+    uint32_t left = mask;
+    mask = 0;
+    while (left) {
+      const int i = __ffs(left) - 1;
+      left &= left - 1u;
+      const float *a = (const float *) S->t.p[i >> 2] + (i & 3);
+      const float dx = __fadd_rn(a[0], -T.bx), dy = __fadd_rn(a[4], -T.by),
+                  dz = __fadd_rn(a[8], -T.bz);
+      float s2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+      if (!IS_SPI(BIN) || GEOM == FCFCG_GEOM_SURVEY) s2 = __fmaf_rn(dz, dz, s2);
+      float dm = 0.f, mm = 0.f;
+      if (GEOM == FCFCG_GEOM_SURVEY) {
+        const float mx = __fadd_rn(T.vx, dx), my = __fadd_rn(T.vy, dy),
+                    mz = __fadd_rn(T.vz, dz);
+        dm = __fmaf_rn(dz, mz, __fmaf_rn(dy, my, __fmul_rn(dx, mx)));
+        mm = __fmaf_rn(mz, mz, __fmaf_rn(my, my, __fmul_rn(mx, mx)));
+      }
+      const PairBin p = pair_bin<GEOM, BIN>(lin_const(L), ES, EP, dup2(s2),
+                                            dup2(dz), dup2(dm), dup2(mm));
+      bool plain = (fabsf(unpack2(p.f).x) < unpack2(p.h).x) &
+                   (fabsf(unpack2(p.g).x) < unpack2(p.k).x);
+      if (GEOM == FCFCG_GEOM_SURVEY && !IS_ISO(BIN)) plain &= mm >= L.m2min;
+      if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && !(p.pi.x < L.p_lim))
+        continue;
+      int b = -1;
+      if (plain) {
+        const int s = (int) (__float_as_uint(unpack2(p.col).x) - TMAGIC_BITS) -
+                      L.hcol0,
+                  q = (int) -unpack2(p.nq).x - L.hrow0;
+        if (s >= 0 && s < L.ns && q >= 0 && q < L.hrows) b = s + q * L.ns;
+      }
+      if (!plain) {
+        mask |= 1u << i;
+      } else if (b >= 0) {
+        n_in++;
+        if (WT) {
+          const float4 wa = S->aw[i];
+          add128((M ? M->gwt : L.gwt) + 2 * b,
+                 fix_prod(__float_as_int(wa.x), wa.y, wa.z, T.wi, T.wr, T.wf));
+        } else {
+          atomicAdd((M ? M->gcnt : L.gcnt) + b, 1ull);
+        }
+      }
+    }
+  }
+  const uint32_t c = (uint32_t) __popc(mask);
+  uint32_t inc = c;
+  for (int s = 1; s < 32; s <<= 1) {
+    const uint32_t u = __shfl_up_sync(FULLMASK, inc, s);
+    if (lane >= s) inc += u;
+  }
+  const uint32_t n = __shfl_sync(FULLMASK, inc, 31);
+  unsigned long long slot = 0;
+  if (lane == 0 && n) slot = atomicAdd(L.qcount, (unsigned long long) n);
+  slot = __shfl_sync(FULLMASK, slot, 0) + (inc - c);
+  for (; mask; mask &= mask - 1u, slot++) {
+    const uint32_t a = T.first + (uint32_t) (__ffs(mask) - 1);
+    if (slot < L.qcap) {
+      ((uint4 *) L.queue)[slot] = make_uint4(a, T.bj, T.code, T.mock);
+      continue;
+    }
+    n_inl++;
+    const int bin = ref_bin_pair(L, a, T.bj, T.code, M ? M->box : L.box);
+    if (bin < 0) continue;
+    n_in++;
+    if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, T.bj));
+    else atomicAdd((M ? M->gcnt : L.gcnt) + bin, 1ull);
+  }
+  __syncwarp();
+  n_in = __reduce_add_sync(FULLMASK, n_in);
+  n_inl = __reduce_add_sync(FULLMASK, n_inl);
+  if (lane == 0) {
+    S->t.cnt[1] += n_in;
+    S->t.cnt[2] += n;
+    S->t.cnt[3] += n_inl;
+  }
+  __syncwarp();
+}
+
+/*
+ * The pairs of one tile: this lane's point against every point of A, four
+ * at a time with packed FP32.  A step none of whose pairs is within the
+ * outer range ends after the distance test.  Returns the pairs left for
+ * tile_rest.
+ *
+ * The columns and rows around the bins (hcol0, hrow0 before the first and
+ * one after the last) take the pairs out of range and are dropped when the
+ * histogram is handed over, so no pair is tested against the range's ends.
+ * s^2 near zero needs no test: tl_q1 makes the mu test fail there
+ * (ctx.c:tile_bounds), and without mu a separation's error is bounded for
+ * every s.
+ *
+ * SP: pairs i >= ilim are left out (blocks meeting themselves) and, for
+ * surveys, the line of sight is tested for pairs next to the observer; the
+ * plain variant is for the other tiles.
+ */
+template <int GEOM, int BIN, int WT, bool SP>
+__device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
+    const LinConst &C, const Tile &T, const TileWarpW *S, uint32_t hb,
+    const EdgeTab &ES, const EdgeTab &EP, uint32_t &n_in) {
+  constexpr bool SURVEY = GEOM == FCFCG_GEOM_SURVEY;
+  constexpr bool TWO = !IS_ISO(BIN);     /* a second axis */
+  constexpr bool LOS = SURVEY && !IS_ISO(BIN), CUT = LOSCUT(GEOM, BIN);
+  const f2 nbx = dup2(-T.bx), nby = dup2(-T.by), nbz = dup2(-T.bz);
+  uint32_t rest = 0;
+  const ulonglong2 *P = S->t.p[0];
+#pragma unroll 1
+  for (int k = 0; k < T.m; k += 4, P += 3) {
+    const ulonglong2 X = P[0], Y = P[1], Z = P[2];
+    const f2 dx[2] = {add2(X.x, nbx), add2(X.y, nbx)};
+    const f2 dy[2] = {add2(Y.x, nby), add2(Y.y, nby)};
+    const f2 dz[2] = {add2(Z.x, nbz), add2(Z.y, nbz)};
+    f2 s2[2];
+    bool c[4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      s2[h] = fma2(dy[h], dy[h], mul2(dx[h], dx[h]));
+      if (IS_SPI(BIN) && !SURVEY) {
+        const float2 v = unpack2(s2[h]), z = unpack2(dz[h]);
+        c[2 * h] = (fabsf(z.x) < L.p_lim) & (v.x < L.s_lim);
+        c[2 * h + 1] = (fabsf(z.y) < L.p_lim) & (v.y < L.s_lim);
+      } else {
+        s2[h] = fma2(dz[h], dz[h], s2[h]);
+        const float2 v = unpack2(s2[h]);
+        c[2 * h] = v.x < C.slim;
+        c[2 * h + 1] = v.y < C.slim;
+        if (CUT) {
+          /* not beyond pi_max for sure */
+          const float2 t = unpack2(fma2(dz[h], dup2(T.uz),
+              fma2(dy[h], dup2(T.uy), mul2(dx[h], dup2(T.ux)))));
+          const float2 r = unpack2(fma2(s2[h], dup2(T.lh), dup2(T.lP)));
+          c[2 * h] = c[2 * h] & (fabsf(t.x) < r.x);
+          c[2 * h + 1] = c[2 * h + 1] & (fabsf(t.y) < r.y);
+        }
+      }
+      if (SP) {
+        c[2 * h] = c[2 * h] & (k + 2 * h < T.ilim);
+        c[2 * h + 1] = c[2 * h + 1] & (k + 2 * h + 1 < T.ilim);
+      }
+    }
+    if (!__ballot_sync(FULLMASK, (c[0] | c[1]) | (c[2] | c[3]))) continue;
+    uint32_t r4 = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      f2 dm = 0, mm = 0;
+      if (LOS) {
+        /* line of sight m = x_a + x_b = (2 b + 2 c_A) + d */
+        const f2 mx = add2(dup2(T.vx), dx[h]), my = add2(dup2(T.vy), dy[h]),
+                 mz = add2(dup2(T.vz), dz[h]);
+        dm = fma2(dz[h], mz, fma2(dy[h], my, mul2(dx[h], mx)));
+        mm = fma2(mz, mz, fma2(my, my, mul2(mx, mx)));
+      }
+      const PairBin p = pair_bin<GEOM, BIN>(C, ES, EP, s2[h], dz[h], dm, mm);
+      const float2 v = unpack2(p.v), f = unpack2(p.f), fh = unpack2(p.h),
+                   g = unpack2(p.g), gk = unpack2(p.k), mm2 = unpack2(mm);
+      uint32_t wat[2];        /* weighted pairs: their bins' addresses */
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        bool in = c[2 * h + e];
+        if (SURVEY && IS_SPI(BIN)) in = in & ((e ? p.pi.y : p.pi.x) < L.p_lim);
+        /* the shared bin's byte address */
+        const uint32_t at = __float_as_uint(e ? v.y : v.x) * 4u + C.ha;
+        const float fe = e ? f.y : f.x,
+                    he = LINS(BIN) ? C.hs : (e ? fh.y : fh.x),
+                    ge = IS_SPI(BIN) && !LINP(BIN) ? C.hp : (e ? g.y : g.x),
+                    ke = LINP(BIN) ? C.hp : (e ? gk.y : gk.x);
+        if (!WT && !SP) {
+          if (TWO) {
+            if (h == 0 && e == 0) red_pair<1>(at, C.spare, in, fe, he, ge, ke, r4);
+            if (h == 0 && e == 1) red_pair<2>(at, C.spare, in, fe, he, ge, ke, r4);
+            if (h == 1 && e == 0) red_pair<4>(at, C.spare, in, fe, he, ge, ke, r4);
+            if (h == 1 && e == 1) red_pair<8>(at, C.spare, in, fe, he, ge, ke, r4);
+          } else {
+            if (h == 0 && e == 0) red_pair<1>(at, C.spare, in, fe, he, r4);
+            if (h == 0 && e == 1) red_pair<2>(at, C.spare, in, fe, he, r4);
+            if (h == 1 && e == 0) red_pair<4>(at, C.spare, in, fe, he, r4);
+            if (h == 1 && e == 1) red_pair<8>(at, C.spare, in, fe, he, r4);
+          }
+          continue;
+        }
+        bool plain = fabsf(fe) < he;
+        if (TWO) plain = plain & (fabsf(ge) < ke);
+        if (LOS && SP) plain = plain & ((e ? mm2.y : mm2.x) >= L.m2min);
+        const bool ok = in & plain;
+        if (in & !plain) r4 |= 1u << (2 * h + e);
+        if (!WT) {
+          red_inc(at, C.spare, ok);
+          continue;
+        }
+        /* counted as in range unless in a row or column around the bins
+         * (above them, only a survey's s_perp can be) */
+        const float2 s1 = unpack2(p.s);
+        const float se = e ? s1.y : s1.x;
+        bool inside = ok & (se >= L.tl_slo);
+        if (IS_SPI(BIN)) {
+          inside = inside & ((e ? p.pi.y : p.pi.x) >= L.tl_plo);
+          if (SURVEY) inside = inside & (se < L.tl_shi);
+        }
+        n_in += (uint32_t) inside;
+        wat[e] = ok ? at : C.spare;
+      }
+      if (WT) {
+        const float4 w0 = S->aw[k + 2 * h], w1 = S->aw[k + 2 * h + 1];
+        tile_add_w2(L, T.mock, hb, wat[0], wat[1],
+                    tile_prod(__float_as_int(w0.x), w0.y, w0.z, T.wi, T.wr,
+                              T.wf),
+                    tile_prod(__float_as_int(w1.x), w1.y, w1.z, T.wi, T.wr,
+                              T.wf));
+      }
+    }
+    rest |= r4 << k;
+  }
+  return rest;
+}
+
+/* Add the shared histogram to a global one and clear it, by threads t0,
+ * t0 + nt, ... (whole warps); unweighted counts handed over are counted as
+ * in range.  Exchanges, so that other warps may go on adding meanwhile. */
+template <int WT>
+__device__ __noinline__ void tile_handover(const fcfcg_launch &L,
+    uint32_t *h, uint32_t mock, int t0, int nt, TileWarp *S) {
+  unsigned long long *g = WT ? (L.mocks ? L.mocks[mock].gwt : L.gwt)
+                             : (L.mocks ? L.mocks[mock].gcnt : L.gcnt);
+  unsigned long long sum = 0;
+  for (uint32_t x = (uint32_t) t0; x < (uint32_t) L.hlen; x += (uint32_t) nt) {
+    const int b = tile_gbin(L, x);
+    if (WT) {
+      const long long v = ((long long) ((int *) h)[L.hlen + 32 + x] << 32) +
+                          (long long) h[x];
+      h[x] = 0;
+      h[L.hlen + 32 + x] = 0;
+      if (v && b >= 0) add128(g + 2 * b, v);
+    } else {
+      const uint32_t v = atomicExch(h + x, 0u);
+      if (v && b >= 0) {
+        atomicAdd(g + b, (unsigned long long) v);
+        sum += v;
+      }
+    }
+  }
+  if (!WT) {
+    __syncwarp();
+    for (int o = 16; o > 0; o >>= 1)
+      sum += __shfl_xor_sync(FULLMASK, sum, o);
+    if ((threadIdx.x & 31) == 0) S->cnt[1] += sum;
+    __syncwarp();
+  }
+}
+
+/* The catalogue a CTA of a batched launch is working on (shared memory). */
+struct TileMock {
+  int nc[3];
+  uint32_t base;
+  float cwf[3], cwl[3];  /* cell widths: float + float residual */
+};
+
+/* Items a CTA of a batch takes at once: a share of those left, so that the
+ * runs shrink towards the end and the histogram changes hands rarely. */
+#define TILE_RUN_MIN 16u
+#ifndef TILE_CTAS
+#define TILE_CTAS 4
+#endif
+
+template <int GEOM, int BIN, int WT, int BATCH>
+__global__ void __launch_bounds__(CT32_THREADS, TILE_CTAS)
+k_tile32(const __grid_constant__ fcfcg_launch L) {
+  constexpr bool SURVEY = GEOM == FCFCG_GEOM_SURVEY;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ TileMock sh_mock;
+  __shared__ uint32_t sh_run[3];     /* batch: next item, end, catalogue */
+  /* edge tables: the cells in use, then the entry for all below them */
+  float2 *te = (float2 *) smem;
+  const EdgeTab ES = {te, L.se_lg, L.se_off, (uint32_t) L.nse - 1u},
+                EP = {te + L.nse, L.pe_lg, L.pe_off, (uint32_t) L.npe - 1u};
+  size_t o = ((size_t) (L.nse + L.npe) * 8 + 15) & ~(size_t) 15;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  TileWarpW *S = (TileWarpW *) (smem + o + (size_t) warp * tile_warp_bytes(WT));
+  o += (size_t) (CT32_THREADS / 32) * tile_warp_bytes(WT);
+  uint32_t *h = (uint32_t *) (smem + o);
+  const uint32_t hb = (uint32_t) __cvta_generic_to_shared(h);
+  /* bias of the bins' byte addresses formed from a rounded value's bits */
+  LinConst C = lin_const(L);
+  C.ha = hb - 4u * TMAGIC_BITS;
+  /* the lane's word behind the bins for the pairs that are not binned */
+  C.spare = pin(hb + 4u * (uint32_t) ((L.hist_smem ? L.hlen : 0) + lane));
+  C.ha = pin(C.ha);
+  C.slim = pin(C.slim);
+  if (LINS(BIN)) {
+    /* without a shared histogram every pair goes to tile_rest */
+    C.hs = pin(L.hist_smem ? L.tl_h : -1.f);
+    C.inv = pin(C.inv);
+    C.s0 = pin(C.s0);
+  } else {
+    C.ea = pin(C.ea);
+    C.eb = pin(L.hist_smem ? C.eb : __int_as_float(0x7f800000));
+    for (int i = threadIdx.x; i < L.nse; i += blockDim.x)
+      te[i] = __ldg((const float2 *) L.se + (i < L.nse - 1 ? L.se_skip + i : L.se_last));
+  }
+  if (IS_SMU(BIN)) {
+    C.q0 = pin(C.q0);
+    C.nmu = pin(C.nmu);
+    C.q1 = pin(C.q1);
+    C.qc = pin(C.qc);
+  }
+  if (IS_SPI(BIN) && !LINP(BIN))
+    for (int i = threadIdx.x; i < L.npe; i += blockDim.x)
+      te[L.nse + i] = __ldg((const float2 *) L.pe + (i < L.npe - 1 ? L.pe_skip + i : L.pe_last));
+  if (L.hist_smem)
+    for (int i = threadIdx.x; i < (L.hlen + 32) * (WT ? 2 : 1); i += blockDim.x)
+      h[i] = 0;
+  const uint32_t nitem = __ldg(L.nblk_dev) << L.pshift;
+  const uint32_t np = 1u << L.pshift;
+  /* a warp's share of the pairs a 32-bit bin holds, less what it can add
+   * between two looks at it */
+  const unsigned long long share = L.hs_limit / (CT32_THREADS / 32);
+  const unsigned long long lim = share > 65536u ? share - 65536u : 0u;
+  if (lane < 4) S->t.cnt[lane] = 0;
+  unsigned long long added = 0;
+  uint32_t cur = ~0u;
+  __syncthreads();
+
+  for (;;) {
+    uint32_t item = 0;
+    if (BATCH) {
+      /* the CTA's run of items of one catalogue; when it is used up the
+       * warps meet, and a change of catalogue hands the histogram over */
+      if (lane == 0) item = atomicAdd(&sh_run[0], cur == ~0u ? 0u : 1u);
+      item = __shfl_sync(FULLMASK, item, 0);
+      if (cur == ~0u || item >= sh_run[1]) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          const uint32_t end = sh_run[2];
+          uint32_t s0 = sh_run[1], s1 = s0;
+          if (cur == ~0u || s0 >= end) {
+            uint32_t r = *(volatile uint32_t *) L.chunk_head;
+            for (;;) {
+              if (r >= nitem) break;
+              uint32_t sz = (nitem - r) / (2u * gridDim.x);
+              sz = sz < TILE_RUN_MIN ? TILE_RUN_MIN : sz;
+              sz = sz < nitem - r ? sz : nitem - r;
+              const uint32_t old = atomicCAS(L.chunk_head, r, r + sz);
+              if (old == r) {
+                s0 = r;
+                s1 = r + sz;
+                break;
+              }
+              r = old;
+            }
+            if (r >= nitem) s0 = s1 = ~0u;
+            sh_run[2] = s1;
+          } else {
+            s1 = end;
+          }
+          if (s0 != ~0u) {
+            /* cut at the end of the first item's catalogue */
+            const uint32_t mk = ((const uint2 *) L.A.bcell)[s0 >> L.pshift].y;
+            const uint32_t e =
+                __ldg(L.A.bstart + __ldg(L.mbase + mk + 1)) << L.pshift;
+            if (e < s1) s1 = e;
+          }
+          sh_run[0] = s0;
+          sh_run[1] = s1;
+        }
+        __syncthreads();
+        const uint32_t s0 = sh_run[0];
+        const uint32_t mk = s0 == ~0u ? ~0u
+            : ((const uint2 *) L.A.bcell)[s0 >> L.pshift].y;
+        if (mk != cur && cur != ~0u && L.hist_smem)
+          tile_handover<WT>(L, h, cur, threadIdx.x, CT32_THREADS, &S->t);
+        if (s0 == ~0u) break;
+        if (mk != cur) {
+          if (threadIdx.x < 3) {
+            const fcfcg_mock *M = L.mocks + mk;
+            const int k = threadIdx.x;
+            sh_mock.nc[k] = M->ncell[k];
+            const float f = (float) M->cw[k];
+            sh_mock.cwf[k] = f;
+            sh_mock.cwl[k] = (float) (M->cw[k] - (double) f);
+            if (k == 0) sh_mock.base = M->cell_base;
+          }
+          added = 0;
+        }
+        __syncthreads();
+        cur = mk;
+        continue;
+      }
+    } else {
+      if (lane == 0) item = atomicAdd(L.chunk_head, 1u);
+      item = __shfl_sync(FULLMASK, item, 0);
+      if (item >= nitem) break;
+    }
+    const uint32_t ab = item >> L.pshift, part = item & (np - 1u);
+    const uint2 ci = __ldg((const uint2 *) L.A.bcell + ab);
+    const float4 *Ab = (const float4 *) L.A.blk + 2 * (size_t) ab;
+    Tile T;
+    T.first = __float_as_uint(__ldg(&Ab[0].w));
+    T.m = (int) __float_as_uint(__ldg(&Ab[1].w));
+    T.mock = ci.y;
+    float c2x = 0.f, c2y = 0.f, c2z = 0.f;
+    if (SURVEY) {
+      /* twice A's cell centre: the FP64 centre the local coordinates are
+       * relative to, rounded once */
+      const int cx = (int) (ci.x % (uint32_t) L.ncell[0]);
+      const int cy = (int) ((ci.x / (uint32_t) L.ncell[0]) % (uint32_t) L.ncell[1]);
+      const int cz = (int) (ci.x / ((uint32_t) L.ncell[0] * (uint32_t) L.ncell[1]));
+      c2x = (float) (2.0 * (L.lo[0] + ((double) cx + 0.5) * L.cw[0]));
+      c2y = (float) (2.0 * (L.lo[1] + ((double) cy + 0.5) * L.cw[1]));
+      c2z = (float) (2.0 * (L.lo[2] + ((double) cz + 0.5) * L.cw[2]));
+    }
+    __syncwarp();
+    {
+      /* places past the block's points: a point no test passes (its squared
+       * separation overflows) */
+      float4 v = make_float4(-1e30f, -1e30f, -1e30f, 0.f);
+      if (lane < T.m) v = __ldg((const float4 *) L.A.l4 + T.first + lane);
+      float *p = (float *) S->t.p[lane >> 2] + (lane & 3);
+      p[0] = v.x;
+      p[4] = v.y;
+      p[8] = v.z;
+      if (WT && lane < T.m) {
+        const int2 w = __ldg((const int2 *) L.A.wq + T.first + lane);
+        S->aw[lane] = make_float4(__int_as_float(w.x), __int_as_float(w.y),
+                                  v.w, 0.f);
+      }
+    }
+    __syncwarp();
+    uint32_t seq = 0;
+    for (int t0 = 0; t0 < L.nsten; t0 += 32) {
+      /* 32 stencil entries, one per lane: the neighbour cell's blocks */
+      uint32_t nb = 0, b0 = 0, ecode = 0;
+      float4 D = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t0 + lane < L.nsten) {
+        int nc[3] = {L.ncell[0], L.ncell[1], L.ncell[2]};
+        uint32_t cbase = 0;
+        if (BATCH) {
+          nc[0] = sh_mock.nc[0];
+          nc[1] = sh_mock.nc[1];
+          nc[2] = sh_mock.nc[2];
+          cbase = sh_mock.base;
+        }
+        const uint32_t lc = ci.x - cbase;
+        const int4 so = __ldg((const int4 *) L.sten + t0 + lane);
+        int q[3] = {(int) (lc % (uint32_t) nc[0]) + so.x,
+                    (int) ((lc / (uint32_t) nc[0]) % (uint32_t) nc[1]) + so.y,
+                    (int) (lc / ((uint32_t) nc[0] * (uint32_t) nc[1])) + so.z};
+        bool in = true;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          int w = 1;
+          if (SURVEY) {
+            in &= (q[k] >= 0) & (q[k] < nc[k]);
+          } else {
+            while (q[k] < 0) { q[k] += nc[k]; w--; }
+            while (q[k] >= nc[k]) { q[k] -= nc[k]; w++; }
+            ecode |= (uint32_t) w << (2 * k);
+          }
+        }
+        if (in) {
+          const uint32_t cb = cbase +
+              ((uint32_t) q[2] * nc[1] + q[1]) * nc[0] + q[0];
+          b0 = __ldg(L.B.bstart + cb);
+          nb = __ldg(L.B.bstart + cb + 1) - b0;
+          if (L.isauto && t0 + lane == L.tzero) {
+            /* A's own cell: its block and those after it */
+            nb -= ab - b0;
+            b0 = ab;
+          }
+        }
+        if (BATCH) {
+          /* -offset * cell width, rounded once: the width is held as a
+           * float plus its float residual */
+          D.x = __fmaf_rn((float) -so.x, sh_mock.cwf[0], __fmul_rn((float) -so.x, sh_mock.cwl[0]));
+          D.y = __fmaf_rn((float) -so.y, sh_mock.cwf[1], __fmul_rn((float) -so.y, sh_mock.cwl[1]));
+          D.z = __fmaf_rn((float) -so.z, sh_mock.cwf[2], __fmul_rn((float) -so.z, sh_mock.cwl[2]));
+        } else {
+          D = __ldg((const float4 *) L.stenD + t0 + lane);
+        }
+        D.w = __uint_as_float(ecode);
+      }
+      /* entries that hold blocks and whose cell can hold a pair */
+      bool visit = nb > 0;
+      if (visit) {
+        const float4 ac = __ldg(Ab), ah = __ldg(Ab + 1);
+        const float hx = 0.5001f * (BATCH ? sh_mock.cwf[0] : L.cwf[0]),
+                    hy = 0.5001f * (BATCH ? sh_mock.cwf[1] : L.cwf[1]),
+                    hz = 0.5001f * (BATCH ? sh_mock.cwf[2] : L.cwf[2]);
+        const float gx = fmaxf(fabsf(ac.x + D.x) - (ah.x + hx) - L.box_eps, 0.f),
+                    gy = fmaxf(fabsf(ac.y + D.y) - (ah.y + hy) - L.box_eps, 0.f),
+                    gz = fmaxf(fabsf(ac.z + D.z) - (ah.z + hz) - L.box_eps, 0.f);
+        if (IS_SPI(BIN) && !SURVEY)
+          visit = (gz < L.p_lim) & (fmaf(gy, gy, gx * gx) < L.s_lim);
+        else
+          visit = fmaf(gz, gz, fmaf(gy, gy, gx * gx)) < L.s_lim;
+      }
+      uint32_t cells = __ballot_sync(FULLMASK, visit);
+      __syncwarp();
+      S->t.sd[lane] = D;
+      S->t.si[lane] = make_uint2(b0, nb);
+      __syncwarp();
+      while (cells) {
+       const int e = __ffs(cells) - 1;
+       cells &= cells - 1u;
+       const float4 d = S->t.sd[e];
+       const uint2 eb = S->t.si[e];
+       const bool own = L.isauto && t0 + e == L.tzero;
+       T.code = __float_as_uint(d.w);
+       for (uint32_t g = 0; g < eb.y; g += 32) {
+        /* 32 blocks, one per lane: can a pair with A's block count? */
+        bool near = false;
+        uint32_t bfirst = 0;
+        int bcnt = 0;
+        if (g + lane < eb.y) {
+          const float4 ac = __ldg(Ab), ah = __ldg(Ab + 1);
+          const float4 *Bb = (const float4 *) L.B.blk +
+              2 * (size_t) (eb.x + g + lane);
+          const float4 bc = __ldg(Bb), bh = __ldg(Bb + 1);
+          bfirst = __float_as_uint(bc.w);
+          bcnt = (int) __float_as_uint(bh.w);
+          /* the boxes' distance, less a slack above its rounding and the
+           * pair arithmetic's: no pair of the blocks is closer */
+          const float gx = fmaxf(fabsf(ac.x - (bc.x - d.x)) - (ah.x + bh.x) - L.box_eps, 0.f),
+                      gy = fmaxf(fabsf(ac.y - (bc.y - d.y)) - (ah.y + bh.y) - L.box_eps, 0.f),
+                      gz = fmaxf(fabsf(ac.z - (bc.z - d.z)) - (ah.z + bh.z) - L.box_eps, 0.f);
+          if (IS_SPI(BIN) && !SURVEY)
+            near = (gz < L.p_lim) & (fmaf(gy, gy, gx * gx) < L.s_lim);
+          else
+            near = fmaf(gz, gz, fmaf(gy, gy, gx * gx)) < L.s_lim;
+        }
+        uint32_t todo = __ballot_sync(FULLMASK, near), cand = 0, n_in = 0;
+        while (todo) {
+          const int j = __ffs(todo) - 1;
+          todo &= todo - 1u;
+          if (np > 1 && (seq++ & (np - 1u)) != part) continue;
+          const uint32_t f = __shfl_sync(FULLMASK, bfirst, j);
+          const int n = __shfl_sync(FULLMASK, bcnt, j);
+          const bool self = own && g + (uint32_t) j == 0;
+          /* lanes past the block: a point no test passes */
+          T.bx = T.by = T.bz = 1e30f;
+          T.bj = f + (uint32_t) lane;
+          T.wi = 0;
+          T.wr = T.wf = 0.f;
+          if (lane < n) {
+            const float4 v = __ldg((const float4 *) L.B.l4 + T.bj);
+            T.bx = v.x - d.x;
+            T.by = v.y - d.y;
+            T.bz = v.z - d.z;
+            if (WT) {
+              const int2 w = __ldg((const int2 *) L.B.wq + T.bj);
+              T.wi = w.x;
+              T.wr = __int_as_float(w.y);
+              T.wf = v.w;
+            }
+          }
+          T.ilim = self ? lane : 32;
+          bool sp = self;
+          if (SURVEY) {
+            T.vx = fmaf(2.f, T.bx, c2x);
+            T.vy = fmaf(2.f, T.by, c2y);
+            T.vz = fmaf(2.f, T.bz, c2z);
+            const float r2 = 0.25f * fmaf(T.vz, T.vz, fmaf(T.vy, T.vy, T.vx * T.vx));
+            if (!IS_ISO(BIN))
+              sp |= __any_sync(FULLMASK, r2 < L.near2) != 0;
+            if (LOSCUT(GEOM, BIN)) {
+              T.ux = T.uy = T.uz = T.lh = 0.f;
+              T.lP = FLT_MAX;          /* near the observer: no cut */
+              if (r2 > L.los_r2min && lane < n) {
+                const float ir = rsq_ftz(r2);
+                T.ux = 0.5f * T.vx * ir;
+                T.uy = 0.5f * T.vy * ir;
+                T.uz = 0.5f * T.vz * ir;
+                T.lh = L.los_h * ir;
+                T.lP = fmaf(L.los_pr, ir, L.los_p);
+              }
+            }
+          }
+          cand += (uint32_t) (T.m * n);
+          uint32_t rest;
+          if (sp)
+            rest = tile_pairs<GEOM, BIN, WT, true>(L, C, T, S, hb, ES, EP,
+                                                   n_in);
+          else
+            rest = tile_pairs<GEOM, BIN, WT, false>(L, C, T, S, hb, ES, EP,
+                                                    n_in);
+          if (__any_sync(FULLMASK, rest != 0u))
+            tile_rest<GEOM, BIN, WT>(L, T, S, rest, ES, EP);
+        }
+        if (lane == 0) S->t.cnt[0] += cand;
+        added += cand;
+        if (!WT && added > lim && L.hist_smem) {
+          /* a warp that may have added its share of what a 32-bit bin holds
+           * hands the CTA's bins over */
+          tile_handover<WT>(L, h, T.mock, lane, 32, &S->t);
+          added = 0;
+        }
+        if (WT) {
+          n_in = __reduce_add_sync(FULLMASK, n_in);
+          if (lane == 0) S->t.cnt[1] += n_in;
+        }
+       }
+      }
+    }
+  }
+  if (!BATCH) {
+    __syncthreads();
+    if (L.hist_smem)
+      tile_handover<WT>(L, h, 0, threadIdx.x, CT32_THREADS, &S->t);
+  }
+  __syncwarp();
+  if (lane < 4) atomicAdd(L.stats + lane, S->t.cnt[lane]);
+}
+
+#endif
