@@ -142,7 +142,6 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
   kfun_t f;
   size_t smem;
   int threads;
-  fcfcg_launch Lq = *L;
   cudaError_t e;
   int per_sm = 0;
   if (precision == FCFCG_PREC_FP64) {
@@ -157,86 +156,31 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
              &per_sm, (const void *) f, threads, smem)))
       return (int) e;
   } else {
-    if (!L->adjoint) {
-      int bin = L->bintype;
-      if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
-      if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
-      if (bin == FCFCG_BIN_SPI && L->tplin) bin = BIN_SPILIN;
-      f = L->geometry == FCFCG_GEOM_SURVEY
-              ? fcfcg_pick32_survey(bin, L->withwt)
-              : (L->mocks ? fcfcg_pick32_batch(bin, L->withwt)
-                          : fcfcg_pick32_box(bin, L->withwt));
-      if (!f) return (int) cudaErrorInvalidValue;
-      const size_t sm = fcfcg_k_tile32_tab(L) +
-          fcfcg_k_tile32_stage(L->withwt) +
-          fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
-      if ((e = cudaFuncSetAttribute((const void *) f,
-               cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm)) ||
-          (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-               &per_sm, (const void *) f, CT32_THREADS, sm)))
-        return (int) e;
-      if (per_sm < 1) return (int) cudaErrorInvalidConfiguration;
-      if (smem_used) *smem_used = sm;
-      if (qwarp_used) *qwarp_used = L->qwarp ? L->qwarp : QWARP_MAX;
-      f<<<nsm * per_sm, CT32_THREADS, sm, (cudaStream_t) stream>>>(Lq);
-      return (int) cudaGetLastError();
-    }
-    /* a bit-pattern s table selects the kernel's log variant */
-    int bin = !L->fslog ? L->bintype
-        : (L->bintype == FCFCG_BIN_SPI ? BIN_SPIL
-           : (L->bintype == FCFCG_BIN_ISO ? BIN_ISOL : BIN_SMUL));
-    /* linear s bins: the s bin from s itself */
-    if (L->slin && L->bintype == FCFCG_BIN_ISO) bin = BIN_ISOLIN;
-    if (L->slin && L->bintype == FCFCG_BIN_SMU) bin = BIN_SMULIN;
-    f = fcfcg_pick32_adj(L->geometry, bin);
+    int bin = L->bintype;
+    if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
+    if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
+    if (bin == FCFCG_BIN_SPI && L->tplin) bin = BIN_SPILIN;
+    f = L->adjoint ? fcfcg_pick32_adj(L->geometry, bin)
+        : (L->geometry == FCFCG_GEOM_SURVEY
+               ? fcfcg_pick32_survey(bin, L->withwt)
+               : (L->mocks ? fcfcg_pick32_batch(bin, L->withwt)
+                           : fcfcg_pick32_box(bin, L->withwt)));
     if (!f) return (int) cudaErrorInvalidValue;
-    size_t tab = fcfcg_k_count32_tab_bytes(L->nfs, L->nfp, L->nsb, L->npb);
-    size_t fixed = tab + (L->hist_smem ? (size_t) L->ntot * (L->withwt ? 8 : 4)
-                                        : 0);
-    fixed = (fixed + 15) & ~(size_t) 15;
+    smem = fcfcg_k_tile32_tab(L) +
+        fcfcg_k_tile32_stage(L->adjoint ? 2 : L->withwt) +
+        fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
     threads = CT32_THREADS;
-    /* the warp queue: as given, or the largest of 1024 / 512 / 256 entries
-     * that reaches the most CTAs per SM the kernel can hold (a smaller
-     * queue can free shared memory for another CTA) */
-    const uint32_t cand[3] = {QWARP_MAX, 512u, QWARP_MIN};
-    uint32_t q = 0;
-    int best = 0, occ[3] = {0, 0, 0};
-    for (int k = 0; k < 3; k++) {
-      if (L->qwarp && cand[k] != L->qwarp) continue;
-      const size_t sm = fixed + stage_bytes(L->nsten, L->withwt + L->adjoint,
-                                            cand[k]);
-      if ((e = cudaFuncSetAttribute((const void *) f,
-               cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm)))
-        return (int) e;
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-               &occ[k], (const void *) f, threads, sm)))
-        return (int) e;
-      if (occ[k] > best) best = occ[k];
-    }
-    for (int k = 0; k < 3 && !q; k++)
-      if ((!L->qwarp || cand[k] == L->qwarp) && occ[k] == best && best > 0)
-        q = cand[k];
-    if (!q) return (int) cudaErrorInvalidConfiguration;
-    smem = fixed + stage_bytes(L->nsten, L->withwt + L->adjoint, q);
-    Lq.qwarp = q;
     if ((e = cudaFuncSetAttribute((const void *) f,
-             cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)))
+             cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+             &per_sm, (const void *) f, threads, smem)))
       return (int) e;
-    per_sm = best;
-    if (qwarp_used) *qwarp_used = q;
+    if (qwarp_used) *qwarp_used = L->qwarp ? L->qwarp : QWARP_MAX;
   }
   if (per_sm < 1) return (int) cudaErrorInvalidConfiguration;
   if (smem_used) *smem_used = smem;
-  f<<<nsm * per_sm, threads, smem, (cudaStream_t) stream>>>(Lq);
+  f<<<nsm * per_sm, threads, smem, (cudaStream_t) stream>>>(*L);
   return (int) cudaGetLastError();
-}
-
-/* Shared memory of the FP32 tables and edges (aligned for the histogram). */
-extern "C" size_t fcfcg_k_count32_tab_bytes(int nfs, int nfp, int nsb,
-    int npb) {
-  size_t n = (((size_t) (nfs + nfp) * 2 + 3) & ~(size_t) 3);
-  n += sizeof(float) * ((size_t) nsb + 1 + (npb ? (size_t) npb + 1 : 0));
-  return (n + 15) & ~(size_t) 15;
 }
 
 extern "C" size_t fcfcg_k_tile32_tab(const fcfcg_launch *L) {
@@ -249,12 +193,6 @@ extern "C" size_t fcfcg_k_tile32_stage(int withwt) {
 
 extern "C" size_t fcfcg_k_tile32_hist(int hlen, int withwt) {
   return ((size_t) hlen + 32) * (withwt ? 8 : 4);
-}
-
-/* Shared memory the FP32 kernel needs beyond its histogram, with the
- * smallest warp queue (whether the kernel fits at all). */
-extern "C" size_t fcfcg_k_count32_stage(int nsten, int withwt) {
-  return stage_bytes(nsten, withwt, QWARP_MIN);
 }
 
 extern "C" int fcfcg_k_recheck(void *stream, const fcfcg_launch *L,

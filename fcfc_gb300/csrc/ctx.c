@@ -61,7 +61,8 @@ struct fcfcg_ctx {
   float *d_stenD;
   unsigned long long *d_cnt, *d_wt, *d_stats, *d_bbox;
   double *d_wd;
-  double *d_gfix;                /* adjoint: the scaled cotangent */
+  int *d_gtab;                   /* adjoint: the scaled cotangent */
+  size_t gtab_cap;
   uint32_t *d_head, *d_queue;      /* d_head: chunk counter, pad, fill */
   unsigned long long *d_qcount;    /* queue fill (64-bit), in d_head */
   size_t qcap, qcap_alloc;
@@ -208,7 +209,7 @@ void fcfcg_destroy(fcfcg_ctx *c) {
                  c->d_fpe, c->d_fs,
                  c->d_se, c->d_pe, c->d_fp, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
                  c->d_sten, c->d_stenD, c->d_cnt, c->d_wt, c->d_stats,
-                 c->d_bbox, c->d_wd, c->d_gfix, c->d_head, c->d_queue, c->d_cnvt,
+                 c->d_bbox, c->d_wd, c->d_gtab, c->d_head, c->d_queue, c->d_cnvt,
                  c->d_mock, c->d_mbase, c->d_bout, c->d_bstat, c->d_grad,
                  c->d_wpart, c->d_pcat, c->d_bpart};
     for (size_t i = 0; i < sizeof p / sizeof p[0]; i++)
@@ -301,7 +302,6 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
   CK(cudaMalloc((void **) &c->d_cnt, sizeof(unsigned long long) * b->ntot));
   CK(cudaMalloc((void **) &c->d_wt, sizeof(unsigned long long) * 2 * b->ntot));
   CK(cudaMalloc((void **) &c->d_wd, sizeof(double) * b->ntot));
-  CK(cudaMalloc((void **) &c->d_gfix, sizeof(double) * b->ntot));
   CK(cudaMalloc((void **) &c->d_stats, sizeof(unsigned long long) * 8));
   CK(cudaMalloc((void **) &c->d_wpart,
                 sizeof(double) * (fcfcg_prep_partials() + 1)));
@@ -1648,7 +1648,7 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
    * chunk kernels' finer cells where the FP32 windows do not fit; then the
    * all-FP64 kernel on the latter. */
   int prec = precision;
-  const int tile = (precision == FCFCG_PREC_FP32_RECHECK && !adj);
+  const int tile = (precision == FCFCG_PREC_FP32_RECHECK);
   size_t tabbytes = 0, stage = 0;
   for (int att = tile ? 0 : 2; ; att++) {
     if ((rc = grid_setup(c, g, A, B, att < 2, att == 0))) return rc;
@@ -1659,12 +1659,8 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
     memset(L, 0, sizeof *L);
     if (prec == FCFCG_PREC_FP64) break;
     if (!fp32_bounds(c, g, dmax, A, B, tile, L)) {
-      if (!tile) launch_fp32_tables(c, L);
-      tabbytes = tile ? fcfcg_k_tile32_tab(L)
-                      : fcfcg_k_count32_tab_bytes(L->nfs, L->nfp, L->nsb,
-                                                  L->npb);
-      stage = tile ? fcfcg_k_tile32_stage(withwt)
-                   : fcfcg_k_count32_stage(P->nsten, withwt + (adj ? 1 : 0));
+      tabbytes = fcfcg_k_tile32_tab(L);
+      stage = fcfcg_k_tile32_stage(adj ? 2 : withwt);
       if (tabbytes + stage <= 200 * 1024) break;
     }
     if (att >= 2) {
@@ -1874,6 +1870,7 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
   const int sort_a = !slot_in_grid(A, &P.g);
   const int sort_b = (B != A) && !slot_in_grid(B, &P.g);
   fcfcg_launch *L = &P.L;
+  int gtab_exp = 0;
   if (adj) {
     const size_t ng = A->n + (isauto ? 0 : B->n);
     GROW(c->d_grad, c->d_grad_cap, sizeof(double) * 2 * ng);
@@ -1893,37 +1890,50 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
       if (fabs(adj->g[k]) > gmax) gmax = fabs(adj->g[k]);
     }
     if (P.prec == FCFCG_PREC_FP32_RECHECK) {
-      /* unit of the integer gradient sums: 2^-S with |w| |g| 2^S <= 2^50
-       * for every weight and cotangent entry */
+      /* the cotangent is scaled by 2^-gexp to at most 1, as the weights are:
+       * a term's unit is 2^-51 of the scales' product */
       int gexp = 0;
       if (gmax > 0) {
         gexp = (int) ceil(log2(gmax));
         if (ldexp(1.0, gexp) < gmax) gexp++;
       }
       const int wexp = A->wexp > B->wexp ? A->wexp : B->wexp;
-      int S = 50 - wexp - gexp;
+      const int S = 50 - wexp - gexp;
       if (S < -1000) {
         set_err(c, "weights times cotangent out of range");
         return FCFCG_ERR_ARG;
       }
-      if (S > 1000) S = 1000;   /* products stay below 2^50 */
-      double *gf = malloc(sizeof(double) * b->ntot);
-      if (!gf) return FCFCG_ERR_MEMORY;
-      for (size_t k = 0; k < (size_t) b->ntot; k++)
-        gf[k] = ldexp(adj->g[k], S);
-      cudaError_t ce = cudaMemcpyAsync(c->d_gfix, gf,
-          sizeof(double) * b->ntot, cudaMemcpyHostToDevice, c->stream);
-      if (ce == cudaSuccess) ce = cudaStreamSynchronize(c->stream);
-      free(gf);
-      CK(ce);
-      L->gfix = c->d_gfix;
-      L->gunit = ldexp(1.0, -S);
+      if (S > 1000) gexp += S - 1000;   /* units stay above 2^-1001 */
+      L->gunitA = ldexp(1.0, B->wexp + gexp - 51);
+      L->gunitB = ldexp(1.0, A->wexp + gexp - 51);
+      gtab_exp = gexp;
     }
   }
-  size_t rbytes = sizeof(unsigned long long) * (2 * b->ntot + STAT_WORDS);
-  if ((rc = ensure_pinned(c, rbytes))) return rc;
+  const size_t rbytes = sizeof(unsigned long long) * (2 * b->ntot + STAT_WORDS);
+  const size_t gbytes = (adj && P.tile) ? sizeof(int) * 2 * ((size_t) L->hlen + 32)
+                                        : 0;
+  if ((rc = ensure_pinned(c, rbytes + gbytes))) return rc;
   unsigned long long *hres = (unsigned long long *) c->h_pinned;
   unsigned long long *hstats = hres + 2 * b->ntot;
+  if (gbytes) {
+    /* per shared bin: the entry as an integer and a remainder; 0 around the
+     * bins and in the spare words */
+    int *gt = (int *) ((char *) c->h_pinned + rbytes);
+    memset(gt, 0, gbytes);
+    for (long k = 0; k < b->ntot; k++) {
+      const double gs = ldexp(adj->g[k], -gtab_exp);
+      const int gi = (int) llrint(gs * 1073741824.0);
+      const float gr = (float) (gs - gi * (1.0 / 1073741824.0));
+      const size_t x = (size_t) (k / b->ns + L->hrow0) * (size_t) L->hcols +
+                       (size_t) (k % b->ns + L->hcol0);
+      gt[2 * x] = gi;
+      memcpy(gt + 2 * x + 1, &gr, 4);
+    }
+    GROW(c->d_gtab, c->gtab_cap, gbytes);
+    CK(cudaMemcpyAsync(c->d_gtab, gt, gbytes, cudaMemcpyHostToDevice,
+                       c->stream));
+    L->gtab = c->d_gtab;
+  }
   rc = count_launch(c, &P, sort_a, sort_b, 1, adj ? NULL : hres, hstats);
   if (rc) return rc;
   slot_mark(A, &P.g);

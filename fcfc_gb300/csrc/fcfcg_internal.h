@@ -226,11 +226,11 @@ typedef struct {
   int adjoint;
   const double *gadj;
   double *dA, *dB;
-  /* the FP32 kernel's integer accumulation: gfix[k] = gadj[k] 2^S with S
-   * chosen so that every |w g 2^S| <= 2^50; a product w gfix rounds to an
-   * int64 and integer sums convert back with gunit = 2^-S */
-  const double *gfix;
-  double gunit;
+  /* the FP32 kernel: per shared bin (hlen, and 32 zeros) the cotangent
+   * scaled to at most 1 as round(g 2^30) and the remainder's float bits; a
+   * term's unit in the gradients of A and of B */
+  const int *gtab;
+  double gunitA, gunitB;
 } fcfcg_launch;
 
 /* Launchers implemented in the .cu files; return 0 or a CUDA error code. */

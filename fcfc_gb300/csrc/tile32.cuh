@@ -67,8 +67,17 @@ struct TileWarpW {
   float4 aw[32];
 };
 
+/* adjoint: partial gradients of A's points, one word per lane and step (a
+ * lane's is that of point 4 step + (lane & 3), over a quarter of the lanes) */
+struct TileWarpA {
+  TileWarpW w;
+  long long ga[8][32];
+};
+
+/* wt: 0 unweighted, 1 weighted, 2 adjoint */
 __host__ __device__ __forceinline__ size_t tile_warp_bytes(int wt) {
-  return wt ? sizeof(TileWarpW) : sizeof(TileWarp);
+  return wt == 2 ? sizeof(TileWarpA)
+                 : (wt ? sizeof(TileWarpW) : sizeof(TileWarp));
 }
 
 /* Two FP32 values in a 64-bit register, for the packed instructions: each
@@ -196,6 +205,55 @@ __device__ __forceinline__ long long tile_prod(int ia, float ra, float fa,
   const long long p = (long long) ia * (long long) ib +
       (256ll - ((long long) TMAGIC_BITS << 9));
   return (p + (long long) __float_as_int(t) * 512ll) >> 9;
+}
+
+/*
+ * Adjoint: the product of a weight and a cotangent entry, both scaled to at
+ * most 1, in units of 2^-51 as tile_prod forms that of two weights: the
+ * integer parts (round(x 2^30)) multiply exactly, the cross terms with the
+ * remainders (weight's: ra, scaled by 2^-30; entry's: rb) are rounded to an
+ * integer, the product of the remainders (2^-11 of a unit) is left out.  An
+ * FP64 multiply-add per product kept the FP64 pipe the bound (32 cycles of
+ * an SM per pair of a warp; GB300 has 2 FP64 lanes per SM).
+ */
+__device__ __forceinline__ long long adj_prod(int ia, float ra, float fa,
+    int ib, float rb, float ib_f) {
+  const float c = __fmaf_rn(fa, rb, __fmul_rn(ra, ib_f));
+  const float t = __fmaf_rn(c, 2251799813685248.0f /* 2^51 */, TMAGIC);
+  const long long p = (long long) ia * (long long) ib +
+      (256ll - ((long long) TMAGIC_BITS << 9));
+  return (p + (long long) __float_as_int(t) * 512ll) >> 9;
+}
+
+__device__ __forceinline__ long long shfl_xor64(long long v, int o) {
+  const uint32_t lo = __shfl_xor_sync(FULLMASK, (uint32_t) v, o),
+                 hi = __shfl_xor_sync(FULLMASK, (uint32_t) (v >> 32), o);
+  return (long long) (((unsigned long long) hi << 32) | lo);
+}
+
+/* Four values per lane to one: lane l gets the sum of value l & 3 over the
+ * lanes that differ from it in the low two bits. */
+__device__ __forceinline__ long long reduce4(const long long v[4], int lane) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+  long long r[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+    r[i] = (b0 ? v[2 * i + 1] : v[2 * i]) +
+           shfl_xor64(b0 ? v[2 * i] : v[2 * i + 1], 1);
+  return (b1 ? r[1] : r[0]) + shfl_xor64(b1 ? r[0] : r[1], 2);
+}
+
+/* Add A's gradients to the global ones and clear them. */
+__device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
+    uint32_t first, int m) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  long long v = 0;
+  for (int i = 0; i < 8; i++) v += S->ga[lane >> 2][(lane & 3) + 4 * i];
+  if (lane < m && v) atomicAdd(L.dA + first + lane, (double) v * L.gunitA);
+  __syncwarp();
+  for (int i = 0; i < 8; i++) S->ga[i][lane] = 0;
+  __syncwarp();
 }
 
 /* Weighted sums in shared memory: two 32-bit words per bin (the high words
@@ -395,13 +453,13 @@ __device__ __forceinline__ LinConst lin_const(const fcfcg_launch &L) {
  * twice.  Without a shared histogram every pair in range arrives here, and
  * the unambiguous ones are counted in global memory.
  */
-template <int GEOM, int BIN, int WT>
+template <int GEOM, int BIN, int WT, int ADJ>
 __device__ __noinline__ void tile_rest(const fcfcg_launch &L, const Tile T,
     TileWarpW *S, uint32_t mask, const EdgeTab ES, const EdgeTab EP) {
   const int lane = threadIdx.x & 31;
   const fcfcg_mock *M = L.mocks ? L.mocks + T.mock : NULL;
   uint32_t n_in = 0, n_inl = 0;
-  if (!L.hist_smem) {
+  if (!ADJ && !L.hist_smem) {
     uint32_t left = mask;
     mask = 0;
     while (left) {
@@ -467,7 +525,8 @@ __device__ __noinline__ void tile_rest(const fcfcg_launch &L, const Tile T,
     const int bin = ref_bin_pair(L, a, T.bj, T.code, M ? M->box : L.box);
     if (bin < 0) continue;
     n_in++;
-    if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, T.bj));
+    if (ADJ) adj_pair(L, a, T.bj, bin);
+    else if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, T.bj));
     else atomicAdd((M ? M->gcnt : L.gcnt) + bin, 1ull);
   }
   __syncwarp();
@@ -498,10 +557,10 @@ __device__ __noinline__ void tile_rest(const fcfcg_launch &L, const Tile T,
  * surveys, the line of sight is tested for pairs next to the observer; the
  * plain variant is for the other tiles.
  */
-template <int GEOM, int BIN, int WT, bool SP>
+template <int GEOM, int BIN, int WT, int ADJ, bool SP>
 __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
-    const LinConst &C, const Tile &T, const TileWarpW *S, uint32_t hb,
-    const EdgeTab &ES, const EdgeTab &EP, uint32_t &n_in) {
+    const LinConst &C, const Tile &T, TileWarpW *S, uint32_t hb,
+    const EdgeTab &ES, const EdgeTab &EP, uint32_t &n_in, long long &gb) {
   constexpr bool SURVEY = GEOM == FCFCG_GEOM_SURVEY;
   constexpr bool TWO = !IS_ISO(BIN);     /* a second axis */
   constexpr bool LOS = SURVEY && !IS_ISO(BIN), CUT = LOSCUT(GEOM, BIN);
@@ -544,6 +603,7 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
     }
     if (!__ballot_sync(FULLMASK, (c[0] | c[1]) | (c[2] | c[3]))) continue;
     uint32_t r4 = 0;
+    long long ga[4];          /* adjoint: terms of A's four points */
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       f2 dm = 0, mm = 0;
@@ -603,7 +663,23 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
         n_in += (uint32_t) inside;
         wat[e] = ok ? at : C.spare;
       }
-      if (WT) {
+      if (ADJ) {
+        /* d/dw_a of w_a w_b g[bin] is w_b g[bin], and the other way round;
+         * spare and outer bins hold g = 0 */
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          int2 g;
+          if (L.hist_smem)
+            asm("ld.shared.v2.s32 {%0, %1}, [%2];"
+                : "=r"(g.x), "=r"(g.y) : "r"(2u * wat[e] - hb));
+          else
+            g = __ldg((const int2 *) L.gtab + ((wat[e] - hb) >> 2));
+          const float4 wa = S->aw[k + 2 * h + e];
+          const float gf = (float) g.x, gr = __int_as_float(g.y);
+          ga[2 * h + e] = adj_prod(T.wi, T.wr, T.wf, g.x, gr, gf);
+          gb += adj_prod(__float_as_int(wa.x), wa.y, wa.z, g.x, gr, gf);
+        }
+      } else if (WT) {
         const float4 w0 = S->aw[k + 2 * h], w1 = S->aw[k + 2 * h + 1];
         tile_add_w2(L, T.mock, hb, wat[0], wat[1],
                     tile_prod(__float_as_int(w0.x), w0.y, w0.z, T.wi, T.wr,
@@ -611,6 +687,11 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
                     tile_prod(__float_as_int(w1.x), w1.y, w1.z, T.wi, T.wr,
                               T.wf));
       }
+    }
+    if (ADJ) {
+      long long *acc = ((TileWarpA *) S)->ga[k >> 2];
+      const int lane = threadIdx.x & 31;
+      acc[lane] += reduce4(ga, lane);
     }
     rest |= r4 << k;
   }
@@ -665,8 +746,8 @@ struct TileMock {
 #define TILE_CTAS 4
 #endif
 
-template <int GEOM, int BIN, int WT, int BATCH>
-__global__ void __launch_bounds__(CT32_THREADS, TILE_CTAS)
+template <int GEOM, int BIN, int WT, int BATCH, int ADJ = 0>
+__global__ void __launch_bounds__(CT32_THREADS, ADJ ? 3 : TILE_CTAS)
 k_tile32(const __grid_constant__ fcfcg_launch L) {
   constexpr bool SURVEY = GEOM == FCFCG_GEOM_SURVEY;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -678,25 +759,25 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
                 EP = {te + L.nse, L.pe_lg, L.pe_off, (uint32_t) L.npe - 1u};
   size_t o = ((size_t) (L.nse + L.npe) * 8 + 15) & ~(size_t) 15;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  TileWarpW *S = (TileWarpW *) (smem + o + (size_t) warp * tile_warp_bytes(WT));
-  o += (size_t) (CT32_THREADS / 32) * tile_warp_bytes(WT);
+  TileWarpW *S = (TileWarpW *) (smem + o + (size_t) warp * tile_warp_bytes(WT + ADJ));
+  o += (size_t) (CT32_THREADS / 32) * tile_warp_bytes(WT + ADJ);
   uint32_t *h = (uint32_t *) (smem + o);
   const uint32_t hb = (uint32_t) __cvta_generic_to_shared(h);
   /* bias of the bins' byte addresses formed from a rounded value's bits */
   LinConst C = lin_const(L);
   C.ha = hb - 4u * TMAGIC_BITS;
   /* the lane's word behind the bins for the pairs that are not binned */
-  C.spare = pin(hb + 4u * (uint32_t) ((L.hist_smem ? L.hlen : 0) + lane));
+  C.spare = pin(hb + 4u * (uint32_t) ((ADJ || L.hist_smem ? L.hlen : 0) + lane));
   C.ha = pin(C.ha);
   C.slim = pin(C.slim);
   if (LINS(BIN)) {
     /* without a shared histogram every pair goes to tile_rest */
-    C.hs = pin(L.hist_smem ? L.tl_h : -1.f);
+    C.hs = pin(ADJ || L.hist_smem ? L.tl_h : -1.f);
     C.inv = pin(C.inv);
     C.s0 = pin(C.s0);
   } else {
     C.ea = pin(C.ea);
-    C.eb = pin(L.hist_smem ? C.eb : __int_as_float(0x7f800000));
+    C.eb = pin(ADJ || L.hist_smem ? C.eb : __int_as_float(0x7f800000));
     for (int i = threadIdx.x; i < L.nse; i += blockDim.x)
       te[i] = __ldg((const float2 *) L.se + (i < L.nse - 1 ? L.se_skip + i : L.se_last));
   }
@@ -709,9 +790,16 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
   if (IS_SPI(BIN) && !LINP(BIN))
     for (int i = threadIdx.x; i < L.npe; i += blockDim.x)
       te[L.nse + i] = __ldg((const float2 *) L.pe + (i < L.npe - 1 ? L.pe_skip + i : L.pe_last));
-  if (L.hist_smem)
+  if (ADJ) {
+    /* the scaled cotangent of the shared bins takes the histogram's place */
+    if (L.hist_smem)
+      for (int i = threadIdx.x; i < L.hlen + 32; i += blockDim.x)
+        ((int2 *) h)[i] = __ldg((const int2 *) L.gtab + i);
+    for (int i = 0; i < 8; i++) ((TileWarpA *) S)->ga[i][lane] = 0;
+  } else if (L.hist_smem) {
     for (int i = threadIdx.x; i < (L.hlen + 32) * (WT ? 2 : 1); i += blockDim.x)
       h[i] = 0;
+  }
   const uint32_t nitem = __ldg(L.nblk_dev) << L.pshift;
   const uint32_t np = 1u << L.pshift;
   /* a warp's share of the pairs a 32-bit bin holds, less what it can add
@@ -821,14 +909,16 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
       p[0] = v.x;
       p[4] = v.y;
       p[8] = v.z;
-      if (WT && lane < T.m) {
-        const int2 w = __ldg((const int2 *) L.A.wq + T.first + lane);
-        S->aw[lane] = make_float4(__int_as_float(w.x), __int_as_float(w.y),
-                                  v.w, 0.f);
+      if (WT) {
+        int2 w = make_int2(0, 0);
+        if (lane < T.m) w = __ldg((const int2 *) L.A.wq + T.first + lane);
+        S->aw[lane] = make_float4(__int_as_float(w.x), __int_as_float(w.y) *
+                                  (ADJ ? 0x1p-30f : 1.f), v.w, 0.f);
       }
     }
     __syncwarp();
     uint32_t seq = 0;
+    int ntile = 0;
     for (int t0 = 0; t0 < L.nsten; t0 += 32) {
       /* 32 stencil entries, one per lane: the neighbour cell's blocks */
       uint32_t nb = 0, b0 = 0, ecode = 0;
@@ -951,7 +1041,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             if (WT) {
               const int2 w = __ldg((const int2 *) L.B.wq + T.bj);
               T.wi = w.x;
-              T.wr = __int_as_float(w.y);
+              T.wr = __int_as_float(w.y) * (ADJ ? 0x1p-30f : 1.f);
               T.wf = v.w;
             }
           }
@@ -979,18 +1069,29 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           }
           cand += (uint32_t) (T.m * n);
           uint32_t rest;
+          long long gb = 0;       /* adjoint: this lane's point's terms */
           if (sp)
-            rest = tile_pairs<GEOM, BIN, WT, true>(L, C, T, S, hb, ES, EP,
-                                                   n_in);
+            rest = tile_pairs<GEOM, BIN, WT, ADJ, true>(L, C, T, S, hb, ES,
+                                                        EP, n_in, gb);
           else
-            rest = tile_pairs<GEOM, BIN, WT, false>(L, C, T, S, hb, ES, EP,
-                                                    n_in);
+            rest = tile_pairs<GEOM, BIN, WT, ADJ, false>(L, C, T, S, hb, ES,
+                                                         EP, n_in, gb);
+          if (ADJ && gb) atomicAdd(L.dB + T.bj, (double) gb * L.gunitB);
           if (__any_sync(FULLMASK, rest != 0u))
-            tile_rest<GEOM, BIN, WT>(L, T, S, rest, ES, EP);
+            tile_rest<GEOM, BIN, WT, ADJ>(L, T, S, rest, ES, EP);
+        }
+        if (ADJ) {
+          /* a term is below 2^51, a step adds 4 of them to a word and a
+           * group of blocks 32 steps' worth: out before 2^60 */
+          ntile += 32;
+          if (ntile >= 128) {
+            adj_flush(L, (TileWarpA *) S, T.first, T.m);
+            ntile = 0;
+          }
         }
         if (lane == 0) S->t.cnt[0] += cand;
         added += cand;
-        if (!WT && added > lim && L.hist_smem) {
+        if (!WT && !ADJ && added > lim && L.hist_smem) {
           /* a warp that may have added its share of what a 32-bit bin holds
            * hands the CTA's bins over */
           tile_handover<WT>(L, h, T.mock, lane, 32, &S->t);
@@ -1003,8 +1104,9 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
        }
       }
     }
+    if (ADJ) adj_flush(L, (TileWarpA *) S, T.first, T.m);
   }
-  if (!BATCH) {
+  if (!BATCH && !ADJ) {
     __syncthreads();
     if (L.hist_smem)
       tile_handover<WT>(L, h, 0, threadIdx.x, CT32_THREADS, &S->t);
