@@ -53,6 +53,9 @@ struct fcfcg_ctx {
   size_t cfill_cap, scan_cap, cchunk_cap, chunk_cap;
   uint32_t *fstart;               /* fine (sub-cell) starts of a grid sort */
   size_t fstart_cap;
+  uint32_t *rank;                 /* sort scratch: rank in the sub-cell, */
+  float *key;                     /* coordinates and index by sub-cell */
+  size_t rank_cap, key_cap;
   uint16_t *d_fs, *d_fp, *d_rs, *d_rp;
   float *d_fse, *d_fpe;
   double *d_s2edge, *d_pedge;
@@ -205,7 +208,7 @@ void fcfcg_destroy(fcfcg_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (int i = 0; i <= FCFCG_MAX_SLOT; i++) slot_free(c->slot + i);
-    void *p[] = {c->cfill, c->fstart, c->scan_tmp, c->cchunk, c->chunks, c->d_fse,
+    void *p[] = {c->cfill, c->fstart, c->rank, c->key, c->scan_tmp, c->cchunk, c->chunks, c->d_fse,
                  c->d_fpe, c->d_fs,
                  c->d_se, c->d_pe, c->d_fp, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
                  c->d_sten, c->d_stenD, c->d_cnt, c->d_wt, c->d_stats,
@@ -958,29 +961,34 @@ static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   const size_t nf = nc << fcfcg_grid_curve_bits(nc, n);
   GROW(c->cfill, c->cfill_cap, sizeof(uint32_t) * (nf + 1));
   GROW(c->fstart, c->fstart_cap, sizeof(uint32_t) * (nf + 1));
+  GROW(c->rank, c->rank_cap, sizeof(uint32_t) * m);
+  GROW(c->key, c->key_cap, sizeof(float) * 4 * m);
   size_t st = fcfcg_scan_tmp_len(nf + 1) + 16;
   GROW(c->scan_tmp, c->scan_cap, sizeof(uint32_t) * st);
   GROW(c->cchunk, c->cchunk_cap, sizeof(uint32_t) * 2 * (nc + 1));
   return FCFCG_OK;
 }
 
+/* The buffers of a sort of slot s. */
+static fcfcg_sort slot_buffers(const fcfcg_ctx *c, const slot_t *s) {
+  const int survey = (c->bins.geometry == FCFCG_GEOM_SURVEY);
+  fcfcg_sort b = {s->cell_of, c->rank, c->cfill, c->fstart, c->scan_tmp,
+                  c->key, s->cstart, s->bstart, s->l4, s->wq, s->sx, s->sy,
+                  s->sz, survey ? s->ss : NULL, s->sw, s->sid, s->blk,
+                  s->bcell};
+  return b;
+}
+
 /* Queue the sort of slot s into grid g (stream work only). */
 static int slot_sort(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   const size_t nc = (size_t) g->n[0] * g->n[1] * g->n[2];
   const size_t n = s->n;
-  const int sb = fcfcg_grid_curve_bits(nc, n);
-  size_t st = fcfcg_scan_tmp_len((nc << sb) + 1) + 16;
   const int survey = (c->bins.geometry == FCFCG_GEOM_SURVEY);
+  const fcfcg_sort b = slot_buffers(c, s);
   CKK(fcfcg_k_grid(c->stream, n, s->x, s->y, s->z, survey ? s->s : NULL,
-                   s->w, s->has_w, s->wexp, g->n, g->cw, g->lo, sb,
-                   s->cell_of, s->cstart, c->fstart, c->cfill, c->scan_tmp,
-                   st, s->l4, s->wq, s->sx, s->sy, s->sz,
-                   survey ? s->ss : NULL, s->sw, s->sid));
-  c->launches += n ? 6 : 4;
-  CKK(fcfcg_k_blocks(c->stream, s->cstart, (uint32_t) nc, n, c->cchunk,
-                     c->scan_tmp, s->l4, s->bstart, s->blk, s->bcell, NULL,
-                     0));
-  c->launches += 5;
+                   s->w, s->has_w, s->wexp, g->n, g->cw, g->lo,
+                   fcfcg_grid_curve_bits(nc, n), &b));
+  c->launches += n ? 7 : 5;
   return FCFCG_OK;
 }
 
@@ -1536,27 +1544,6 @@ static void launch_bins(const fcfcg_ctx *c, fcfcg_launch *L) {
   L->qcount = c->d_qcount;
   L->qcap = (uint32_t) c->qcap;
   L->stats = c->d_stats;
-}
-
-/* Launch fields of the FP32 edge-window tables. */
-static void launch_fp32_tables(const fcfcg_ctx *c, fcfcg_launch *L) {
-  const fcfcg_bins *b = &c->bins;
-  L->fs = c->d_fs;
-  L->nfs = (int) b->s.nftab;
-  L->fsoff = (int) b->s.foff;
-  L->fslog = b->s.flog;
-  L->fsinv = (float) ldexp(1.0, b->s.flog ? -b->s.flog : -b->s.fshift);
-  L->fse = c->d_fse;
-  L->nsb = b->s.nbin;
-  if (b->bintype == FCFCG_BIN_SPI) {
-    L->fp = c->d_fp;
-    L->nfp = (int) b->p.nftab;
-    L->fpoff = (int) b->p.foff;
-    L->fplog = b->p.flog;
-    L->fpinv = (float) ldexp(1.0, b->p.flog ? -b->p.flog : -b->p.fshift);
-    L->fpe = c->d_fpe;
-    L->npb = b->p.nbin;
-  }
 }
 
 static int ensure_pinned(fcfcg_ctx *c, size_t bytes) {
@@ -2769,22 +2756,19 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   BGROW(c->fstart, c->fstart_cap, sizeof(uint32_t) * (nf + 1));
   const size_t stl = fcfcg_scan_tmp_len(nf + 1) + 16;
   BGROW(c->scan_tmp, c->scan_cap, sizeof(uint32_t) * stl);
-  BCK(cudaMemsetAsync(c->cfill, 0, sizeof(uint32_t) * (nf + 1), c->stream));
+  BGROW(c->rank, c->rank_cap, sizeof(uint32_t) * m);
+  BGROW(c->key, c->key_cap, sizeof(float) * 4 * m);
   /* the table again, with the grids (the stream is idle: the range checks
    * synchronised it) */
   BCK(cudaMemcpyAsync(c->d_pcat, P, sizeof(fcfcg_prep_cat) * na,
                       cudaMemcpyHostToDevice, c->stream));
-  BCKK(fcfcg_k_cell_batch(c->stream, (const fcfcg_prep_cat *) c->d_pcat, na,
-                          ntile, sb, S->x, S->y, S->z, S->cell_of, c->cfill));
-  BCKK(fcfcg_scan(c->stream, c->cfill, nf, c->fstart, c->scan_tmp));
-  BCKK(fcfcg_k_cstart(c->stream, cells, sb, c->fstart, S->cstart));
-  BCK(cudaMemsetAsync(c->cfill, 0, sizeof(uint32_t) * (nf + 1), c->stream));
-  BCKK(fcfcg_k_scatter_batch(c->stream, (const fcfcg_prep_cat *) c->d_pcat,
-                             na, ntile, sb, S->x, S->y, S->z,
-                             withwt ? S->w : NULL, withwt, S->cell_of,
-                             c->fstart, c->cfill, S->l4, S->wq, S->sx, S->sy,
-                             S->sz, S->sw, S->sid));
-  c->launches += 6;
+  BCK(cudaMemcpyAsync(c->d_mbase, hbase, sizeof(uint32_t) * (na + 1),
+                      cudaMemcpyHostToDevice, c->stream));
+  const fcfcg_sort sbuf = slot_buffers(c, S);
+  BCKK(fcfcg_k_grid_batch(c->stream, (const fcfcg_prep_cat *) c->d_pcat, na,
+                          ntile, cells, N, c->d_mbase, sb, S->x, S->y, S->z,
+                          withwt ? S->w : NULL, withwt, &sbuf));
+  c->launches += 7;
   /* 6. per-catalogue histograms and the catalogue table */
   const size_t per = (size_t) b->ntot * (withwt ? 2 : 1);
   BGROW(c->d_bout, c->d_bout_cap, sizeof(unsigned long long) * per * na);
@@ -2796,8 +2780,6 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   }
   BGROW(c->d_mock, c->d_mock_cap, sizeof(fcfcg_mock) * na);
   BCK(cudaMemcpyAsync(c->d_mock, c->h_mock, sizeof(fcfcg_mock) * na,
-                      cudaMemcpyHostToDevice, c->stream));
-  BCK(cudaMemcpyAsync(c->d_mbase, hbase, sizeof(uint32_t) * (na + 1),
                       cudaMemcpyHostToDevice, c->stream));
   /* the copies read host memory that is freed below */
   BCK(cudaStreamSynchronize(c->stream));
@@ -2841,12 +2823,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   }
   L.sten = c->d_sten;
   L.stenD = c->d_stenD;
-  /* 8. blocks of every catalogue, in catalogue order */
-  BGROW(c->cchunk, c->cchunk_cap, sizeof(uint32_t) * 2 * (cells + 1));
-  BCKK(fcfcg_k_blocks(c->stream, S->cstart, (uint32_t) cells, N, c->cchunk,
-                      c->scan_tmp, S->l4, S->bstart, S->blk, S->bcell,
-                      c->d_mbase, na));
-  c->launches += 5;
+  /* 8. count */
   BCK(cudaEventRecord(c->ev[1], c->stream));
   L.chunk_head = c->d_head;
   BCK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * 4,

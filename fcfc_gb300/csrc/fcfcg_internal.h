@@ -95,8 +95,8 @@ typedef struct {
   const uint32_t *id;    /* input index */
   const uint32_t *cstart;/* ncell + 1 */
   /* blocks of at most 32 points of a cell: two float4 each, (box centre,
-   * bits of the first sorted index) and (half extents, bits of the count);
-   * bstart: the cells' first blocks (ncell + 1); bcell: (cell, catalogue of
+   * bits of the first sorted index) and (half extents, bits of the count; 0
+   * for a place left unused); bstart: the cells' first blocks (ncell + 1); bcell: (cell, catalogue of
    * a batch) per block */
   const float *blk;
   const uint32_t *bstart, *bcell;
@@ -247,30 +247,34 @@ size_t fcfcg_prep_partials(void);
  * 15 where cells hold many points. */
 int fcfcg_grid_sub_bits(size_t ncell, size_t npoint);
 int fcfcg_grid_curve_bits(size_t ncell, size_t npoint);
-/* Counting sort into the grid, cells in order and, within a cell, by
- * sub-cell (sb bits); cstart[0..nc] the cells' first sorted points.
- * Scratch: cell_of (n), fstart and cfill ((nc << sb) + 1 each), scan_tmp
- * (fcfcg_scan_tmp_len((nc << sb) + 1)). */
+/* Buffers of a sort into a grid of nc cells (sb sub-cell bits) of n points:
+ * scratch cell_of, rank (n), key (float4, n), cfill and fstart ((nc << sb) +
+ * 1), scan_tmp (fcfcg_scan_tmp_len of that); results cstart and bstart (nc +
+ * 1), the sorted arrays (n) and blk, bcell (fcfcg_max_blocks). */
+typedef struct {
+  uint32_t *cell_of, *rank, *cfill, *fstart, *scan_tmp;
+  float *key;
+  uint32_t *cstart, *bstart;
+  float *l4;
+  int *wq;
+  double *sx, *sy, *sz, *ss, *sw;
+  uint32_t *sid;
+  float *blk;
+  uint32_t *bcell;
+} fcfcg_sort;
+
+/* Sort into the grid: cells in order, within a cell runs along a Hilbert
+ * curve of its sub-cells, within a run blocks of 32 (prep.cu:k_runs).
+ * cstart[0..nc]: the cells' first sorted points; bstart: their first blocks;
+ * blk, bcell: see fcfcg_dcat. */
+size_t fcfcg_max_blocks(size_t n, size_t ncell);
 int fcfcg_k_grid(void *stream, size_t n, const double *x, const double *y,
     const double *z, const double *s, const double *w, int has_w, int wexp,
     const int ncell[3], const double cw[3], const double lo[3], int sb,
-    uint32_t *cell_of, uint32_t *cstart, uint32_t *fstart, uint32_t *cfill,
-    uint32_t *scan_tmp, size_t scan_tmp_len, float *l4, int *wq, double *sx,
-    double *sy, double *sz, double *ss, double *sw, uint32_t *sid);
-/* cstart[c] = fstart[c << sb] for c = 0..nc. */
-int fcfcg_k_cstart(void *stream, size_t nc, int sb, const uint32_t *fstart,
-    uint32_t *cstart);
+    const fcfcg_sort *S);
 int fcfcg_k_chunks(void *stream, const uint32_t *cstart, uint32_t ncell,
     uint32_t clen, uint32_t *cchunk, uint32_t *scan_tmp, size_t scan_tmp_len,
     uint32_t *chunks, uint32_t *nchunk_out, const uint32_t *mock_cell_base,
-    int nmock);
-/* Blocks of at most 32 points of the cells of a sorted catalogue (see
- * fcfcg_dcat): bstart (ncell + 1 entries), blk and bcell (at most n / 32 +
- * min(n, ncell) blocks); count: ncell scratch words; mbase as above. */
-size_t fcfcg_max_blocks(size_t n, size_t ncell);
-int fcfcg_k_blocks(void *stream, const uint32_t *cstart, uint32_t ncell,
-    size_t n, uint32_t *count, uint32_t *scan_tmp, const float *l4,
-    uint32_t *bstart, float *blk, uint32_t *bcell, const uint32_t *mbase,
     int nmock);
 /* One catalogue of a batch for the preparation kernels: its inputs (device
  * or GPU-readable host memory), its place o in the batch slot, its first
@@ -295,19 +299,13 @@ size_t fcfcg_batch_tile(void);
 int fcfcg_k_prep_batch(void *stream, const fcfcg_prep_cat *d_cat, int ncat,
     uint32_t ntile, double rescale, int withwt, double *ox, double *oy,
     double *oz, double *ow, unsigned long long *bstat, double *partial);
-/* Batch grid: every live catalogue's fine indices (cell numbered from its
- * cell_base, shifted by sb, with the sub-cell) counted into a shared array
- * (k_cell_batch), and its points scattered into the shared sorted arrays
- * after the global scan of the fine counts (k_scatter_batch); the id of
- * slot point i is i. */
-int fcfcg_k_cell_batch(void *stream, const fcfcg_prep_cat *d_cat, int ncat,
-    uint32_t ntile, int sb, const double *x, const double *y,
-    const double *z, uint32_t *cell_of, uint32_t *count);
-int fcfcg_k_scatter_batch(void *stream, const fcfcg_prep_cat *d_cat,
-    int ncat, uint32_t ntile, int sb, const double *x, const double *y,
-    const double *z, const double *w, int has_w, const uint32_t *cell_of,
-    const uint32_t *fstart, uint32_t *cfill, float *l4, int *wq, double *sx,
-    double *sy, double *sz, double *sw, uint32_t *sid);
+/* The same for a batch: every live catalogue's cells numbered from its
+ * cell_base (mbase: the catalogues' first cells, ncat + 1), one sorted array;
+ * the id of slot point i is i. */
+int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat, int ncat,
+    uint32_t ntile, size_t ncell, size_t n, const uint32_t *mbase, int sb,
+    const double *x, const double *y, const double *z, const double *w,
+    int has_w, const fcfcg_sort *S);
 /* out[sid[p]] = in[p] for p < n (sorted order back to input order). */
 int fcfcg_k_unsort(void *stream, size_t n, const uint32_t *sid,
     const double *in, double *out);

@@ -8,6 +8,7 @@
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "fcfcg_internal.h"
 
@@ -334,77 +335,327 @@ __device__ __forceinline__ uint32_t fine_of_point(const FineGrid &g,
 __global__ void k_cell(size_t n, const double *__restrict__ x,
     const double *__restrict__ y, const double *__restrict__ z,
     const FineGrid g, uint32_t *__restrict__ cell_of,
-    uint32_t *__restrict__ count) {
+    uint32_t *__restrict__ rank, uint32_t *__restrict__ count) {
   for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n;
        i += (size_t) gridDim.x * blockDim.x) {
     const uint32_t c = fine_of_point(g, x[i], y[i], z[i]);
     cell_of[i] = c;
-    atomicAdd(count + c, 1u);
+    rank[i] = atomicAdd(count + c, 1u);
   }
 }
 
-/* Point i (input order) of a grid to its sorted place pos: the FP32
- * offsets from its cell centre and its weight's scaled high part (l4), the
- * weight's fixed-point split (wq), FP64 copies and its id. */
-__device__ __forceinline__ void scatter_point(uint32_t c, uint32_t pos,
-    double a, double b, double d, double wv, int wexp, int nx, int ny,
-    double cwx, double cwy, double cwz, double lox, double loy, double loz,
-    uint32_t cell_base, uint32_t id, float4 *__restrict__ l4,
-    int2 *__restrict__ wq, double *__restrict__ sx, double *__restrict__ sy,
-    double *__restrict__ sz, double *__restrict__ sw,
-    uint32_t *__restrict__ sid) {
-  const uint32_t cl = c - cell_base;
-  int cx = (int) (cl % (uint32_t) nx);
-  int cy = (int) ((cl / (uint32_t) nx) % (uint32_t) ny);
-  int cz = (int) (cl / ((uint32_t) nx * (uint32_t) ny));
-  double ccx = lox + (cx + 0.5) * cwx;
-  double ccy = loy + (cy + 0.5) * cwy;
-  double ccz = loz + (cz + 0.5) * cwz;
-  double ws = ldexp(wv, -wexp);            /* |ws| <= 1 */
-  int wi = (int) __double2ll_rn(ws * 1073741824.0);
-  float wr = (float) (ws - (double) wi * (1.0 / 1073741824.0));
-  float4 v;
-  v.x = (float) (a - ccx);
-  v.y = (float) (b - ccy);
-  v.z = (float) (d - ccz);
-  v.w = (float) ws;
-  l4[pos] = v;
-  wq[pos] = make_int2(wi, __float_as_int(wr));
-  sx[pos] = a;
-  sy[pos] = b;
-  sz[pos] = d;
-  sw[pos] = wv;
-  sid[pos] = id;
-}
-
-__global__ void k_scatter(size_t n, const double *__restrict__ x,
+/* Every point to its place by cell and sub-cell: FP32 coordinates (for the
+ * ordering within a run, k_runs) and the input index. */
+__global__ void k_keys(size_t n, const double *__restrict__ x,
     const double *__restrict__ y, const double *__restrict__ z,
-    const double *__restrict__ s, const double *__restrict__ w, int has_w,
-    int wexp, int nx, int ny, double cwx, double cwy, double cwz, double lox,
-    double loy, double loz, uint32_t cell_base, uint32_t id_base, int sb,
-    const uint32_t *__restrict__ cell_of,
-    const uint32_t *__restrict__ fstart, uint32_t *__restrict__ cfill,
-    float4 *__restrict__ l4, int2 *__restrict__ wq, double *__restrict__ sx,
-    double *__restrict__ sy, double *__restrict__ sz, double *__restrict__ ss,
-    double *__restrict__ sw, uint32_t *__restrict__ sid) {
+    const uint32_t *__restrict__ cell_of, const uint32_t *__restrict__ rank,
+    const uint32_t *__restrict__ fstart, float4 *__restrict__ key) {
   for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n;
-       i += (size_t) gridDim.x * blockDim.x) {
-    const uint32_t f = cell_of[i];
-    uint32_t pos = fstart[f] + atomicAdd(cfill + f, 1u);
-    scatter_point(f >> sb, pos, x[i], y[i], z[i], has_w ? w[i] : 1.0, wexp, nx, ny,
-                  cwx, cwy, cwz, lox, loy, loz, cell_base,
-                  id_base + (uint32_t) i, l4, wq, sx, sy, sz, sw, sid);
-    if (ss) ss[pos] = s[i];
-  }
+       i += (size_t) gridDim.x * blockDim.x)
+    key[fstart[cell_of[i]] + rank[i]] = make_float4((float) x[i], (float) y[i],
+        (float) z[i], __uint_as_float((uint32_t) i));
 }
 
 /* cstart[c] = fstart[c << sb], c = 0..nc: the cells' first sorted points
- * from the fine (sub-cell) starts. */
+ * from the fine (sub-cell) starts.  bstart, if given: the cells' first
+ * blocks, numbered with at most one place left unused per cell:
+ * floor(cstart / 32) + c grows from cell to cell by more than the cell's
+ * points / 32. */
 __global__ void k_cstart(size_t nc, int sb, const uint32_t *__restrict__ fstart,
-    uint32_t *__restrict__ cstart) {
+    uint32_t *__restrict__ cstart, uint32_t *__restrict__ bstart) {
   for (size_t c = blockIdx.x * (size_t) blockDim.x + threadIdx.x; c <= nc;
-       c += (size_t) gridDim.x * blockDim.x)
-    cstart[c] = fstart[c << sb];
+       c += (size_t) gridDim.x * blockDim.x) {
+    const uint32_t v = fstart[c << sb];
+    cstart[c] = v;
+    if (bstart) bstart[c] = v / 32u + (uint32_t) c;
+  }
+}
+
+__global__ void k_block_count(const uint32_t *__restrict__ cstart,
+    uint32_t ncell, uint32_t *__restrict__ count) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
+       c += gridDim.x * blockDim.x)
+    count[c] = (cstart[c + 1] - cstart[c] + 31u) / 32u;
+}
+
+/*
+ * The sorted arrays and the blocks.  A cell's points come in runs of at most
+ * RUN_LEN along the Hilbert curve; a warp orders a run so that each block of
+ * 32 has a compact box: it is halved along its longest axis, the halves
+ * along theirs, down to 32 (a bitonic sort of 23-bit coordinates and 9-bit
+ * indices in registers, 16 per lane).  Consecutive runs of 32 points of the
+ * curve itself have boxes of about twice the volume; with this order the
+ * tiles of a uniform box fell by a fifth.  Then the run is gathered from the
+ * input arrays and written in order: the FP32 offsets from the cell centre
+ * and the weight's scaled high part (l4), the weight's fixed-point split
+ * (wq), FP64 copies and ids, and the blocks' boxes of the FP32 offsets (half
+ * extents rounded up).
+ *
+ * Warps: groups of `group` consecutive cells, `share` warps to a group, which
+ * deal the cells' runs among themselves.
+ */
+#define RUN_LEN 512
+#define RUN_WARPS 4
+struct RunArgs {
+  const uint32_t *cstart, *bstart;
+  uint32_t ncell;
+  uint32_t group, share;
+  const float4 *key;
+  const double *x, *y, *z, *s, *w;
+  int has_w, wexp;
+  int nx, ny;
+  double cw[3], lo[3];
+  const fcfcg_prep_cat *cat;      /* a batch: per catalogue */
+  const uint32_t *mbase;
+  int ncat;
+  float4 *l4;
+  int2 *wq;
+  double *sx, *sy, *sz, *ss, *sw;
+  uint32_t *sid;
+  float4 *blk;
+  uint2 *bcell;
+};
+struct RunSh {
+  float c[3][RUN_LEN];
+  uint32_t id[RUN_LEN];
+  uint16_t ord[RUN_LEN];
+};
+
+/* Compare-exchange of keys i and i ^ J of a lane, ascending. */
+template <int J>
+__device__ __forceinline__ void run_step(uint32_t k[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i++)
+    if (!(i & J)) {
+      const uint32_t a = k[i], b = k[i | J];
+      k[i] = a < b ? a : b;
+      k[i | J] = a < b ? b : a;
+    }
+}
+
+/* Sort segments of S keys (16 S / 16 lanes), ascending; S = 64 .. 512. */
+__device__ __forceinline__ void run_sort(uint32_t k[16], int S, int lane) {
+  /* bitonic runs of 2, 4, 8 within the lane: descending where bit K of the
+   * index is set (the keys complemented) */
+#pragma unroll
+  for (int K = 2; K < 16; K <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (i & K) k[i] = ~k[i];
+    if (K > 4) run_step<4>(k);
+    if (K > 2) run_step<2>(k);
+    run_step<1>(k);
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (i & K) k[i] = ~k[i];
+  }
+#pragma unroll 1
+  for (int K = 16; K <= S; K <<= 1) {
+    const uint32_t m = (K < S && ((lane << 4) & K)) ? 0xffffffffu : 0u;
+#pragma unroll
+    for (int i = 0; i < 16; i++) k[i] ^= m;
+#pragma unroll 1
+    for (int o = K >> 5; o > 0; o >>= 1) {
+      const bool low = !(lane & o);
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const uint32_t b = __shfl_xor_sync(0xffffffffu, k[i], o);
+        k[i] = (low == (k[i] < b)) ? k[i] : b;
+      }
+    }
+    run_step<8>(k);
+    run_step<4>(k);
+    run_step<2>(k);
+    run_step<1>(k);
+#pragma unroll
+    for (int i = 0; i < 16; i++) k[i] ^= m;
+  }
+}
+
+/* One run: points [a, a + n) of the cell's, its first block b0. */
+__device__ __forceinline__ void run_order(RunSh *S, const float4 *key,
+    uint32_t a, int n, int lane) {
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    const float4 v = key[a + i];
+    S->c[0][i] = v.x;
+    S->c[1][i] = v.y;
+    S->c[2][i] = v.z;
+    S->id[i] = __float_as_uint(v.w);
+    S->ord[i] = (uint16_t) i;
+  }
+  __syncwarp();
+  if (n <= 32) return;
+  uint32_t k[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) k[i] = (uint32_t) (16 * lane + i);
+#pragma unroll 1
+  for (int L = RUN_LEN; L >= 64; L >>= 1) {
+    if (n <= L / 2) continue;       /* all in the first half already */
+    /* the longest axis of each segment of L */
+    float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int e = (int) (k[i] & (RUN_LEN - 1u));
+      if (e < n)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          const float v = S->c[d][e];
+          lo[d] = fminf(lo[d], v);
+          hi[d] = fmaxf(hi[d], v);
+        }
+    }
+    for (int o = L >> 5; o > 0; o >>= 1)
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+    const float ex = hi[0] - lo[0], ey = hi[1] - lo[1], ez = hi[2] - lo[2];
+    const int d = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
+    const float l = lo[d], w = hi[d] - lo[d];
+    const float f = w > 0 ? 8388606.f / w : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t e = k[i] & (RUN_LEN - 1u);
+      uint32_t q = 0x7fffffu;
+      if ((int) e < n) {
+        q = (uint32_t) ((S->c[d][e] - l) * f);
+        q = q < 0x7ffffeu ? q : 0x7ffffeu;
+      }
+      k[i] = q << 9 | e;
+    }
+    run_sort(k, L, lane);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; i++)
+    S->ord[16 * lane + i] = (uint16_t) (k[i] & (RUN_LEN - 1u));
+  __syncwarp();
+}
+
+template <int BATCH>
+__global__ void __launch_bounds__(32 * RUN_WARPS) k_runs(const RunArgs A) {
+  __shared__ RunSh sh[RUN_WARPS];
+  const int lane = threadIdx.x & 31;
+  RunSh *S = sh + (threadIdx.x >> 5);
+  const uint32_t wid = blockIdx.x * RUN_WARPS + (threadIdx.x >> 5);
+  const uint32_t r0 = wid % A.share, c0 = wid / A.share * A.group;
+  if (c0 >= A.ncell) return;
+  const uint32_t c1 = c0 + A.group < A.ncell ? c0 + A.group : A.ncell;
+  for (uint32_t c = c0; c < c1; c++) {
+    const uint32_t a = __ldg(A.cstart + c), n = __ldg(A.cstart + c + 1) - a;
+    const uint32_t b = __ldg(A.bstart + c), nb = (n + 31u) / 32u;
+    const uint32_t nrun = (n + RUN_LEN - 1u) / RUN_LEN;
+    const bool gap = r0 == 0 && __ldg(A.bstart + c + 1) - b > nb;
+    if (r0 >= nrun && !gap) continue;
+    int nx = A.nx, ny = A.ny, wexp = A.wexp;
+    uint32_t lc = c, mk = 0;
+    double cw[3] = {A.cw[0], A.cw[1], A.cw[2]},
+           lo[3] = {A.lo[0], A.lo[1], A.lo[2]};
+    if (BATCH) {
+      int l = 0, h = A.ncat;        /* last l with mbase[l] <= c */
+      while (h - l > 1) {
+        const int mid = (l + h) >> 1;
+        if (__ldg(A.mbase + mid) <= c) l = mid;
+        else h = mid;
+      }
+      mk = (uint32_t) l;
+      const fcfcg_prep_cat *C = A.cat + l;
+      nx = C->ncell[0];
+      ny = C->ncell[1];
+      wexp = C->wexp;
+      lc = c - C->cell_base;
+      for (int k = 0; k < 3; k++) {
+        cw[k] = C->cw[k];
+        lo[k] = 0.0;
+      }
+    }
+    if (gap && lane == 0) {
+      /* the place left unused: far from everything, no points */
+      A.blk[2 * (size_t) (b + nb)] = make_float4(1e30f, 1e30f, 1e30f, 0.f);
+      A.blk[2 * (size_t) (b + nb) + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      A.bcell[b + nb] = make_uint2(c, mk);
+    }
+    const double cc[3] = {
+        lo[0] + ((double) (int) (lc % (uint32_t) nx) + 0.5) * cw[0],
+        lo[1] + ((double) (int) ((lc / (uint32_t) nx) % (uint32_t) ny) + 0.5) * cw[1],
+        lo[2] + ((double) (int) (lc / ((uint32_t) nx * (uint32_t) ny)) + 0.5) * cw[2]};
+    for (uint32_t r = r0; r < nrun; r += A.share) {
+      const uint32_t q0 = r * RUN_LEN;
+      const int m = (int) (n - q0 < RUN_LEN ? n - q0 : RUN_LEN);
+      run_order(S, A.key, a + q0, m, lane);
+      for (int j0 = 0; j0 < m; j0 += 32) {
+        const int j = j0 + lane;
+        float mn[3] = {3e38f, 3e38f, 3e38f}, mx[3] = {-3e38f, -3e38f, -3e38f};
+        const uint32_t pos = a + q0 + (uint32_t) j;
+        if (j < m) {
+          const uint32_t i = S->id[S->ord[j]];
+          const double v[3] = {A.x[i], A.y[i], A.z[i]};
+          const double wv = A.has_w ? A.w[i] : 1.0;
+          double ws = wv;
+          int wi = 1 << 30;
+          float wr = 0.f;
+          if (A.has_w) {
+            ws = ldexp(wv, -wexp);               /* |ws| <= 1 */
+            wi = (int) __double2ll_rn(ws * 1073741824.0);
+            wr = (float) (ws - (double) wi * (1.0 / 1073741824.0));
+          }
+          float4 p;
+          p.x = (float) (v[0] - cc[0]);
+          p.y = (float) (v[1] - cc[1]);
+          p.z = (float) (v[2] - cc[2]);
+          p.w = (float) ws;
+          A.l4[pos] = p;
+          A.wq[pos] = make_int2(wi, __float_as_int(wr));
+          A.sx[pos] = v[0];
+          A.sy[pos] = v[1];
+          A.sz[pos] = v[2];
+          if (A.ss) A.ss[pos] = A.s[i];
+          A.sw[pos] = wv;
+          A.sid[pos] = i;
+          mn[0] = mx[0] = p.x;
+          mn[1] = mx[1] = p.y;
+          mn[2] = mx[2] = p.z;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+            mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+          }
+        if (lane == 0) {
+          float ce[3], e[3];
+          for (int k = 0; k < 3; k++) {
+            ce[k] = 0.5f * mn[k] + 0.5f * mx[k];
+            e[k] = __fmul_ru(fmaxf(__fsub_ru(mx[k], ce[k]),
+                                   __fsub_ru(ce[k], mn[k])), 1.000001f);
+          }
+          const size_t B = b + (q0 + (uint32_t) j0) / 32u;
+          const int cnt = m - j0 < 32 ? m - j0 : 32;
+          A.blk[2 * B] = make_float4(ce[0], ce[1], ce[2],
+                                     __uint_as_float(pos));
+          A.blk[2 * B + 1] = make_float4(e[0], e[1], e[2],
+                                         __uint_as_float((uint32_t) cnt));
+          A.bcell[B] = make_uint2(c, mk);
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+/* Warps of k_runs for ncell cells of n points: 32 cells to a group where
+ * there are many, and as many warps to a group as its cells have runs. */
+static void launch_runs(RunArgs *A, size_t n, cudaStream_t st) {
+  A->group = A->ncell > 32u * 4864u ? 32u : (A->ncell > 4u * 4864u ? 4u : 1u);
+  const size_t per = n / A->ncell / RUN_LEN + 1;
+  A->share = (uint32_t) (per * 2 < 256 ? per * 2 : 256);
+  const uint64_t warps =
+      ((uint64_t) A->ncell + A->group - 1) / A->group * A->share;
+  const unsigned nb = (unsigned) ((warps + RUN_WARPS - 1) / RUN_WARPS);
+  if (A->cat) k_runs<1><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
+  else k_runs<0><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
 }
 
 extern "C" int fcfcg_grid_sub_bits(size_t ncell, size_t npoint) {
@@ -427,44 +678,82 @@ extern "C" int fcfcg_grid_curve_bits(size_t ncell, size_t npoint) {
   return fcfcg_grid_sub_bits(ncell, npoint);
 }
 
+/* The blocks' numbering from the cells' points: with gaps (k_cstart) unless
+ * cells far outnumber the blocks, where it is compacted by a scan. */
+static int gaps_ok(size_t n, size_t nc) { return nc <= 4096 || nc <= n / 16; }
+
+extern "C" size_t fcfcg_max_blocks(size_t n, size_t ncell) {
+  return n / 32 + (n < ncell && !gaps_ok(n, ncell) ? n : ncell) + 1;
+}
+
+/* Fine counts (in cfill) to cell starts, keys and the block numbering. */
+static int sort_rest(cudaStream_t st, size_t nc, size_t n, int sb,
+    uint32_t *cfill, uint32_t *fstart, uint32_t *scan_tmp, uint32_t *cstart,
+    uint32_t *bstart) {
+  int r = scan_u32(st, cfill, nc << sb, fstart, scan_tmp);
+  if (r) return r;
+  const int gaps = gaps_ok(n, nc);
+  k_cstart<<<grid_for(nc + 1, PREP_THREADS), PREP_THREADS, 0, st>>>(
+      nc, sb, fstart, cstart, gaps ? bstart : NULL);
+  cudaError_t e = cudaGetLastError();
+  if (e || gaps) return (int) e;
+  k_block_count<<<grid_for(nc, PREP_THREADS), PREP_THREADS, 0, st>>>(
+      cstart, (uint32_t) nc, cfill);
+  if ((e = cudaGetLastError())) return (int) e;
+  return scan_u32(st, cfill, nc, bstart, scan_tmp);
+}
+
 extern "C" int fcfcg_k_grid(void *stream, size_t n, const double *x,
     const double *y, const double *z, const double *s, const double *w,
     int has_w, int wexp, const int ncell[3], const double cw[3],
-    const double lo[3], int sb, uint32_t *cell_of, uint32_t *cstart,
-    uint32_t *fstart, uint32_t *cfill, uint32_t *scan_tmp,
-    size_t scan_tmp_len, float *l4, int *wq, double *sx, double *sy,
-    double *sz, double *ss, double *sw, uint32_t *sid) {
+    const double lo[3], int sb, const fcfcg_sort *S) {
   cudaStream_t st = (cudaStream_t) stream;
   const size_t nc = (size_t) ncell[0] * ncell[1] * ncell[2];
-  const size_t nf = nc << sb;
-  (void) scan_tmp_len;
-  cudaError_t e = cudaMemsetAsync(cfill, 0, sizeof(uint32_t) * nf, st);
+  cudaError_t e = cudaMemsetAsync(S->cfill, 0, sizeof(uint32_t) * (nc << sb), st);
   if (e) return (int) e;
   if (n) {
     k_cell<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0, st>>>(
-        n, x, y, z, fine_grid(ncell, cw, lo, sb), cell_of, cfill);
+        n, x, y, z, fine_grid(ncell, cw, lo, sb), S->cell_of, S->rank, S->cfill);
     if ((e = cudaGetLastError())) return (int) e;
   }
-  int r = scan_u32(st, cfill, nf, fstart, scan_tmp);
+  int r = sort_rest(st, nc, n, sb, S->cfill, S->fstart, S->scan_tmp, S->cstart,
+                    S->bstart);
   if (r) return r;
-  k_cstart<<<grid_for(nc + 1, PREP_THREADS), PREP_THREADS, 0, st>>>(
-      nc, sb, fstart, cstart);
-  if ((e = cudaGetLastError())) return (int) e;
-  if ((e = cudaMemsetAsync(cfill, 0, sizeof(uint32_t) * nf, st))) return (int) e;
   if (n) {
-    k_scatter<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0, st>>>(
-        n, x, y, z, s, w, has_w, wexp, ncell[0], ncell[1], cw[0], cw[1],
-        cw[2], lo[0], lo[1], lo[2], 0u, 0u, sb, cell_of, fstart, cfill,
-        (float4 *) l4, (int2 *) wq, sx, sy, sz, ss, sw, sid);
+    k_keys<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0, st>>>(
+        n, x, y, z, S->cell_of, S->rank, S->fstart, (float4 *) S->key);
     if ((e = cudaGetLastError())) return (int) e;
   }
-  return 0;
-}
-
-extern "C" int fcfcg_k_cstart(void *stream, size_t nc, int sb,
-    const uint32_t *fstart, uint32_t *cstart) {
-  k_cstart<<<grid_for(nc + 1, PREP_THREADS), PREP_THREADS, 0,
-             (cudaStream_t) stream>>>(nc, sb, fstart, cstart);
+  RunArgs A;
+  memset(&A, 0, sizeof A);
+  A.cstart = S->cstart;
+  A.bstart = S->bstart;
+  A.ncell = (uint32_t) nc;
+  A.key = (const float4 *) S->key;
+  A.x = x;
+  A.y = y;
+  A.z = z;
+  A.s = s;
+  A.w = w;
+  A.has_w = has_w;
+  A.wexp = wexp;
+  A.nx = ncell[0];
+  A.ny = ncell[1];
+  for (int k = 0; k < 3; k++) {
+    A.cw[k] = cw[k];
+    A.lo[k] = lo[k];
+  }
+  A.l4 = (float4 *) S->l4;
+  A.wq = (int2 *) S->wq;
+  A.sx = S->sx;
+  A.sy = S->sy;
+  A.sz = S->sz;
+  A.ss = s ? S->ss : NULL;
+  A.sw = S->sw;
+  A.sid = S->sid;
+  A.blk = (float4 *) S->blk;
+  A.bcell = (uint2 *) S->bcell;
+  launch_runs(&A, n, st);
   return (int) cudaGetLastError();
 }
 
@@ -610,7 +899,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_cell_batch(
     const fcfcg_prep_cat *__restrict__ cat, int ncat, int sb,
     const double *__restrict__ x, const double *__restrict__ y,
     const double *__restrict__ z, uint32_t *__restrict__ cell_of,
-    uint32_t *__restrict__ count) {
+    uint32_t *__restrict__ rank, uint32_t *__restrict__ count) {
   const uint32_t t = blockIdx.x;
   const fcfcg_prep_cat *C = cat + batch_cat(cat, ncat, t);
   if (!C->live) return;
@@ -628,58 +917,70 @@ __global__ void __launch_bounds__(PREP_THREADS) k_cell_batch(
   for (size_t i = o + i0 + threadIdx.x; i < o + i1; i += PREP_THREADS) {
     const uint32_t c = fine_of_point(g, x[i], y[i], z[i]);
     cell_of[i] = c;
-    atomicAdd(count + c, 1u);
+    rank[i] = atomicAdd(count + c, 1u);
   }
 }
 
-/* Every live catalogue's points to their sorted places (as k_scatter); the
- * id of point i of the slot is i. */
-__global__ void __launch_bounds__(PREP_THREADS) k_scatter_batch(
-    const fcfcg_prep_cat *__restrict__ cat, int ncat, int sb,
+/* k_keys for every live catalogue; the index of point i of the slot is i. */
+__global__ void __launch_bounds__(PREP_THREADS) k_keys_batch(
+    const fcfcg_prep_cat *__restrict__ cat, int ncat,
     const double *__restrict__ x, const double *__restrict__ y,
-    const double *__restrict__ z, const double *__restrict__ w, int has_w,
-    const uint32_t *__restrict__ cell_of,
-    const uint32_t *__restrict__ fstart, uint32_t *__restrict__ cfill,
-    float4 *__restrict__ l4, int2 *__restrict__ wq, double *__restrict__ sx,
-    double *__restrict__ sy, double *__restrict__ sz, double *__restrict__ sw,
-    uint32_t *__restrict__ sid) {
+    const double *__restrict__ z, const uint32_t *__restrict__ cell_of,
+    const uint32_t *__restrict__ rank, const uint32_t *__restrict__ fstart,
+    float4 *__restrict__ key) {
   const uint32_t t = blockIdx.x;
   const fcfcg_prep_cat *C = cat + batch_cat(cat, ncat, t);
   if (!C->live) return;
   const size_t o = C->o, n = C->n;
   const size_t i0 = (size_t) (t - C->tile0) * BATCH_TILE;
   const size_t i1 = (i0 + BATCH_TILE < n) ? i0 + BATCH_TILE : n;
-  const int nx = C->ncell[0], ny = C->ncell[1], wexp = C->wexp;
-  const double cwx = C->cw[0], cwy = C->cw[1], cwz = C->cw[2];
-  const uint32_t base = C->cell_base;
-  for (size_t i = o + i0 + threadIdx.x; i < o + i1; i += PREP_THREADS) {
-    const uint32_t f = cell_of[i];
-    const uint32_t pos = fstart[f] + atomicAdd(cfill + f, 1u);
-    scatter_point(f >> sb, pos, x[i], y[i], z[i], has_w ? w[i] : 1.0, wexp, nx, ny,
-                  cwx, cwy, cwz, 0.0, 0.0, 0.0, base, (uint32_t) i, l4, wq,
-                  sx, sy, sz, sw, sid);
-  }
+  for (size_t i = o + i0 + threadIdx.x; i < o + i1; i += PREP_THREADS)
+    key[fstart[cell_of[i]] + rank[i]] = make_float4((float) x[i], (float) y[i],
+        (float) z[i], __uint_as_float((uint32_t) i));
 }
 
-extern "C" int fcfcg_k_cell_batch(void *stream, const fcfcg_prep_cat *d_cat,
-    int ncat, uint32_t ntile, int sb, const double *x, const double *y,
-    const double *z, uint32_t *cell_of, uint32_t *count) {
+extern "C" int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat,
+    int ncat, uint32_t ntile, size_t ncell, size_t n, const uint32_t *mbase,
+    int sb, const double *x, const double *y, const double *z,
+    const double *w, int has_w, const fcfcg_sort *S) {
   if (!ncat || !ntile) return 0;
-  k_cell_batch<<<ntile, PREP_THREADS, 0, (cudaStream_t) stream>>>(
-      d_cat, ncat, sb, x, y, z, cell_of, count);
-  return (int) cudaGetLastError();
-}
-
-extern "C" int fcfcg_k_scatter_batch(void *stream,
-    const fcfcg_prep_cat *d_cat, int ncat, uint32_t ntile, int sb,
-    const double *x, const double *y, const double *z, const double *w,
-    int has_w, const uint32_t *cell_of, const uint32_t *fstart,
-    uint32_t *cfill, float *l4, int *wq, double *sx, double *sy, double *sz,
-    double *sw, uint32_t *sid) {
-  if (!ncat || !ntile) return 0;
-  k_scatter_batch<<<ntile, PREP_THREADS, 0, (cudaStream_t) stream>>>(
-      d_cat, ncat, sb, x, y, z, w, has_w, cell_of, fstart, cfill, (float4 *) l4,
-      (int2 *) wq, sx, sy, sz, sw, sid);
+  cudaStream_t st = (cudaStream_t) stream;
+  cudaError_t e = cudaMemsetAsync(S->cfill, 0,
+                                  sizeof(uint32_t) * (ncell << sb), st);
+  if (e) return (int) e;
+  k_cell_batch<<<ntile, PREP_THREADS, 0, st>>>(d_cat, ncat, sb, x, y, z,
+                                               S->cell_of, S->rank, S->cfill);
+  if ((e = cudaGetLastError())) return (int) e;
+  int r = sort_rest(st, ncell, n, sb, S->cfill, S->fstart, S->scan_tmp,
+                    S->cstart, S->bstart);
+  if (r) return r;
+  k_keys_batch<<<ntile, PREP_THREADS, 0, st>>>(d_cat, ncat, x, y, z,
+      S->cell_of, S->rank, S->fstart, (float4 *) S->key);
+  if ((e = cudaGetLastError())) return (int) e;
+  RunArgs A;
+  memset(&A, 0, sizeof A);
+  A.cstart = S->cstart;
+  A.bstart = S->bstart;
+  A.ncell = (uint32_t) ncell;
+  A.key = (const float4 *) S->key;
+  A.x = x;
+  A.y = y;
+  A.z = z;
+  A.w = w;
+  A.has_w = has_w;
+  A.cat = d_cat;
+  A.mbase = mbase;
+  A.ncat = ncat;
+  A.l4 = (float4 *) S->l4;
+  A.wq = (int2 *) S->wq;
+  A.sx = S->sx;
+  A.sy = S->sy;
+  A.sz = S->sz;
+  A.sw = S->sw;
+  A.sid = S->sid;
+  A.blk = (float4 *) S->blk;
+  A.bcell = (uint2 *) S->bcell;
+  launch_runs(&A, n, st);
   return (int) cudaGetLastError();
 }
 
@@ -747,97 +1048,6 @@ extern "C" int fcfcg_k_chunks(void *stream, const uint32_t *cstart,
                              cudaMemcpyDeviceToHost, st)))
       return (int) e;
   return 0;
-}
-
-/* ------------------------------------------------------------------------ */
-/* Blocks of at most 32 points. */
-
-__global__ void k_block_count(const uint32_t *__restrict__ cstart,
-    uint32_t ncell, uint32_t *__restrict__ count) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += gridDim.x * blockDim.x)
-    count[c] = (cstart[c + 1] - cstart[c] + 31u) / 32u;
-}
-
-/* A warp per block: the points of a cell are cut as evenly as possible, and
- * the block's box is that of its FP32 offsets from the cell centre (half
- * extents rounded up). */
-__global__ void __launch_bounds__(PREP_THREADS) k_blocks(
-    const uint32_t *__restrict__ cstart, uint32_t ncell,
-    const uint32_t *__restrict__ bstart, const float4 *__restrict__ l4,
-    float4 *__restrict__ blk, uint2 *__restrict__ bcell,
-    const uint32_t *__restrict__ mbase, int nmock) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t nblk = __ldg(bstart + ncell);
-  const uint32_t nw = gridDim.x * (PREP_THREADS / 32);
-  for (uint32_t b = blockIdx.x * (PREP_THREADS / 32) + (threadIdx.x >> 5);
-       b < nblk; b += nw) {
-    uint32_t lo = 0, hi = ncell;    /* last lo with bstart[lo] <= b */
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (__ldg(bstart + mid) <= b) lo = mid;
-      else hi = mid;
-    }
-    const uint32_t a = __ldg(cstart + lo), n = __ldg(cstart + lo + 1) - a;
-    const uint32_t q = b - __ldg(bstart + lo), nq = (n + 31u) / 32u;
-    const uint32_t i0 = (uint32_t) (((unsigned long long) n * q) / nq),
-                   i1 = (uint32_t) (((unsigned long long) n * (q + 1)) / nq);
-    const uint32_t m = i1 - i0;
-    const float4 v = __ldg(l4 + a + i0 + (lane < (int) m ? lane : 0));
-    float mn[3] = {v.x, v.y, v.z}, mx[3] = {v.x, v.y, v.z};
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-        mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-      }
-    if (lane == 0) {
-      float c[3], e[3];
-      for (int k = 0; k < 3; k++) {
-        c[k] = 0.5f * mn[k] + 0.5f * mx[k];
-        e[k] = __fmul_ru(fmaxf(__fsub_ru(mx[k], c[k]), __fsub_ru(c[k], mn[k])),
-                         1.000001f);
-      }
-      blk[2 * (size_t) b] = make_float4(c[0], c[1], c[2],
-                                        __uint_as_float(a + i0));
-      blk[2 * (size_t) b + 1] = make_float4(e[0], e[1], e[2],
-                                            __uint_as_float(m));
-      uint32_t mk = 0;
-      if (mbase) {
-        int l = 0, h = nmock;       /* last l with mbase[l] <= the cell */
-        while (h - l > 1) {
-          const int mid = (l + h) >> 1;
-          if (__ldg(mbase + mid) <= lo) l = mid;
-          else h = mid;
-        }
-        mk = (uint32_t) l;
-      }
-      bcell[b] = make_uint2(lo, mk);
-    }
-  }
-}
-
-extern "C" size_t fcfcg_max_blocks(size_t n, size_t ncell) {
-  return n / 32 + (n < ncell ? n : ncell) + 1;
-}
-
-extern "C" int fcfcg_k_blocks(void *stream, const uint32_t *cstart,
-    uint32_t ncell, size_t n, uint32_t *count, uint32_t *scan_tmp,
-    const float *l4, uint32_t *bstart, float *blk, uint32_t *bcell,
-    const uint32_t *mbase, int nmock) {
-  cudaStream_t st = (cudaStream_t) stream;
-  k_block_count<<<grid_for(ncell, PREP_THREADS), PREP_THREADS, 0, st>>>(
-      cstart, ncell, count);
-  cudaError_t e = cudaGetLastError();
-  if (e) return (int) e;
-  int r = scan_u32(st, count, ncell, bstart, scan_tmp);
-  if (r) return r;
-  k_blocks<<<grid_for(fcfcg_max_blocks(n, ncell) * 32, PREP_THREADS),
-             PREP_THREADS, 0, st>>>(cstart, ncell, bstart,
-                                    (const float4 *) l4, (float4 *) blk,
-                                    (uint2 *) bcell, mbase, nmock);
-  return (int) cudaGetLastError();
 }
 
 /* Occupancy of a coarse grid over a catalogue's bounding box: one bit per

@@ -888,6 +888,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
     T.first = __float_as_uint(__ldg(&Ab[0].w));
     T.m = (int) __float_as_uint(__ldg(&Ab[1].w));
     T.mock = ci.y;
+    if (T.m == 0) continue;        /* a place left unused */
     float c2x = 0.f, c2y = 0.f, c2z = 0.f;
     if (SURVEY) {
       /* twice A's cell centre: the FP64 centre the local coordinates are
