@@ -325,12 +325,12 @@ def mocks_cpu_sample(cats, boxes, subset, steps=1, warmup=0):
 
 
 def kernel_source_sha256():
-    """sha256 over the FP32 count kernel's sources (count32.cuh, then
+    """sha256 over the FP32 count kernel's sources (tile32.cuh, then
     count_common.cuh): a committed ncu summary records the value it was
     captured on."""
     import hashlib
     h = hashlib.sha256()
-    for f in ("count32.cuh", "count_common.cuh"):
+    for f in ("tile32.cuh", "count_common.cuh"):
         h.update(open(os.path.join(ROOT, "fcfc_gb300", "csrc", f), "rb").read())
     return h.hexdigest()
 
@@ -490,7 +490,7 @@ def run_mocks(args, rank, world, local, dist):
         "roofline": {"bound": "issue", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": traffic,
-                     "kernel": "k_count32<box,smu,unweighted,batch>",
+                     "kernel": "k_tile32<box,smu,unweighted,batch>",
                      "kernel_ms": k_ms,
                      "peak_source": "measured cuBLAS SGEMM (TF32 off) on this GPU",
                      "flops_per_pair": FLOPS_PER_PAIR["smu"],
@@ -674,7 +674,7 @@ def run_survey(args, rank, world, local, dist):
                 "d2h_bytes_per_step": 3 * (p1.ntot + p2.ntot) * 8},
         "roofline": {"bound": "issue", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
-                     "kernel": "k_count32<survey,smu,weighted> (RR)",
+                     "kernel": "k_tile32<survey,smu,weighted> (RR)",
                      "kernel_ms": k_rr,
                      "peak_source": "measured cuBLAS SGEMM (TF32 off) on this GPU",
                      "flops_per_pair": FLOPS_PER_PAIR["smu"],
@@ -1081,7 +1081,7 @@ def main():
         "roofline": {"bound": "issue", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": traffic,
-                     "kernel": "k_count32<box,smu,weighted>",
+                     "kernel": "k_tile32<box,smu,weighted>",
                      "kernel_ms": k1_ms,
                      "peak_source": "measured cuBLAS SGEMM (TF32 off) on this GPU",
                      "flops_per_pair": FLOPS_PER_PAIR["smu"],

@@ -19,7 +19,7 @@ OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libfcfcg.so")
 
 CU_SOURCES = ["prep.cu", "count.cu", "count32_box.cu", "count32_survey.cu",
-              "count32_batch.cu", "count32_adj.cu", "cnvt.cu", "probe.cu"]
+              "count32_batch.cu", "count32_adj.cu", "count32_f64.cu", "cnvt.cu", "probe.cu"]
 C_SOURCES = ["bins.c", "ctx.c", "epilogue.c", "cnvt.c"]
 HEADERS = ["fcfcg_internal.h", "legauss_tab.h", "count_common.cuh", "tile32.cuh",
            os.path.join("..", "..", "include", "fcfcg.h")]
@@ -69,7 +69,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
         o = os.path.join(OBJDIR, s + ".o")
         jobs.append([nvcc, *ARCH, "-O3", "-lineinfo", "-std=c++17",
                      "-Xcompiler", "-fPIC", "-Xptxas", "-v" if verbose else "-O3",
-                     *os.environ.get("FCFCG_NVCC_FLAGS", "").split(),
                      "-I", CSRC, "-c", os.path.join(CSRC, s), "-o", o])
     for s in C_SOURCES:
         o = os.path.join(OBJDIR, s + ".o")

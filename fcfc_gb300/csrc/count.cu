@@ -1,85 +1,9 @@
 /*
- * count.cu -- host-side launchers of the counting kernels, the all-FP64
- * counting kernel, the FP64 recheck of queued pairs, and the
- * allocation-free FP64 counter.  The FP32 counting kernel is count32.cuh,
- * instantiated by the count32_*.cu files.
+ * count.cu -- host-side launchers of the counting kernels, the FP64 recheck
+ * of queued pairs, and the allocation-free FP64 counter.  The tile kernel is
+ * tile32.cuh, instantiated by the count32_*.cu files.
  */
 #include "tile32.cuh"
-
-/*
- * FP64 counting kernel: the same traversal, every pair binned by the
- * reference's FP64 formula.  Weighted sums are FP64 products accumulated
- * in FP64.
- */
-template <int GEOM, int WT, int ADJ>
-__global__ void __launch_bounds__(CT_THREADS)
-k_count64(const fcfcg_launch L) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  uint32_t *h32 = (uint32_t *) smem;
-  double *hd = (double *) smem;
-  if (!ADJ && L.hist_smem) {
-    if (WT)
-      for (long i = threadIdx.x; i < L.ntot; i += blockDim.x) hd[i] = 0;
-    else
-      for (long i = threadIdx.x; i < L.ntot; i += blockDim.x) h32[i] = 0;
-  }
-  __syncthreads();
-  unsigned long long n_cand = 0, n_in = 0;
-  WarpChunk w;
-  while (next_chunk(L, w)) {
-    double ga = 0;      /* adjoint: this lane's share of dL/dw of its point */
-    for (int t = 0; t < L.nsten; t++) {
-      const int4 o = __ldg((const int4 *) L.sten + t);
-      uint32_t cb, code;
-      if (!neighbour(L, w, o, cb, code)) continue;
-      const uint32_t bstart = __ldg(L.B.cstart + cb);
-      const uint32_t bend = __ldg(L.B.cstart + cb + 1);
-      if (bstart == bend || !w.active) continue;
-      const bool self = L.isauto && o.x == 0 && o.y == 0 && o.z == 0;
-      const int nb = (int) (bend - bstart);
-      for (int j = first_j(w, self, bstart); j < nb; j += w.G) {
-        const uint32_t bj = bstart + (uint32_t) j;
-        n_cand++;
-        int bin = ref_bin_pair(L, w.ai, bj, code, L.box);
-        if (bin < 0) continue;
-        n_in++;
-        if (ADJ) {
-          const double g = __ldg(L.gadj + bin);
-          ga = __dadd_rn(ga, __dmul_rn(L.B.w[bj], g));
-          atomicAdd(L.dB + bj, __dmul_rn(L.A.w[w.ai], g));
-        } else if (WT) {
-          double v = __dmul_rn(L.A.w[w.ai], L.B.w[bj]);
-          if (L.hist_smem) atomicAdd(hd + bin, v);
-          else atomicAdd(L.gwd + bin, v);
-        } else {
-          if (L.hist_smem) hist_add_count(h32, L.gcnt, bin);
-          else atomicAdd(L.gcnt + bin, 1ull);
-        }
-      }
-    }
-    if (ADJ && ga != 0.0) atomicAdd(L.dA + w.ai, ga);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    n_cand += __shfl_xor_sync(FULLMASK, n_cand, o);
-    n_in += __shfl_xor_sync(FULLMASK, n_in, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(L.stats + 0, n_cand);
-    atomicAdd(L.stats + 1, n_in);
-  }
-  __syncthreads();
-  if (!ADJ && L.hist_smem) {
-    for (long i = threadIdx.x; i < L.ntot; i += blockDim.x) {
-      if (WT) {
-        double v = hd[i];
-        if (v != 0) atomicAdd(L.gwd + i, v);
-      } else {
-        uint32_t v = h32[i];
-        if (v) atomicAdd(L.gcnt + i, (unsigned long long) v);
-      }
-    }
-  }
-}
 
 /* Queued pairs to recheck: the queue's fill, at most its capacity. */
 __device__ __forceinline__ uint32_t queue_len(const fcfcg_launch &L) {
@@ -124,62 +48,54 @@ __global__ void k_recheck(const fcfcg_launch L) {
   if ((threadIdx.x & 31) == 0 && n_in) atomicAdd(L.stats + 1, n_in);
 }
 
-/* ------------------------------------------------------------------------ */
-
-static kfun_t pick64(int geom, int wt, int adj) {
-  if (adj)
-    return geom == FCFCG_GEOM_BOX ? (kfun_t) k_count64<FCFCG_GEOM_BOX, 1, 1>
-                                  : (kfun_t) k_count64<FCFCG_GEOM_SURVEY, 1, 1>;
-  if (geom == FCFCG_GEOM_BOX)
-    return wt ? (kfun_t) k_count64<FCFCG_GEOM_BOX, 1, 0>
-              : (kfun_t) k_count64<FCFCG_GEOM_BOX, 0, 0>;
-  return wt ? (kfun_t) k_count64<FCFCG_GEOM_SURVEY, 1, 0>
-            : (kfun_t) k_count64<FCFCG_GEOM_SURVEY, 0, 0>;
+/* FP64 sums: the copies in pairs, then those sums, ... into the first. */
+__global__ void k_gwd_fold(double *gwd, long ntot, int copies) {
+  const long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
+  if (i >= ntot) return;
+  double v[FCFCG_GWD_COPIES];
+#pragma unroll
+  for (int k = 0; k < FCFCG_GWD_COPIES; k++)
+    v[k] = k < copies ? gwd[(size_t) k * ntot + i] : 0;
+#pragma unroll
+  for (int o = FCFCG_GWD_COPIES / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < o; k++) v[k] = __dadd_rn(v[k], v[k + o]);
+  gwd[i] = v[0];
 }
 
+/* ------------------------------------------------------------------------ */
+
 extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
-    int precision, int nsm, size_t *smem_used, uint32_t *qwarp_used) {
-  kfun_t f;
-  size_t smem;
-  int threads;
-  cudaError_t e;
+    int precision, int nsm, size_t *smem_used) {
+  int bin = L->bintype;
+  if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
+  if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
+  if (bin == FCFCG_BIN_SPI && L->tplin) bin = BIN_SPILIN;
+  const int f64 = (precision == FCFCG_PREC_FP64);
+  const kfun_t f = f64 ? fcfcg_pick64(L->geometry, L->withwt, L->adjoint)
+      : L->adjoint ? fcfcg_pick32_adj(L->geometry, bin)
+      : L->geometry == FCFCG_GEOM_SURVEY ? fcfcg_pick32_survey(bin, L->withwt)
+      : L->mocks ? fcfcg_pick32_batch(bin, L->withwt)
+                 : fcfcg_pick32_box(bin, L->withwt);
+  if (!f) return (int) cudaErrorInvalidValue;
+  const size_t smem = (f64 ? 0 : fcfcg_k_tile32_tab(L)) +
+      fcfcg_k_tile32_stage(f64 ? 3 : L->adjoint ? 2 : L->withwt) +
+      fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
+  const int threads = CT32_THREADS;
   int per_sm = 0;
-  if (precision == FCFCG_PREC_FP64) {
-    f = pick64(L->geometry, L->withwt, L->adjoint);
-    smem = (L->hist_smem && !L->adjoint)
-               ? (size_t) L->ntot * (L->withwt ? 8 : 4) : 0;
-    threads = CT_THREADS;
-    if (!f) return (int) cudaErrorInvalidValue;
-    if ((e = cudaFuncSetAttribute((const void *) f,
-             cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-             &per_sm, (const void *) f, threads, smem)))
-      return (int) e;
-  } else {
-    int bin = L->bintype;
-    if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
-    if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
-    if (bin == FCFCG_BIN_SPI && L->tplin) bin = BIN_SPILIN;
-    f = L->adjoint ? fcfcg_pick32_adj(L->geometry, bin)
-        : (L->geometry == FCFCG_GEOM_SURVEY
-               ? fcfcg_pick32_survey(bin, L->withwt)
-               : (L->mocks ? fcfcg_pick32_batch(bin, L->withwt)
-                           : fcfcg_pick32_box(bin, L->withwt)));
-    if (!f) return (int) cudaErrorInvalidValue;
-    smem = fcfcg_k_tile32_tab(L) +
-        fcfcg_k_tile32_stage(L->adjoint ? 2 : L->withwt) +
-        fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
-    threads = CT32_THREADS;
-    if ((e = cudaFuncSetAttribute((const void *) f,
-             cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-             &per_sm, (const void *) f, threads, smem)))
-      return (int) e;
-    if (qwarp_used) *qwarp_used = L->qwarp ? L->qwarp : QWARP_MAX;
-  }
+  cudaError_t e;
+  if ((e = cudaFuncSetAttribute((const void *) f,
+           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) ||
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+           &per_sm, (const void *) f, threads, smem)))
+    return (int) e;
   if (per_sm < 1) return (int) cudaErrorInvalidConfiguration;
   if (smem_used) *smem_used = smem;
   f<<<nsm * per_sm, threads, smem, (cudaStream_t) stream>>>(*L);
+  const int copies = fcfcg_gwd_copies(L->ntot);
+  if (f64 && L->withwt && !L->adjoint && copies > 1)
+    k_gwd_fold<<<(unsigned) ((L->ntot + 127) / 128), 128, 0,
+                 (cudaStream_t) stream>>>(L->gwd, L->ntot, copies);
   return (int) cudaGetLastError();
 }
 
@@ -187,8 +103,8 @@ extern "C" size_t fcfcg_k_tile32_tab(const fcfcg_launch *L) {
   return ((size_t) (L->nse + L->npe) * 8 + 15) & ~(size_t) 15;
 }
 
-extern "C" size_t fcfcg_k_tile32_stage(int withwt) {
-  return (size_t) (CT32_THREADS / 32) * tile_warp_bytes(withwt);
+extern "C" size_t fcfcg_k_tile32_stage(int kind) {
+  return (size_t) (CT32_THREADS / 32) * tile_warp_bytes(kind);
 }
 
 extern "C" size_t fcfcg_k_tile32_hist(int hlen, int withwt) {

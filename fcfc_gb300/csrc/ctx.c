@@ -49,15 +49,14 @@ struct fcfcg_ctx {
   int kcell;
   slot_t slot[FCFCG_MAX_SLOT + 1];   /* the last one holds batches */
   /* shared scratch */
-  uint32_t *cfill, *scan_tmp, *cchunk, *chunks;
-  size_t cfill_cap, scan_cap, cchunk_cap, chunk_cap;
+  uint32_t *cfill, *scan_tmp;
+  size_t cfill_cap, scan_cap;
   uint32_t *fstart;               /* fine (sub-cell) starts of a grid sort */
   size_t fstart_cap;
   uint32_t *rank;                 /* sort scratch: rank in the sub-cell, */
   float *key;                     /* coordinates and index by sub-cell */
   size_t rank_cap, key_cap;
-  uint16_t *d_fs, *d_fp, *d_rs, *d_rp;
-  float *d_fse, *d_fpe;
+  uint16_t *d_rs, *d_rp;
   double *d_s2edge, *d_pedge;
   float *d_se, *d_pe;             /* edge tables of the tile kernel */
   int *d_sten;
@@ -80,12 +79,9 @@ struct fcfcg_ctx {
   /* autotuned grid refinement, keyed on the expected neighbours per object */
   int tuned_k;
   int tuned_key;
-  /* FP32 kernel's warp queue: forced (fcfcg_set_warp_queue), or autotuned
-   * for a key and weighting, else the launcher's choice; the last used */
-  uint32_t qwarp_force, tuned_q, last_qwarp;
+  uint32_t qwarp_force;           /* fcfcg_set_warp_queue: reported only */
   /* hand-over threshold of the unweighted shared histogram (0: 2^32 - 1) */
   unsigned long long hs_limit;
-  int tuned_q_key, tuned_q_wt;
   /* RA/Dec/z conversion scratch */
   void *d_cnvt;
   size_t cnvt_cap;
@@ -208,9 +204,8 @@ void fcfcg_destroy(fcfcg_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (int i = 0; i <= FCFCG_MAX_SLOT; i++) slot_free(c->slot + i);
-    void *p[] = {c->cfill, c->fstart, c->rank, c->key, c->scan_tmp, c->cchunk, c->chunks, c->d_fse,
-                 c->d_fpe, c->d_fs,
-                 c->d_se, c->d_pe, c->d_fp, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
+    void *p[] = {c->cfill, c->fstart, c->rank, c->key, c->scan_tmp,
+                 c->d_se, c->d_pe, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
                  c->d_sten, c->d_stenD, c->d_cnt, c->d_wt, c->d_stats,
                  c->d_bbox, c->d_wd, c->d_gtab, c->d_head, c->d_queue, c->d_cnvt,
                  c->d_mock, c->d_mbase, c->d_bout, c->d_bstat, c->d_grad,
@@ -275,12 +270,6 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
   rc = upload(c, (void **) &c->d_s2edge, b->s.edge,
               sizeof(double) * (b->s.nbin + 1));
   if (rc) return rc;
-  if (b->s.ftab) {
-    rc = upload(c, (void **) &c->d_fs, b->s.ftab, sizeof(uint16_t) * b->s.nftab);
-    if (rc) return rc;
-    rc = upload(c, (void **) &c->d_fse, b->s.fedge, sizeof(float) * (b->s.nbin + 1));
-    if (rc) return rc;
-  }
   rc = upload(c, (void **) &c->d_se, b->s.etab,
               sizeof(float) * 2 * (b->s.netab + 2));
   if (rc) return rc;
@@ -293,18 +282,11 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
     rc = upload(c, (void **) &c->d_pedge, b->p.edge,
                 sizeof(double) * (b->p.nbin + 1));
     if (rc) return rc;
-    if (b->p.ftab) {
-      rc = upload(c, (void **) &c->d_fp, b->p.ftab,
-                  sizeof(uint16_t) * b->p.nftab);
-      if (rc) return rc;
-      rc = upload(c, (void **) &c->d_fpe, b->p.fedge,
-                  sizeof(float) * (b->p.nbin + 1));
-      if (rc) return rc;
-    }
   }
   CK(cudaMalloc((void **) &c->d_cnt, sizeof(unsigned long long) * b->ntot));
   CK(cudaMalloc((void **) &c->d_wt, sizeof(unsigned long long) * 2 * b->ntot));
-  CK(cudaMalloc((void **) &c->d_wd, sizeof(double) * b->ntot));
+  CK(cudaMalloc((void **) &c->d_wd,
+                sizeof(double) * b->ntot * fcfcg_gwd_copies(b->ntot)));
   CK(cudaMalloc((void **) &c->d_stats, sizeof(unsigned long long) * 8));
   CK(cudaMalloc((void **) &c->d_wpart,
                 sizeof(double) * (fcfcg_prep_partials() + 1)));
@@ -792,17 +774,11 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
 }
 
 /* Cell offsets whose cell pairs can hold a counted pair; half of them (with
- * the zero offset) for auto counts.  D = -offset * cell width.  The offsets
- * whose cell pairs lie entirely within the counting range (for cells up to
- * cw_far wide; NULL: the grid's) come first, nin of them: their candidates
- * need no distance test (the binning still checks every pair). */
+ * the zero offset) for auto counts.  D = -offset * cell width. */
 static int stencil_build(fcfcg_ctx *c, const grid_t *g, int isauto, int *sten,
-    float *stD, int *nsten, double *dmax, const double *cw_far, int *nin) {
+    float *stD, int *nsten, double *dmax) {
   const fcfcg_bins *b = &c->bins;
   const int box = (b->geometry == FCFCG_GEOM_BOX);
-  if (!cw_far) cw_far = g->cw;
-  unsigned char *ins = malloc(FCFCG_MAX_STENCIL);
-  if (!ins) return FCFCG_ERR_MEMORY;
   const double margin = 1 + 1e-9;
   int r[3];
   for (int d = 0; d < 3; d++) {
@@ -843,19 +819,8 @@ static int stencil_build(fcfcg_ctx *c, const grid_t *g, int isauto, int *sten,
         }
         if (cnt >= FCFCG_MAX_STENCIL) {
           set_err(c, "cell stencil too large");
-          free(ins);
           return FCFCG_ERR_UNSUPPORTED;
         }
-        /* every pair of the cell pair within range (outer limits only) */
-        double fz[3];
-        for (int d = 0; d < 3; d++) fz[d] = (abs(o[d]) + 1) * cw_far[d];
-        if (b->bintype == FCFCG_BIN_SPI && box)
-          ins[cnt] = (fz[0] * fz[0] + fz[1] * fz[1] < b->s.vmax) &&
-                     (fz[2] < b->p.vmax);
-        else
-          ins[cnt] = (fz[0] * fz[0] + fz[1] * fz[1] + fz[2] * fz[2] <
-                      ((b->bintype == FCFCG_BIN_SPI) ? b->s.vmax + b->p.vmax
-                                                     : b->s.vmax));
         sten[4 * cnt + 0] = ox;
         sten[4 * cnt + 1] = oy;
         sten[4 * cnt + 2] = oz;
@@ -868,32 +833,7 @@ static int stencil_build(fcfcg_ctx *c, const grid_t *g, int isauto, int *sten,
         stD[4 * cnt + 3] = 0;
         cnt++;
       }
-  /* the offsets within range first (stable) */
-  int *ts = malloc(sizeof(int) * 4 * (cnt ? cnt : 1));
-  float *td = malloc(sizeof(float) * 4 * (cnt ? cnt : 1));
-  if (!ts || !td) {
-    free(ts);
-    free(td);
-    free(ins);
-    return FCFCG_ERR_MEMORY;
-  }
-  int k = 0;
-  for (int pass = 1; pass >= 0; pass--)
-    for (int t = 0; t < cnt; t++)
-      if (ins[t] == pass) {
-        memcpy(ts + 4 * k, sten + 4 * t, sizeof(int) * 4);
-        memcpy(td + 4 * k, stD + 4 * t, sizeof(float) * 4);
-        k++;
-      }
-  int n1 = 0;
-  for (int t = 0; t < cnt; t++) n1 += ins[t];
-  memcpy(sten, ts, sizeof(int) * 4 * cnt);
-  memcpy(stD, td, sizeof(float) * 4 * cnt);
-  free(ts);
-  free(td);
-  free(ins);
   *nsten = cnt;
-  *nin = n1;
   return FCFCG_OK;
 }
 
@@ -965,7 +905,6 @@ static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   GROW(c->key, c->key_cap, sizeof(float) * 4 * m);
   size_t st = fcfcg_scan_tmp_len(nf + 1) + 16;
   GROW(c->scan_tmp, c->scan_cap, sizeof(uint32_t) * st);
-  GROW(c->cchunk, c->cchunk_cap, sizeof(uint32_t) * 2 * (nc + 1));
   return FCFCG_OK;
 }
 
@@ -990,23 +929,6 @@ static int slot_sort(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
                    fcfcg_grid_curve_bits(nc, n), &b));
   c->launches += n ? 7 : 5;
   return FCFCG_OK;
-}
-
-
-/* Are the s bins linear as FCFC's integer table sees them: rescaled edges
- * a + k d, integers, a >= 0, d >= 1? */
-static int linear_edges(const fcfcg_bins *b, double *a, double *d) {
-  if (b->bintype == FCFCG_BIN_SPI || b->s.tabtype != FCFCG_TAB_INT ||
-      b->s.nbin < 1)
-    return 0;
-  for (int k = 0; k <= b->s.nbin; k++) {
-    const double e = sqrt(b->s.edge[k]);
-    if (!(e == floor(e) && e * e == b->s.edge[k] && e < 1e6)) return 0;
-    if (k == 0) *a = e;
-    else if (k == 1) *d = e - *a;
-    else if (e != *a + k * *d) return 0;
-  }
-  return *d >= 1;
 }
 
 /* Lower end of cell c of a bit-pattern table (FP32 bits c << sh). */
@@ -1095,8 +1017,7 @@ static int etab_use(const fcfcg_axis *x, double w0, double w1, double vmax,
  * tl_ea s^2 + tl_eb; the edge's rounding and the difference's add 2 u v.
  */
 static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
-    double K2a, double hw, double dmax, double R, double dmr, double sabs,
-    fcfcg_launch *L) {
+    double K2a, double R, double dmr, double sabs, fcfcg_launch *L) {
   const fcfcg_bins *b = &c->bins;
   const int box = (b->geometry == FCFCG_GEOM_BOX);
   const int spi = (b->bintype == FCFCG_BIN_SPI);
@@ -1105,10 +1026,6 @@ static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
   const double nmu = b->nmu;
   double a = 0, d = 0;
   L->tlin = L->tplin = 0;
-  /* boxes' distance: the blocks' points, D, their difference and the
-   * extents, each rounded to u of at most hw, dmax or R */
-  L->box_eps = (float) (16 * u * (2 * hw + dmax + R));
-  L->near2 = (float) (1.52 * R * 1.52 * R);
   const double st = fmax(80 * dc, sqrt(40 * K0a));
   int rows = 1;
   L->hrow0 = 0;
@@ -1232,14 +1149,12 @@ static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
   return 0;
 }
 
-/* Rounding bounds of the FP32 path; returns 0 when the FP32 windows stay
- * below half a table unit, i.e. the FP32 path applies. */
 /*
- * Error windows of the FP32 kernels (every constant below is derived here;
- * the kernels' arithmetic is in count32.cuh bin_pair / lin_bin / mu_bin /
- * ftab_bin).  u = 2^-24, v = 2^-53; CUDA's documented maximum errors:
- * rsqrtf 2 ulp (relative <= 2^-22), __fdividef 2 ulp for divisors in
- * [2^-126, 2^126]; every other FP32 operation is correctly rounded.
+ * Rounding bounds of the tile kernel: the outer limits of s^2 (s_perp^2) and
+ * pi that no pair in range exceeds and, unless every pair is taken in FP64
+ * (f64), its windows (tile_bounds above); -1 where these exceed what it
+ * takes.  Every constant below is derived here; the arithmetic is in
+ * tile32.cuh.  u = 2^-24, v = 2^-53.
  *
  * 1. One separation component.  The reference forms dx_ref = fl(X_a (+
  *    shift) - X_b) from FP64 rescaled coordinates X.  The kernel forms
@@ -1256,31 +1171,14 @@ static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
  *    <= 2 sqrt(3) dc s + 3 dc^2 (Cauchy-Schwarz).  Survey pairs add the
  *    reference's S - t rounding: s_i (3v |x|^2), S (2v sabs), t (6v sabs),
  *    S - t exact (Sterbenz) or v s^2: <= 14 v sabs, carried as refs2 =
- *    64 v sabs.  Hence |s2 - s2_ref| <= E = K2' s^2 + K1 s + K0' with
- *      K2' = 3.0002 u + 3.0001 v   (taken as 4 u),
- *      K1  = 1.1 * 2 sqrt(3) dc    (2 sqrt(2) for s_perp^2; the 1.1 covers
- *            E's own FP32 evaluation and s = s2 rsqrtf(s2) against the
- *            exact root),
- *      K0' = 4 dc^2 + refs2.
- *    The kernel's table lookup of an FP32 value adds the rounding of its
- *    cell position, fl(v / w) (u v), and of 1 - fr against the window
- *    (u w / 2): the table windows use K2 = K2' + u, K0 = K0' + u w.
- * 3. mu in a box: FCFC's bin is floor(sqrt(Q)), Q = fl(fl(dz^2 / s^2)
- *    nmu^2) (the (int) cut and the mu table reduce to that); sqrt(Q) is
- *    within 1.5 v of nmu |dz_ref| / sqrt(s2_ref).  The kernel's q =
- *    fl(fl(nmu |dz|) rsqrtf(s2)) is within 3 2^-23 q (rsqrtf and two
- *    products) of nmu |dz| / sqrt(s2); |dz - dz_ref| <= dc contributes
- *    nmu dc / s, the root of s2 against s2_ref contributes q E / (2 s^2) =
- *    q (K2'/2 + K1 / (2 s) + K0' / (2 s^2)), q <= nmu.  So
- *      Eq = Q1 / s + Q2 q + Q0, Q1 = 1.25 nmu (dc + K1 / 2),
- *      Q2 = 1.25 (K2' / 2 + 2^-21 + 2 v + 2 u), Q0 = 1e-6 + u,
- *    the 1e-6 covering nmu K0' / (2 s^2) <= 5e-7 (pairs with s^2 < tiny =
- *    1e6 K0' nmu are rechecked whatever their value); the kernel tests
- *    the window's ends fl(q -+ Eq), each within u (q + Eq) of q -+ Eq
- *    (Eq < 1/2): the 2 u of Q2 and the u of Q0.
- * 4. Survey mu and pi^2 use the line of sight m = x_a + x_b.  The kernel
+ *    64 v sabs.  Hence |s2 - s2_ref| <= E = K2 s^2 + K1 s + K0 with
+ *      K2 = 3.0002 u + 3.0001 v   (taken as 4 u),
+ *      K1 = 1.1 * 2 sqrt(3) dc    (2 sqrt(2) for s_perp^2; the 1.1 covers
+ *           E's own evaluation at the FP32 s),
+ *      K0 = 4 dc^2 + refs2.
+ * 3. Survey mu and pi^2 use the line of sight m = x_a + x_b.  The kernel
  *    forms m = fl(fl(2 b + c2) + d) with b the neighbour's offset from the
- *    chunk cell's centre c and c2 = fl32(2 c) (the centre in FP64, rounded
+ *    block's cell centre c and c2 = fl32(2 c) (the centre in FP64, rounded
  *    once): per component |dm| <= 3 dc + 2u |c| + u (|m| + s) + u |m|,
  *    and with |x_a| <= (|m| + s) / 2, |c| <= |x_a| + hw:
  *      |dm| / |m| <= dmr = sqrt(3) (3 dc + 2 u (hw + R)) / |m| +
@@ -1288,29 +1186,22 @@ static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
  *    bounded by requiring |m| >= 2 R (pairs with |m|^2 < m2min = (2.01
  *    R)^2, i.e. next to the observer, are rechecked).  The direction m/|m|
  *    moves by <= 2 dmr.  The reference's dd = s1 - s2 = d.m carries
- *    6 v sabs, its S + t = |m|^2 carries 8 v sabs.
- *    mu: q = nmu |d.m| / (|m| s): d contributes nmu sqrt(3) dc / s (the
- *    length of d is E's business), m 2 nmu dmr, the kernel's roundings
- *    (dm 3u absolute, mm, the product, rsqrtf, two products: 8u relative)
- *    and the reference's (6 v nmu sabs / (2 R s), 4 v sabs / |m|^2):
- *      Q1 = 1.25 nmu (sqrt(3) dc + K1 / 2 + 3 v sabs / R),
- *      Q2 = 1.25 (K2' / 2 + 8 u + v sabs / R^2 + 2 v + 2 u),
- *      Q0 = 1.25 nmu (3 u + 2 dmr) + 1e-6 + u (the ends, as in a box).
- *    pi^2 = (d.m)^2 / |m|^2: |d pi| <= sqrt(3) dc + s (2 dmr + 3u), so
+ *    6 v sabs, its S + t = |m|^2 carries 8 v sabs.  pi^2 = (d.m)^2 /
+ *    |m|^2: |d pi| <= sqrt(3) dc + s (2 dmr + 3u), so its error is
  *      Ep = P2 s^2 + P1 s + P0, P1 = 1.25 (2 sqrt(3) dc + 6 v sabs / R),
- *      P2 = 1.25 (4 dmr + 14 u + 2 v sabs / R^2 + 2 v + u) (dm^2, mm and
- *      __fdividef: 8u relative; the table position: u),
- *      P0 = 1.25 (6 dc^2 + u w_pi) + 1e-12.
+ *      P2 = 1.25 (4 dmr + 15 u + 2 v sabs / R^2 + 2 v), P0 = 7.5 dc^2 +
+ *      1e-12;
  *    s_perp^2 = s^2 - pi^2 takes E + Ep.
- * 5. pi in a box is |dz|: P0 = 1.25 (dc + u w_pi).
+ * 4. pi in a box is |dz|: Ep = 1.25 dc.
  * Every constant carries a factor >= 1.1 over its derived value; the
  * near-edge tests place pairs on every bin edge and check that each one is
  * rechecked.
  */
 static int fp32_bounds(const fcfcg_ctx *c, const grid_t *g, double dmax,
-    const slot_t *A, const slot_t *B, int tile, fcfcg_launch *L) {
+    const slot_t *A, const slot_t *B, int f64, fcfcg_launch *L) {
   const fcfcg_bins *b = &c->bins;
   const int box = (b->geometry == FCFCG_GEOM_BOX);
+  const int spi = (b->bintype == FCFCG_BIN_SPI);
   const double u = ldexp(1.0, -24), v = ldexp(1.0, -53);
   double hw = 0;
   for (int d = 0; d < 3; d++) hw = fmax(hw, 0.5 * g->cw[d] * (1 + 1e-6));
@@ -1322,175 +1213,66 @@ static int fp32_bounds(const fcfcg_ctx *c, const grid_t *g, double dmax,
                     1e-300;
   const double refs2 = box ? 0 : 64 * v * sabs;
   const double s3 = sqrt(3.0);
-  /* cell widths of the FP32 tables (uniform ones; 0 for bit patterns) */
-  const double ws = b->s.ftab && !b->s.flog ? ldexp(1.0, b->s.fshift) : 0;
-  const double wp = (b->bintype == FCFCG_BIN_SPI && b->p.ftab && !b->p.flog)
-                        ? ldexp(1.0, b->p.fshift) : 0;
-  const double K2a = 4 * u, K0a = 4 * dc * dc + refs2;   /* arithmetic */
-  const double K1 = 1.1 * 2 * ((b->bintype == FCFCG_BIN_SPI && box)
-                                   ? sqrt(2.0) : s3) * dc;
-  L->K2 = (float) (K2a + u);
-  L->K1 = (float) K1;
-  L->K0 = (float) (K0a + u * ws + 1e-30);
-  double nmu = b->nmu;
-  L->fnmu = (float) nmu;
+  const double K2 = 4 * u, K0 = 4 * dc * dc + refs2;
+  const double K1 = 1.1 * 2 * (spi && box ? sqrt(2.0) : s3) * dc;
+  L->fnmu = (float) b->nmu;
   /* survey: relative error of the line of sight for |m| >= 2 R */
   const double dmr = s3 * (3 * dc + 2 * u * (hw + R)) / (2 * R) +
                      3.0001 * s3 * u;
   L->m2min = box ? 0.f : (float) (2.01 * R * 2.01 * R);
-  if (box) {
-    L->Q1 = (float) (1.25 * nmu * (dc + 0.5 * K1));
-    L->Q2 = (float) (1.25 * (0.5 * K2a + ldexp(1.0, -21) + 2 * v + 2 * u));
-    L->Q0 = (float) (1e-6 + u);
-  } else {
-    L->Q1 = (float) (1.25 * nmu * (s3 * dc + 0.5 * K1 + 3 * v * sabs / R));
-    L->Q2 = (float) (1.25 * (0.5 * K2a + 8 * u + v * sabs / (R * R) + 2 * v +
-                             2 * u));
-    L->Q0 = (float) (1.25 * nmu * (3 * u + 2 * dmr) + 1e-6 + u);
-  }
-  double tiny = 1e6 * K0a * (nmu > 1 ? nmu : 1);
-  if (tiny < 1e-20) tiny = 1e-20;
-  L->tiny = (float) tiny;
-  /*
-   * Linear s bins as FCFC's integer table sees them: rescaled edges
-   * e_k = a + k d with integers a >= 0, d >= 1, so that the table's edges
-   * e_k^2 are integers and FCFC's bin is the k with e_k <= sqrt(s2_ref) <
-   * e_k+1.  The kernel then bins s itself: k = floor(t), t = (s - a) / d.
-   * Window of t, for a pair with s^2 >= tiny (smaller ones are rechecked):
-   *   |s_32 - sqrt(s2_ref)| <= eta s_32 (1 + 2 eta) + E(s) / sqrt(s2_32),
-   *   with eta = 2^-22 + 2^-24 (s_32 = fl(s2 rsqrtf(s2)): rsqrtf within 2
-   *   ulp, CUDA's documented bound, then the product's rounding), E(s) =
-   *   K2 s^2 + K1 s + K0 the bound on |s2_32 - s2_ref| above, and
-   *   sqrt(s2_32) >= s_32 / (1 + eta), K0 / s <= K0 / sqrt(tiny);
-   *   t = fl(fma(s, fl(1 / d), fl(-a / d))) adds u (s + a) / d + u |t|,
-   *   |t| <= ns + 1 where the window matters; the kernel tests the ends
-   *   fl(t -+ W), each within u (|t| + W) <= u (ns + 2) of t -+ W (W <
-   *   0.45), plus 3 u of slack.  The factor 1.01 covers W's own FP32
-   *   evaluation.
-   */
-  L->slin = 0;
-  {
-    double a = 0, d = 0;
-    if (linear_edges(b, &a, &d)) {
-      const double eta = ldexp(1.0, -22) + ldexp(1.0, -24);
-      const double uu = ldexp(1.0, -24);
-      const double A = 1.01 * (eta * (1 + 2 * eta) + (double) L->K2 * (1 + eta)
-                               + uu) / d;
-      const double Bw = 1.01 * (((double) L->K1 + (double) L->K0 /
-                                 sqrt((double) L->tiny)) * (1 + eta) / d +
-                                uu * a / d + uu * (b->s.nbin + 1) +
-                                uu * (b->s.nbin + 2) + 3 * uu);
-      const double smax = a + d * b->s.nbin;
-      if (A * (smax + d) + Bw < 0.45) {
-        L->slin = 1;
-        L->lin_inv = (float) (1.0 / d);
-        L->lin_off = (float) (-a / d);
-        L->lin_A = (float) A;
-        if ((double) L->lin_A < A) L->lin_A = nextafterf(L->lin_A, INFINITY);
-        L->lin_B = (float) Bw;
-        if ((double) L->lin_B < Bw) L->lin_B = nextafterf(L->lin_B, INFINITY);
-        L->lin_k0 = b->s.min0 ? 0 : -1;
-      }
-    }
-  }
-  /* worst windows at the top of the ranges */
-  double smax2 = b->s.vmax;
-  double Es = L->K2 * smax2 + L->K1 * sqrt(smax2) + L->K0;
+  /* boxes' distance: the blocks' points, D, their difference and the
+   * extents, each rounded to u of at most hw, dmax or R */
+  L->box_eps = (float) (16 * u * (2 * hw + dmax + R));
+  L->near2 = (float) (1.52 * R * 1.52 * R);
+  /* the outer limits, with the errors at the top of the ranges */
+  const double r2 = b->s.vmax + (spi && !box ? b->p.vmax : 0);
+  const double Es = K2 * r2 + K1 * sqrt(r2) + K0;
   double Ep = 0;
-  if (b->bintype == FCFCG_BIN_SPI) {
-    if (box) {
-      L->P0 = (float) (1.25 * (dc + u * wp));
-      L->P1 = L->P2 = 0;
-      Ep = L->P0;
-      L->p_lim = (float) (b->p.vmax + Ep + 1e-6 * (1 + b->p.vmax));
-      L->s_lim = (float) (smax2 + Es + 1e-6 * (1 + smax2));
-    } else {
-      double r2 = b->s.vmax + b->p.vmax;
-      L->P0 = (float) (1.25 * (6 * dc * dc + u * wp) + 1e-12);
-      L->P1 = (float) (1.25 * (2 * s3 * dc + 6 * v * sabs / R));
-      L->P2 = (float) (1.25 * (4 * dmr + 15 * u + 2 * v * sabs / (R * R) +
-                               2 * v));
-      Ep = L->P2 * r2 + L->P1 * sqrt(r2) + L->P0;
-      Es = L->K2 * r2 + L->K1 * sqrt(r2) + L->K0 + Ep;
-      L->s_lim = (float) (r2 + Es + 1e-6 * (1 + r2));
-      L->p_lim = 0;
-      /* line-of-sight prefilter.  With m = x_a + x_b = 2 x_b + d,
-       * pi = |d.m| / |m| and |m| <= 2 |x_b| + s, pi < pi_max implies
-       *   |d.u_b| < pi_max + (pi_max s + s^2) / (2 |x_b|),
-       * and s <= Rs, the outer range.  The constants carry a factor
-       * 1 + 2^-8 and an absolute slack far above the FP32 rounding of d,
-       * u_b and |x_b| (below 1e-5 relative where the test applies,
-       * |x_b| >= Rs) */
-      const double pm = sqrt(b->p.vmax), Rs = sqrt((double) L->s_lim);
-      const double f = 1 + ldexp(1.0, -8);
-      L->los_p = (float) (pm * f + ldexp(Rs, -12) + 1e-6);
-      L->los_pr = (float) (0.5 * f * pm * Rs);
-      L->los_h = (float) (0.5 * f);
-      L->los_r2min = (float) (Rs * Rs);
-    }
-  } else {
-    L->s_lim = (float) (smax2 + Es + 1e-6 * (1 + smax2));
+  if (spi && box) {
+    Ep = 1.25 * dc;
+    L->p_lim = (float) (b->p.vmax + Ep + 1e-6 * (1 + b->p.vmax));
+    Ep = 0;
+  } else if (spi) {
+    const double P0 = 1.25 * 6 * dc * dc + 1e-12;
+    const double P1 = 1.25 * (2 * s3 * dc + 6 * v * sabs / R);
+    const double P2 = 1.25 * (4 * dmr + 15 * u + 2 * v * sabs / (R * R) +
+                              2 * v);
+    Ep = P2 * r2 + P1 * sqrt(r2) + P0;
   }
-  L->Emax = (float) (Es * 1.01);
-  if (tile)
-    return tile_bounds(c, dc, K1, K0a, K2a, hw, dmax, R, dmr, sabs, L);
-  if (b->s.nbin > FCFCG_FTAB_MAXBIN || !b->s.ftab) return -1;
-  if (b->bintype == FCFCG_BIN_SPI &&
-      (b->p.nbin > FCFCG_FTAB_MAXBIN || !b->p.ftab))
-    return -1;
-  /* windows below half a table cell: over the whole uniform tables; for a
-   * bit-pattern table, whose cells shrink with the value, from a threshold
-   * up -- values below it are sent to the recheck */
-  L->fsamb = L->fpamb = -1.f;
-  if (b->s.flog) {
-    /* the window the s-axis lookups use at value v (an upper bound): with
-     * a bit-pattern table every kernel variant takes it per pair (only
-     * boxes get such tables, so p2, for a survey's s_perp^2 = s^2 - pi^2,
-     * is 0 today) */
-    const double p2 = (b->bintype == FCFCG_BIN_SPI && !box) ? b->p.vmax : 0;
-    double amb = -1;
-    for (long c = b->s.nftab - 1; c >= 0; c--) {
-      const double x0 = ftab_cell_value(b->s.foff + c, b->s.flog);
-      const double x1 = ftab_cell_value(b->s.foff + c + 1, b->s.flog);
-      const double v = x1 + p2;
-      double W = (double) L->K2 * v + (double) L->K1 * sqrt(v) + (double) L->K0;
-      if (p2 > 0)
-        W += (double) L->P2 * v + (double) L->P1 * sqrt(v) + (double) L->P0;
-      W *= 1.01;
-      if (!(W < 0.45 * (x1 - x0))) {
-        amb = x1;
-        break;
-      }
-    }
-    L->fsamb = (float) amb;
-    if (amb > 0 && (double) L->fsamb < amb)   /* round up: still ambiguous */
-      L->fsamb = nextafterf(L->fsamb, INFINITY);
-  } else if (!(Es < 0.45 * ldexp(1.0, b->s.fshift))) {
-    return -1;
+  L->s_lim = (float) (r2 + Es + Ep + 1e-6 * (1 + r2));
+  if (spi && !box) {
+    /* line-of-sight prefilter.  With m = x_a + x_b = 2 x_b + d,
+     * pi = |d.m| / |m| and |m| <= 2 |x_b| + s, pi < pi_max implies
+     *   |d.u_b| < pi_max + (pi_max s + s^2) / (2 |x_b|),
+     * and s <= Rs, the outer range.  The constants carry a factor
+     * 1 + 2^-8 and an absolute slack far above the FP32 rounding of d,
+     * u_b and |x_b| (below 1e-5 relative where the test applies,
+     * |x_b| >= Rs) */
+    const double pm = sqrt(b->p.vmax), Rs = sqrt((double) L->s_lim);
+    const double f = 1 + ldexp(1.0, -8);
+    L->los_p = (float) (pm * f + ldexp(Rs, -12) + 1e-6);
+    L->los_pr = (float) (0.5 * f * pm * Rs);
+    L->los_h = (float) (0.5 * f);
+    L->los_r2min = (float) (Rs * Rs);
   }
-  if (b->bintype == FCFCG_BIN_SPI) {
-    if (b->p.flog) {
-      double amb = -1;
-      for (long c = b->p.nftab - 1; c >= 0; c--) {
-        const double x0 = ftab_cell_value(b->p.foff + c, b->p.flog);
-        const double x1 = ftab_cell_value(b->p.foff + c + 1, b->p.flog);
-        if (!(Ep * 1.01 < 0.45 * (x1 - x0))) {
-          amb = x1;
-          break;
-        }
-      }
-      L->fpamb = (float) amb;
-      if (amb > 0 && (double) L->fpamb < amb)
-        L->fpamb = nextafterf(L->fpamb, INFINITY);
-    } else if (!(Ep < 0.45 * ldexp(1.0, b->p.fshift))) {
-      return -1;
-    }
+  if (!f64)
+    return tile_bounds(c, dc, K1, K0, K2, R, dmr, sabs, L);
+  if (!(R > 1e-12 && R < 1e12 && hw < 1e12 && dmax < 1e12)) {
+    /* squares that FP32 cannot hold: no pair is left out by them */
+    L->s_lim = L->p_lim = L->box_eps = INFINITY;
   }
-  /* Values beyond either end of an FP32 table need no check: a table runs
-   * from at least one cell below its lowest edge to at least one cell above
-   * its highest (fcfcg_axis_ftab), so an FP32 value outside it is more than
-   * a cell, hence more than its window, away from every edge. */
+  /* the shared histogram is the bins */
+  L->hcols = b->ns;
+  L->hcol0 = L->hrow0 = 0;
+  L->hrows = (int) (b->ntot / b->ns);
+  L->hlen = (int) b->ntot;
   return 0;
+}
+
+/* The candidate queue of fcfcg_stats: the one set, or the largest.  (The tile
+ * kernel has none; the counts never depended on it.) */
+static int warp_queue(const fcfcg_ctx *c) {
+  return c->qwarp_force ? (int) c->qwarp_force : 1024;
 }
 
 /* Launch fields of a sorted catalogue. */
@@ -1536,7 +1318,6 @@ static void launch_bins(const fcfcg_ctx *c, fcfcg_launch *L) {
     L->pmax = b->p.vmax;
     L->pmin0 = b->p.min0;
   }
-  L->fixF = FCFCG_FIX_F;
   L->gcnt = c->d_cnt;
   L->gwt = c->d_wt;
   L->gwd = c->d_wd;
@@ -1594,10 +1375,8 @@ typedef struct {
   int hwa, hwb;
   int isauto, withwt, prec;
   grid_t g;
-  int tile;                      /* the tile kernel counts */
-  int nsten, nin;                /* stencil entries, those within range */
+  int nsten;                     /* stencil entries */
   uint32_t ncell;
-  size_t st;                     /* scan scratch length of the chunk list */
   fcfcg_launch L;                /* stencil pointers: set by the caller */
 } count_plan;
 
@@ -1635,39 +1414,27 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
    * chunk kernels' finer cells where the FP32 windows do not fit; then the
    * all-FP64 kernel on the latter. */
   int prec = precision;
-  const int tile = (precision == FCFCG_PREC_FP32_RECHECK);
   size_t tabbytes = 0, stage = 0;
-  for (int att = tile ? 0 : 2; ; att++) {
+  for (int att = 0; ; att++) {
     if ((rc = grid_setup(c, g, A, B, att < 2, att == 0))) return rc;
     double dmax = 0;
-    if ((rc = stencil_build(c, g, isauto, sten, stD, &P->nsten, &dmax, NULL,
-                            &P->nin)))
+    if ((rc = stencil_build(c, g, isauto, sten, stD, &P->nsten, &dmax)))
       return rc;
     memset(L, 0, sizeof *L);
-    if (prec == FCFCG_PREC_FP64) break;
-    if (!fp32_bounds(c, g, dmax, A, B, tile, L)) {
-      tabbytes = fcfcg_k_tile32_tab(L);
-      stage = fcfcg_k_tile32_stage(adj ? 2 : withwt);
+    const int f64 = (prec == FCFCG_PREC_FP64);
+    if (!fp32_bounds(c, g, dmax, A, B, f64, L)) {
+      tabbytes = f64 ? 0 : fcfcg_k_tile32_tab(L);
+      stage = fcfcg_k_tile32_stage(f64 ? 3 : adj ? 2 : withwt);
       if (tabbytes + stage <= 200 * 1024) break;
     }
     if (att >= 2) {
       prec = FCFCG_PREC_FP64;
-      tabbytes = stage = 0;
-      break;
+      att = -1;                  /* the first grid again, in FP64 */
     }
   }
-  P->tile = (tile && prec == FCFCG_PREC_FP32_RECHECK);
   if ((rc = slot_reserve(c, A, g))) return rc;
   if (B != A && (rc = slot_reserve(c, B, g))) return rc;
   P->ncell = (uint32_t) ((size_t) g->n[0] * g->n[1] * g->n[2]);
-  GROW(c->cchunk, c->cchunk_cap,
-       sizeof(uint32_t) * 2 * ((size_t) P->ncell + 1));
-  P->st = fcfcg_scan_tmp_len(P->ncell + 1) + 16;
-  GROW(c->scan_tmp, c->scan_cap, sizeof(uint32_t) * P->st);
-  if (!P->tile) {
-    size_t maxchunk = A->n / FCFCG_CHUNK + P->ncell + 1;
-    GROW(c->chunks, c->chunk_cap, sizeof(uint32_t) * 4 * maxchunk);
-  }
   L->geometry = b->geometry;
   L->bintype = b->bintype;
   L->isauto = isauto;
@@ -1681,28 +1448,18 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
     L->lof[d] = (float) g->lo[d];
   }
   L->nsten = P->nsten;
-  L->nin = P->nin;
   L->tzero = -1;
   for (int t = 0; t < P->nsten; t++)
     if (!sten[4 * t] && !sten[4 * t + 1] && !sten[4 * t + 2]) L->tzero = t;
-  L->chunks = P->tile ? NULL : c->chunks;
   L->chunk_head = c->d_head;
-  /* the number of blocks, or of chunks: k_chunks leaves it after the ncell
-   * + 1 counts and ncell offsets in cchunk */
   L->nblk_dev = A->bstart + P->ncell;
-  L->nchunk_dev = P->tile ? L->nblk_dev
-                          : c->cchunk + ((size_t) P->ncell + 1) + P->ncell;
   launch_cat(&L->A, A);
   launch_cat(&L->B, B);
   launch_bins(c, L);
-  const size_t hbytes = P->tile ? fcfcg_k_tile32_hist(L->hlen, withwt)
-                                : (size_t) b->ntot * (withwt ? 8 : 4);
+  const size_t hbytes = fcfcg_k_tile32_hist(L->hlen, withwt);
   L->hist_smem = (tabbytes + stage + hbytes <= 200 * 1024);
   L->pshift = tile_parts(A->n, P->ncell, c->nsm);
   L->hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
-  L->qwarp = c->qwarp_force ? c->qwarp_force
-      : ((c->tuned_q && c->tuned_q_key == g->key && c->tuned_q_wt == withwt)
-             ? c->tuned_q : 0);
   P->prec = prec;
   return FCFCG_OK;
 }
@@ -1719,28 +1476,21 @@ static int count_launch(fcfcg_ctx *c, const count_plan *P, int sort_a,
   if (timed) CK(cudaEventRecord(c->ev[0], c->stream));
   if (sort_a && (rc = slot_sort(c, P->A, &P->g))) return rc;
   if (sort_b && P->B != P->A && (rc = slot_sort(c, P->B, &P->g))) return rc;
-  /* work chunks: 64 points per CTA in the FP32 kernel, 32 per warp in the
-   * FP64 kernel */
-  if (!P->tile) {
-    const uint32_t clen = (P->prec == FCFCG_PREC_FP32_RECHECK)
-                              ? FCFCG_CHUNK32 : FCFCG_CHUNK;
-    CKK(fcfcg_k_chunks(c->stream, P->A->cstart, P->ncell, clen, c->cchunk,
-                       c->scan_tmp, P->st, c->chunks, NULL, NULL, 0));
-    c->launches += 5;
-  }
   if (timed) CK(cudaEventRecord(c->ev[1], c->stream));
   CK(cudaMemsetAsync(c->d_cnt, 0, sizeof(unsigned long long) * b->ntot,
                      c->stream));
   CK(cudaMemsetAsync(c->d_wt, 0, sizeof(unsigned long long) * 2 * b->ntot,
                      c->stream));
-  if (!L->adjoint)
-    CK(cudaMemsetAsync(c->d_wd, 0, sizeof(double) * b->ntot, c->stream));
+  if (L->withwt && !L->adjoint && P->prec == FCFCG_PREC_FP64)
+    CK(cudaMemsetAsync(c->d_wd, 0,
+                       sizeof(double) * b->ntot * fcfcg_gwd_copies(b->ntot),
+                       c->stream));
   CK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * 4,
                      c->stream));
   CK(cudaMemsetAsync(c->d_head, 0, sizeof(uint32_t) * 4, c->stream));
   if (timed) CK(cudaEventRecord(c->ev[2], c->stream));
   size_t smem = 0;
-  CKK(fcfcg_k_count(c->stream, L, P->prec, c->nsm, &smem, &c->last_qwarp));
+  CKK(fcfcg_k_count(c->stream, L, P->prec, c->nsm, &smem));
   c->launches += 1;
   if (timed) CK(cudaEventRecord(c->ev[3], c->stream));
   if (P->prec == FCFCG_PREC_FP32_RECHECK) {
@@ -1764,9 +1514,9 @@ static int count_launch(fcfcg_ctx *c, const count_plan *P, int sort_a,
   if (stats) {
     CK(cudaMemcpyAsync(stats, c->d_stats, sizeof(unsigned long long) * 4,
                        cudaMemcpyDeviceToHost, c->stream));
-    /* the chunk count (32 bits) into the low half of the last word */
+    /* the block count (32 bits) into the low half of the last word */
     stats[4] = 0;
-    CK(cudaMemcpyAsync(stats + 4, L->nchunk_dev, sizeof(uint32_t),
+    CK(cudaMemcpyAsync(stats + 4, L->nblk_dev, sizeof(uint32_t),
                        cudaMemcpyDeviceToHost, c->stream));
   }
   return FCFCG_OK;
@@ -1781,7 +1531,7 @@ static void count_finish(fcfcg_ctx *c, const count_plan *P, const void *res,
   if (P->withwt && P->prec == FCFCG_PREC_FP64) {
     memcpy(wcnt, res, sizeof(double) * b->ntot);
   } else if (P->withwt) {
-    const int ex = P->A->wexp + P->B->wexp - P->L.fixF;
+    const int ex = P->A->wexp + P->B->wexp - FCFCG_FIX_F;
     for (long i = 0; i < b->ntot; i++) {
       __int128 v = (__int128) (((unsigned __int128) hres[2 * i + 1] << 64) |
                                (unsigned __int128) hres[2 * i]);
@@ -1800,7 +1550,7 @@ static void count_finish(fcfcg_ctx *c, const count_plan *P, const void *res,
   o->nstencil = P->nsten;
   o->nchunks = (uint32_t) stats[4];
   o->precision_used = P->prec;
-  o->warp_queue = P->prec == FCFCG_PREC_FP32_RECHECK ? (int) c->last_qwarp : 0;
+  o->warp_queue = P->prec == FCFCG_PREC_FP32_RECHECK ? warp_queue(c) : 0;
   o->launches = c->launches;
 }
 
@@ -1897,7 +1647,7 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
     }
   }
   const size_t rbytes = sizeof(unsigned long long) * (2 * b->ntot + STAT_WORDS);
-  const size_t gbytes = (adj && P.tile) ? sizeof(int) * 2 * ((size_t) L->hlen + 32)
+  const size_t gbytes = (adj && P.prec == FCFCG_PREC_FP32_RECHECK) ? sizeof(int) * 2 * ((size_t) L->hlen + 32)
                                         : 0;
   if ((rc = ensure_pinned(c, rbytes + gbytes))) return rc;
   unsigned long long *hres = (unsigned long long *) c->h_pinned;
@@ -1949,7 +1699,7 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
     o->cells_per_smax = P.g.k;
     o->nchunks = (uint32_t) hstats[4];
     o->precision_used = P.prec;
-    o->warp_queue = P.prec == FCFCG_PREC_FP32_RECHECK ? (int) c->last_qwarp : 0;
+    o->warp_queue = P.prec == FCFCG_PREC_FP32_RECHECK ? warp_queue(c) : 0;
     o->launches = c->launches;
   } else {
     count_finish(c, &P, hres, hstats, icnt, wcnt);
@@ -2248,29 +1998,6 @@ int fcfcg_autotune(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
       bk = k;
     }
   }
-  /* then the warp queue at that refinement */
-  uint32_t bq = 0;
-  const uint32_t saved_q = c->qwarp_force;
-  if (rc == FCFCG_OK && bk) {
-    c->kcell = bk;
-    static const uint32_t qs[3] = {1024, 512, 256};
-    double qms = 1e300;
-    for (int i = 0; i < 3 && rc == FCFCG_OK; i++) {
-      c->qwarp_force = qs[i];
-      double ms = 0;
-      for (int rep = 0; rep < 2 && rc == FCFCG_OK; rep++) {
-        rc = fcfcg_count(c, sa, sb, isauto, withwt, FCFCG_PREC_FP32_RECHECK,
-                         ic, wc);
-        ms = c->stats.ms_count + c->stats.ms_recheck;
-      }
-      if (rc == FCFCG_OK && ms < qms) {
-        qms = ms;
-        bq = qs[i];
-      }
-    }
-    if (qms < bms) bms = qms;
-  }
-  c->qwarp_force = saved_q;
   c->kcell = saved;
   if (rc == FCFCG_OK && bk) {
     /* the key of this catalogue pair, as the grid set-up computes it */
@@ -2280,9 +2007,6 @@ int fcfcg_autotune(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
     key = g.key;
     c->tuned_k = bk;
     c->tuned_key = key;
-    c->tuned_q = bq;
-    c->tuned_q_key = key;
-    c->tuned_q_wt = withwt;
   }
   free(ic);
   free(wc);
@@ -2600,7 +2324,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   }
   fcfcg_launch L;
   grid_t gmin, gmax;
-  int nsten = 0, nin = 0, prec = FCFCG_PREC_FP32_RECHECK;
+  int nsten = 0, prec = FCFCG_PREC_FP32_RECHECK;
   size_t cells = 0;
   S->s2abs = 0;
   S->wexp = 0;
@@ -2663,8 +2387,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
       free(hbase);
       goto out;
     }
-    if ((rc = stencil_build(c, &gmin, 1, c->sten, c->stD, &nsten, &dmin,
-                            gmax.cw, &nin))) {
+    if ((rc = stencil_build(c, &gmin, 1, c->sten, c->stD, &nsten, &dmin))) {
       free(wexp);
       free(hbase);
       goto out;
@@ -2675,7 +2398,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
         dmax = fmax(dmax, fabs((double) c->sten[4 * t + d]) * gmax.cw[d]);
     S->xabs = xabs;
     memset(&L, 0, sizeof L);
-    if (!fp32_bounds(c, &gmax, dmax, S, S, 1, &L) &&
+    if (!fp32_bounds(c, &gmax, dmax, S, S, 0, &L) &&
         fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt) <= 200 * 1024)
       break;
     if (att >= 2) {
@@ -2806,7 +2529,6 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   L.nblk_dev = S->bstart + cells;
   L.hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
   L.nsten = nsten;
-  L.nin = nin;
   L.tzero = -1;
   for (int t = 0; t < nsten; t++)
     if (!c->sten[4 * t] && !c->sten[4 * t + 1] && !c->sten[4 * t + 2])
@@ -2831,10 +2553,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   BCK(cudaMemsetAsync(c->d_head, 0, sizeof(uint32_t) * 4, c->stream));
   BCK(cudaEventRecord(c->ev[2], c->stream));
   size_t smem = 0;
-  L.qwarp = c->qwarp_force ? c->qwarp_force
-      : ((c->tuned_q && c->tuned_q_key == key && c->tuned_q_wt == withwt)
-             ? c->tuned_q : 0);
-  BCKK(fcfcg_k_count(c->stream, &L, prec, c->nsm, &smem, &c->last_qwarp));
+  BCKK(fcfcg_k_count(c->stream, &L, prec, c->nsm, &smem));
   c->launches += 1;
   BCK(cudaEventRecord(c->ev[3], c->stream));
   unsigned long long nq = 0;
@@ -2872,7 +2591,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
       if (J->status) continue;
       const unsigned long long *r = hres + per * a;
       if (withwt) {
-        const int ex = 2 * wexp[a] - L.fixF;
+        const int ex = 2 * wexp[a] - FCFCG_FIX_F;
         for (long i = 0; i < b->ntot; i++) {
           __int128 v = (__int128) (((unsigned __int128) r[2 * i + 1] << 64) |
                                    (unsigned __int128) r[2 * i]);
@@ -2901,7 +2620,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
     o->nstencil = nsten;
     o->nchunks = nblk;
     o->precision_used = prec;
-    o->warp_queue = prec == FCFCG_PREC_FP32_RECHECK ? (int) c->last_qwarp : 0;
+    o->warp_queue = prec == FCFCG_PREC_FP32_RECHECK ? warp_queue(c) : 0;
     o->launches = c->launches;
     if (hstats[3]) queue_grow(c, hstats[2] + hstats[2] / 4);
   }
@@ -2940,29 +2659,6 @@ int fcfcg_autotune_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs,
       bk = k;
     }
   }
-  /* then the warp queue at that refinement */
-  uint32_t bq = 0;
-  const uint32_t saved_q = c->qwarp_force;
-  if (rc == FCFCG_OK && bk) {
-    c->kcell = bk;
-    static const uint32_t qs[3] = {1024, 512, 256};
-    double qms = 1e300;
-    for (int i = 0; i < 3 && rc == FCFCG_OK; i++) {
-      c->qwarp_force = qs[i];
-      double ms = 0;
-      for (int rep = 0; rep < 2 && rc == FCFCG_OK; rep++) {
-        rc = fcfcg_count_batch(c, jobs, njobs, withwt,
-                               FCFCG_PREC_FP32_RECHECK, on_device);
-        ms = c->stats.ms_count + c->stats.ms_recheck;
-      }
-      if (rc == FCFCG_OK && ms > 0 && ms < qms) {
-        qms = ms;
-        bq = qs[i];
-      }
-    }
-    if (qms < bms) bms = qms;
-  }
-  c->qwarp_force = saved_q;
   c->kcell = saved;
   if (rc == FCFCG_OK && bk) {
     /* the key fcfcg_count_batch computes for this batch */
@@ -2979,9 +2675,6 @@ int fcfcg_autotune_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs,
     }
     c->tuned_k = bk;
     c->tuned_key = tune_key(nsum / (vol > 0 ? vol : 1), gr.reach) + 1000;
-    c->tuned_q = bq;
-    c->tuned_q_key = c->tuned_key;
-    c->tuned_q_wt = withwt;
   }
   if (best_k) *best_k = bk;
   if (best_ms) *best_ms = bms;

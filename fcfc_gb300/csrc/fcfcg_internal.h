@@ -15,8 +15,6 @@ extern "C" {
 #endif
 
 #define FCFCG_MAX_SLOT 8
-#define FCFCG_CHUNK 32            /* chunk length of the FP64 kernel */
-#define FCFCG_CHUNK32 64          /* chunk length of the FP32 kernel */
 #define FCFCG_MAX_STENCIL 4096
 #define FCFCG_FIX_F 51            /* fractional bits of a weight product */
 /* FP32 edge-window tables: one uint16 per cell of width w = 2^-shift units
@@ -121,14 +119,8 @@ typedef struct {
   float cwf[3], lof[3];
   /* stencil: nsten entries of int4 (ox, oy, oz, 0) and float4 (-o * cw) */
   int nsten;
-  int nin;          /* the first nin entries: cell pairs within range */
   const int *sten;
   const float *stenD;
-  /* chunks: uint4 (cell, first sorted index, count, 0); their number is
-   * nchunk, or *nchunk_dev when set (written by an earlier launch) */
-  uint32_t nchunk;
-  const uint32_t *nchunk_dev;
-  const uint32_t *chunks;
   uint32_t *chunk_head;
   /* tile kernel: the number of A blocks (device), log2 of the parts a
    * block's tiles are dealt to, slack of the block box distance, and for a
@@ -141,27 +133,11 @@ typedef struct {
   /* bins */
   int ns, nmu, np;
   long ntot;
-  /* FP32 tables (copied to shared memory) */
-  const uint16_t *fs, *fp;
-  int nfs, nfp, fsoff, fpoff;
-  float fsinv, fpinv;          /* 1 / cell width of the FP32 tables, or
-                                  2^-flog for bit-pattern tables */
-  int fslog, fplog;            /* the axes' flog (0: uniform cells) */
-  float fsamb, fpamb;          /* bit-pattern tables: values below are
-                                  ambiguous (the window exceeds the cell) */
-  const float *fse, *fpe;      /* FP32 edges (nbin + 1 each) */
-  int nsb, npb;                /* bins of the s and pi axes */
   float s_lim, p_lim;          /* values at/above: out of range for sure */
   /* survey (s_perp, pi): a pair with |d.u_b| >= los_p + (los_pr + los_h
    * s^2) / |x_b| (u_b = x_b / |x_b|) has pi >= pi_max for sure; the test
    * is skipped for |x_b|^2 <= los_r2min */
   float los_p, los_pr, los_h, los_r2min;
-  float K0, K1, K2;            /* E(s^2) = K2 s^2 + K1 s + K0 */
-  /* linear s bins (slin): t = s lin_inv + lin_off, bin floor(t), window
-   * lin_A s + lin_B in units of t; lin_k0: bins above it have a lower edge
-   * that is a boundary */
-  int slin, lin_k0;
-  float lin_inv, lin_off, lin_A, lin_B;
   /* the tile kernel's linear bins: column rn((s + tl_s0) tl_inv), an edge
    * within the window at a distance >= tl_h from the column's middle; mu:
    * rn((mu + tl_q0) nmu) and >= tl_qc - tl_q1 / s; |x_b|^2 below near2: the line of sight is
@@ -183,12 +159,8 @@ typedef struct {
   int nse, npe, se_lg, pe_lg, se_off, pe_off, se_skip, pe_skip, se_last,
       pe_last;
   int hcols, hcol0, hrow0, hrows, hlen;
-  float P0, P1, P2;            /* E(pi) (box) or E(pi^2) (survey) */
-  float Q0, Q1, Q2;            /* E(q), q = nmu mu: Q1 / s + Q2 q + Q0 */
   float m2min;                 /* survey: |m|^2 below (next to the observer):
                                   mu and pi^2 are rechecked */
-  float tiny;                  /* s^2 below: always recheck */
-  float Emax;                  /* E at the top of the s axis (iso, spi) */
   int tzero;                   /* stencil index of the zero offset */
   float fnmu;
   /* FP64 reference binning */
@@ -199,18 +171,15 @@ typedef struct {
   double s2min, s2max, pmin, pmax;
   int smin0, pmin0;
   int mu_one;                  /* WITH_MU_ONE: clamp the mu bin, not drop */
-  /* weights: fixed point with F fractional bits */
-  int fixF;
   /* outputs */
   unsigned long long *gcnt;    /* ntot counts */
   unsigned long long *gwt;     /* 2 * ntot: lo, hi words of int128 */
-  double *gwd;                 /* ntot FP64 sums (FP64 path) */
+  double *gwd;                 /* FP64 sums (FP64 path): fcfcg_gwd_copies of
+                                  ntot, the sum of all in the first */
   /* recheck queue: uint4 (a, b, code, 0) */
   uint32_t *queue;
   unsigned long long *qcount;  /* fill: 64 bits, so it cannot wrap */
   uint32_t qcap;
-  uint32_t qwarp;              /* FP32 kernel: entries of a warp's candidate
-                                  queue (256..1024; 0: the launcher picks) */
   unsigned long long *stats;   /* [0] candidates [1] in-range [2] recheck
                                   [3] inline rechecks */
   int hist_smem;               /* histogram in shared memory */
@@ -232,6 +201,12 @@ typedef struct {
   const int *gtab;
   double gunitA, gunitB;
 } fcfcg_launch;
+
+/* Copies of the FP64 sums the CTAs spread their shared ones over: a bin's
+ * chain of additions in memory, of rounding errors each as large as the sum's,
+ * is as much shorter.  One where the sums do not fit in shared memory. */
+#define FCFCG_GWD_COPIES 32
+#define fcfcg_gwd_copies(ntot) ((ntot) <= 25600 ? FCFCG_GWD_COPIES : 1)
 
 /* Launchers implemented in the .cu files; return 0 or a CUDA error code. */
 /* Rescale, |x|^2, max |w|; with w and wsum, also the sum of the weights in
@@ -272,10 +247,6 @@ int fcfcg_k_grid(void *stream, size_t n, const double *x, const double *y,
     const double *z, const double *s, const double *w, int has_w, int wexp,
     const int ncell[3], const double cw[3], const double lo[3], int sb,
     const fcfcg_sort *S);
-int fcfcg_k_chunks(void *stream, const uint32_t *cstart, uint32_t ncell,
-    uint32_t clen, uint32_t *cchunk, uint32_t *scan_tmp, size_t scan_tmp_len,
-    uint32_t *chunks, uint32_t *nchunk_out, const uint32_t *mock_cell_base,
-    int nmock);
 /* One catalogue of a batch for the preparation kernels: its inputs (device
  * or GPU-readable host memory), its place o in the batch slot, its first
  * tile (tiles of fcfcg_batch_tile() points, numbered across the batch) and,
@@ -312,21 +283,17 @@ int fcfcg_k_unsort(void *stream, size_t n, const uint32_t *sid,
 int fcfcg_scan(void *stream, const uint32_t *in, size_t n, uint32_t *out,
     uint32_t *tmp);
 /* Shared memory of the tile kernel: its tables, and besides them and its
- * histogram. */
+ * histogram (kind: 0 unweighted, 1 weighted, 2 adjoint, 3 all-FP64). */
 size_t fcfcg_k_tile32_tab(const fcfcg_launch *L);
-size_t fcfcg_k_tile32_stage(int withwt);
+size_t fcfcg_k_tile32_stage(int kind);
 /* And its histogram's, with a spare word per lane. */
 size_t fcfcg_k_tile32_hist(int hlen, int withwt);
-/* withwt: 0 unweighted, 1 weighted, 2 adjoint */
-size_t fcfcg_k_count32_stage(int nsten, int withwt);
-size_t fcfcg_k_count32_tab_bytes(int nfs, int nfp, int nsb, int npb);
 int fcfcg_k_bbox(void *stream, size_t n, const double *x, const double *y,
     const double *z, unsigned long long *bits6);
-/* The count kernel of a launch.  FP32: L->qwarp 0 lets the launcher pick
- * the warp queue (the largest of 1024 / 512 / 256 entries at the most CTAs
- * per SM); the one used goes to *qwarp_used. */
+/* The count kernel of a launch; *smem_used (may be NULL): its shared memory
+ * per CTA. */
 int fcfcg_k_count(void *stream, const fcfcg_launch *L, int precision,
-    int nsm, size_t *smem_used, uint32_t *qwarp_used);
+    int nsm, size_t *smem_used);
 /* Bits of the coarse cells (dim, cells of 1 / inv_cell from lo) that hold
  * an object, and their number (count). */
 int fcfcg_k_occupancy(void *stream, size_t n, const double *x,

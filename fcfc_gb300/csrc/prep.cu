@@ -984,72 +984,6 @@ extern "C" int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat,
   return (int) cudaGetLastError();
 }
 
-/* Work chunks: every cell is cut into pieces of at most clen points, as
- * evenly as possible. */
-__global__ void k_chunk_count(const uint32_t *__restrict__ cstart,
-    uint32_t ncell, uint32_t clen, uint32_t *__restrict__ cchunk) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += gridDim.x * blockDim.x) {
-    uint32_t m = cstart[c + 1] - cstart[c];
-    cchunk[c] = (m + clen - 1) / clen;
-  }
-}
-
-/* mbase (nmock + 1 entries, may be NULL): first cell of each catalogue of a
- * batch; the chunk's .w is the catalogue holding its cell. */
-__global__ void k_chunk_emit(const uint32_t *__restrict__ cstart,
-    uint32_t ncell, uint32_t clen, const uint32_t *__restrict__ coff,
-    uint4 *__restrict__ chunks, const uint32_t *__restrict__ mbase,
-    int nmock) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += gridDim.x * blockDim.x) {
-    uint32_t a = cstart[c], m = cstart[c + 1] - a;
-    uint32_t k = coff[c];
-    uint32_t nch = (m + clen - 1) / clen;
-    uint32_t mk = 0;
-    if (mbase) {
-      int lo = 0, hi = nmock;   /* last lo with mbase[lo] <= c */
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (mbase[mid] <= c) lo = mid;
-        else hi = mid;
-      }
-      mk = (uint32_t) lo;
-    }
-    for (uint32_t q = 0; q < nch; q++) {
-      uint32_t b0 = (uint32_t) (((unsigned long long) m * q) / nch);
-      uint32_t b1 = (uint32_t) (((unsigned long long) m * (q + 1)) / nch);
-      chunks[k++] = make_uint4(c, a + b0, b1 - b0, mk);
-    }
-  }
-}
-
-extern "C" int fcfcg_k_chunks(void *stream, const uint32_t *cstart,
-    uint32_t ncell, uint32_t clen, uint32_t *cchunk, uint32_t *scan_tmp,
-    size_t scan_tmp_len, uint32_t *chunks, uint32_t *nchunk_out,
-    const uint32_t *mock_cell_base, int nmock) {
-  cudaStream_t st = (cudaStream_t) stream;
-  (void) scan_tmp_len;
-  k_chunk_count<<<grid_for(ncell, PREP_THREADS), PREP_THREADS, 0, st>>>(
-      cstart, ncell, clen, cchunk);
-  cudaError_t e = cudaGetLastError();
-  if (e) return (int) e;
-  /* cchunk holds ncell + 1 slots: scan in place via the offset array */
-  uint32_t *coff = cchunk + ncell + 1;
-  int r = scan_u32(st, cchunk, ncell, coff, scan_tmp);
-  if (r) return r;
-  if (chunks) {
-    k_chunk_emit<<<grid_for(ncell, PREP_THREADS), PREP_THREADS, 0, st>>>(
-        cstart, ncell, clen, coff, (uint4 *) chunks, mock_cell_base, nmock);
-    if ((e = cudaGetLastError())) return (int) e;
-  }
-  if (nchunk_out)
-    if ((e = cudaMemcpyAsync(nchunk_out, coff + ncell, sizeof(uint32_t),
-                             cudaMemcpyDeviceToHost, st)))
-      return (int) e;
-  return 0;
-}
-
 /* Occupancy of a coarse grid over a catalogue's bounding box: one bit per
  * cell that holds an object (the occupied-volume estimate of a survey). */
 __global__ void k_occupy(size_t n, const double *__restrict__ x,

@@ -1,5 +1,6 @@
 /*
- * tile32.cuh -- the FP32 pair-counting kernel (instantiated by count32_*.cu).
+ * tile32.cuh -- the pair-counting kernel (instantiated by count32_*.cu): FP32
+ * separations with an FP64 recheck, or (BIN_F64) every pair in FP64.
  *
  * Work decomposition (replaces FCFC's dual k-d tree, src/fcfc/2pt_box/
  * dual_tree.c:245-373, and its OpenMP/MPI node-pair scheduler,
@@ -74,9 +75,20 @@ struct TileWarpA {
   long long ga[8][32];
 };
 
-/* wt: 0 unweighted, 1 weighted, 2 adjoint */
+/* all-FP64: pairs within the outer range, to be binned 32 at a time; and the
+ * adjoint's FP64 gradients of A's points */
+#define Q64 160
+struct TileWarp64 {
+  TileWarpW w;
+  uint2 q[Q64];            /* sorted indices */
+  uint8_t code[Q64];       /* image codes */
+  double ga[32];
+};
+
+/* wt: 0 unweighted, 1 weighted, 2 adjoint, 3 all-FP64 */
 __host__ __device__ __forceinline__ size_t tile_warp_bytes(int wt) {
-  return wt == 2 ? sizeof(TileWarpA)
+  return wt == 3 ? sizeof(TileWarp64)
+      : wt == 2 ? sizeof(TileWarpA)
                  : (wt ? sizeof(TileWarpW) : sizeof(TileWarp));
 }
 
@@ -256,6 +268,7 @@ __device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
   __syncwarp();
 }
 
+#define HI_LIMIT (1 << 30)
 /* Weighted sums in shared memory: two 32-bit words per bin (the high words
  * hlen + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed;
  * the carry out of lo is read from the returned value, and 2^30 of hi (2^62)
@@ -698,12 +711,116 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
   return rest;
 }
 
+/* All-FP64: bin n <= 32 queued pairs by the reference's formula, every lane
+ * busy. */
+template <int WT>
+__device__ __forceinline__ void bin64(const fcfcg_launch &L, TileWarp64 *S,
+    uint32_t *h, int first, int n, uint32_t &n_in) {
+  const int lane = threadIdx.x & 31;
+  if (lane >= n) return;
+  const uint2 e = S->q[first + lane];
+  const int bin = ref_bin_pair(L, e.x, e.y, S->code[first + lane], L.box);
+  if (bin < 0) return;
+  if (WT) {
+    n_in++;
+    const double v = __dmul_rn(L.A.w[e.x], L.B.w[e.y]);
+    if (L.hist_smem) atomicAdd((double *) h + bin, v);
+    else atomicAdd(L.gwd + bin, v);
+  } else if (L.hist_smem) {
+    atomicAdd(h + bin, 1u);
+  } else {
+    n_in++;
+    atomicAdd(L.gcnt + bin, 1ull);
+  }
+}
+
+/*
+ * The pairs of one tile in FP64.  The FP32 distances, with their rounding
+ * bound, only leave out pairs beyond the outer range (half of a tile's are
+ * within it, and an FP64 instruction takes an SM 16 cycles whether its lanes
+ * are active or not); the others are collected and binned 32 at a time.  nq:
+ * pairs collected.  The adjoint bins a point of A against the lanes' points
+ * and sums its terms across them.
+ *
+ * Bound by the FP64 pipe (2 lanes per SM and clock): 8 operations per pair
+ * for the separation, and few others since the mu bin is taken from FP32
+ * where that is certain (ref_mu).  Weighted (s, mu) count of a box of 3e4
+ * points, 2.6e7 pairs: 15.0 -> 2.0 ms against a kernel that took every pair
+ * of the neighbouring cells, with an FP64 division each.
+ */
+template <int GEOM, int WT, int ADJ>
+__device__ __forceinline__ void tile_pairs64(const fcfcg_launch &L,
+    const Tile &T, TileWarp64 *S, uint32_t *h, int &nq, uint32_t &n_in) {
+  const int lane = threadIdx.x & 31;
+  const bool cyl = GEOM == FCFCG_GEOM_BOX && L.bintype == FCFCG_BIN_SPI;
+  double gb = 0;
+#pragma unroll 1
+  for (int k = 0; k < T.m; k += 4) {
+    const float *P = (const float *) S->w.t.p[k >> 2];
+#pragma unroll 1
+    for (int e = 0; e < 4; e++) {
+      const float dx = P[e] - T.bx, dy = P[4 + e] - T.by, dz = P[8 + e] - T.bz;
+      float s2 = fmaf(dy, dy, dx * dx);
+      if (!cyl) s2 = fmaf(dz, dz, s2);
+      /* (an infinite limit keeps every pair) */
+      const bool in = (k + e < T.ilim) & !(s2 > L.s_lim) &
+                      (!cyl | !(fabsf(dz) > L.p_lim));
+      const uint32_t bal = __ballot_sync(FULLMASK, in);
+      if (!bal) continue;
+      const uint32_t a = T.first + (uint32_t) (k + e);
+      if (ADJ) {
+        double va = 0;
+        const int bin = in ? ref_bin_pair(L, a, T.bj, T.code, L.box) : -1;
+        if (bin >= 0) {
+          n_in++;
+          const double g = __ldg(L.gadj + bin);
+          va = __dmul_rn(L.B.w[T.bj], g);
+          gb = __dadd_rn(gb, __dmul_rn(L.A.w[a], g));
+        }
+        for (int o = 16; o > 0; o >>= 1)
+          va = __dadd_rn(va, __shfl_xor_sync(FULLMASK, va, o));
+        if (lane == 0) S->ga[k + e] = __dadd_rn(S->ga[k + e], va);
+        continue;
+      }
+      if (in) {
+        const int q = nq + __popc(bal & ((1u << lane) - 1u));
+        S->q[q] = make_uint2(a, T.bj);
+        S->code[q] = (uint8_t) T.code;
+      }
+      nq += __popc(bal);
+    }
+    if (!ADJ && nq >= 32) {
+      __syncwarp();
+      int f = 0;
+      for (; f + 32 <= nq; f += 32) bin64<WT>(L, S, h, f, 32, n_in);
+      __syncwarp();
+      if (f + lane < nq) {
+        const uint2 q = S->q[f + lane];
+        const uint8_t c = S->code[f + lane];
+        S->q[lane] = q;
+        S->code[lane] = c;
+      }
+      nq -= f;
+      __syncwarp();
+    }
+  }
+  if (ADJ && gb != 0.0) atomicAdd(L.dB + T.bj, gb);
+}
+
 /* Add the shared histogram to a global one and clear it, by threads t0,
  * t0 + nt, ... (whole warps); unweighted counts handed over are counted as
  * in range.  Exchanges, so that other warps may go on adding meanwhile. */
-template <int WT>
+template <int WT, bool F64 = false>
 __device__ __noinline__ void tile_handover(const fcfcg_launch &L,
     uint32_t *h, uint32_t mock, int t0, int nt, TileWarp *S) {
+  if (WT && F64) {
+    double *g = L.gwd + (size_t) (blockIdx.x % fcfcg_gwd_copies(L.ntot)) * L.ntot;
+    for (int x = t0; x < L.hlen; x += nt) {
+      const double v = ((double *) h)[x];
+      if (v != 0) atomicAdd(g + x, v);
+    }
+    return;
+  }
   unsigned long long *g = WT ? (L.mocks ? L.mocks[mock].gwt : L.gwt)
                              : (L.mocks ? L.mocks[mock].gcnt : L.gcnt);
   unsigned long long sum = 0;
@@ -750,6 +867,9 @@ template <int GEOM, int BIN, int WT, int BATCH, int ADJ = 0>
 __global__ void __launch_bounds__(CT32_THREADS, ADJ ? 3 : TILE_CTAS)
 k_tile32(const __grid_constant__ fcfcg_launch L) {
   constexpr bool SURVEY = GEOM == FCFCG_GEOM_SURVEY;
+  constexpr bool F64 = BIN == BIN_F64;
+  constexpr int KIND = F64 ? 3 : WT + ADJ;
+  const bool cyl = !SURVEY && (F64 ? L.bintype == FCFCG_BIN_SPI : IS_SPI(BIN));
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ TileMock sh_mock;
   __shared__ uint32_t sh_run[3];     /* batch: next item, end, catalogue */
@@ -759,8 +879,8 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
                 EP = {te + L.nse, L.pe_lg, L.pe_off, (uint32_t) L.npe - 1u};
   size_t o = ((size_t) (L.nse + L.npe) * 8 + 15) & ~(size_t) 15;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  TileWarpW *S = (TileWarpW *) (smem + o + (size_t) warp * tile_warp_bytes(WT + ADJ));
-  o += (size_t) (CT32_THREADS / 32) * tile_warp_bytes(WT + ADJ);
+  TileWarpW *S = (TileWarpW *) (smem + o + (size_t) warp * tile_warp_bytes(KIND));
+  o += (size_t) (CT32_THREADS / 32) * tile_warp_bytes(KIND);
   uint32_t *h = (uint32_t *) (smem + o);
   const uint32_t hb = (uint32_t) __cvta_generic_to_shared(h);
   /* bias of the bins' byte addresses formed from a rounded value's bits */
@@ -770,7 +890,9 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
   C.spare = pin(hb + 4u * (uint32_t) ((ADJ || L.hist_smem ? L.hlen : 0) + lane));
   C.ha = pin(C.ha);
   C.slim = pin(C.slim);
-  if (LINS(BIN)) {
+  if (F64) {
+    /* no tables */
+  } else if (LINS(BIN)) {
     /* without a shared histogram every pair goes to tile_rest */
     C.hs = pin(ADJ || L.hist_smem ? L.tl_h : -1.f);
     C.inv = pin(C.inv);
@@ -790,7 +912,9 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
   if (IS_SPI(BIN) && !LINP(BIN))
     for (int i = threadIdx.x; i < L.npe; i += blockDim.x)
       te[L.nse + i] = __ldg((const float2 *) L.pe + (i < L.npe - 1 ? L.pe_skip + i : L.pe_last));
-  if (ADJ) {
+  if (ADJ && F64) {
+    ((TileWarp64 *) S)->ga[lane] = 0;
+  } else if (ADJ) {
     /* the scaled cotangent of the shared bins takes the histogram's place */
     if (L.hist_smem)
       for (int i = threadIdx.x; i < L.hlen + 32; i += blockDim.x)
@@ -809,6 +933,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
   if (lane < 4) S->t.cnt[lane] = 0;
   unsigned long long added = 0;
   uint32_t cur = ~0u;
+  int nq = 0;              /* all-FP64: pairs collected */
   __syncthreads();
 
   for (;;) {
@@ -858,7 +983,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
         const uint32_t mk = s0 == ~0u ? ~0u
             : ((const uint2 *) L.A.bcell)[s0 >> L.pshift].y;
         if (mk != cur && cur != ~0u && L.hist_smem)
-          tile_handover<WT>(L, h, cur, threadIdx.x, CT32_THREADS, &S->t);
+          tile_handover<WT, F64>(L, h, cur, threadIdx.x, CT32_THREADS, &S->t);
         if (s0 == ~0u) break;
         if (mk != cur) {
           if (threadIdx.x < 3) {
@@ -910,7 +1035,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
       p[0] = v.x;
       p[4] = v.y;
       p[8] = v.z;
-      if (WT) {
+      if (WT && !F64) {
         int2 w = make_int2(0, 0);
         if (lane < T.m) w = __ldg((const int2 *) L.A.wq + T.first + lane);
         S->aw[lane] = make_float4(__int_as_float(w.x), __int_as_float(w.y) *
@@ -982,7 +1107,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
         const float gx = fmaxf(fabsf(ac.x + D.x) - (ah.x + hx) - L.box_eps, 0.f),
                     gy = fmaxf(fabsf(ac.y + D.y) - (ah.y + hy) - L.box_eps, 0.f),
                     gz = fmaxf(fabsf(ac.z + D.z) - (ah.z + hz) - L.box_eps, 0.f);
-        if (IS_SPI(BIN) && !SURVEY)
+        if (cyl)
           visit = (gz < L.p_lim) & (fmaf(gy, gy, gx * gx) < L.s_lim);
         else
           visit = fmaf(gz, gz, fmaf(gy, gy, gx * gx)) < L.s_lim;
@@ -1016,7 +1141,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           const float gx = fmaxf(fabsf(ac.x - (bc.x - d.x)) - (ah.x + bh.x) - L.box_eps, 0.f),
                       gy = fmaxf(fabsf(ac.y - (bc.y - d.y)) - (ah.y + bh.y) - L.box_eps, 0.f),
                       gz = fmaxf(fabsf(ac.z - (bc.z - d.z)) - (ah.z + bh.z) - L.box_eps, 0.f);
-          if (IS_SPI(BIN) && !SURVEY)
+          if (cyl)
             near = (gz < L.p_lim) & (fmaf(gy, gy, gx * gx) < L.s_lim);
           else
             near = fmaf(gz, gz, fmaf(gy, gy, gx * gx)) < L.s_lim;
@@ -1039,7 +1164,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             T.bx = v.x - d.x;
             T.by = v.y - d.y;
             T.bz = v.z - d.z;
-            if (WT) {
+            if (WT && !F64) {
               const int2 w = __ldg((const int2 *) L.B.wq + T.bj);
               T.wi = w.x;
               T.wr = __int_as_float(w.y) * (ADJ ? 0x1p-30f : 1.f);
@@ -1047,8 +1172,9 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             }
           }
           T.ilim = self ? lane : 32;
+          if (F64) T.ilim = lane < n ? min(T.ilim, T.m) : 0;
           bool sp = self;
-          if (SURVEY) {
+          if (SURVEY && !F64) {
             T.vx = fmaf(2.f, T.bx, c2x);
             T.vy = fmaf(2.f, T.by, c2y);
             T.vz = fmaf(2.f, T.bz, c2z);
@@ -1069,19 +1195,23 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             }
           }
           cand += (uint32_t) (T.m * n);
-          uint32_t rest;
-          long long gb = 0;       /* adjoint: this lane's point's terms */
-          if (sp)
-            rest = tile_pairs<GEOM, BIN, WT, ADJ, true>(L, C, T, S, hb, ES,
-                                                        EP, n_in, gb);
-          else
-            rest = tile_pairs<GEOM, BIN, WT, ADJ, false>(L, C, T, S, hb, ES,
-                                                         EP, n_in, gb);
-          if (ADJ && gb) atomicAdd(L.dB + T.bj, (double) gb * L.gunitB);
-          if (__any_sync(FULLMASK, rest != 0u))
-            tile_rest<GEOM, BIN, WT, ADJ>(L, T, S, rest, ES, EP);
+          if constexpr (F64) {
+            tile_pairs64<GEOM, WT, ADJ>(L, T, (TileWarp64 *) S, h, nq, n_in);
+          } else {
+            uint32_t rest;
+            long long gb = 0;     /* adjoint: this lane's point's terms */
+            if (sp)
+              rest = tile_pairs<GEOM, BIN, WT, ADJ, true>(L, C, T, S, hb, ES,
+                                                          EP, n_in, gb);
+            else
+              rest = tile_pairs<GEOM, BIN, WT, ADJ, false>(L, C, T, S, hb, ES,
+                                                           EP, n_in, gb);
+            if (ADJ && gb) atomicAdd(L.dB + T.bj, (double) gb * L.gunitB);
+            if (__any_sync(FULLMASK, rest != 0u))
+              tile_rest<GEOM, BIN, WT, ADJ>(L, T, S, rest, ES, EP);
+          }
         }
-        if (ADJ) {
+        if (ADJ && !F64) {
           /* a term is below 2^51, a step adds 4 of them to a word and a
            * group of blocks 32 steps' worth: out before 2^60 */
           ntile += 32;
@@ -1098,19 +1228,34 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           tile_handover<WT>(L, h, T.mock, lane, 32, &S->t);
           added = 0;
         }
-        if (WT) {
+        if (WT || (F64 && !L.hist_smem)) {
           n_in = __reduce_add_sync(FULLMASK, n_in);
           if (lane == 0) S->t.cnt[1] += n_in;
         }
        }
       }
     }
-    if (ADJ) adj_flush(L, (TileWarpA *) S, T.first, T.m);
+    if (ADJ && F64) {
+      double &ga = ((TileWarp64 *) S)->ga[lane];
+      __syncwarp();
+      if (lane < T.m && ga != 0.0) atomicAdd(L.dA + T.first + lane, ga);
+      ga = 0;
+      __syncwarp();
+    } else if (ADJ) {
+      adj_flush(L, (TileWarpA *) S, T.first, T.m);
+    }
+  }
+  if (F64 && !ADJ) {
+    uint32_t n_in = 0;
+    __syncwarp();
+    bin64<WT>(L, (TileWarp64 *) S, h, 0, nq, n_in);
+    n_in = __reduce_add_sync(FULLMASK, n_in);
+    if (lane == 0) S->t.cnt[1] += n_in;
   }
   if (!BATCH && !ADJ) {
     __syncthreads();
     if (L.hist_smem)
-      tile_handover<WT>(L, h, 0, threadIdx.x, CT32_THREADS, &S->t);
+      tile_handover<WT, F64>(L, h, 0, threadIdx.x, CT32_THREADS, &S->t);
   }
   __syncwarp();
   if (lane < 4) atomicAdd(L.stats + lane, S->t.cnt[lane]);

@@ -111,3 +111,45 @@ def test_one_cell_and_global_histogram():
         np.testing.assert_array_equal(cnt[0], want)
         np.testing.assert_array_equal(cnt[1], ob.count(x[:40], mode=1))
         assert cnt[2].sum() == 0
+
+
+@pytest.mark.parametrize("name", sorted(BINS))
+@pytest.mark.parametrize("geom", ["box", "survey"])
+def test_tile_fp64(geom, name):
+    """The tiles with every pair in FP64: catalogues around a block, integer
+    coordinates (separations and mu on the bin edges), and lengths whose
+    squares FP32 does not hold.  Weighted sums: FP64 additions in any order,
+    at most 2e6 terms of at most 10 each, of which a bin's sum loses less
+    than 2e6 eps = 4.4e-10 of their absolute sum."""
+    import fcfc_gb300 as fg
+    for n, m, scale in ((1, 1, 1.0), (31, 33, 1.0), (97, 700, 1.0),
+                        (2049, 130, 1.0), (300, 65, 1e20)):
+        if scale != 1.0 and (geom == "survey" or name not in ("smu", "iso_smin")):
+            continue
+        kw = dict(BINS[name])
+        if scale != 1.0:
+            kw.update(smin=kw["smin"] * scale, ds=kw["ds"] * scale)
+        box = 130.0 * scale if geom == "box" else None
+        pc, ob = _pair(geom, kw, box)
+        for whole in (False, True):
+            a, b = _points(geom, n, 130.0, n), _points(geom, m, 130.0, 1000 + m)
+            if whole:
+                a, b = np.floor(a), np.floor(b)
+            a, b = a * scale, b * scale
+            w = np.random.default_rng(5).normal(1.0, 0.6, n)
+            pc.load(0, a, w)
+            pc.load(1, b)
+            for other, want, wantw, tot in (
+                    (None, ob.count(a, mode=1), ob.count(a, wa=w, mode=1),
+                     ob.count(a, wa=np.abs(w), mode=1)),
+                    (1, ob.count(a, b, mode=1), ob.count(a, b, wa=w, mode=1),
+                     ob.count(a, b, wa=np.abs(w), mode=1))):
+                got = pc.count_pairs(0, other, precision=fg.PREC_FP64)
+                np.testing.assert_array_equal(got, want)
+                st = pc.stats()
+                assert st["precision_used"] == fg.PREC_FP64
+                assert st["in_range"] == want.sum()
+                got = pc.count_pairs(0, other, weighted=True,
+                                     precision=fg.PREC_FP64)
+                assert (np.abs(got - wantw) <= 4.4e-10 * tot).all()
+                assert pc.stats()["in_range"] == want.sum()
