@@ -100,7 +100,8 @@ struct fcfcg_ctx {
   size_t d_pcat_cap;
   double *d_bpart;               /* per-tile weight sums of a batch */
   size_t d_bpart_cap;
-  double *d_wpart;               /* weight-sum partials; [0] the sum */
+  double *d_wpart;               /* weight-sum partials */
+  unsigned long long *h_load;    /* pinned: the results of a load */
   double *d_grad;                /* adjoint: sorted and input-order gradients */
   size_t d_grad_cap;
   unsigned long long *d_bout, *d_bstat;
@@ -213,6 +214,7 @@ void fcfcg_destroy(fcfcg_ctx *c) {
     for (size_t i = 0; i < sizeof p / sizeof p[0]; i++)
       if (p[i]) cudaFree(p[i]);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
+    if (c->h_load) cudaFreeHost(c->h_load);
     for (int i = 0; i < 5; i++)
       if (c->ev[i]) cudaEventDestroy(c->ev[i]);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -289,8 +291,13 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
                 sizeof(double) * b->ntot * fcfcg_gwd_copies(b->ntot)));
   CK(cudaMalloc((void **) &c->d_stats, sizeof(unsigned long long) * 8));
   CK(cudaMalloc((void **) &c->d_wpart,
-                sizeof(double) * (fcfcg_prep_partials() + 1)));
-  CK(cudaMalloc((void **) &c->d_bbox, sizeof(unsigned long long) * 6));
+                sizeof(double) * fcfcg_prep_partials()));
+  CK(cudaMallocHost((void **) &c->h_load, sizeof(unsigned long long) * 8));
+  memset(c->h_load, 0, sizeof(unsigned long long) * 8);
+  for (int k = 0; k < 3; k++) c->h_load[k] = ~0ull;
+  rc = upload(c, (void **) &c->d_bbox, c->h_load,
+              sizeof(unsigned long long) * 8);
+  if (rc) return rc;
   CK(cudaMalloc((void **) &c->d_head, sizeof(uint32_t) * 4));
   c->d_qcount = (unsigned long long *) (c->d_head + 2);
   c->qcap = c->qcap_alloc = (size_t) 1 << 25;   /* 32M pairs, 512 MiB */
@@ -423,10 +430,10 @@ static int occupied_volume(fcfcg_ctx *c, slot_t *s) {
   CKK(fcfcg_k_occupancy(c->stream, s->n, s->x, s->y, s->z, s->bmin, dim, inv,
                         c->cfill, nw, dcount));
   c->launches += 2;
-  unsigned long long K = 0;
-  CK(cudaMemcpyAsync(&K, dcount, sizeof K, cudaMemcpyDeviceToHost,
-                     c->stream));
+  CK(cudaMemcpyAsync(c->h_load, dcount, sizeof *c->h_load,
+                     cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  const unsigned long long K = *c->h_load;
   const double n = (double) s->n, T = (double) tot;
   double M;
   if (T * -expm1(-n / T) <= (double) K) {
@@ -509,27 +516,15 @@ static int load_common(fcfcg_ctx *c, int slot, size_t n, const double *x,
     iy = s->y;
     iz = s->z;
   }
-  unsigned long long *wbits = c->d_stats + 7;
-  CK(cudaMemsetAsync(wbits, 0, sizeof(unsigned long long), c->stream));
+  /* one pass, its results in pinned memory */
+  unsigned long long *hb = c->h_load;
   CKK(fcfcg_k_prep(c->stream, n, ix, iy, iz, iw, c->bins.rescale, survey,
-                   s->x, s->y, s->z, s->s, s->w, wbits, c->d_wpart + 1,
-                   c->d_wpart));
-  c->launches += n ? (w ? 3 : 2) : 0;
-  /* bounding box of the rescaled catalogue and max |w| */
-  unsigned long long init[6] = {~0ull, ~0ull, ~0ull, 0, 0, 0};
-  CK(cudaMemcpyAsync(c->d_bbox, init, sizeof init, cudaMemcpyHostToDevice,
-                     c->stream));
-  CKK(fcfcg_k_bbox(c->stream, n, s->x, s->y, s->z, c->d_bbox));
-  unsigned long long hb[7];
-  CK(cudaMemcpyAsync(hb, c->d_bbox, sizeof(unsigned long long) * 6,
-                     cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(hb + 6, wbits, sizeof(unsigned long long),
-                     cudaMemcpyDeviceToHost, c->stream));
+                   s->x, s->y, s->z, s->s, s->w, c->d_bbox, c->d_wpart, hb));
+  c->launches += n ? 1 : 0;
+  if (n) CK(cudaStreamSynchronize(c->stream));
+  else memset(hb, 0, sizeof *hb * 8);
   double wsum = 0;
-  if (w && n)
-    CK(cudaMemcpyAsync(&wsum, c->d_wpart, sizeof(double),
-                       cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  if (w && n) memcpy(&wsum, hb + 7, sizeof wsum);
   double mn[3], mx[3];
   for (int k = 0; k < 3; k++) {
     unsigned long long a = hb[k], bb = hb[3 + k];
@@ -927,7 +922,7 @@ static int slot_sort(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   CKK(fcfcg_k_grid(c->stream, n, s->x, s->y, s->z, survey ? s->s : NULL,
                    s->w, s->has_w, s->wexp, g->n, g->cw, g->lo,
                    fcfcg_grid_curve_bits(nc, n), &b));
-  c->launches += n ? 7 : 5;
+  c->launches += n ? 5 : 3;
   return FCFCG_OK;
 }
 
@@ -2491,7 +2486,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   BCKK(fcfcg_k_grid_batch(c->stream, (const fcfcg_prep_cat *) c->d_pcat, na,
                           ntile, cells, N, c->d_mbase, sb, S->x, S->y, S->z,
                           withwt ? S->w : NULL, withwt, &sbuf));
-  c->launches += 7;
+  c->launches += 5;
   /* 6. per-catalogue histograms and the catalogue table */
   const size_t per = (size_t) b->ntot * (withwt ? 2 : 1);
   BGROW(c->d_bout, c->d_bout_cap, sizeof(unsigned long long) * per * na);

@@ -209,12 +209,15 @@ typedef struct {
 #define fcfcg_gwd_copies(ntot) ((ntot) <= 25600 ? FCFCG_GWD_COPIES : 1)
 
 /* Launchers implemented in the .cu files; return 0 or a CUDA error code. */
-/* Rescale, |x|^2, max |w|; with w and wsum, also the sum of the weights in
- * a fixed order (partial: fcfcg_prep_partials() doubles of scratch). */
+/* Rescale and |x|^2 (surveys); out[0..5] the bounding box (order-preserving
+ * keys, min then max), out[6] max |w| bits and, with w, out[7] the sum of the
+ * weights (a double, in a fixed order).  out: memory the device can write;
+ * acc: 8 words, three ~0 and five 0, left so; partial:
+ * fcfcg_prep_partials() doubles of scratch. */
 int fcfcg_k_prep(void *stream, size_t n, const double *x, const double *y,
     const double *z, const double *w, double rescale, int survey,
     double *ox, double *oy, double *oz, double *os, double *ow,
-    unsigned long long *wmax_bits, double *partial, double *wsum);
+    unsigned long long *acc, double *partial, unsigned long long *out);
 size_t fcfcg_prep_partials(void);
 /* Sub-cell bits of a grid of ncell cells holding npoint points: 6 (4 x 4
  * x 4 sub-cells), 3 (2 x 2 x 2) or 0; the sort then uses (ncell << sb) fine
@@ -288,8 +291,6 @@ size_t fcfcg_k_tile32_tab(const fcfcg_launch *L);
 size_t fcfcg_k_tile32_stage(int kind);
 /* And its histogram's, with a spare word per lane. */
 size_t fcfcg_k_tile32_hist(int hlen, int withwt);
-int fcfcg_k_bbox(void *stream, size_t n, const double *x, const double *y,
-    const double *z, unsigned long long *bits6);
 /* The count kernel of a launch; *smem_used (may be NULL): its shared memory
  * per CTA. */
 int fcfcg_k_count(void *stream, const fcfcg_launch *L, int precision,

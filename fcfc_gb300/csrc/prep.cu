@@ -24,72 +24,61 @@ static int grid_for(size_t n, int threads) {
   return (int) b;
 }
 
-/* Order-preserving map of a double to an unsigned key. */
+/* Order-preserving map of a double to an unsigned key.  The bits are taken
+ * in PTX: with __double_as_longlong the compiler sets the sign by a negation
+ * of the double, which leaves a NaN's alone. */
 __device__ __forceinline__ unsigned long long dkey(double v) {
-  unsigned long long b = (unsigned long long) __double_as_longlong(v);
+  unsigned long long b;
+  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(v));
   return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-__global__ void k_prep(size_t n, const double *__restrict__ x,
-    const double *__restrict__ y, const double *__restrict__ z,
-    const double *__restrict__ w, double rescale, int survey,
-    double *__restrict__ ox, double *__restrict__ oy, double *__restrict__ oz,
-    double *__restrict__ os, double *__restrict__ ow,
-    unsigned long long *wmax_bits, double *__restrict__ partial) {
-  __shared__ double sh_sum[PREP_THREADS];
-  unsigned long long wm = 0;
-  double ws = 0;
-  for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n;
-       i += (size_t) gridDim.x * blockDim.x) {
-    double a = x[i], b = y[i], c = z[i];
-    if (rescale != 1) {
-      a = __dmul_rn(a, rescale);
-      b = __dmul_rn(b, rescale);
-      c = __dmul_rn(c, rescale);
+/* Smallest and largest over the block of lo[k] and hi[k], and the largest of
+ * wm, into the accumulators acc[0..2], acc[3..5] and acc[6]: one atomic per
+ * block, and only where it would change the value (by then most blocks would
+ * not; one per warp, 6 words each, took 73 us for 6e5 points). */
+__device__ __forceinline__ void block_range(unsigned long long lo[3],
+    unsigned long long hi[3], unsigned long long wm, unsigned long long *acc) {
+  __shared__ unsigned long long sh[PREP_THREADS / 32][7];
+  const int lane = threadIdx.x & 31;
+  for (int o = 16; o > 0; o >>= 1) {
+    unsigned long long t;
+    for (int k = 0; k < 3; k++) {
+      t = __shfl_xor_sync(0xffffffffu, lo[k], o);
+      lo[k] = t < lo[k] ? t : lo[k];
+      t = __shfl_xor_sync(0xffffffffu, hi[k], o);
+      hi[k] = t > hi[k] ? t : hi[k];
     }
-    ox[i] = a;
-    oy[i] = b;
-    oz[i] = c;
-    if (survey)
-      os[i] = __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)),
-                        __dmul_rn(c, c));
-    if (w) {
-      double v = w[i];
-      ow[i] = v;
-      ws = __dadd_rn(ws, v);
-      unsigned long long bits =
-          (unsigned long long) __double_as_longlong(fabs(v));
-      wm = bits > wm ? bits : wm;
-    }
+    t = __shfl_xor_sync(0xffffffffu, wm, o);
+    wm = t > wm ? t : wm;
   }
-  if (w && partial) {
-    /* this block's weight sum, in a fixed order (deterministic) */
-    sh_sum[threadIdx.x] = ws;
-    __syncthreads();
-    for (int o = PREP_THREADS / 2; o > 0; o >>= 1) {
-      if ((int) threadIdx.x < o)
-        sh_sum[threadIdx.x] = __dadd_rn(sh_sum[threadIdx.x],
-                                        sh_sum[threadIdx.x + o]);
-      __syncthreads();
+  if (lane == 0) {
+    for (int k = 0; k < 3; k++) {
+      sh[threadIdx.x >> 5][k] = lo[k];
+      sh[threadIdx.x >> 5][3 + k] = hi[k];
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = sh_sum[0];
+    sh[threadIdx.x >> 5][6] = wm;
   }
-  if (w) {
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long t = __shfl_xor_sync(0xffffffffu, wm, o);
-      wm = t > wm ? t : wm;
+  __syncthreads();
+  if (threadIdx.x < 7) {
+    const int k = threadIdx.x;
+    unsigned long long v = sh[0][k];
+    for (int i = 1; i < PREP_THREADS / 32; i++) {
+      const unsigned long long t = sh[i][k];
+      v = k < 3 ? (t < v ? t : v) : (t > v ? t : v);
     }
-    if ((threadIdx.x & 31) == 0 && wm) atomicMax(wmax_bits, wm);
+    const unsigned long long old = *(volatile unsigned long long *) (acc + k);
+    if (k < 3) {
+      if (v < old) atomicMin(acc + k, v);
+    } else if (v > old) {
+      atomicMax(acc + k, v);
+    }
   }
 }
 
-/* Sum of the per-block partial sums, in a fixed order. */
-__global__ void k_sum_partials(int nb, const double *__restrict__ partial,
-    double *out) {
+/* The block's sum of v, in a fixed order, by thread 0. */
+__device__ __forceinline__ double block_sum(double v) {
   __shared__ double sh[PREP_THREADS];
-  double v = 0;
-  for (int i = threadIdx.x; i < nb; i += PREP_THREADS)
-    v = __dadd_rn(v, partial[i]);
   sh[threadIdx.x] = v;
   __syncthreads();
   for (int o = PREP_THREADS / 2; o > 0; o >>= 1) {
@@ -97,7 +86,77 @@ __global__ void k_sum_partials(int nb, const double *__restrict__ partial,
       sh[threadIdx.x] = __dadd_rn(sh[threadIdx.x], sh[threadIdx.x + o]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = sh[0];
+  return sh[0];
+}
+
+/* A catalogue in one pass: rescaled, |x|^2, its bounding box, max |w| and
+ * the sum of the weights, in a fixed order: the blocks' sums, added by the
+ * block that finishes last, which also hands the results over and leaves the
+ * accumulators as it found them.  (With the box, the sum and the copies as
+ * operations of their own, a small catalogue's load was 7 of them.) */
+__global__ void k_prep(size_t n, const double *__restrict__ x,
+    const double *__restrict__ y, const double *__restrict__ z,
+    const double *__restrict__ w, double rescale, int survey,
+    double *__restrict__ ox, double *__restrict__ oy, double *__restrict__ oz,
+    double *__restrict__ os, double *__restrict__ ow,
+    unsigned long long *acc, double *__restrict__ partial,
+    unsigned long long *out) {
+  __shared__ uint32_t sh_last;
+  unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
+  unsigned long long wm = 0;
+  double ws = 0;
+  for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n;
+       i += (size_t) gridDim.x * blockDim.x) {
+    double v[3] = {x[i], y[i], z[i]};
+    if (rescale != 1)
+      for (int k = 0; k < 3; k++) v[k] = __dmul_rn(v[k], rescale);
+    ox[i] = v[0];
+    oy[i] = v[1];
+    oz[i] = v[2];
+    if (survey)
+      os[i] = __dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]),
+                                  __dmul_rn(v[1], v[1])),
+                        __dmul_rn(v[2], v[2]));
+    for (int k = 0; k < 3; k++) {
+      const unsigned long long q = dkey(v[k]);
+      lo[k] = q < lo[k] ? q : lo[k];
+      hi[k] = q > hi[k] ? q : hi[k];
+    }
+    if (w) {
+      const double u = w[i];
+      ow[i] = u;
+      ws = __dadd_rn(ws, u);
+      const unsigned long long bits =
+          (unsigned long long) __double_as_longlong(fabs(u));
+      wm = bits > wm ? bits : wm;
+    }
+  }
+  block_range(lo, hi, wm, acc);
+  if (w) {
+    const double s = block_sum(ws);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    sh_last = atomicAdd((uint32_t *) (acc + 7), 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!sh_last) return;
+  __threadfence();
+  double sum = 0;
+  if (w) {
+    double v = 0;
+    for (int i = threadIdx.x; i < (int) gridDim.x; i += PREP_THREADS)
+      v = __dadd_rn(v, __ldcg(partial + i));
+    __syncthreads();
+    sum = block_sum(v);
+  }
+  if (threadIdx.x < 8) {
+    const int k = threadIdx.x;
+    out[k] = k < 7 ? __ldcg(acc + k)
+                   : (unsigned long long) __double_as_longlong(sum);
+    acc[k] = k < 3 ? ~0ull : 0ull;
+  }
 }
 
 extern "C" size_t fcfcg_prep_partials(void) { return 152 * 32; }
@@ -105,51 +164,11 @@ extern "C" size_t fcfcg_prep_partials(void) { return 152 * 32; }
 extern "C" int fcfcg_k_prep(void *stream, size_t n, const double *x,
     const double *y, const double *z, const double *w, double rescale,
     int survey, double *ox, double *oy, double *oz, double *os, double *ow,
-    unsigned long long *wmax_bits, double *partial, double *wsum) {
+    unsigned long long *acc, double *partial, unsigned long long *out) {
   if (!n) return 0;
-  const int nb = grid_for(n, PREP_THREADS);
-  k_prep<<<nb, PREP_THREADS, 0, (cudaStream_t) stream>>>(
-      n, x, y, z, w, rescale, survey, ox, oy, oz, os, ow, wmax_bits,
-      (w && wsum) ? partial : NULL);
-  cudaError_t e = cudaGetLastError();
-  if (e || !w || !wsum) return (int) e;
-  k_sum_partials<<<1, PREP_THREADS, 0, (cudaStream_t) stream>>>(nb, partial,
-                                                                 wsum);
-  return (int) cudaGetLastError();
-}
-
-__global__ void k_bbox(size_t n, const double *__restrict__ x,
-    const double *__restrict__ y, const double *__restrict__ z,
-    unsigned long long *bits6) {
-  unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
-  const double *p[3] = {x, y, z};
-  for (size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < n;
-       i += (size_t) gridDim.x * blockDim.x) {
-    for (int k = 0; k < 3; k++) {
-      unsigned long long v = dkey(p[k][i]);
-      lo[k] = v < lo[k] ? v : lo[k];
-      hi[k] = v > hi[k] ? v : hi[k];
-    }
-  }
-  for (int k = 0; k < 3; k++) {
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long a = __shfl_xor_sync(0xffffffffu, lo[k], o);
-      unsigned long long b = __shfl_xor_sync(0xffffffffu, hi[k], o);
-      lo[k] = a < lo[k] ? a : lo[k];
-      hi[k] = b > hi[k] ? b : hi[k];
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicMin(bits6 + k, lo[k]);
-      atomicMax(bits6 + 3 + k, hi[k]);
-    }
-  }
-}
-
-extern "C" int fcfcg_k_bbox(void *stream, size_t n, const double *x,
-    const double *y, const double *z, unsigned long long *bits6) {
-  if (!n) return 0;
-  k_bbox<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0,
-           (cudaStream_t) stream>>>(n, x, y, z, bits6);
+  k_prep<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0,
+           (cudaStream_t) stream>>>(n, x, y, z, w, rescale, survey, ox, oy,
+                                    oz, os, ow, acc, partial, out);
   return (int) cudaGetLastError();
 }
 
@@ -210,8 +229,25 @@ __global__ void k_scan_sums(uint32_t *__restrict__ tile_sum, size_t ntile) {
   }
 }
 
+__device__ __forceinline__ void scan_put(uint32_t *out, size_t i, uint32_t e,
+    int sb, uint32_t *cstart, uint32_t *bstart) {
+  out[i] = e;
+  if (!cstart || (i & (((size_t) 1 << sb) - 1))) return;
+  const size_t c = i >> sb;
+  cstart[c] = e;
+  if (bstart) bstart[c] = e / 32u + (uint32_t) c;
+}
+
+/* The scan itself.  The items before a block: tile_sum[its] where those are
+ * scanned (sums 2), else their sum taken here, from the tiles' sums (1) or
+ * the items (0).  With cstart, items come (1 << sb) to a cell: cstart[c] the
+ * scan at the cells' first items, c = 0..n >> sb, and bstart, if given: the
+ * cells' first blocks, numbered with at most one place left unused per cell
+ * (floor(cstart / 32) + c grows from cell to cell by more than the cell's
+ * points / 32). */
 __global__ void k_scan_apply(const uint32_t *__restrict__ in, size_t n,
-    const uint32_t *__restrict__ tile_sum, uint32_t *__restrict__ out) {
+    const uint32_t *__restrict__ tile_sum, int sums, uint32_t *__restrict__ out,
+    int sb, uint32_t *__restrict__ cstart, uint32_t *__restrict__ bstart) {
   __shared__ uint32_t shw[32];
   __shared__ uint32_t tot;
   size_t base = (size_t) blockIdx.x * SCAN_TILE;
@@ -223,12 +259,27 @@ __global__ void k_scan_apply(const uint32_t *__restrict__ in, size_t n,
     v[k] = (i < n) ? in[i] : 0;
     s += v[k];
   }
-  uint32_t e = block_excl_scan(s, shw, &tot) + tile_sum[blockIdx.x];
+  uint32_t before = 0;
+  if (sums == 2) {
+    before = tile_sum[blockIdx.x];
+  } else {
+    const uint32_t *__restrict__ q = sums ? tile_sum : in;
+    const size_t m = sums ? (size_t) blockIdx.x : base;
+    uint32_t t = 0;
+#pragma unroll 4
+    for (size_t i = threadIdx.x; i < m; i += SCAN_THREADS) t += q[i];
+    block_excl_scan(t, shw, &tot);
+    before = tot;
+    __syncthreads();
+  }
+  uint32_t e = block_excl_scan(s, shw, &tot) + before;
+  if (n == 0) scan_put(out, 0, 0, sb, cstart, bstart);
   for (int k = 0; k < SCAN_ITEMS; k++) {
-    size_t i = base + (size_t) threadIdx.x * SCAN_ITEMS + k;
-    if (i < n) out[i] = e;
+    const size_t i = base + (size_t) threadIdx.x * SCAN_ITEMS + k;
+    if (i >= n) break;
+    scan_put(out, i, e, sb, cstart, bstart);
     e += v[k];
-    if (i == n - 1) out[n] = e;
+    if (i == n - 1) scan_put(out, n, e, sb, cstart, bstart);
   }
 }
 
@@ -236,16 +287,19 @@ extern "C" size_t fcfcg_scan_tmp_len(size_t n) {
   return (n + SCAN_TILE - 1) / SCAN_TILE + 1;
 }
 
-/* out[0..n] = exclusive scan of in[0..n-1], out[n] = total. */
+/* out[0..n] = exclusive scan of in[0..n-1], out[n] = total; sb, cstart and
+ * bstart as k_scan_apply.  One launch up to 8 tiles, where each block adds
+ * up the items before its own; two up to 4096, where each adds up the tiles'
+ * sums (16 KB from L2); else three. */
 static int scan_u32(cudaStream_t s, const uint32_t *in, size_t n,
-    uint32_t *out, uint32_t *tmp) {
-  if (n == 0) {
-    return (int) cudaMemsetAsync(out, 0, sizeof(uint32_t), s);
-  }
+    uint32_t *out, uint32_t *tmp, int sb = 0, uint32_t *cstart = NULL,
+    uint32_t *bstart = NULL) {
   size_t ntile = (n + SCAN_TILE - 1) / SCAN_TILE;
-  k_scan_tiles<<<(unsigned) ntile, SCAN_THREADS, 0, s>>>(in, n, tmp);
-  k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(tmp, ntile);
-  k_scan_apply<<<(unsigned) ntile, SCAN_THREADS, 0, s>>>(in, n, tmp, out);
+  const int sums = ntile <= 8 ? 0 : (ntile <= 4096 ? 1 : 2);
+  if (sums) k_scan_tiles<<<(unsigned) ntile, SCAN_THREADS, 0, s>>>(in, n, tmp);
+  if (sums == 2) k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(tmp, ntile);
+  k_scan_apply<<<(unsigned) (ntile ? ntile : 1), SCAN_THREADS, 0, s>>>(
+      in, n, tmp, sums, out, sb, cstart, bstart);
   return (int) cudaGetLastError();
 }
 
@@ -356,21 +410,6 @@ __global__ void k_keys(size_t n, const double *__restrict__ x,
         (float) z[i], __uint_as_float((uint32_t) i));
 }
 
-/* cstart[c] = fstart[c << sb], c = 0..nc: the cells' first sorted points
- * from the fine (sub-cell) starts.  bstart, if given: the cells' first
- * blocks, numbered with at most one place left unused per cell:
- * floor(cstart / 32) + c grows from cell to cell by more than the cell's
- * points / 32. */
-__global__ void k_cstart(size_t nc, int sb, const uint32_t *__restrict__ fstart,
-    uint32_t *__restrict__ cstart, uint32_t *__restrict__ bstart) {
-  for (size_t c = blockIdx.x * (size_t) blockDim.x + threadIdx.x; c <= nc;
-       c += (size_t) gridDim.x * blockDim.x) {
-    const uint32_t v = fstart[c << sb];
-    cstart[c] = v;
-    if (bstart) bstart[c] = v / 32u + (uint32_t) c;
-  }
-}
-
 __global__ void k_block_count(const uint32_t *__restrict__ cstart,
     uint32_t ncell, uint32_t *__restrict__ count) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
@@ -380,18 +419,24 @@ __global__ void k_block_count(const uint32_t *__restrict__ cstart,
 
 /*
  * The sorted arrays and the blocks.  A cell's points come in runs of at most
- * RUN_LEN along the Hilbert curve; a warp orders a run so that each block of
- * 32 has a compact box: it is halved along its longest axis, the halves
- * along theirs, down to 32 (a bitonic sort of 23-bit coordinates and 9-bit
- * indices in registers, 16 per lane).  Consecutive runs of 32 points of the
- * curve itself have boxes of about twice the volume; with this order the
- * tiles of a uniform box fell by a fifth.  Then the run is gathered from the
- * input arrays and written in order: the FP32 offsets from the cell centre
- * and the weight's scaled high part (l4), the weight's fixed-point split
- * (wq), FP64 copies and ids, and the blocks' boxes of the FP32 offsets (half
- * extents rounded up).
+ * RUN_LEN along the Hilbert curve; a team of W warps orders a run so that
+ * each block of 32 has a compact box: it is halved along its longest axis,
+ * the halves along theirs, down to 32 (a bitonic sort of 23-bit coordinates
+ * and 9-bit indices in registers, 16 / W per lane).  Consecutive runs of 32
+ * points of the curve itself have boxes of about twice the volume; with this
+ * order the tiles of a uniform box fell by a fifth.  Then the run is gathered
+ * from the input arrays and written in order: the FP32 offsets from the cell
+ * centre and the weight's scaled high part (l4), the weight's fixed-point
+ * split (wq), FP64 copies and ids, and the blocks' boxes of the FP32 offsets
+ * (half extents rounded up).
  *
- * Warps: groups of `group` consecutive cells, `share` warps to a group, which
+ * Bound by latency unless there are many runs: one warp per run took 30 us
+ * for any number of points up to 1e5 (16 gathers one after the other, 40
+ * steps of the sort on 16 keys a lane); four warps share both: 15 us for
+ * 2e3 points, 22 us for 1e5 (31 before), 45 for 6e5 (65).  One warp where
+ * cells hold few points.
+ *
+ * Teams: groups of `group` consecutive cells, `share` teams to a group, which
  * deal the cells' runs among themselves.
  */
 #define RUN_LEN 512
@@ -420,63 +465,98 @@ struct RunSh {
   uint32_t id[RUN_LEN];
   uint16_t ord[RUN_LEN];
 };
+/* a team of four: keys to exchange, and the warps' ranges */
+struct RunX {
+  uint32_t k[2][RUN_LEN];
+  float r[RUN_WARPS][6];
+};
+
+template <int W>
+__device__ __forceinline__ void team_sync() {
+  if (W == 1) __syncwarp();
+  else __syncthreads();
+}
 
 /* Compare-exchange of keys i and i ^ J of a lane, ascending. */
-template <int J>
-__device__ __forceinline__ void run_step(uint32_t k[16]) {
+template <int J, int E>
+__device__ __forceinline__ void run_step(uint32_t k[E]) {
 #pragma unroll
-  for (int i = 0; i < 16; i++)
+  for (int i = 0; i < E; i++)
     if (!(i & J)) {
       const uint32_t a = k[i], b = k[i | J];
       k[i] = a < b ? a : b;
       k[i | J] = a < b ? b : a;
     }
 }
+template <int E>
+__device__ __forceinline__ void run_steps(uint32_t k[E]) {
+  if (E > 8) run_step<8, E>(k);
+  if (E > 4) run_step<4, E>(k);
+  run_step<2, E>(k);
+  run_step<1, E>(k);
+}
 
-/* Sort segments of S keys (16 S / 16 lanes), ascending; S = 64 .. 512. */
-__device__ __forceinline__ void run_sort(uint32_t k[16], int S, int lane) {
-  /* bitonic runs of 2, 4, 8 within the lane: descending where bit K of the
-   * index is set (the keys complemented) */
+/* Sort segments of S keys (thread t's are E t to E t + E - 1), ascending;
+ * S = 64 .. 512. */
+template <int W>
+__device__ __forceinline__ void run_sort(uint32_t k[16 / W], int S, int t,
+    RunX *X) {
+  constexpr int E = 16 / W;
+  /* bitonic runs within the thread: descending where bit K of the index is
+   * set (the keys complemented) */
 #pragma unroll
-  for (int K = 2; K < 16; K <<= 1) {
+  for (int K = 2; K < E; K <<= 1) {
 #pragma unroll
-    for (int i = 0; i < 16; i++)
+    for (int i = 0; i < E; i++)
       if (i & K) k[i] = ~k[i];
-    if (K > 4) run_step<4>(k);
-    if (K > 2) run_step<2>(k);
-    run_step<1>(k);
+    if (K > 4) run_step<4, E>(k);
+    if (K > 2) run_step<2, E>(k);
+    run_step<1, E>(k);
 #pragma unroll
-    for (int i = 0; i < 16; i++)
+    for (int i = 0; i < E; i++)
       if (i & K) k[i] = ~k[i];
   }
+  int buf = 0;
 #pragma unroll 1
-  for (int K = 16; K <= S; K <<= 1) {
-    const uint32_t m = (K < S && ((lane << 4) & K)) ? 0xffffffffu : 0u;
+  for (int K = E; K <= S; K <<= 1) {
+    const uint32_t m = (K < S && ((t * E) & K)) ? 0xffffffffu : 0u;
 #pragma unroll
-    for (int i = 0; i < 16; i++) k[i] ^= m;
+    for (int i = 0; i < E; i++) k[i] ^= m;
 #pragma unroll 1
-    for (int o = K >> 5; o > 0; o >>= 1) {
-      const bool low = !(lane & o);
+    for (int o = K / (2 * E); o > 0; o >>= 1) {
+      const bool low = !(t & o);
+      if (W > 1 && o >= 32) {
+        /* across warps */
+        uint32_t *x = X->k[buf];
+        buf ^= 1;
+        *(uint4 *) (x + E * t) = make_uint4(k[0], k[1], k[2], k[3]);
+        __syncthreads();
+        const uint4 q = *(const uint4 *) (x + E * (t ^ o));
+        const uint32_t b[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        const uint32_t b = __shfl_xor_sync(0xffffffffu, k[i], o);
-        k[i] = (low == (k[i] < b)) ? k[i] : b;
+        for (int i = 0; i < 4; i++)
+          k[i] = (low == (k[i] < b[i])) ? k[i] : b[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < E; i++) {
+          const uint32_t b = __shfl_xor_sync(0xffffffffu, k[i], o);
+          k[i] = (low == (k[i] < b)) ? k[i] : b;
+        }
       }
     }
-    run_step<8>(k);
-    run_step<4>(k);
-    run_step<2>(k);
-    run_step<1>(k);
+    run_steps<E>(k);
 #pragma unroll
-    for (int i = 0; i < 16; i++) k[i] ^= m;
+    for (int i = 0; i < E; i++) k[i] ^= m;
   }
 }
 
-/* One run: points [a, a + n) of the cell's, its first block b0. */
-__device__ __forceinline__ void run_order(RunSh *S, const float4 *key,
-    uint32_t a, int n, int lane) {
-  __syncwarp();
-  for (int i = lane; i < n; i += 32) {
+/* The order of one run, the n points from key[a] on. */
+template <int W>
+__device__ __forceinline__ void run_order(RunSh *S, RunX *X, const float4 *key,
+    uint32_t a, int n, int t) {
+  constexpr int E = 16 / W;
+  team_sync<W>();
+  for (int i = t; i < n; i += 32 * W) {
     const float4 v = key[a + i];
     S->c[0][i] = v.x;
     S->c[1][i] = v.y;
@@ -484,18 +564,18 @@ __device__ __forceinline__ void run_order(RunSh *S, const float4 *key,
     S->id[i] = __float_as_uint(v.w);
     S->ord[i] = (uint16_t) i;
   }
-  __syncwarp();
+  team_sync<W>();
   if (n <= 32) return;
-  uint32_t k[16];
+  uint32_t k[E];
 #pragma unroll
-  for (int i = 0; i < 16; i++) k[i] = (uint32_t) (16 * lane + i);
+  for (int i = 0; i < E; i++) k[i] = (uint32_t) (E * t + i);
 #pragma unroll 1
   for (int L = RUN_LEN; L >= 64; L >>= 1) {
     if (n <= L / 2) continue;       /* all in the first half already */
     /* the longest axis of each segment of L */
     float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
+    for (int i = 0; i < E; i++) {
       const int e = (int) (k[i] & (RUN_LEN - 1u));
       if (e < n)
 #pragma unroll
@@ -505,18 +585,35 @@ __device__ __forceinline__ void run_order(RunSh *S, const float4 *key,
           hi[d] = fmaxf(hi[d], v);
         }
     }
-    for (int o = L >> 5; o > 0; o >>= 1)
+    for (int o = L / (2 * E) < 16 ? L / (2 * E) : 16; o > 0; o >>= 1)
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
         hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
       }
+    if (W > 1 && L > 32 * E) {
+      const int w = t >> 5, nw = L / (32 * E);
+      __syncthreads();
+      if ((t & 31) == 0)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          X->r[w][d] = lo[d];
+          X->r[w][3 + d] = hi[d];
+        }
+      __syncthreads();
+      for (int q = w & ~(nw - 1), e = q + nw; q < e; q++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          lo[d] = fminf(lo[d], X->r[q][d]);
+          hi[d] = fmaxf(hi[d], X->r[q][3 + d]);
+        }
+    }
     const float ex = hi[0] - lo[0], ey = hi[1] - lo[1], ez = hi[2] - lo[2];
     const int d = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
     const float l = lo[d], w = hi[d] - lo[d];
     const float f = w > 0 ? 8388606.f / w : 0.f;
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
+    for (int i = 0; i < E; i++) {
       const uint32_t e = k[i] & (RUN_LEN - 1u);
       uint32_t q = 0x7fffffu;
       if ((int) e < n) {
@@ -525,20 +622,25 @@ __device__ __forceinline__ void run_order(RunSh *S, const float4 *key,
       }
       k[i] = q << 9 | e;
     }
-    run_sort(k, L, lane);
+    run_sort<W>(k, L, t, X);
   }
 #pragma unroll
-  for (int i = 0; i < 16; i++)
-    S->ord[16 * lane + i] = (uint16_t) (k[i] & (RUN_LEN - 1u));
-  __syncwarp();
+  for (int i = 0; i < E; i++)
+    S->ord[E * t + i] = (uint16_t) (k[i] & (RUN_LEN - 1u));
+  team_sync<W>();
 }
 
-template <int BATCH>
+template <int BATCH, int W>
 __global__ void __launch_bounds__(32 * RUN_WARPS) k_runs(const RunArgs A) {
-  __shared__ RunSh sh[RUN_WARPS];
-  const int lane = threadIdx.x & 31;
-  RunSh *S = sh + (threadIdx.x >> 5);
-  const uint32_t wid = blockIdx.x * RUN_WARPS + (threadIdx.x >> 5);
+  static_assert(W == 1 || W == RUN_WARPS, "a team is a warp or the block");
+  __shared__ RunSh sh[RUN_WARPS / W];
+  __shared__ __align__(16) unsigned char shx[W > 1 ? sizeof(RunX) : 16];
+  RunX *X = (RunX *) shx;
+  const int lane = threadIdx.x & 31, wt = W > 1 ? threadIdx.x >> 5 : 0;
+  const int t = W > 1 ? (int) threadIdx.x : lane;
+  RunSh *S = sh + (W > 1 ? 0 : threadIdx.x >> 5);
+  const uint32_t wid = W > 1 ? blockIdx.x
+      : blockIdx.x * RUN_WARPS + (threadIdx.x >> 5);
   const uint32_t r0 = wid % A.share, c0 = wid / A.share * A.group;
   if (c0 >= A.ncell) return;
   const uint32_t c1 = c0 + A.group < A.ncell ? c0 + A.group : A.ncell;
@@ -570,7 +672,7 @@ __global__ void __launch_bounds__(32 * RUN_WARPS) k_runs(const RunArgs A) {
         lo[k] = 0.0;
       }
     }
-    if (gap && lane == 0) {
+    if (gap && t == 0) {
       /* the place left unused: far from everything, no points */
       A.blk[2 * (size_t) (b + nb)] = make_float4(1e30f, 1e30f, 1e30f, 0.f);
       A.blk[2 * (size_t) (b + nb) + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -583,79 +685,105 @@ __global__ void __launch_bounds__(32 * RUN_WARPS) k_runs(const RunArgs A) {
     for (uint32_t r = r0; r < nrun; r += A.share) {
       const uint32_t q0 = r * RUN_LEN;
       const int m = (int) (n - q0 < RUN_LEN ? n - q0 : RUN_LEN);
-      run_order(S, A.key, a + q0, m, lane);
-      for (int j0 = 0; j0 < m; j0 += 32) {
-        const int j = j0 + lane;
-        float mn[3] = {3e38f, 3e38f, 3e38f}, mx[3] = {-3e38f, -3e38f, -3e38f};
-        const uint32_t pos = a + q0 + (uint32_t) j;
-        if (j < m) {
-          const uint32_t i = S->id[S->ord[j]];
-          const double v[3] = {A.x[i], A.y[i], A.z[i]};
-          const double wv = A.has_w ? A.w[i] : 1.0;
-          double ws = wv;
-          int wi = 1 << 30;
-          float wr = 0.f;
-          if (A.has_w) {
-            ws = ldexp(wv, -wexp);               /* |ws| <= 1 */
-            wi = (int) __double2ll_rn(ws * 1073741824.0);
-            wr = (float) (ws - (double) wi * (1.0 / 1073741824.0));
+      run_order<W>(S, X, A.key, a + q0, m, t);
+      /* blocks j = wt, wt + W, ..., up to four gathers in flight */
+#pragma unroll 1
+      for (int jb = 32 * wt; jb < m; jb += 128 * W) {
+        double v[4][3], wv[4], sv[4];
+        uint32_t id[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int j = jb + 32 * W * u + lane;
+          wv[u] = 1.0;
+          if (j < m) {
+            const uint32_t i = id[u] = S->id[S->ord[j]];
+            v[u][0] = __ldg(A.x + i);
+            v[u][1] = __ldg(A.y + i);
+            v[u][2] = __ldg(A.z + i);
+            if (A.has_w) wv[u] = __ldg(A.w + i);
+            if (A.ss) sv[u] = __ldg(A.s + i);
           }
-          float4 p;
-          p.x = (float) (v[0] - cc[0]);
-          p.y = (float) (v[1] - cc[1]);
-          p.z = (float) (v[2] - cc[2]);
-          p.w = (float) ws;
-          A.l4[pos] = p;
-          A.wq[pos] = make_int2(wi, __float_as_int(wr));
-          A.sx[pos] = v[0];
-          A.sy[pos] = v[1];
-          A.sz[pos] = v[2];
-          if (A.ss) A.ss[pos] = A.s[i];
-          A.sw[pos] = wv;
-          A.sid[pos] = i;
-          mn[0] = mx[0] = p.x;
-          mn[1] = mx[1] = p.y;
-          mn[2] = mx[2] = p.z;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int u = 0; u < 4; u++) {
+          const int j0 = jb + 32 * W * u, j = j0 + lane;
+          if (j0 >= m) break;
+          float mn[3] = {3e38f, 3e38f, 3e38f}, mx[3] = {-3e38f, -3e38f, -3e38f};
+          const uint32_t pos = a + q0 + (uint32_t) j;
+          if (j < m) {
+            double ws = wv[u];
+            int wi = 1 << 30;
+            float wr = 0.f;
+            if (A.has_w) {
+              ws = ldexp(wv[u], -wexp);          /* |ws| <= 1 */
+              wi = (int) __double2ll_rn(ws * 1073741824.0);
+              wr = (float) (ws - (double) wi * (1.0 / 1073741824.0));
+            }
+            float4 p;
+            p.x = (float) (v[u][0] - cc[0]);
+            p.y = (float) (v[u][1] - cc[1]);
+            p.z = (float) (v[u][2] - cc[2]);
+            p.w = (float) ws;
+            A.l4[pos] = p;
+            A.wq[pos] = make_int2(wi, __float_as_int(wr));
+            A.sx[pos] = v[u][0];
+            A.sy[pos] = v[u][1];
+            A.sz[pos] = v[u][2];
+            if (A.ss) A.ss[pos] = sv[u];
+            A.sw[pos] = wv[u];
+            A.sid[pos] = id[u];
+            mn[0] = mx[0] = p.x;
+            mn[1] = mx[1] = p.y;
+            mn[2] = mx[2] = p.z;
+          }
 #pragma unroll
-          for (int k = 0; k < 3; k++) {
-            mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+              mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+              mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+            }
+          if (lane == 0) {
+            float ce[3], e[3];
+            for (int k = 0; k < 3; k++) {
+              ce[k] = 0.5f * mn[k] + 0.5f * mx[k];
+              e[k] = __fmul_ru(fmaxf(__fsub_ru(mx[k], ce[k]),
+                                     __fsub_ru(ce[k], mn[k])), 1.000001f);
+            }
+            const size_t B = b + (q0 + (uint32_t) j0) / 32u;
+            const int cnt = m - j0 < 32 ? m - j0 : 32;
+            A.blk[2 * B] = make_float4(ce[0], ce[1], ce[2],
+                                       __uint_as_float(pos));
+            A.blk[2 * B + 1] = make_float4(e[0], e[1], e[2],
+                                           __uint_as_float((uint32_t) cnt));
+            A.bcell[B] = make_uint2(c, mk);
           }
-        if (lane == 0) {
-          float ce[3], e[3];
-          for (int k = 0; k < 3; k++) {
-            ce[k] = 0.5f * mn[k] + 0.5f * mx[k];
-            e[k] = __fmul_ru(fmaxf(__fsub_ru(mx[k], ce[k]),
-                                   __fsub_ru(ce[k], mn[k])), 1.000001f);
-          }
-          const size_t B = b + (q0 + (uint32_t) j0) / 32u;
-          const int cnt = m - j0 < 32 ? m - j0 : 32;
-          A.blk[2 * B] = make_float4(ce[0], ce[1], ce[2],
-                                     __uint_as_float(pos));
-          A.blk[2 * B + 1] = make_float4(e[0], e[1], e[2],
-                                         __uint_as_float((uint32_t) cnt));
-          A.bcell[B] = make_uint2(c, mk);
         }
       }
-      __syncwarp();
+      team_sync<W>();
     }
   }
 }
 
-/* Warps of k_runs for ncell cells of n points: 32 cells to a group where
- * there are many, and as many warps to a group as its cells have runs. */
+/* Teams of k_runs for ncell cells of n points: four warps where cells hold
+ * RUN_TEAM points on average; 32 cells to a group where there are many, and
+ * twice as many teams to a group as a cell has runs on average. */
+#define RUN_TEAM 96
 static void launch_runs(RunArgs *A, size_t n, cudaStream_t st) {
   A->group = A->ncell > 32u * 4864u ? 32u : (A->ncell > 4u * 4864u ? 4u : 1u);
   const size_t per = n / A->ncell / RUN_LEN + 1;
   A->share = (uint32_t) (per * 2 < 256 ? per * 2 : 256);
-  const uint64_t warps =
+  const uint64_t teams =
       ((uint64_t) A->ncell + A->group - 1) / A->group * A->share;
-  const unsigned nb = (unsigned) ((warps + RUN_WARPS - 1) / RUN_WARPS);
-  if (A->cat) k_runs<1><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
-  else k_runs<0><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
+  if (n >= (size_t) RUN_TEAM * A->ncell) {
+    const unsigned nb = (unsigned) teams;
+    if (A->cat) k_runs<1, RUN_WARPS><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
+    else k_runs<0, RUN_WARPS><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
+  } else {
+    const unsigned nb = (unsigned) ((teams + RUN_WARPS - 1) / RUN_WARPS);
+    if (A->cat) k_runs<1, 1><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
+    else k_runs<0, 1><<<nb, 32 * RUN_WARPS, 0, st>>>(*A);
+  }
 }
 
 extern "C" int fcfcg_grid_sub_bits(size_t ncell, size_t npoint) {
@@ -678,7 +806,7 @@ extern "C" int fcfcg_grid_curve_bits(size_t ncell, size_t npoint) {
   return fcfcg_grid_sub_bits(ncell, npoint);
 }
 
-/* The blocks' numbering from the cells' points: with gaps (k_cstart) unless
+/* The blocks' numbering from the cells' points: with gaps (k_scan_apply) unless
  * cells far outnumber the blocks, where it is compacted by a scan. */
 static int gaps_ok(size_t n, size_t nc) { return nc <= 4096 || nc <= n / 16; }
 
@@ -690,13 +818,11 @@ extern "C" size_t fcfcg_max_blocks(size_t n, size_t ncell) {
 static int sort_rest(cudaStream_t st, size_t nc, size_t n, int sb,
     uint32_t *cfill, uint32_t *fstart, uint32_t *scan_tmp, uint32_t *cstart,
     uint32_t *bstart) {
-  int r = scan_u32(st, cfill, nc << sb, fstart, scan_tmp);
-  if (r) return r;
   const int gaps = gaps_ok(n, nc);
-  k_cstart<<<grid_for(nc + 1, PREP_THREADS), PREP_THREADS, 0, st>>>(
-      nc, sb, fstart, cstart, gaps ? bstart : NULL);
-  cudaError_t e = cudaGetLastError();
-  if (e || gaps) return (int) e;
+  int r = scan_u32(st, cfill, nc << sb, fstart, scan_tmp, sb, cstart,
+                   gaps ? bstart : NULL);
+  if (r || gaps) return r;
+  cudaError_t e;
   k_block_count<<<grid_for(nc, PREP_THREADS), PREP_THREADS, 0, st>>>(
       cstart, (uint32_t) nc, cfill);
   if ((e = cudaGetLastError())) return (int) e;
@@ -791,7 +917,6 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep_batch(
     const fcfcg_prep_cat *__restrict__ cat, int ncat, double rescale,
     int withwt, double *ox, double *oy, double *oz, double *ow,
     unsigned long long *bstat, double *__restrict__ partial) {
-  __shared__ double sh_sum[PREP_THREADS];
   const uint32_t t = blockIdx.x;
   const int a = batch_cat(cat, ncat, t);
   const fcfcg_prep_cat *C = cat + a;
@@ -823,34 +948,10 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep_batch(
       wm = bits > wm ? bits : wm;
     }
   }
-  unsigned long long *B = bstat + 8 * (size_t) a;
-  for (int k = 0; k < 3; k++) {
-    for (int s = 16; s > 0; s >>= 1) {
-      const unsigned long long p = __shfl_xor_sync(0xffffffffu, lo[k], s);
-      const unsigned long long q = __shfl_xor_sync(0xffffffffu, hi[k], s);
-      lo[k] = p < lo[k] ? p : lo[k];
-      hi[k] = q > hi[k] ? q : hi[k];
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicMin(B + k, lo[k]);
-      atomicMax(B + 3 + k, hi[k]);
-    }
-  }
+  block_range(lo, hi, wm, bstat + 8 * (size_t) a);
   if (!withwt) return;
-  for (int s = 16; s > 0; s >>= 1) {
-    const unsigned long long p = __shfl_xor_sync(0xffffffffu, wm, s);
-    wm = p > wm ? p : wm;
-  }
-  if ((threadIdx.x & 31) == 0 && wm) atomicMax(B + 6, wm);
-  sh_sum[threadIdx.x] = ws;
-  __syncthreads();
-  for (int s = PREP_THREADS / 2; s > 0; s >>= 1) {
-    if ((int) threadIdx.x < s)
-      sh_sum[threadIdx.x] = __dadd_rn(sh_sum[threadIdx.x],
-                                      sh_sum[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[t] = sh_sum[0];
+  const double s = block_sum(ws);
+  if (threadIdx.x == 0) partial[t] = s;
 }
 
 /* Block a: catalogue a's weight sum from its tiles' sums, in a fixed order,
@@ -858,23 +959,16 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep_batch(
 __global__ void __launch_bounds__(PREP_THREADS) k_sum_batch(
     const fcfcg_prep_cat *__restrict__ cat, int ncat, uint32_t ntile,
     const double *__restrict__ partial, unsigned long long *bstat) {
-  __shared__ double sh[PREP_THREADS];
   const int a = blockIdx.x;
   const uint32_t t0 = cat[a].tile0;
   const uint32_t t1 = (a + 1 < ncat) ? cat[a + 1].tile0 : ntile;
   double v = 0;
   for (uint32_t t = t0 + threadIdx.x; t < t1; t += PREP_THREADS)
     v = __dadd_rn(v, partial[t]);
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = PREP_THREADS / 2; s > 0; s >>= 1) {
-    if ((int) threadIdx.x < s)
-      sh[threadIdx.x] = __dadd_rn(sh[threadIdx.x], sh[threadIdx.x + s]);
-    __syncthreads();
-  }
+  const double s = block_sum(v);
   if (threadIdx.x == 0)
     bstat[8 * (size_t) a + 7] =
-        (unsigned long long) __double_as_longlong(sh[0]);
+        (unsigned long long) __double_as_longlong(s);
 }
 
 extern "C" int fcfcg_k_prep_batch(void *stream, const fcfcg_prep_cat *d_cat,
