@@ -48,6 +48,10 @@ __global__ void k_recheck(const fcfcg_launch L) {
   if ((threadIdx.x & 31) == 0 && n_in) atomicAdd(L.stats + 1, n_in);
 }
 
+/* Shared memory of a launch: 200 KB (ctx.c: count_plan_make) and the spare
+ * words. */
+#define SMEM_MAX (201 * 1024)
+
 /* FP64 sums: the copies in pairs, then those sums, ... into the first. */
 __global__ void k_gwd_fold(double *gwd, long ntot, int copies) {
   const long i = blockIdx.x * (long) blockDim.x + threadIdx.x;
@@ -66,7 +70,7 @@ __global__ void k_gwd_fold(double *gwd, long ntot, int copies) {
 /* ------------------------------------------------------------------------ */
 
 extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
-    int precision, int nsm, size_t *smem_used) {
+    int precision, int nsm, fcfcg_occ *occ) {
   int bin = L->bintype;
   if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
   if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
@@ -83,14 +87,26 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
       fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
   const int threads = CT32_THREADS;
   int per_sm = 0;
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute((const void *) f,
-           cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-           &per_sm, (const void *) f, threads, smem)))
-    return (int) e;
-  if (per_sm < 1) return (int) cudaErrorInvalidConfiguration;
-  if (smem_used) *smem_used = smem;
+  for (int i = 0; i < FCFCG_OCC; i++)
+    if (occ->f[i] == (const void *) f && occ->smem[i] == smem)
+      per_sm = occ->per_sm[i];
+  if (!per_sm) {
+    /* (the attribute is the device's, for every context: always the most
+     * that any launch takes) */
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute((const void *) f,
+             cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX)) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+             &per_sm, (const void *) f, threads, smem)))
+      return (int) e;
+    if (per_sm < 1 || smem > SMEM_MAX)
+      return (int) cudaErrorInvalidConfiguration;
+    const int i = occ->next;
+    occ->f[i] = (const void *) f;
+    occ->smem[i] = smem;
+    occ->per_sm[i] = per_sm;
+    occ->next = (i + 1) % FCFCG_OCC;
+  }
   f<<<nsm * per_sm, threads, smem, (cudaStream_t) stream>>>(*L);
   const int copies = fcfcg_gwd_copies(L->ntot);
   if (f64 && L->withwt && !L->adjoint && copies > 1)
@@ -111,11 +127,14 @@ extern "C" size_t fcfcg_k_tile32_hist(int hlen, int withwt) {
   return ((size_t) hlen + 32) * (withwt ? 8 : 4);
 }
 
+#define RECHECK_CTAS 4
 extern "C" int fcfcg_k_recheck(void *stream, const fcfcg_launch *L,
     uint32_t nq_bound) {
   if (!nq_bound) return 0;
+  /* (a queue is mostly short, or empty: more blocks than fit at once cost a
+   * launch more than they gain a long one) */
   unsigned blocks = (nq_bound + 255) / 256;
-  if (blocks > 152 * 16) blocks = 152 * 16;
+  if (blocks > 152 * RECHECK_CTAS) blocks = 152 * RECHECK_CTAS;
   if (L->adjoint)
     k_recheck_adj<<<blocks, 256, 0, (cudaStream_t) stream>>>(*L);
   else if (L->withwt)

@@ -59,14 +59,18 @@ struct fcfcg_ctx {
   uint16_t *d_rs, *d_rp;
   double *d_s2edge, *d_pedge;
   float *d_se, *d_pe;             /* edge tables of the tile kernel */
-  int *d_sten;
-  float *d_stenD;
-  unsigned long long *d_cnt, *d_wt, *d_stats, *d_bbox;
+  int *d_sten;                    /* the stencil's entries, displacements */
+  int sten_up;                    /* entries there (h_sten holds them) */
+  int *h_sten;                    /* pinned: what was copied there */
+  /* RES_HDR words (statistics, then the work counter and the queue's fill),
+   * then the histogram: ntot counts, or 2 ntot words of weighted sums */
+  unsigned long long *d_res;
+  unsigned long long *d_hist, *d_stats, *d_bbox;
+  fcfcg_occ occ;                  /* launch shapes of the count kernels */
   double *d_wd;
   int *d_gtab;                   /* adjoint: the scaled cotangent */
   size_t gtab_cap;
-  uint32_t *d_head, *d_queue;      /* d_head: chunk counter, pad, fill */
-  unsigned long long *d_qcount;    /* queue fill (64-bit), in d_head */
+  uint32_t *d_queue;
   size_t qcap, qcap_alloc;
   int qcap_user;                  /* capacity set by fcfcg_set_queue_capacity */
   void *h_pinned;
@@ -181,6 +185,11 @@ static int grow(fcfcg_ctx *c, void **p, size_t *cap, size_t need) {
     (capv) = cap_;                                                          \
   } while (0)
 
+#define RES_HDR 16
+#define RES_HEAD 8                /* words: the work counter (32 bits), */
+#define RES_FILL 9                /* the recheck queue's fill */
+#define STEN_BYTES ((size_t) 32 * FCFCG_MAX_STENCIL)
+
 static int upload(fcfcg_ctx *c, void **dst, const void *src, size_t bytes) {
   if (*dst) cudaFree(*dst);
   *dst = NULL;
@@ -207,8 +216,8 @@ void fcfcg_destroy(fcfcg_ctx *c) {
     for (int i = 0; i <= FCFCG_MAX_SLOT; i++) slot_free(c->slot + i);
     void *p[] = {c->cfill, c->fstart, c->rank, c->key, c->scan_tmp,
                  c->d_se, c->d_pe, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
-                 c->d_sten, c->d_stenD, c->d_cnt, c->d_wt, c->d_stats,
-                 c->d_bbox, c->d_wd, c->d_gtab, c->d_head, c->d_queue, c->d_cnvt,
+                 c->d_sten, c->d_res,
+                 c->d_bbox, c->d_wd, c->d_gtab, c->d_queue, c->d_cnvt,
                  c->d_mock, c->d_mbase, c->d_bout, c->d_bstat, c->d_grad,
                  c->d_wpart, c->d_pcat, c->d_bpart};
     for (size_t i = 0; i < sizeof p / sizeof p[0]; i++)
@@ -285,21 +294,23 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
                 sizeof(double) * (b->p.nbin + 1));
     if (rc) return rc;
   }
-  CK(cudaMalloc((void **) &c->d_cnt, sizeof(unsigned long long) * b->ntot));
-  CK(cudaMalloc((void **) &c->d_wt, sizeof(unsigned long long) * 2 * b->ntot));
+  CK(cudaMalloc((void **) &c->d_res,
+                sizeof(unsigned long long) * (RES_HDR + 2 * b->ntot)));
+  c->d_stats = c->d_res;
+  c->d_hist = c->d_res + RES_HDR;
   CK(cudaMalloc((void **) &c->d_wd,
                 sizeof(double) * b->ntot * fcfcg_gwd_copies(b->ntot)));
-  CK(cudaMalloc((void **) &c->d_stats, sizeof(unsigned long long) * 8));
   CK(cudaMalloc((void **) &c->d_wpart,
                 sizeof(double) * fcfcg_prep_partials()));
-  CK(cudaMallocHost((void **) &c->h_load, sizeof(unsigned long long) * 8));
+  CK(cudaMalloc((void **) &c->d_sten, STEN_BYTES));
+  CK(cudaMallocHost((void **) &c->h_load,
+                    sizeof(unsigned long long) * 8 + STEN_BYTES));
+  c->h_sten = (int *) (c->h_load + 8);
   memset(c->h_load, 0, sizeof(unsigned long long) * 8);
   for (int k = 0; k < 3; k++) c->h_load[k] = ~0ull;
   rc = upload(c, (void **) &c->d_bbox, c->h_load,
               sizeof(unsigned long long) * 8);
   if (rc) return rc;
-  CK(cudaMalloc((void **) &c->d_head, sizeof(uint32_t) * 4));
-  c->d_qcount = (unsigned long long *) (c->d_head + 2);
   c->qcap = c->qcap_alloc = (size_t) 1 << 25;   /* 32M pairs, 512 MiB */
   CK(cudaMalloc((void **) &c->d_queue, sizeof(uint32_t) * 4 * c->qcap));
   CK(cudaStreamSynchronize(c->stream));
@@ -1270,6 +1281,24 @@ static int warp_queue(const fcfcg_ctx *c) {
   return c->qwarp_force ? (int) c->qwarp_force : 1024;
 }
 
+/* The context's stencil (c->sten, c->stD) to the device, in one copy from
+ * pinned memory; not where the device holds the same entries already.
+ * Called with the stream idle. */
+static int stencil_upload(fcfcg_ctx *c, int nsten, fcfcg_launch *L) {
+  const size_t m = (size_t) nsten * 4;
+  L->sten = c->d_sten;
+  L->stenD = (const float *) (c->d_sten + m);
+  if (nsten == c->sten_up && !memcmp(c->h_sten, c->sten, sizeof(int) * m) &&
+      !memcmp(c->h_sten + m, c->stD, sizeof(float) * m))
+    return FCFCG_OK;
+  memcpy(c->h_sten, c->sten, sizeof(int) * m);
+  memcpy(c->h_sten + m, c->stD, sizeof(float) * m);
+  c->sten_up = nsten;
+  CK(cudaMemcpyAsync(c->d_sten, c->h_sten, sizeof(int) * 2 * m,
+                     cudaMemcpyHostToDevice, c->stream));
+  return FCFCG_OK;
+}
+
 /* Launch fields of a sorted catalogue. */
 static void launch_cat(fcfcg_dcat *D, const slot_t *S) {
   D->l4 = S->l4;
@@ -1313,11 +1342,12 @@ static void launch_bins(const fcfcg_ctx *c, fcfcg_launch *L) {
     L->pmax = b->p.vmax;
     L->pmin0 = b->p.min0;
   }
-  L->gcnt = c->d_cnt;
-  L->gwt = c->d_wt;
+  L->gcnt = c->d_hist;
+  L->gwt = c->d_hist;
   L->gwd = c->d_wd;
   L->queue = c->d_queue;
-  L->qcount = c->d_qcount;
+  L->qcount = c->d_res + RES_FILL;
+  L->chunk_head = (uint32_t *) (c->d_res + RES_HEAD);
   L->qcap = (uint32_t) c->qcap;
   L->stats = c->d_stats;
 }
@@ -1387,7 +1417,6 @@ static int tile_parts(size_t n, size_t ncell, int nsm) {
   return p;
 }
 
-#define STAT_WORDS 5   /* candidates, in range, rechecked, inline, chunks */
 
 static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
     int withwt, int precision, int adj, int *sten, float *stD,
@@ -1446,7 +1475,6 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   L->tzero = -1;
   for (int t = 0; t < P->nsten; t++)
     if (!sten[4 * t] && !sten[4 * t + 1] && !sten[4 * t + 2]) L->tzero = t;
-  L->chunk_head = c->d_head;
   L->nblk_dev = A->bstart + P->ncell;
   launch_cat(&L->A, A);
   launch_cat(&L->B, B);
@@ -1459,33 +1487,34 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   return FCFCG_OK;
 }
 
+/* Words of a count's result on the device, from d_res on. */
+static size_t res_words(const fcfcg_bins *b, int withwt) {
+  return RES_HDR + (size_t) b->ntot * (withwt ? 2 : 1);
+}
+
 /* Stream side of a count.  sort_a / sort_b: sort that catalogue into the
  * plan's grid first.  timed: record the context's events (not while
- * capturing).  res (pinned, 2 ntot words) and stats (pinned, STAT_WORDS
- * words): where the histogram and the statistics go; NULL for none. */
+ * capturing).  res (pinned, RES_HDR + 2 ntot words): where the statistics
+ * and (hist) the histogram go, in one copy. */
 static int count_launch(fcfcg_ctx *c, const count_plan *P, int sort_a,
-    int sort_b, int timed, void *res, unsigned long long *stats) {
+    int sort_b, int timed, unsigned long long *res, int hist) {
   const fcfcg_bins *b = &c->bins;
   const fcfcg_launch *L = &P->L;
+  const int wd = P->withwt && P->prec == FCFCG_PREC_FP64;
   int rc;
   if (timed) CK(cudaEventRecord(c->ev[0], c->stream));
   if (sort_a && (rc = slot_sort(c, P->A, &P->g))) return rc;
   if (sort_b && P->B != P->A && (rc = slot_sort(c, P->B, &P->g))) return rc;
   if (timed) CK(cudaEventRecord(c->ev[1], c->stream));
-  CK(cudaMemsetAsync(c->d_cnt, 0, sizeof(unsigned long long) * b->ntot,
+  const size_t words = res_words(b, P->withwt);
+  CK(cudaMemsetAsync(c->d_res, 0, sizeof(unsigned long long) * words,
                      c->stream));
-  CK(cudaMemsetAsync(c->d_wt, 0, sizeof(unsigned long long) * 2 * b->ntot,
-                     c->stream));
-  if (L->withwt && !L->adjoint && P->prec == FCFCG_PREC_FP64)
+  if (wd && hist)
     CK(cudaMemsetAsync(c->d_wd, 0,
                        sizeof(double) * b->ntot * fcfcg_gwd_copies(b->ntot),
                        c->stream));
-  CK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * 4,
-                     c->stream));
-  CK(cudaMemsetAsync(c->d_head, 0, sizeof(uint32_t) * 4, c->stream));
   if (timed) CK(cudaEventRecord(c->ev[2], c->stream));
-  size_t smem = 0;
-  CKK(fcfcg_k_count(c->stream, L, P->prec, c->nsm, &smem));
+  CKK(fcfcg_k_count(c->stream, L, P->prec, c->nsm, &c->occ));
   c->launches += 1;
   if (timed) CK(cudaEventRecord(c->ev[3], c->stream));
   if (P->prec == FCFCG_PREC_FP32_RECHECK) {
@@ -1494,37 +1523,23 @@ static int count_launch(fcfcg_ctx *c, const count_plan *P, int sort_a,
     c->launches += 1;
   }
   if (timed) CK(cudaEventRecord(c->ev[4], c->stream));
-  if (res) {
-    if (P->withwt && P->prec == FCFCG_PREC_FP64)
-      CK(cudaMemcpyAsync(res, c->d_wd, sizeof(double) * b->ntot,
-                         cudaMemcpyDeviceToHost, c->stream));
-    else if (P->withwt)
-      CK(cudaMemcpyAsync(res, c->d_wt,
-                         sizeof(unsigned long long) * 2 * b->ntot,
-                         cudaMemcpyDeviceToHost, c->stream));
-    else
-      CK(cudaMemcpyAsync(res, c->d_cnt, sizeof(unsigned long long) * b->ntot,
-                         cudaMemcpyDeviceToHost, c->stream));
-  }
-  if (stats) {
-    CK(cudaMemcpyAsync(stats, c->d_stats, sizeof(unsigned long long) * 4,
+  CK(cudaMemcpyAsync(res, c->d_res,
+                     sizeof(unsigned long long) * (hist && !wd ? words : RES_HDR),
+                     cudaMemcpyDeviceToHost, c->stream));
+  if (hist && wd)
+    CK(cudaMemcpyAsync(res + RES_HDR, c->d_wd, sizeof(double) * b->ntot,
                        cudaMemcpyDeviceToHost, c->stream));
-    /* the block count (32 bits) into the low half of the last word */
-    stats[4] = 0;
-    CK(cudaMemcpyAsync(stats + 4, L->nblk_dev, sizeof(uint32_t),
-                       cudaMemcpyDeviceToHost, c->stream));
-  }
   return FCFCG_OK;
 }
 
 /* Host side after the stream finished: the caller's histogram and the
  * statistics (timings are the caller's). */
-static void count_finish(fcfcg_ctx *c, const count_plan *P, const void *res,
+static void count_finish(fcfcg_ctx *c, const count_plan *P,
     const unsigned long long *stats, int64_t *icnt, double *wcnt) {
   const fcfcg_bins *b = &c->bins;
-  const unsigned long long *hres = (const unsigned long long *) res;
+  const unsigned long long *hres = stats + RES_HDR;
   if (P->withwt && P->prec == FCFCG_PREC_FP64) {
-    memcpy(wcnt, res, sizeof(double) * b->ntot);
+    memcpy(wcnt, hres, sizeof(double) * b->ntot);
   } else if (P->withwt) {
     const int ex = P->A->wexp + P->B->wexp - FCFCG_FIX_F;
     for (long i = 0; i < b->ntot; i++) {
@@ -1593,12 +1608,6 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
   rc = count_plan_make(c, A, B, isauto, withwt, precision, adj != NULL,
                        c->sten, c->stD, &P);
   if (rc) return rc;
-  rc = upload(c, (void **) &c->d_sten, c->sten, sizeof(int) * 4 * P.nsten);
-  if (rc) return rc;
-  rc = upload(c, (void **) &c->d_stenD, c->stD, sizeof(float) * 4 * P.nsten);
-  if (rc) return rc;
-  P.L.sten = c->d_sten;
-  P.L.stenD = c->d_stenD;
   const int sort_a = !slot_in_grid(A, &P.g);
   const int sort_b = (B != A) && !slot_in_grid(B, &P.g);
   fcfcg_launch *L = &P.L;
@@ -1641,12 +1650,11 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
       gtab_exp = gexp;
     }
   }
-  const size_t rbytes = sizeof(unsigned long long) * (2 * b->ntot + STAT_WORDS);
+  const size_t rbytes = sizeof(unsigned long long) * (RES_HDR + 2 * b->ntot);
   const size_t gbytes = (adj && P.prec == FCFCG_PREC_FP32_RECHECK) ? sizeof(int) * 2 * ((size_t) L->hlen + 32)
                                         : 0;
   if ((rc = ensure_pinned(c, rbytes + gbytes))) return rc;
-  unsigned long long *hres = (unsigned long long *) c->h_pinned;
-  unsigned long long *hstats = hres + 2 * b->ntot;
+  unsigned long long *hstats = (unsigned long long *) c->h_pinned;
   if (gbytes) {
     /* per shared bin: the entry as an integer and a remainder; 0 around the
      * bins and in the spare words */
@@ -1666,7 +1674,8 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
                        c->stream));
     L->gtab = c->d_gtab;
   }
-  rc = count_launch(c, &P, sort_a, sort_b, 1, adj ? NULL : hres, hstats);
+  if ((rc = stencil_upload(c, P.nsten, &P.L))) return rc;
+  rc = count_launch(c, &P, sort_a, sort_b, 1, hstats, !adj);
   if (rc) return rc;
   slot_mark(A, &P.g);
   if (B != A) slot_mark(B, &P.g);
@@ -1697,7 +1706,7 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
     o->warp_queue = P.prec == FCFCG_PREC_FP32_RECHECK ? warp_queue(c) : 0;
     o->launches = c->launches;
   } else {
-    count_finish(c, &P, hres, hstats, icnt, wcnt);
+    count_finish(c, &P, hstats, icnt, wcnt);
   }
   if (hstats[3]) queue_grow(c, hstats[2] + hstats[2] / 4);
   fcfcg_stats *o = &c->stats;
@@ -1724,7 +1733,7 @@ struct fcfcg_graph {
   int empty[FCFCG_MAX_GRAPH_ITEMS];
   int *d_sten[FCFCG_MAX_GRAPH_ITEMS];
   float *d_stenD[FCFCG_MAX_GRAPH_ITEMS];
-  unsigned long long *h_stage;   /* pinned: per item 2 ntot + STAT_WORDS */
+  unsigned long long *h_stage;   /* pinned: per item RES_HDR + 2 ntot */
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   unsigned long bufgen;          /* the context's, when captured */
@@ -1749,7 +1758,7 @@ static void graph_release(fcfcg_graph *G) {
 }
 
 static unsigned long long *stage_of(const fcfcg_graph *G, int i) {
-  return G->h_stage + (size_t) i * (2 * (size_t) G->c->bins.ntot + STAT_WORDS);
+  return G->h_stage + (size_t) i * (RES_HDR + 2 * (size_t) G->c->bins.ntot);
 }
 
 /* Plan every item and capture their launches as one graph. */
@@ -1795,9 +1804,7 @@ static int graph_build(fcfcg_graph *G) {
   int rc = FCFCG_OK;
   for (int i = 0; i < G->n && !rc; i++) {
     if (G->empty[i]) continue;
-    unsigned long long *st = stage_of(G, i);
-    rc = count_launch(c, G->plan + i, 1, 1, 0, st,
-                      st + 2 * (size_t) c->bins.ntot);
+    rc = count_launch(c, G->plan + i, 1, 1, 0, stage_of(G, i), 1);
   }
   cudaGraph_t gr = NULL;
   cudaError_t e = cudaStreamEndCapture(c->stream, &gr);
@@ -1850,7 +1857,7 @@ int fcfcg_graph_create(fcfcg_ctx *c, const fcfcg_count_item *items,
   G->n = nitem;
   G->precision = precision;
   memcpy(G->item, items, sizeof *items * nitem);
-  const size_t words = (size_t) nitem * (2 * (size_t) c->bins.ntot + STAT_WORDS);
+  const size_t words = (size_t) nitem * (RES_HDR + 2 * (size_t) c->bins.ntot);
   cudaError_t e = cudaMallocHost((void **) &G->h_stage,
                                  sizeof(unsigned long long) * words);
   if (e != cudaSuccess) {
@@ -1916,8 +1923,7 @@ int fcfcg_graph_run(fcfcg_graph *G) {
       if (it->wcnt) memset(it->wcnt, 0, sizeof(double) * ntot);
       continue;
     }
-    const unsigned long long *st = stage_of(G, i);
-    count_finish(c, G->plan + i, st, st + 2 * (size_t) ntot,
+    count_finish(c, G->plan + i, stage_of(G, i),
                  it->withwt ? NULL : it->icnt, it->withwt ? it->wcnt : NULL);
   }
   for (int s = 0; s < FCFCG_MAX_SLOT; s++)
@@ -1926,7 +1932,7 @@ int fcfcg_graph_run(fcfcg_graph *G) {
    * (which capture again) */
   unsigned long long need = 0;
   for (int i = 0; i < G->n; i++) {
-    const unsigned long long *st = stage_of(G, i) + 2 * (size_t) c->bins.ntot;
+    const unsigned long long *st = stage_of(G, i);
     if (!G->empty[i] && st[3] && st[2] > need) need = st[2];
   }
   if (need) queue_grow(c, need + need / 4);
@@ -2528,51 +2534,32 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   for (int t = 0; t < nsten; t++)
     if (!c->sten[4 * t] && !c->sten[4 * t + 1] && !c->sten[4 * t + 2])
       L.tzero = t;
-  if ((rc = upload(c, (void **) &c->d_sten, c->sten,
-                   sizeof(int) * 4 * nsten))) {
+  if ((rc = stencil_upload(c, nsten, &L))) {
     free(wexp);
     goto out;
   }
-  if ((rc = upload(c, (void **) &c->d_stenD, c->stD,
-                   sizeof(float) * 4 * nsten))) {
-    free(wexp);
-    goto out;
-  }
-  L.sten = c->d_sten;
-  L.stenD = c->d_stenD;
   /* 8. count */
   BCK(cudaEventRecord(c->ev[1], c->stream));
-  L.chunk_head = c->d_head;
-  BCK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * 4,
+  BCK(cudaMemsetAsync(c->d_res, 0, sizeof(unsigned long long) * RES_HDR,
                       c->stream));
-  BCK(cudaMemsetAsync(c->d_head, 0, sizeof(uint32_t) * 4, c->stream));
   BCK(cudaEventRecord(c->ev[2], c->stream));
-  size_t smem = 0;
-  BCKK(fcfcg_k_count(c->stream, &L, prec, c->nsm, &smem));
+  BCKK(fcfcg_k_count(c->stream, &L, prec, c->nsm, &c->occ));
   c->launches += 1;
   BCK(cudaEventRecord(c->ev[3], c->stream));
-  unsigned long long nq = 0;
-  BCK(cudaMemcpyAsync(&nq, c->d_qcount, sizeof nq, cudaMemcpyDeviceToHost,
-                      c->stream));
-  BCK(cudaStreamSynchronize(c->stream));
-  if (nq > c->qcap) nq = c->qcap;
-  BCKK(fcfcg_k_recheck(c->stream, &L, (uint32_t) nq));
-  c->launches += nq ? 1 : 0;
+  BCKK(fcfcg_k_recheck(c->stream, &L, (uint32_t) c->qcap));
+  c->launches += 1;
   BCK(cudaEventRecord(c->ev[4], c->stream));
   /* 9. results */
   {
     unsigned long long *hres = malloc(sizeof(unsigned long long) * per * na);
-    unsigned long long hstats[4];
+    unsigned long long hstats[RES_HDR];
     if (!hres) {
       free(wexp);
       BFAIL(FCFCG_ERR_MEMORY);
     }
-    uint32_t nblk = 0;
     cudaError_t e = cudaMemcpyAsync(hres, c->d_bout,
                                     sizeof(unsigned long long) * per * na,
                                     cudaMemcpyDeviceToHost, c->stream);
-    if (!e) e = cudaMemcpyAsync(&nblk, L.nblk_dev, sizeof nblk,
-                                cudaMemcpyDeviceToHost, c->stream);
     if (!e) e = cudaMemcpyAsync(hstats, c->d_stats, sizeof hstats,
                                 cudaMemcpyDeviceToHost, c->stream);
     if (!e) e = cudaStreamSynchronize(c->stream);
@@ -2613,7 +2600,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
     o->ms_total = ms;
     o->cells_per_smax = k;
     o->nstencil = nsten;
-    o->nchunks = nblk;
+    o->nchunks = (uint32_t) hstats[4];
     o->precision_used = prec;
     o->warp_queue = prec == FCFCG_PREC_FP32_RECHECK ? warp_queue(c) : 0;
     o->launches = c->launches;

@@ -181,7 +181,7 @@ typedef struct {
   unsigned long long *qcount;  /* fill: 64 bits, so it cannot wrap */
   uint32_t qcap;
   unsigned long long *stats;   /* [0] candidates [1] in-range [2] recheck
-                                  [3] inline rechecks */
+                                  [3] inline rechecks [4] blocks */
   int hist_smem;               /* histogram in shared memory */
   /* unweighted shared histogram: pairs a CTA adds between hand-overs to
    * the global counters, at most 2^32 - 1 (u32 bins) */
@@ -291,10 +291,16 @@ size_t fcfcg_k_tile32_tab(const fcfcg_launch *L);
 size_t fcfcg_k_tile32_stage(int kind);
 /* And its histogram's, with a spare word per lane. */
 size_t fcfcg_k_tile32_hist(int hlen, int withwt);
-/* The count kernel of a launch; *smem_used (may be NULL): its shared memory
- * per CTA. */
+/* The count kernel of a launch.  occ: the CTAs per SM of the launches so
+ * far (a context's; the last FCFCG_OCC shapes). */
+#define FCFCG_OCC 8
+typedef struct {
+  const void *f[FCFCG_OCC];
+  size_t smem[FCFCG_OCC];
+  int per_sm[FCFCG_OCC], next;
+} fcfcg_occ;
 int fcfcg_k_count(void *stream, const fcfcg_launch *L, int precision,
-    int nsm, size_t *smem_used);
+    int nsm, fcfcg_occ *occ);
 /* Bits of the coarse cells (dim, cells of 1 / inv_cell from lo) that hold
  * an object, and their number (count). */
 int fcfcg_k_occupancy(void *stream, size_t n, const double *x,

@@ -925,6 +925,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
       h[i] = 0;
   }
   const uint32_t nitem = __ldg(L.nblk_dev) << L.pshift;
+  if (blockIdx.x == 0 && threadIdx.x == 0) L.stats[4] = nitem >> L.pshift;
   const uint32_t np = 1u << L.pshift;
   /* a warp's share of the pairs a 32-bit bin holds, less what it can add
    * between two looks at it */
