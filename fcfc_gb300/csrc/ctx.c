@@ -1405,18 +1405,37 @@ typedef struct {
   fcfcg_launch L;                /* stencil pointers: set by the caller */
 } count_plan;
 
-/* log2 of the parts the tiles of a block are dealt to, so that a small
- * catalogue still gives every warp of the GPU a few items: 8 items per
- * warp (32 warps per SM), at most 16 parts (a part repeats the box tests of
- * its block's neighbours). */
-static int tile_parts(size_t n, size_t ncell, int nsm) {
-  const double blocks = (double) n / 32 + 0.5 * (double) (n < ncell ? n : ncell);
-  const double want = 8.0 * 32 * nsm;
-  int p = 0;
-  while (p < 4 && blocks * (double) (1 << p) < want) p++;
-  return p;
+/*
+ * The items of the tile kernel: the blocks of na points in ncell cells, the
+ * last nsplit of them (all, of a small catalogue) in 2^pshift parts, by groups
+ * of 32 neighbour blocks.  Whole blocks cost the least, but a warp's last one
+ * is a sixteenth of a count of 1e6 points; with the last 2 blocks per warp (32
+ * warps per SM) in parts none is left waiting long (2e6 points, (s, mu): 24.0
+ * -> 23.5 ms; before, every block was dealt tile by tile, each part testing
+ * the boxes of all: 1e5 points 827 -> 655 us a pass).  As many parts as make 8
+ * items per warp, but while that suffices for 4, none below 3.5 groups (nb:
+ * points of the neighbour side; nsten cells each).  Where 16 parts make less
+ * than an item per warp (16 with f64, whose tiles are long), up to 8 times as
+ * many by single tiles (tshift of the log).  A batch, whose CTAs wait for
+ * their last warp at the end of every run of items: all blocks, 16 items per
+ * warp (48 mocks of 2e4 to 6e4 points: 6.81 ms; 7.08 with 8, 7.16 with 64,
+ * 6.94 with the last ones in parts).
+ */
+static void tile_parts(size_t na, size_t nb, size_t ncell, int nsten, int nsm,
+    int f64, int batch, fcfcg_launch *L) {
+  const double warps = 32.0 * nsm, want = batch ? 16 : 8;
+  double blocks = (double) na / 32 + 0.5 * (double) (na < ncell ? na : ncell);
+  if (!batch && blocks > 2 * warps) blocks = 2 * warps;
+  const double groups = nsten * ceil((double) nb / 32 / 32 / (double) ncell);
+  int p = 0, t = 0;
+  while (p < 4 && blocks * (double) (1 << p) <
+                      (groups >= 7.0 * (1 << p) ? want : 4) * warps) p++;
+  while (p == 4 && t < 3 &&
+         blocks * (double) (1 << (p + t)) < (f64 ? 16 : 1) * warps) t++;
+  L->pshift = p + t;
+  L->tshift = t;
+  L->nsplit = batch ? 0xFFFFFFFFu : (uint32_t) (2 * warps);
 }
-
 
 static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
     int withwt, int precision, int adj, int *sten, float *stD,
@@ -1481,7 +1500,8 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   launch_bins(c, L);
   const size_t hbytes = fcfcg_k_tile32_hist(L->hlen, withwt);
   L->hist_smem = (tabbytes + stage + hbytes <= 200 * 1024);
-  L->pshift = tile_parts(A->n, P->ncell, c->nsm);
+  tile_parts(A->n, B->n, P->ncell, P->nsten, c->nsm,
+             prec == FCFCG_PREC_FP64, 0, L);
   L->hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
   P->prec = prec;
   return FCFCG_OK;
@@ -2526,10 +2546,10 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   const size_t hbytes = fcfcg_k_tile32_hist(L.hlen, withwt);
   L.hist_smem = (fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt) +
                      hbytes <= 200 * 1024);
-  L.pshift = tile_parts(N, cells, c->nsm);
   L.nblk_dev = S->bstart + cells;
   L.hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
   L.nsten = nsten;
+  tile_parts(N, N, cells, nsten, c->nsm, 0, 1, &L);
   L.tzero = -1;
   for (int t = 0; t < nsten; t++)
     if (!c->sten[4 * t] && !c->sten[4 * t + 1] && !c->sten[4 * t + 2])

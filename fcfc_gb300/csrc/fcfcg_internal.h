@@ -126,7 +126,8 @@ typedef struct {
    * block's tiles are dealt to, slack of the block box distance, and for a
    * batch the catalogues' first cells (nmock + 1) */
   const uint32_t *nblk_dev;
-  int pshift;
+  int pshift, tshift;
+  uint32_t nsplit;       /* the blocks dealt in parts, the last ones */
   float box_eps;
   const uint32_t *mbase;
   fcfcg_dcat A, B;

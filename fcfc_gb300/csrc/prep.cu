@@ -497,7 +497,7 @@ __device__ __forceinline__ void run_steps(uint32_t k[E]) {
 }
 
 /* Sort segments of S keys (thread t's are E t to E t + E - 1), ascending;
- * S = 64 .. 512. */
+ * S = E .. 512. */
 template <int W>
 __device__ __forceinline__ void run_sort(uint32_t k[16 / W], int S, int t,
     RunX *X) {
@@ -554,7 +554,7 @@ __device__ __forceinline__ void run_sort(uint32_t k[16 / W], int S, int t,
 template <int W>
 __device__ __forceinline__ void run_order(RunSh *S, RunX *X, const float4 *key,
     uint32_t a, int n, int t) {
-  constexpr int E = 16 / W;
+  constexpr int E = 16 / W, LMIN = W == 1 ? 16 : 8;
   team_sync<W>();
   for (int i = t; i < n; i += 32 * W) {
     const float4 v = key[a + i];
@@ -565,12 +565,12 @@ __device__ __forceinline__ void run_order(RunSh *S, RunX *X, const float4 *key,
     S->ord[i] = (uint16_t) i;
   }
   team_sync<W>();
-  if (n <= 32) return;
+  if (n <= 4) return;
   uint32_t k[E];
 #pragma unroll
   for (int i = 0; i < E; i++) k[i] = (uint32_t) (E * t + i);
 #pragma unroll 1
-  for (int L = RUN_LEN; L >= 64; L >>= 1) {
+  for (int L = RUN_LEN; L >= LMIN; L >>= 1) {
     if (n <= L / 2) continue;       /* all in the first half already */
     /* the longest axis of each segment of L */
     float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
