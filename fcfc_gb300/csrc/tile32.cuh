@@ -65,6 +65,9 @@ struct TileWarp {
   float4 sd[32];           /* stencil entry: -offset * width, image code */
   uint2 si[32];            /* its first block and their number */
   unsigned long long cnt[4];   /* as fcfcg_launch.stats */
+  /* pairs to recheck, nrest of them: A's and B's index, image code and (from
+   * bit 6) the catalogue */
+  uint32_t ra[32], rb[32], rc[32], nrest, pad[3];
 };
 /* with weights: (round(w 2^30), remainder, w) of each point of A */
 struct TileWarpW {
@@ -462,100 +465,131 @@ __device__ __forceinline__ LinConst lin_const(const fcfcg_launch &L) {
 }
 
 /*
- * The tile's pairs that could not be binned in FP32 (bit i of mask: A point
- * i of this lane): those with an edge within the rounding bound go to the
- * FP64 recheck queue -- the warp reserves their places with one atomic --
- * and those beyond the queue's capacity are binned here by the FP64
- * formula.  Every ambiguous pair takes a ticket from the 64-bit fill
- * counter, queued or not, so the counter cannot wrap and hand out slots
- * twice.  Without a shared histogram every pair in range arrives here, and
- * the unambiguous ones are counted in global memory.
+ * Without a shared histogram: the pairs of a tile (mask: this lane's) into
+ * the global one, by FP32 where the windows allow; the others are returned.
  */
-template <int GEOM, int BIN, int WT, int ADJ>
-__device__ __noinline__ void tile_rest(const fcfcg_launch &L, const Tile T,
-    TileWarpW *S, uint32_t mask, const EdgeTab ES, const EdgeTab EP) {
-  const int lane = threadIdx.x & 31;
+template <int GEOM, int BIN, int WT>
+__device__ __noinline__ uint32_t tile_global(const fcfcg_launch &L,
+    const Tile T, TileWarpW *S, uint32_t mask, const EdgeTab ES,
+    const EdgeTab EP) {
   const fcfcg_mock *M = L.mocks ? L.mocks + T.mock : NULL;
-  uint32_t n_in = 0, n_inl = 0;
-  if (!ADJ && !L.hist_smem) {
-    uint32_t left = mask;
-    mask = 0;
-    while (left) {
-      const int i = __ffs(left) - 1;
-      left &= left - 1u;
-      const float *a = (const float *) S->t.p[i >> 2] + (i & 3);
-      const float dx = __fadd_rn(a[0], -T.bx), dy = __fadd_rn(a[4], -T.by),
-                  dz = __fadd_rn(a[8], -T.bz);
-      float s2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
-      if (!IS_SPI(BIN) || GEOM == FCFCG_GEOM_SURVEY) s2 = __fmaf_rn(dz, dz, s2);
-      float dm = 0.f, mm = 0.f;
-      if (GEOM == FCFCG_GEOM_SURVEY) {
-        const float mx = __fadd_rn(T.vx, dx), my = __fadd_rn(T.vy, dy),
-                    mz = __fadd_rn(T.vz, dz);
-        dm = __fmaf_rn(dz, mz, __fmaf_rn(dy, my, __fmul_rn(dx, mx)));
-        mm = __fmaf_rn(mz, mz, __fmaf_rn(my, my, __fmul_rn(mx, mx)));
-      }
-      const PairBin p = pair_bin<GEOM, BIN>(lin_const(L), ES, EP, dup2(s2),
-                                            dup2(dz), dup2(dm), dup2(mm));
-      bool plain = (fabsf(unpack2(p.f).x) < unpack2(p.h).x) &
-                   (fabsf(unpack2(p.g).x) < unpack2(p.k).x);
-      if (GEOM == FCFCG_GEOM_SURVEY && !IS_ISO(BIN)) plain &= mm >= L.m2min;
-      if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && !(p.pi.x < L.p_lim))
-        continue;
-      int b = -1;
-      if (plain) {
-        const int s = (int) (__float_as_uint(unpack2(p.col).x) - TMAGIC_BITS) -
-                      L.hcol0,
-                  q = (int) -unpack2(p.nq).x - L.hrow0;
-        if (s >= 0 && s < L.ns && q >= 0 && q < L.hrows) b = s + q * L.ns;
-      }
-      if (!plain) {
-        mask |= 1u << i;
-      } else if (b >= 0) {
-        n_in++;
-        if (WT) {
-          const float4 wa = S->aw[i];
-          add128((M ? M->gwt : L.gwt) + 2 * b,
-                 fix_prod(__float_as_int(wa.x), wa.y, wa.z, T.wi, T.wr, T.wf));
-        } else {
-          atomicAdd((M ? M->gcnt : L.gcnt) + b, 1ull);
-        }
-      }
+  uint32_t n_in = 0;
+  uint32_t left = mask;
+  mask = 0;
+  while (left) {
+    const int i = __ffs(left) - 1;
+    left &= left - 1u;
+    const float *a = (const float *) S->t.p[i >> 2] + (i & 3);
+    const float dx = __fadd_rn(a[0], -T.bx), dy = __fadd_rn(a[4], -T.by),
+                dz = __fadd_rn(a[8], -T.bz);
+    float s2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+    if (!IS_SPI(BIN) || GEOM == FCFCG_GEOM_SURVEY) s2 = __fmaf_rn(dz, dz, s2);
+    float dm = 0.f, mm = 0.f;
+    if (GEOM == FCFCG_GEOM_SURVEY) {
+      const float mx = __fadd_rn(T.vx, dx), my = __fadd_rn(T.vy, dy),
+                  mz = __fadd_rn(T.vz, dz);
+      dm = __fmaf_rn(dz, mz, __fmaf_rn(dy, my, __fmul_rn(dx, mx)));
+      mm = __fmaf_rn(mz, mz, __fmaf_rn(my, my, __fmul_rn(mx, mx)));
     }
-  }
-  const uint32_t c = (uint32_t) __popc(mask);
-  uint32_t inc = c;
-  for (int s = 1; s < 32; s <<= 1) {
-    const uint32_t u = __shfl_up_sync(FULLMASK, inc, s);
-    if (lane >= s) inc += u;
-  }
-  const uint32_t n = __shfl_sync(FULLMASK, inc, 31);
-  unsigned long long slot = 0;
-  if (lane == 0 && n) slot = atomicAdd(L.qcount, (unsigned long long) n);
-  slot = __shfl_sync(FULLMASK, slot, 0) + (inc - c);
-  for (; mask; mask &= mask - 1u, slot++) {
-    const uint32_t a = T.first + (uint32_t) (__ffs(mask) - 1);
-    if (slot < L.qcap) {
-      ((uint4 *) L.queue)[slot] = make_uint4(a, T.bj, T.code, T.mock);
+    const PairBin p = pair_bin<GEOM, BIN>(lin_const(L), ES, EP, dup2(s2),
+                                          dup2(dz), dup2(dm), dup2(mm));
+    bool plain = (fabsf(unpack2(p.f).x) < unpack2(p.h).x) &
+                 (fabsf(unpack2(p.g).x) < unpack2(p.k).x);
+    if (GEOM == FCFCG_GEOM_SURVEY && !IS_ISO(BIN)) plain &= mm >= L.m2min;
+    if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && !(p.pi.x < L.p_lim))
       continue;
+    int b = -1;
+    if (plain) {
+      const int s = (int) (__float_as_uint(unpack2(p.col).x) - TMAGIC_BITS) -
+                    L.hcol0,
+                q = (int) -unpack2(p.nq).x - L.hrow0;
+      if (s >= 0 && s < L.ns && q >= 0 && q < L.hrows) b = s + q * L.ns;
     }
-    n_inl++;
-    const int bin = ref_bin_pair(L, a, T.bj, T.code, M ? M->box : L.box);
-    if (bin < 0) continue;
-    n_in++;
-    if (ADJ) adj_pair(L, a, T.bj, bin);
-    else if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, T.bj));
-    else atomicAdd((M ? M->gcnt : L.gcnt) + bin, 1ull);
+    if (!plain) {
+      mask |= 1u << i;
+    } else if (b >= 0) {
+      n_in++;
+      if (WT) {
+        const float4 wa = S->aw[i];
+        add128((M ? M->gwt : L.gwt) + 2 * b,
+               fix_prod(__float_as_int(wa.x), wa.y, wa.z, T.wi, T.wr, T.wf));
+      } else {
+        atomicAdd((M ? M->gcnt : L.gcnt) + b, 1ull);
+      }
+    }
   }
   __syncwarp();
   n_in = __reduce_add_sync(FULLMASK, n_in);
-  n_inl = __reduce_add_sync(FULLMASK, n_inl);
-  if (lane == 0) {
-    S->t.cnt[1] += n_in;
-    S->t.cnt[2] += n;
-    S->t.cnt[3] += n_inl;
+  if ((threadIdx.x & 31) == 0) S->t.cnt[1] += n_in;
+  __syncwarp();
+  return mask;
+}
+
+/*
+ * The collected pairs to the FP64 recheck queue -- the warp reserves their
+ * places with one atomic -- and those beyond the queue's capacity are binned
+ * here by the FP64 formula.  Every pair counts in the queue's 64-bit fill
+ * counter, queued or not, so the counter cannot wrap and hand out slots twice.
+ */
+template <int WT, int ADJ>
+__device__ __noinline__ void rest_flush(const fcfcg_launch &L, TileWarp *t) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  const uint32_t n = t->nrest;
+  unsigned long long slot = 0;
+  if (lane == 0 && n) slot = atomicAdd(L.qcount, (unsigned long long) n);
+  slot = __shfl_sync(FULLMASK, slot, 0) + (unsigned long long) lane;
+  const bool mine = (uint32_t) lane < n, full = mine && slot >= L.qcap;
+  if (mine) {
+    const uint32_t a = t->ra[lane], b = t->rb[lane], c = t->rc[lane];
+    if (!full) ((uint4 *) L.queue)[slot] = make_uint4(a, b, c & 63u, c >> 6);
+  }
+  uint32_t n_in = 0;
+  if (full) {
+    const uint32_t a = t->ra[lane], b = t->rb[lane], c = t->rc[lane];
+    const fcfcg_mock *M = L.mocks ? L.mocks + (c >> 6) : NULL;
+    const int bin = ref_bin_pair(L, a, b, c & 63u, M ? M->box : L.box);
+    if (bin >= 0) {
+      n_in = 1;
+      if (ADJ) adj_pair(L, a, b, bin);
+      else if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, b));
+      else atomicAdd((M ? M->gcnt : L.gcnt) + bin, 1ull);
+    }
   }
   __syncwarp();
+  n_in = __reduce_add_sync(FULLMASK, n_in);
+  const uint32_t n_inl = (uint32_t) __popc(__ballot_sync(FULLMASK, full));
+  if (lane == 0) {
+    t->cnt[1] += n_in;
+    t->cnt[2] += n;
+    t->cnt[3] += n_inl;
+    t->nrest = 0;
+  }
+  __syncwarp();
+}
+
+/* Collect the pairs a tile left (bit i of rest: this lane's point and A's i).
+ * Every second tile has one or two: they go to the queue 32 at a time, whose
+ * atomic and writes took a tile's turn 150 instructions otherwise. */
+template <int WT, int ADJ>
+__device__ __forceinline__ void tile_rest(const fcfcg_launch &L, const Tile &T,
+    TileWarp *t, uint32_t rest) {
+  const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
+  uint32_t bal;
+  while ((bal = __ballot_sync(FULLMASK, rest != 0u)) != 0u) {
+    const uint32_t n = (uint32_t) __popc(bal);
+    if (t->nrest + n > 32u) rest_flush<WT, ADJ>(L, t);
+    const uint32_t at = t->nrest + (uint32_t) __popc(bal & below);
+    if (rest) {
+      t->ra[at] = T.first + (uint32_t) (__ffs((int) rest) - 1);
+      t->rb[at] = T.bj;
+      t->rc[at] = T.code | T.mock << 6;
+      rest &= rest - 1u;
+    }
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) t->nrest += n;
+    __syncwarp();
+  }
 }
 
 /*
@@ -1007,6 +1041,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
   const unsigned long long share = L.hs_limit / (CT32_THREADS / 32);
   const unsigned long long lim = share > 65536u ? share - 65536u : 0u;
   if (lane < 4) S->t.cnt[lane] = 0;
+  if (lane == 0) S->t.nrest = 0;
   unsigned long long added = 0;
   uint32_t cur = ~0u;
   int nq = 0;              /* all-FP64: pairs collected */
@@ -1322,8 +1357,11 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
               rest = tile_pairs<GEOM, BIN, WT, ADJ, false>(L, C, T, S, hb, ES,
                                                            EP, n_in, gb);
             if (ADJ && gb) atomicAdd(L.dB + T.bj, (double) gb * L.gunitB);
-            if (__any_sync(FULLMASK, rest != 0u))
-              tile_rest<GEOM, BIN, WT, ADJ>(L, T, S, rest, ES, EP);
+            if (__any_sync(FULLMASK, rest != 0u)) {
+              if (!ADJ && !L.hist_smem)
+                rest = tile_global<GEOM, BIN, WT>(L, T, S, rest, ES, EP);
+              tile_rest<WT, ADJ>(L, T, &S->t, rest);
+            }
           }
         }
         if (ADJ && !F64) {
@@ -1372,6 +1410,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
     if (L.hist_smem)
       tile_handover<WT, F64>(L, h, 0, threadIdx.x, CT32_THREADS, &S->t);
   }
+  if (!F64) rest_flush<WT, ADJ>(L, &S->t);
   __syncwarp();
   if (lane < 4) atomicAdd(L.stats + lane, S->t.cnt[lane]);
 }
