@@ -572,8 +572,8 @@ __device__ __noinline__ void rest_flush(const fcfcg_launch &L, TileWarp *t) {
  * Every second tile has one or two: they go to the queue 32 at a time, whose
  * atomic and writes took a tile's turn 150 instructions otherwise. */
 template <int WT, int ADJ>
-__device__ __forceinline__ void tile_rest(const fcfcg_launch &L, const Tile &T,
-    TileWarp *t, uint32_t rest) {
+__device__ __forceinline__ void tile_rest(const fcfcg_launch &L, TileWarp *t,
+    uint32_t rest, uint32_t first, uint32_t bj, uint32_t code) {
   const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
   uint32_t bal;
   while ((bal = __ballot_sync(FULLMASK, rest != 0u)) != 0u) {
@@ -581,15 +581,21 @@ __device__ __forceinline__ void tile_rest(const fcfcg_launch &L, const Tile &T,
     if (t->nrest + n > 32u) rest_flush<WT, ADJ>(L, t);
     const uint32_t at = t->nrest + (uint32_t) __popc(bal & below);
     if (rest) {
-      t->ra[at] = T.first + (uint32_t) (__ffs((int) rest) - 1);
-      t->rb[at] = T.bj;
-      t->rc[at] = T.code | T.mock << 6;
+      t->ra[at] = first + (uint32_t) (__ffs((int) rest) - 1);
+      t->rb[at] = bj;
+      t->rc[at] = code;
       rest &= rest - 1u;
     }
     __syncwarp();
     if ((threadIdx.x & 31) == 0) t->nrest += n;
     __syncwarp();
   }
+}
+
+template <int WT, int ADJ>
+__device__ __noinline__ void tile_rest_call(const fcfcg_launch &L,
+    TileWarp *t, uint32_t rest, uint32_t first, uint32_t bj, uint32_t code) {
+  tile_rest<WT, ADJ>(L, t, rest, first, bj, code);
 }
 
 /*
@@ -1360,7 +1366,14 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             if (__any_sync(FULLMASK, rest != 0u)) {
               if (!ADJ && !L.hist_smem)
                 rest = tile_global<GEOM, BIN, WT>(L, T, S, rest, ES, EP);
-              tile_rest<WT, ADJ>(L, T, &S->t, rest);
+              /* (in place where the loop has many values to keep: the call
+               * saves them, 0.9 % of a weighted (s, mu) count; the others
+               * gain 2 % by the registers) */
+              const uint32_t code = T.code | T.mock << 6;
+              if (WT && (SURVEY || !IS_SPI(BIN)))
+                tile_rest<WT, ADJ>(L, &S->t, rest, T.first, T.bj, code);
+              else
+                tile_rest_call<WT, ADJ>(L, &S->t, rest, T.first, T.bj, code);
             }
           }
         }
