@@ -52,7 +52,7 @@ __device__ __forceinline__ void add128(unsigned long long *lohi, long long v) {
  * (<= 2^-11 of a unit) is dropped.  No 64-bit float conversions.  The
  * function is symmetric in a and b (two rounded products and a commutative
  * sum, no fused multiply-add), and every path uses it, so a pair adds the
- * same integer whichever point is the chunk's: weighted sums do not depend
+ * same integer whichever point is A's: weighted sums do not depend
  * on the order of the points within a cell.
  */
 __device__ __forceinline__ long long fix_prod(int ia, float ra, float fa,

@@ -661,17 +661,9 @@ static int tune_key(double density, const double reach[3]) {
 
 static double box_volume(const double v[3]) { return v[0] * v[1] * v[2]; }
 
-/* Cells per maximum separation: about 24 objects of the chunk side per
- * cell, 1 to 8.  (Timed over k = 1..8 on boxes and surveys of 1e5 to 1e7
- * objects, the fastest refinement held 15 to 50 objects per cell.) */
-/* Default refinement: about `per_cell` objects per cell at the given
- * density (timed over k = 1..8: boxes 24 objects of the chunk catalogue;
- * survey s and (s, mu) counts 130 at the geometric mean of the two
- * catalogues' densities in their occupied volumes -- on 1e6 data and 1e7
- * randoms with the packed direct binning, RR fastest at k = 6 (2046 ms,
- * 2324 at the old 8), DR at k = 4 (427 ms, 495 at the old 5); survey
- * (s_perp, pi) counts, which keep the candidate test, 30 of the chunk
- * catalogue: RR at k = 5 (430 ms), DR and DD at k = 2 (100, 5.6 ms)). */
+/* Finer cells for counts whose FP32 windows do not fit wide ones (large
+ * separations in units of the bins): about `per_cell` objects per cell, 1 to 8
+ * cells per maximum separation. */
 static int pick_k(double density, double reach, double per_cell) {
   const int k = (int) floor(reach * cbrt(density / per_cell) + 0.5);
   return k < 1 ? 1 : (k > 8 ? 8 : k);
@@ -711,8 +703,8 @@ static double cell_widen(double density, const double reach[3]) {
   return f < 1 ? 1 : (f > CELL_WIDEN ? CELL_WIDEN : f);
 }
 
-/* tile: the grid of the tile kernel (k = 1 unless set or tuned; widen: its
- * cells may be wider than the reach), else of the chunk kernels. */
+/* tile: coarse cells (k = 1 unless set or tuned; widen: they may be wider
+ * than the reach), else the finer ones of pick_k. */
 static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
     const slot_t *B, int tile, int widen) {
   const fcfcg_bins *b = &c->bins;
@@ -734,7 +726,7 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
   }
   double ext[3] = {hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]};
   double vol = box_volume(ext);
-  /* density of the chunk side, in the volume it occupies; surveys take
+  /* density of A's side, in the volume it occupies; surveys take
    * the geometric mean with the neighbour side's */
   const double vbox = vol;
   if (!box && A->vol > 0 && A->vol < vol) vol = A->vol;
@@ -1347,7 +1339,7 @@ static void launch_bins(const fcfcg_ctx *c, fcfcg_launch *L) {
   L->gwd = c->d_wd;
   L->queue = c->d_queue;
   L->qcount = c->d_res + RES_FILL;
-  L->chunk_head = (uint32_t *) (c->d_res + RES_HEAD);
+  L->item_head = (uint32_t *) (c->d_res + RES_HEAD);
   L->qcap = (uint32_t) c->qcap;
   L->stats = c->d_stats;
 }
@@ -1389,8 +1381,8 @@ int fcfcg_adjoint(fcfcg_ctx *c, int sa, int sb, int isauto, const double *g,
  * grid, the stencil, the precision and the launch parameters, with every
  * buffer the launches touch grown to size.  count_launch (stream work only:
  * no allocation and no host synchronisation, so that it can be captured in
- * a CUDA graph): sort the catalogues into the grid, cut its cells into
- * chunks, count, recheck, and copy the histogram and the statistics to
+ * a CUDA graph): sort the catalogues into the grid, count, recheck,
+ * and copy the histogram and the statistics to
  * pinned host memory.  count_finish (once the stream has finished): the
  * caller's histogram and the statistics.
  */
@@ -1453,9 +1445,9 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   P->withwt = withwt;
   grid_t *g = &P->g;
   fcfcg_launch *L = &P->L;
-  /* The tile kernel's coarse grid; cells no wider than the reach, then the
-   * chunk kernels' finer cells where the FP32 windows do not fit; then the
-   * all-FP64 kernel on the latter. */
+  /* The tile kernel's coarse grid; cells no wider than the reach, then
+   * finer cells, where the FP32 windows do not fit; then every pair in FP64 on
+   * the first. */
   int prec = precision;
   size_t tabbytes = 0, stage = 0;
   for (int att = 0; ; att++) {

@@ -121,7 +121,7 @@ typedef struct {
   int nsten;
   const int *sten;
   const float *stenD;
-  uint32_t *chunk_head;
+  uint32_t *item_head;
   /* tile kernel: the number of A blocks (device), log2 of the parts a
    * block's tiles are dealt to, slack of the block box distance, and for a
    * batch the catalogues' first cells (nmock + 1) */
@@ -187,8 +187,7 @@ typedef struct {
   /* unweighted shared histogram: pairs a CTA adds between hand-overs to
    * the global counters, at most 2^32 - 1 (u32 bins) */
   unsigned long long hs_limit;
-  /* batch of catalogues (NULL: one catalogue pair): chunk .w is the
-   * catalogue, queue entries carry it too */
+  /* batch of catalogues (NULL: one catalogue pair) */
   const fcfcg_mock *mocks;
   int nmock;
   /* adjoint of the weighted counts: gadj[ntot] in, FP64 gradients per

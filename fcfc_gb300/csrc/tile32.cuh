@@ -8,7 +8,7 @@
  *   - points are sorted into a coarse cell grid (cells about as wide as the
  *     largest separation that counts) and, inside a cell, along a Hilbert
  *     curve; a cell's points are cut into blocks of at most 32, each with
- *     its bounding box (prep.cu:k_blocks);
+ *     its bounding box (prep.cu:k_runs);
  *   - the unit of work is a tile: the points of one block (A, in shared
  *     memory) against those of another (B, one per lane).  A persistent
  *     warp takes a block A from a global counter, tests the boxes of 32
@@ -962,9 +962,7 @@ struct TileMock {
 /* Items a CTA of a batch takes at once: a share of those left, so that the
  * runs shrink towards the end and the histogram changes hands rarely. */
 #define TILE_RUN_MIN 16u
-#ifndef TILE_CTAS
 #define TILE_CTAS 4
-#endif
 
 /* The block of an item, and the first item of a block. */
 __device__ __forceinline__ uint32_t tile_block(const fcfcg_launch &L,
@@ -1066,13 +1064,13 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           const uint32_t end = sh_run[2];
           uint32_t s0 = sh_run[1], s1 = s0;
           if (cur == ~0u || s0 >= end) {
-            uint32_t r = *(volatile uint32_t *) L.chunk_head;
+            uint32_t r = *(volatile uint32_t *) L.item_head;
             for (;;) {
               if (r >= nitem) break;
               uint32_t sz = (nitem - r) / (2u * gridDim.x);
               sz = sz < TILE_RUN_MIN ? TILE_RUN_MIN : sz;
               sz = sz < nitem - r ? sz : nitem - r;
-              const uint32_t old = atomicCAS(L.chunk_head, r, r + sz);
+              const uint32_t old = atomicCAS(L.item_head, r, r + sz);
               if (old == r) {
                 s0 = r;
                 s1 = r + sz;
@@ -1119,7 +1117,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
         continue;
       }
     } else {
-      if (lane == 0) item = atomicAdd(L.chunk_head, 1u);
+      if (lane == 0) item = atomicAdd(L.item_head, 1u);
       item = __shfl_sync(FULLMASK, item, 0);
       if (item >= nitem) break;
     }

@@ -123,7 +123,7 @@ typedef struct {
   uint64_t nchunks;
   int precision_used;    /* FCFCG_PREC_*: FP32 windows too wide fall to FP64 */
   uint64_t launches;     /* kernels launched by this context since creation */
-  int warp_queue;        /* FP32 kernel: entries of a warp's candidate queue */
+  int warp_queue;        /* as fcfcg_set_warp_queue (FP32 counts) */
 } fcfcg_stats;
 
 const char *fcfcg_strerror(int err);
@@ -198,8 +198,8 @@ typedef struct {
 /*
  * Count DD pairs of many periodic-box catalogues (mocks) with one set of bins
  * in a single persistent FP32 launch: all catalogues are cell-sorted into one
- * array with per-catalogue grids, and the CTAs draw (catalogue, cell chunk)
- * items from one device work counter; ambiguous pairs of every catalogue go
+ * array with per-catalogue grids, and the CTAs draw runs of blocks of 32
+ * points from one device work counter; ambiguous pairs of every catalogue go
  * through one FP64 recheck.  Box contexts only.  precision FCFCG_PREC_FP64
  * counts the catalogues one after the other with the all-FP64 kernel (the
  * comparison path).  Returns FCFCG_OK when the batch ran (per-catalogue
@@ -292,7 +292,7 @@ int fcfcg_count(fcfcg_ctx *ctx, int slot_a, int slot_b, int isauto,
  * typically DD, DR and RR of one survey, the eval_pairs loop of
  * src/fcfc/2pt/eval_cf.c -- captured once as a CUDA graph and replayed.
  * A replay queues, for every item, the sort of its catalogues into the
- * item's cell grid, the chunk list, the count and the FP64 recheck kernels
+ * item's cell grid, the count and the FP64 recheck kernels
  * and the copy of the histogram to pinned host memory, with no host
  * synchronisation in between; fcfcg_graph_run then writes each item's
  * icnt or wcnt exactly as fcfcg_count would.  The graph reads the context's
@@ -347,16 +347,16 @@ int fcfcg_adjoint(fcfcg_ctx *ctx, int slot_a, int slot_b, int isauto,
 
 int fcfcg_stats_get(const fcfcg_ctx *ctx, fcfcg_stats *out);
 
-/* Grid refinement: cells per maximum separation, 1..8 (0 = automatic:
- * about 24 objects of the first catalogue per cell, counted in the volume
- * it occupies -- for a survey estimated at load time, not its bounding
- * box). */
+/* Grid refinement: cells per maximum separation, 1..8 (0 = automatic: one
+ * cell per maximum separation, or wider cells, up to 4 times, where they would
+ * hold fewer than 256 objects of the first catalogue, its density counted in
+ * the volume it occupies -- for a survey estimated at load time, not its
+ * bounding box). */
 int fcfcg_set_cells_per_smax(fcfcg_ctx *ctx, int k);
 
-/* Entries of a warp's candidate queue in the FP32 counting kernel: 256,
- * 512 or 1024, or 0 (default) for automatic -- the value fcfcg_autotune
- * found for this binning and density, else the largest queue that keeps
- * the most CTAs per SM.  The counts do not depend on it. */
+/* Accepted and reported (256, 512, 1024; 0, the default, is reported as
+ * 1024): the entries of a warp's candidate queue.  The counting kernel has no
+ * such queue any more, and the counts never depended on it. */
 int fcfcg_set_warp_queue(fcfcg_ctx *ctx, int entries);
 
 /* Capacity of the FP64 recheck queue in pairs.  By default the queue holds
@@ -371,22 +371,18 @@ int fcfcg_set_queue_capacity(fcfcg_ctx *ctx, size_t cap);
 /* Unweighted counts in the FP32 kernel: a CTA's shared-memory bins are 32
  * bits wide and take their adds unchecked, so the CTA hands them to the
  * global 64-bit counters before the pairs it may have added since the last
- * hand-over (a chunk of m points with t neighbour points adds at most m t)
- * could pass this threshold, and counts a chunk that alone could pass it
- * in global memory.  1..2^32 - 1, or 0 (default) for 2^32 - 1.  The counts
- * do not depend on it; meant for tests of those two paths. */
+ * hand-over (a tile of m by t points adds at most m t) could pass this
+ * threshold.  1..2^32 - 1, or 0 (default) for 2^32 - 1.  The counts do not
+ * depend on it; meant for tests of that path. */
 int fcfcg_set_hist_handover(fcfcg_ctx *ctx, unsigned long long pairs);
 
 /*
- * Autotune the grid refinement and the kernel's tile for this binning and
- * catalogue pair: times the FP32 count at 1..8 cells per maximum
- * separation (stopping two past the fastest), then at the fastest with a
- * warp candidate queue of 1024, 512 and 256 entries (a smaller queue can
- * free shared memory for another CTA per SM or for L1), and keeps both for
- * catalogues of the same number density (key: log2 of the mean number of
- * objects of the first catalogue within the maximum separation box) and
- * weighting.  Later automatic counts of matching density use them;
- * fcfcg_stats.warp_queue reports the queue a count used.
+ * Autotune the grid refinement for this binning and catalogue pair: times
+ * the FP32 count at 1..8 cells per maximum separation (stopping two past the
+ * fastest) and keeps the fastest for catalogues of the same number density
+ * (key: log2 of the mean number of objects of the first catalogue within the
+ * maximum separation box).  Later automatic counts of matching density use
+ * it.
  */
 int fcfcg_autotune(fcfcg_ctx *ctx, int slot_a, int slot_b, int isauto,
     int withwt, int *best_k, double *best_ms);
