@@ -84,7 +84,7 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
   if (!f) return (int) cudaErrorInvalidValue;
   const size_t smem = (f64 ? 0 : fcfcg_k_tile32_tab(L)) +
       fcfcg_k_tile32_stage(f64 ? 3 : L->adjoint ? 2 : L->withwt) +
-      fcfcg_k_tile32_hist(L->hist_smem ? L->hlen : 0, L->withwt);
+      fcfcg_k_tile32_hist(L->hist_smem ? L->hwords : 0, L->withwt);
   const int threads = CT32_THREADS;
   int per_sm = 0;
   for (int i = 0; i < FCFCG_OCC; i++)
@@ -123,8 +123,8 @@ extern "C" size_t fcfcg_k_tile32_stage(int kind) {
   return (size_t) (CT32_THREADS / 32) * tile_warp_bytes(kind);
 }
 
-extern "C" size_t fcfcg_k_tile32_hist(int hlen, int withwt) {
-  return ((size_t) hlen + 32) * (withwt ? 8 : 4);
+extern "C" size_t fcfcg_k_tile32_hist(int hwords, int withwt) {
+  return ((size_t) hwords + 32) * (withwt ? 8 : 4);
 }
 
 #define RECHECK_CTAS 4

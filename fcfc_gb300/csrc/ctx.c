@@ -1429,6 +1429,21 @@ static void tile_parts(size_t na, size_t nb, size_t ncell, int nsten, int nsm,
   L->nsplit = batch ? 0xFFFFFFFFu : (uint32_t) (2 * warps);
 }
 
+/* Is the histogram in shared memory (other: bytes beside it), and, of
+ * weighted s bins, in how many copies: up to one per lane, in a quarter of an
+ * SM's 228 KB. */
+static void hist_shape(fcfcg_launch *L, size_t other, int plain) {
+  L->hlog = 0;
+  L->hist_smem =
+      (other + fcfcg_k_tile32_hist(L->hlen, L->withwt) <= 200 * 1024);
+  if (L->withwt && !plain && L->hist_smem && L->bintype == FCFCG_BIN_ISO)
+    while (L->hlog < 5 &&
+           other + fcfcg_k_tile32_hist(L->hlen << (L->hlog + 1), 1) <=
+               55 * 1024)
+      L->hlog++;
+  L->hwords = L->hlen << L->hlog;
+}
+
 static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
     int withwt, int precision, int adj, int *sten, float *stD,
     count_plan *P) {
@@ -1490,8 +1505,7 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   launch_cat(&L->A, A);
   launch_cat(&L->B, B);
   launch_bins(c, L);
-  const size_t hbytes = fcfcg_k_tile32_hist(L->hlen, withwt);
-  L->hist_smem = (tabbytes + stage + hbytes <= 200 * 1024);
+  hist_shape(L, tabbytes + stage, prec == FCFCG_PREC_FP64 || adj);
   tile_parts(A->n, B->n, P->ncell, P->nsten, c->nsm,
              prec == FCFCG_PREC_FP64, 0, L);
   L->hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
@@ -2535,9 +2549,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   L.mocks = (const fcfcg_mock *) c->d_mock;
   L.nmock = na;
   L.mbase = c->d_mbase;
-  const size_t hbytes = fcfcg_k_tile32_hist(L.hlen, withwt);
-  L.hist_smem = (fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt) +
-                     hbytes <= 200 * 1024);
+  hist_shape(&L, fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt), 0);
   L.nblk_dev = S->bstart + cells;
   L.hs_limit = c->hs_limit ? c->hs_limit : 0xFFFFFFFFull;
   L.nsten = nsten;

@@ -160,6 +160,7 @@ typedef struct {
   int nse, npe, se_lg, pe_lg, se_off, pe_off, se_skip, pe_skip, se_last,
       pe_last;
   int hcols, hcol0, hrow0, hrows, hlen;
+  int hlog, hwords;            /* in 2^hlog copies: hwords = hlen << hlog */
   float m2min;                 /* survey: |m|^2 below (next to the observer):
                                   mu and pi^2 are rechecked */
   int tzero;                   /* stencil index of the zero offset */
@@ -290,7 +291,7 @@ int fcfcg_scan(void *stream, const uint32_t *in, size_t n, uint32_t *out,
 size_t fcfcg_k_tile32_tab(const fcfcg_launch *L);
 size_t fcfcg_k_tile32_stage(int kind);
 /* And its histogram's, with a spare word per lane. */
-size_t fcfcg_k_tile32_hist(int hlen, int withwt);
+size_t fcfcg_k_tile32_hist(int hwords, int withwt);
 /* The count kernel of a launch.  occ: the CTAs per SM of the launches so
  * far (a context's; the last FCFCG_OCC shapes). */
 #define FCFCG_OCC 8

@@ -184,6 +184,11 @@ __device__ __forceinline__ uint32_t pin(uint32_t a) {
   asm volatile("" : "+r"(a));
   return a;
 }
+/* Weighted s histograms are held in 2^hlog copies, a lane's by its number: an
+ * atomic that returns takes a turn per lane on the same word, and the lanes'
+ * separations from one point lie in a bin or two (5.6e5 points, 23 bins: 2.26 ->
+ * 1.58 ms a pass; (s, mu) bins of 4 copies gained nothing). */
+#define HREP(WT, ADJ, B) ((WT) && !(ADJ) && IS_ISO(B))
 struct LinConst {
   float slim;              /* the outer range */
   float inv, s0, hs;       /* linear s bins */
@@ -191,7 +196,7 @@ struct LinConst {
   float p0, pinv, hp;      /* linear pi bins */
   float ea, eb;            /* window of a table's value: ea s^2 + eb */
   float hc;                /* columns of a row */
-  uint32_t ha, spare;
+  uint32_t ha, spare, hm;  /* shared bins: base, the lane's spare, bytes each */
 };
 
 /* An axis by table: cells of the value's FP32 bits >> lg from off on, the
@@ -277,7 +282,7 @@ __device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
 
 #define HI_LIMIT (1 << 30)
 /* Weighted sums in shared memory: two 32-bit words per bin (the high words
- * hlen + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed;
+ * hwords + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed;
  * the carry out of lo is read from the returned value, and 2^30 of hi (2^62)
  * moves to the global 128-bit accumulator when hi crosses +-2^30. */
 __device__ __forceinline__ uint32_t add_lo(uint32_t addr, uint32_t v) {
@@ -300,7 +305,7 @@ __device__ __forceinline__ void hi_moved(const fcfcg_launch &L, uint32_t mock,
       : ((nh <= -HI_LIMIT && oh > -HI_LIMIT) ? -HI_LIMIT : 0);
   if (!d) return;
   asm volatile("red.shared.add.s32 [%0], %1;" :: "r"(ah), "r"(-d));
-  const int b = tile_gbin(L, (addr - hb) >> 2);
+  const int b = tile_gbin(L, (addr - hb) >> (2 + L.hlog));
   if (b >= 0)
     add128((L.mocks ? L.mocks[mock].gwt : L.gwt) + 2 * b,
            (long long) d << 32);
@@ -309,7 +314,7 @@ __device__ __forceinline__ void hi_moved(const fcfcg_launch &L, uint32_t mock,
 __device__ __forceinline__ void tile_add_w2(const fcfcg_launch &L,
     uint32_t mock, uint32_t hb, uint32_t a0, uint32_t a1, long long v0,
     long long v1) {
-  const uint32_t ho = 4u * (uint32_t) ((L.hist_smem ? L.hlen : 0) + 32);
+  const uint32_t ho = 4u * (uint32_t) ((L.hist_smem ? L.hwords : 0) + 32);
   const uint32_t l0 = add_lo(a0, (uint32_t) v0), l1 = add_lo(a1, (uint32_t) v1);
   const int h0 = (int) (v0 >> 32) + ((l0 + (uint32_t) v0) < l0 ? 1 : 0),
             h1 = (int) (v1 >> 32) + ((l1 + (uint32_t) v1) < l1 ? 1 : 0);
@@ -460,7 +465,7 @@ __device__ __forceinline__ LinConst lin_const(const fcfcg_launch &L) {
   C.ea = L.tl_ea;
   C.eb = L.tl_eb;
   C.hc = (float) L.hcols;
-  C.ha = C.spare = 0;
+  C.ha = C.spare = C.hm = 0;
   return C;
 }
 
@@ -681,7 +686,8 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
         bool in = c[2 * h + e];
         if (SURVEY && IS_SPI(BIN)) in = in & ((e ? p.pi.y : p.pi.x) < L.p_lim);
         /* the shared bin's byte address */
-        const uint32_t at = __float_as_uint(e ? v.y : v.x) * 4u + C.ha;
+        const uint32_t at = __float_as_uint(e ? v.y : v.x) *
+                            (HREP(WT, ADJ, BIN) ? C.hm : 4u) + C.ha;
         const float fe = e ? f.y : f.x,
                     he = LINS(BIN) ? C.hs : (e ? fh.y : fh.x),
                     ge = IS_SPI(BIN) && !LINP(BIN) ? C.hp : (e ? g.y : g.x),
@@ -927,13 +933,13 @@ __device__ __noinline__ void tile_handover(const fcfcg_launch &L,
   unsigned long long *g = WT ? (L.mocks ? L.mocks[mock].gwt : L.gwt)
                              : (L.mocks ? L.mocks[mock].gcnt : L.gcnt);
   unsigned long long sum = 0;
-  for (uint32_t x = (uint32_t) t0; x < (uint32_t) L.hlen; x += (uint32_t) nt) {
-    const int b = tile_gbin(L, x);
+  for (uint32_t x = (uint32_t) t0; x < (uint32_t) L.hwords; x += (uint32_t) nt) {
+    const int b = tile_gbin(L, x >> L.hlog);
     if (WT) {
-      const long long v = ((long long) ((int *) h)[L.hlen + 32 + x] << 32) +
+      const long long v = ((long long) ((int *) h)[L.hwords + 32 + x] << 32) +
                           (long long) h[x];
       h[x] = 0;
-      h[L.hlen + 32 + x] = 0;
+      h[L.hwords + 32 + x] = 0;
       if (v && b >= 0) add128(g + 2 * b, v);
     } else {
       const uint32_t v = atomicExch(h + x, 0u);
@@ -996,9 +1002,15 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
   const uint32_t hb = (uint32_t) __cvta_generic_to_shared(h);
   /* bias of the bins' byte addresses formed from a rounded value's bits */
   LinConst C = lin_const(L);
-  C.ha = hb - 4u * TMAGIC_BITS;
+  C.hm = 4u;
+  if (HREP(WT, ADJ, BIN)) {
+    C.hm = pin(4u << L.hlog);
+    C.ha = hb - C.hm * TMAGIC_BITS + 4u * ((uint32_t) lane & ((1u << L.hlog) - 1u));
+  } else {
+    C.ha = hb - 4u * TMAGIC_BITS;
+  }
   /* the lane's word behind the bins for the pairs that are not binned */
-  C.spare = pin(hb + 4u * (uint32_t) ((ADJ || L.hist_smem ? L.hlen : 0) + lane));
+  C.spare = pin(hb + 4u * (uint32_t) ((ADJ || L.hist_smem ? L.hwords : 0) + lane));
   C.ha = pin(C.ha);
   C.slim = pin(C.slim);
   if (F64) {
@@ -1032,7 +1044,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
         ((int2 *) h)[i] = __ldg((const int2 *) L.gtab + i);
     for (int i = 0; i < 8; i++) ((TileWarpA *) S)->ga[i][lane] = 0;
   } else if (L.hist_smem) {
-    for (int i = threadIdx.x; i < (L.hlen + 32) * (WT ? 2 : 1); i += blockDim.x)
+    for (int i = threadIdx.x; i < (L.hwords + 32) * (WT ? 2 : 1); i += blockDim.x)
       h[i] = 0;
   }
   /* items: the blocks up to nwhole, then the rest in parts */

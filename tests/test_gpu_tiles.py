@@ -153,3 +153,23 @@ def test_tile_fp64(geom, name):
                                      precision=fg.PREC_FP64)
                 assert (np.abs(got - wantw) <= 4.4e-10 * tot).all()
                 assert pc.stats()["in_range"] == want.sum()
+
+
+@pytest.mark.parametrize("ns", [1, 20, 190, 191, 500, 3000, 6000])
+def test_weighted_s_histogram_copies(ns):
+    """Weighted s bins: 32 copies of the shared histogram down to one, and
+    none in shared memory, in a box and in a batch."""
+    box = 130.0
+    kw = dict(bintype=0, smin=0.0, ds=40.0 / ns, ns=ns)
+    pc, ob = _pair("box", kw, box)
+    x = _points("box", 2100, box, ns)
+    w = np.random.default_rng(6).normal(1.0, 0.6, len(x))
+    want, tot = ob.count(x, wa=w, mode=1), ob.count(x, wa=np.abs(w), mode=1)
+    pc.load(0, x, w)
+    for _ in range(2):
+        got = pc.count_pairs(0, weighted=True)
+        assert (np.abs(got - want) <= 1e-10 * tot + 1e-300).all()
+    cnt, status, _ = pc.count_batch([x, x[:70]], [box, box],
+                                    weights=[w, w[:70]], weighted=True)
+    assert status == [0, 0]
+    assert (np.abs(cnt[0] - want) <= 1e-10 * tot + 1e-300).all()
