@@ -1407,8 +1407,9 @@ typedef struct {
  * the boxes of all: 1e5 points 827 -> 655 us a pass).  As many parts as make 8
  * items per warp, but while that suffices for 4, none below 3.5 groups (nb:
  * points of the neighbour side; nsten cells each).  Where 16 parts make less
- * than an item per warp (16 with f64, whose tiles are long), up to 8 times as
- * many by single tiles (tshift of the log).  A batch, whose CTAs wait for
+ * than 2 items per warp (16 with f64, whose tiles are long), up to 8 times as
+ * many by single tiles (tshift of the log; survey graph of 1.4e4 x 6.9e4
+ * points: 1.11 -> 1.06 ms).  A batch, whose CTAs wait for
  * their last warp at the end of every run of items: all blocks, 16 items per
  * warp (48 mocks of 2e4 to 6e4 points: 6.81 ms; 7.08 with 8, 7.16 with 64,
  * 6.94 with the last ones in parts).
@@ -1423,7 +1424,7 @@ static void tile_parts(size_t na, size_t nb, size_t ncell, int nsten, int nsm,
   while (p < 4 && blocks * (double) (1 << p) <
                       (groups >= 7.0 * (1 << p) ? want : 4) * warps) p++;
   while (p == 4 && t < 3 &&
-         blocks * (double) (1 << (p + t)) < (f64 ? 16 : 1) * warps) t++;
+         blocks * (double) (1 << (p + t)) < (f64 ? 16 : 2) * warps) t++;
   L->pshift = p + t;
   L->tshift = t;
   L->nsplit = batch ? 0xFFFFFFFFu : (uint32_t) (2 * warps);
