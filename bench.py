@@ -151,7 +151,7 @@ def fp32_peak_tflops(dev):
     return 2.0 * n ** 3 / (best * 1e-3) / 1e12
 
 
-def profile_value(key, name="k_count32_box_smu_wt_ns_box.txt"):
+def profile_value(key, name="k_tile32_box_smu_wt_ns_box.txt"):
     """A figure of a committed ncu summary (DRAM bytes per launch, warp
     instructions per in-range pair), if present; by default the summary of
     the box workload's dominant kernel."""
@@ -169,7 +169,7 @@ def profile_traffic():
     return profile_value("traffic_bytes_per_launch_full_workload")
 
 
-def issue_bound(pairs_per_s, clocks, name="k_count32_box_smu_wt_ns_box.txt"):
+def issue_bound(pairs_per_s, clocks, name="k_tile32_box_smu_wt_ns_box.txt"):
     """The bound the count kernel actually meets: instruction issue.  Warp
     instructions per in-range pair (ncu, committed summary) x pairs/s over
     the issue rate of the GPU (SMs x 4 schedulers x the SM clock sampled
@@ -456,7 +456,7 @@ def run_mocks(args, rank, world, local, dist):
     peak = fp32_peak_tflops(dev)
     apeak = smem_atomic_peak(local)
     achieved = pairs * FLOPS_PER_PAIR["smu"] / (k_ms * 1e-3) / 1e12
-    prof = profile_info("k_count32_batch_mocks32.txt") or {}
+    prof = profile_info("k_tile32_batch_mocks32.txt") or {}
     traffic = None
     if prof.get("traffic_bytes_per_launch_full_workload"):
         traffic = float(prof["traffic_bytes_per_launch_full_workload"])
@@ -508,7 +508,7 @@ def run_mocks(args, rank, world, local, dist):
                          "frac": pairs / (k_ms * 1e-3) * ipp / (152 * 4 * mhz * 1e6),
                          "warp_instructions_per_pair": ipp},
                      "from_profile": {
-                         "file": "profiles/k_count32_batch_mocks32.txt",
+                         "file": "profiles/k_tile32_batch_mocks32.txt",
                          "keys": ["traffic", "issue.warp_instructions_per_pair"],
                          "captured_on_current_source": prof.get("source_matches")}},
         "counters": {"candidates": st["candidates"], "rechecked": st["rechecked"],
@@ -680,12 +680,12 @@ def run_survey(args, rank, world, local, dist):
                      "flops_per_pair": FLOPS_PER_PAIR["smu"],
                      "issue": issue_bound(
                          pairs[("smu", "RR")] / (k_rr * 1e-3), clocks,
-                         "k_count32_survey_smu_wt_rr.txt"),
+                         "k_tile32_survey_smu_wt_rr.txt"),
                      "from_profile": {
-                         "file": "profiles/k_count32_survey_smu_wt_rr.txt",
+                         "file": "profiles/k_tile32_survey_smu_wt_rr.txt",
                          "keys": ["issue.warp_instructions_per_pair"],
                          "captured_on_current_source": (profile_info(
-                             "k_count32_survey_smu_wt_rr.txt") or {}).get(
+                             "k_tile32_survey_smu_wt_rr.txt") or {}).get(
                                  "source_matches")}},
         "counters": {"kernel_ms_%s_%s" % k: v for k, v in kt.items()},
         "clocks": clocks,
@@ -1087,10 +1087,10 @@ def main():
                      "flops_per_pair": FLOPS_PER_PAIR["smu"],
                      "issue": issue_bound(n_in[0] / (k1_ms * 1e-3), clocks),
                      "from_profile": {
-                         "file": "profiles/k_count32_box_smu_wt_ns_box.txt",
+                         "file": "profiles/k_tile32_box_smu_wt_ns_box.txt",
                          "keys": ["traffic", "issue.warp_instructions_per_pair"],
                          "captured_on_current_source": (profile_info(
-                             "k_count32_box_smu_wt_ns_box.txt") or {}).get(
+                             "k_tile32_box_smu_wt_ns_box.txt") or {}).get(
                                  "source_matches")}},
         "counters": {"candidates_smu": st1["candidates"],
                      "rechecked_smu": st1["rechecked"],

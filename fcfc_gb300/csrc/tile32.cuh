@@ -31,15 +31,16 @@
  * of the reference (metric_common.c of src/fcfc/2pt_box and src/fcfc/2pt),
  * so integer counts equal the FP64 build.
  *
- * What bounds it: instruction issue and the FMA pipe (issue slots 78 % used,
- * FMA pipe 50 %, ALU 56 % on an unweighted (s, mu) box).  1.5 warp
- * instructions per in-range pair: 8 per pair slot for the distance test
- * (1.9 slots per in-range pair) and 22 for binning the slots whose step is
- * not empty (67 % of them).  A kernel that tested candidates first, queued
- * them and binned them compacted took 2.7.  Counts of one launch, before and
- * after: (s, mu) box of 2e6 points weighted 32.2 -> 23.8 ms, (s_perp, pi)
- * with log bins 5.5 -> 3.4, log s bins of 4e5 points 3.5 -> 1.3, 256 mocks
- * 607 -> 362 ms, survey (s, mu) RR + DR of 4e6 randoms 407 -> 310.
+ * What bounds it: instruction issue and the FMA pipe (unweighted (s, mu)
+ * mocks: issue slots 81 % used, FMA pipe 52 %, ALU 57 %; weighted: 74 %, with
+ * 64 % of the shared wavefronts).  1.35 warp instructions per in-range pair
+ * (weighted 2.55, survey 3.4): 8 per pair slot for the distance test (1.7
+ * slots per in-range pair) and 22 (54) for binning the slots whose step is not
+ * empty.  A kernel that tested candidates first, queued them and binned them
+ * compacted took 2.8 (3.9, 4.8).  A pass before and after: (s, mu) box of 2e6
+ * points weighted 33.6 -> 22.8 ms, (s_perp, pi) with log bins 6.4 -> 3.6, log
+ * s bins of 4e5 points 3.9 -> 1.3, 256 mocks 631 -> 332, survey (s, mu) of 4e5
+ * + 4e6 433 -> 308.
  *
  * Histograms live in shared memory (u32 counts, or int64 fixed-point weight
  * products) and are merged into global 64/128-bit integer accumulators, so
