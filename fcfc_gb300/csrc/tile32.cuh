@@ -281,11 +281,15 @@ __device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
   __syncwarp();
 }
 
-#define HI_LIMIT (1 << 30)
 /* Weighted sums in shared memory: two 32-bit words per bin (the high words
  * hwords + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed;
- * the carry out of lo is read from the returned value, and 2^30 of hi (2^62)
- * moves to the global 128-bit accumulator when hi crosses +-2^30. */
+ * the carries out of both are read from the returned values: out of lo into
+ * hi, and out of hi, where an add overflows its 32 bits, 2^64 of the overflow's
+ * sign into the global 128-bit accumulator.  Every overflow is seen by the one
+ * add that makes it, whatever the others do, and hi is never changed behind
+ * their backs: moving a part out at a limit instead lost sums of mixed signs,
+ * of which a warp's 32 adds to one word step over the limit several times
+ * before the first move takes effect. */
 __device__ __forceinline__ uint32_t add_lo(uint32_t addr, uint32_t v) {
   uint32_t old;
   asm volatile("atom.shared.add.u32 %0, [%1], %2;"
@@ -298,18 +302,18 @@ __device__ __forceinline__ int add_hi(uint32_t addr, int v) {
                : "=r"(old) : "r"(addr), "r"(v));
   return old;
 }
-/* After hi went from oh to nh: move 2^62 if this add crossed +-2^30 (an add
- * is below 2^20 in magnitude, so the top two bits of oh and nh differ). */
-__device__ __forceinline__ void hi_moved(const fcfcg_launch &L, uint32_t mock,
-    uint32_t addr, uint32_t ah, uint32_t hb, int oh, int nh) {
-  const int d = (nh >= HI_LIMIT && oh < HI_LIMIT) ? HI_LIMIT
-      : ((nh <= -HI_LIMIT && oh > -HI_LIMIT) ? -HI_LIMIT : 0);
-  if (!d) return;
-  asm volatile("red.shared.add.s32 [%0], %1;" :: "r"(ah), "r"(-d));
+/* An add of h that took hi from o to n overflowed iff o and h are of one sign
+ * and n is of the other. */
+__device__ __forceinline__ int hi_wraps(int o, int n, int h) {
+  return (o ^ n) & (h ^ n);
+}
+__device__ __forceinline__ void hi_carry(const fcfcg_launch &L, uint32_t mock,
+    uint32_t addr, uint32_t hb, int o, int n, int h) {
+  if (hi_wraps(o, n, h) >= 0) return;
   const int b = tile_gbin(L, (addr - hb) >> (2 + L.hlog));
   if (b >= 0)
-    add128((L.mocks ? L.mocks[mock].gwt : L.gwt) + 2 * b,
-           (long long) d << 32);
+    atomicAdd((L.mocks ? L.mocks[mock].gwt : L.gwt) + 2 * b + 1,
+              h < 0 ? ~0ull : 1ull);
 }
 /* Two weighted pairs: their atomics overlap. */
 __device__ __forceinline__ void tile_add_w2(const fcfcg_launch &L,
@@ -320,10 +324,11 @@ __device__ __forceinline__ void tile_add_w2(const fcfcg_launch &L,
   const int h0 = (int) (v0 >> 32) + ((l0 + (uint32_t) v0) < l0 ? 1 : 0),
             h1 = (int) (v1 >> 32) + ((l1 + (uint32_t) v1) < l1 ? 1 : 0);
   const int o0 = add_hi(a0 + ho, h0), o1 = add_hi(a1 + ho, h1);
-  const int n0 = o0 + h0, n1 = o1 + h1;
-  if ((((o0 ^ n0) | (o1 ^ n1)) & (int) 0xC0000000) && L.hist_smem) {
-    hi_moved(L, mock, a0, a0 + ho, hb, o0, n0);
-    hi_moved(L, mock, a1, a1 + ho, hb, o1, n1);
+  const int n0 = (int) ((uint32_t) o0 + (uint32_t) h0),
+            n1 = (int) ((uint32_t) o1 + (uint32_t) h1);
+  if ((hi_wraps(o0, n0, h0) | hi_wraps(o1, n1, h1)) < 0 && L.hist_smem) {
+    hi_carry(L, mock, a0, hb, o0, n0, h0);
+    hi_carry(L, mock, a1, hb, o1, n1, h1);
   }
 }
 
