@@ -268,7 +268,7 @@ __device__ __forceinline__ long long reduce4(const long long v[4], int lane) {
   return (b1 ? r[1] : r[0]) + shfl_xor64(b1 ? r[0] : r[1], 2);
 }
 
-/* Add A's gradients to the global ones and clear them. */
+/* Add A's gradients (of at most 127 tiles) to the global ones and clear them. */
 __device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
     uint32_t first, int m) {
   const int lane = threadIdx.x & 31;
@@ -1318,6 +1318,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           }
         }
         uint32_t todo = __ballot_sync(FULLMASK, near), cand = 0, n_in = 0;
+        if (ADJ && !F64) ntile += __popc(todo);
         while (todo) {
           const int j = __ffs(todo) - 1;
           todo &= todo - 1u;
@@ -1394,10 +1395,11 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           }
         }
         if (ADJ && !F64) {
-          /* a term is below 2^51, a step adds 4 of them to a word and a
-           * group of blocks 32 steps' worth: out before 2^60 */
-          ntile += 32;
-          if (ntile >= 128) {
+          /* a term is at most 2^51 (2^51 itself for a weight and an entry of
+           * 1), a tile adds 32 of them to a point's eight words, whose sum
+           * adj_flush forms in 64 bits: out after at most 95 + 32
+           * tiles, 127 x 32 x 2^51 < 2^63 */
+          if (ntile > 127 - 32) {
             adj_flush(L, (TileWarpA *) S, T.first, T.m);
             ntile = 0;
           }
