@@ -370,8 +370,8 @@ __device__ __forceinline__ float tab_col(const EdgeTab &E, float v,
  * (tab_col) of s^2, s_perp^2 or pi (survey: pi^2), the window a linear bound
  * ea s^2 + eb.
  *
- * v: 1.5 2^23 + the shared bin (row hcols + column, exact), so that its low
- * bits are the bin.  No edge lies within the windows when |f| < h and |g| <
+ * v: 1.5 2^23 + the shared bin (row hcols + column, exact below 2^22), so that
+ * its low bits are the bin.  No edge lies within the windows when |f| < h and |g| <
  * k (k = 1, g = 0 without a second axis).
  */
 struct PairBin {
@@ -453,6 +453,16 @@ __device__ __forceinline__ PairBin pair_bin(const LinConst &C,
   p.s = sv;
   p.nq = nq;
   return p;
+}
+
+/* The bin's word of a pair of pair_bin, in integers: p.v holds it in a float,
+ * exact below 2^22, which shared bins are and the adjoint's table in global
+ * memory may not be. */
+__device__ __forceinline__ uint32_t tile_word(const PairBin &p, int e,
+    int hcols) {
+  const float2 c = unpack2(p.col), q = unpack2(p.nq);
+  return __float_as_uint(e ? c.y : c.x) - TMAGIC_BITS +
+         (uint32_t) -(e ? q.y : q.x) * (uint32_t) hcols;
 }
 
 __device__ __forceinline__ LinConst lin_const(const fcfcg_launch &L) {
@@ -743,7 +753,9 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
             asm("ld.shared.v2.s32 {%0, %1}, [%2];"
                 : "=r"(g.x), "=r"(g.y) : "r"(2u * wat[e] - hb));
           else
-            g = __ldg((const int2 *) L.gtab + ((wat[e] - hb) >> 2));
+            g = __ldg((const int2 *) L.gtab +
+                      (wat[e] == C.spare ? (wat[e] - hb) >> 2
+                                         : tile_word(p, e, L.hcols)));
           const float4 wa = S->aw[k + 2 * h + e];
           const float gf = (float) g.x, gr = __int_as_float(g.y);
           ga[2 * h + e] = adj_prod(T.wi, T.wr, T.wf, g.x, gr, gf);
