@@ -517,7 +517,9 @@ __device__ __noinline__ uint32_t tile_global(const fcfcg_launch &L,
     bool plain = (fabsf(unpack2(p.f).x) < unpack2(p.h).x) &
                  (fabsf(unpack2(p.g).x) < unpack2(p.k).x);
     if (GEOM == FCFCG_GEOM_SURVEY && !IS_ISO(BIN)) plain &= mm >= L.m2min;
-    if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && !(p.pi.x < L.p_lim))
+    /* (next to the observer pi's error is not bounded: rechecked) */
+    if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && mm >= L.m2min &&
+        !(p.pi.x < L.p_lim))
       continue;
     int b = -1;
     if (plain) {
@@ -700,7 +702,12 @@ __device__ __forceinline__ uint32_t tile_pairs(const fcfcg_launch &L,
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         bool in = c[2 * h + e];
-        if (SURVEY && IS_SPI(BIN)) in = in & ((e ? p.pi.y : p.pi.x) < L.p_lim);
+        if (SURVEY && IS_SPI(BIN)) {
+          /* (next to the observer pi's error is not bounded: rechecked) */
+          bool cut = (e ? p.pi.y : p.pi.x) < L.p_lim;
+          if (SP) cut = cut | ((e ? mm2.y : mm2.x) < L.m2min);
+          in = in & cut;
+        }
         /* the shared bin's byte address */
         const uint32_t at = __float_as_uint(e ? v.y : v.x) *
                             (HREP(WT, ADJ, BIN) ? C.hm : 4u) + C.ha;

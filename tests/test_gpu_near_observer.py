@@ -1,0 +1,58 @@
+"""Survey (s_perp, pi) counts of pairs on either side of the observer, whose line
+of sight m = x_a + x_b is short and whose pi lies just below pi_max: FP32 cannot
+tell their pi, so that each of them has to be rechecked and none left out.
+Counts equal the oracle's, weighted sums and gradients to rounding."""
+import numpy as np
+import pytest
+
+from oracle import fcfc_oracle as fo
+
+pytestmark = pytest.mark.gpu
+PMAX, SMAX = 27.0, 40.0
+
+
+def _antipodal(n, lengths, seed, below=1e-3):
+    """x_a, x_b with |m| = lengths, pi in (PMAX - below, PMAX)."""
+    rng = np.random.default_rng(seed)
+    u, v = rng.normal(size=(2, n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    v -= (v * u).sum(1)[:, None] * u
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    d = u * (PMAX - below * rng.random(n))[:, None] + \
+        v * rng.uniform(1.0, SMAX - 1.0, n)[:, None]
+    m = u * np.broadcast_to(lengths, n)[:, None]
+    return (m + d) / 2, (m - d) / 2
+
+
+def _counters(ns, dpi):
+    import fcfc_gb300 as fg
+    pc = fg.PairCounter("survey", fg.BIN_SPI, smin=0, smax=SMAX, ds=SMAX / ns,
+                        pmin=0, pmax=PMAX, dpi=dpi)
+    return pc, fo.Bins(True, 2, smin=0, ds=SMAX / ns, ns=ns, pmin=0, dpi=dpi,
+                       np_=round(PMAX / dpi))
+
+
+@pytest.mark.parametrize("ns,dpi", [(10, 3.0), (40, 0.025)],
+                         ids=["shared", "global"])
+@pytest.mark.parametrize("length", [1e-5, 0.003, 0.1, 1.0])
+def test_pairs_across_the_observer(length, ns, dpi):
+    pc, ob = _counters(ns, dpi)
+    a, b = _antipodal(2000, length, 1)
+    far = np.random.default_rng(2).uniform(-200.0, 150.0, (300, 3))
+    a, b = np.concatenate([a, far[:200]]), np.concatenate([b, far[200:]])
+    w = np.random.default_rng(3).normal(1.0, 0.6, len(a))
+    pc.load(0, a, w)
+    pc.load(1, b)
+    both = np.concatenate([a, b])
+    pc.load(2, both)
+    np.testing.assert_array_equal(pc.count_pairs(0, 1), ob.count(a, b, mode=1))
+    assert pc.stats()["precision_used"] == 0
+    np.testing.assert_array_equal(pc.count_pairs(2), ob.count(both, mode=1))
+    np.testing.assert_allclose(pc.count_pairs(0, 1, weighted=True),
+                               ob.count(a, b, wa=w, mode=1), rtol=1e-10,
+                               atol=1e-10)
+    g = np.random.default_rng(4).normal(size=pc.ntot)
+    da, db = pc.adjoint(0, 1, g)
+    wda, wdb = ob.adjoint(a, g, b=b, wa=w)
+    np.testing.assert_allclose(da, wda, rtol=1e-10, atol=1e-9)
+    np.testing.assert_allclose(db, wdb, rtol=1e-10, atol=1e-9)
