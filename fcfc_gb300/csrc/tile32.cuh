@@ -826,9 +826,11 @@ __device__ __forceinline__ void group_box(TileWarp &t, const float4 &v,
  * h = h_a + h_b, of m0 = a0 + b0, its direction within 1.05 |h| / |m0| of u0 =
  * m0 / |m0| where |h| < |m0| / 2, and
  *   pi = |d.m| / |m| >= |(a0 - b0).u0| - sum h_k |u0_k| - Rs 1.05 |h| / |m0|
- * for separations within the outer range Rs (los_p holds a slack far above
- * the rounding).  The sphere alone lets in 1.6 times the tiles of a cylinder
- * of radius 100 and length 2 x 40.
+ * for separations within the outer range Rs.  los_p holds a slack far above the
+ * rounding where |m0| >= 2 R; nearer the observer u0 itself can be rounding
+ * noise (of single points h = 0 and |m0| as small as you like), and the blocks
+ * are kept.  The sphere alone lets in 1.6 times the tiles of a cylinder of
+ * radius 100 and length 2 x 40.
  */
 __device__ __forceinline__ bool los_apart(const fcfcg_launch &L, float c2x,
     float c2y, float c2z, const float4 &ac, const float4 &ah, float bx,
@@ -841,7 +843,7 @@ __device__ __forceinline__ bool los_apart(const fcfcg_launch &L, float c2x,
   const float dm = fmaf(ac.z - bz, mz, fmaf(ac.y - by, my, (ac.x - bx) * mx));
   const float hm = fmaf(hz, fabsf(mz), fmaf(hy, fabsf(my), hx * fabsf(mx))) +
                    1.1f * sqrtf(h2 * L.los_r2min);
-  return h2 < 0.2f * m2 && (fabsf(dm) - hm) * ir >= L.los_p;
+  return m2 >= L.m2min && h2 < 0.2f * m2 && (fabsf(dm) - hm) * ir >= L.los_p;
 }
 
 /* All-FP64: bin n <= 32 queued pairs by the reference's formula, every lane

@@ -56,3 +56,20 @@ def test_pairs_across_the_observer(length, ns, dpi):
     wda, wdb = ob.adjoint(a, g, b=b, wa=w)
     np.testing.assert_allclose(da, wda, rtol=1e-10, atol=1e-9)
     np.testing.assert_allclose(db, wdb, rtol=1e-10, atol=1e-9)
+
+
+@pytest.mark.parametrize("length", [1e-4, 3e-4, 1e-3])
+def test_single_pairs_across_the_observer(length):
+    """One pair at a time: boxes of single points have no extent, and their
+    line of sight is as short as the pair's.  A far third point widens the cells,
+    so that the coordinates are not taken from the pair's own middle."""
+    pc, ob = _counters(10, 3.0)
+    a, b = _antipodal(300, length, 5)
+    rng = np.random.default_rng(6)
+    for i in range(len(a)):
+        far = rng.uniform([400.0, 40.0, 40.0], [450.0, 90.0, 90.0])
+        x, y = a[i:i + 1], np.stack([b[i], far])
+        pc.load(0, x)
+        pc.load(1, y)
+        np.testing.assert_array_equal(pc.count_pairs(0, 1),
+                                      ob.count(x, y, mode=1))
