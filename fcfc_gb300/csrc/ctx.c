@@ -772,9 +772,12 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
 }
 
 /* Cell offsets whose cell pairs can hold a counted pair; half of them (with
- * the zero offset) for auto counts.  D = -offset * cell width. */
-static int stencil_build(fcfcg_ctx *c, const grid_t *g, int isauto, int *sten,
-    float *stD, int *nsten, double *dmax) {
+ * the zero offset) for auto counts.  D = -offset * cell width.  Of several
+ * grids (a batch), g has the narrowest cells, by which an offset can be within
+ * the outer range, and wide the widest widths, by which it can reach the inner
+ * edge. */
+static int stencil_build(fcfcg_ctx *c, const grid_t *g, const double wide[3],
+    int isauto, int *sten, float *stD, int *nsten, double *dmax) {
   const fcfcg_bins *b = &c->bins;
   const int box = (b->geometry == FCFCG_GEOM_BOX);
   const double margin = 1 + 1e-9;
@@ -798,7 +801,7 @@ static int stencil_build(fcfcg_ctx *c, const grid_t *g, int isauto, int *sten,
         for (int d = 0; d < 3; d++) {
           int a = abs(o[d]);
           gap[d] = (a > 0 ? a - 1 : 0) * g->cw[d];
-          far[d] = (a + 1) * g->cw[d];
+          far[d] = (a + 1) * wide[d];
         }
         if (b->bintype == FCFCG_BIN_SPI && box) {
           if (gap[2] > b->p.vmax * margin) continue;
@@ -1469,7 +1472,8 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
   for (int att = 0; ; att++) {
     if ((rc = grid_setup(c, g, A, B, att < 2, att == 0))) return rc;
     double dmax = 0;
-    if ((rc = stencil_build(c, g, isauto, sten, stD, &P->nsten, &dmax)))
+    if ((rc = stencil_build(c, g, g->cw, isauto, sten, stD, &P->nsten,
+                            &dmax)))
       return rc;
     memset(L, 0, sizeof *L);
     const int f64 = (prec == FCFCG_PREC_FP64);
@@ -2406,8 +2410,8 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
       }
     }
     hbase[na] = (uint32_t) cells;
-    /* 4. one stencil for all: built for the narrowest cells (a superset of
-     * every catalogue's own); bounds for the widest */
+    /* 4. one stencil for all, a superset of every catalogue's own; bounds
+     * for the widest cells */
     double dmin = 0;
     gmin.k = gmax.k = k;
     if (gmin.cw[0] > 1e299) {        /* every catalogue failed its checks */
@@ -2415,7 +2419,8 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
       free(hbase);
       goto out;
     }
-    if ((rc = stencil_build(c, &gmin, 1, c->sten, c->stD, &nsten, &dmin))) {
+    if ((rc = stencil_build(c, &gmin, gmax.cw, 1, c->sten, c->stD, &nsten,
+                            &dmin))) {
       free(wexp);
       free(hbase);
       goto out;
