@@ -332,12 +332,14 @@ void fcfcg_graph_destroy(fcfcg_graph *graph);
  * n_a entries) and, for a cross count, dw_b likewise over catalogue b (may
  * be NULL).  For auto counts every unordered pair feeds both of its points.
  * The pair bins are recomputed, exactly as the count bins them (FP32 windows
- * with the FP64 recheck).  Each product w_j g[b] is rounded once (one
- * FP64 fused multiply-add) to an integer multiple of 2^-S, where S makes
- * max|w| max|g| 2^S <= 2^50; those integers are summed exactly (in
- * 32-bit word pairs, with exact spills to FP64), so every gradient is within
- * n 2^-49 max|w| max|g| (plus the rounding of the final FP64 additions) of
- * the exact sum of its n products.  Catalogues
+ * with the FP64 recheck).  Each product w_j g[b] is taken as an integer
+ * multiple of 2^-51 of the scales (the powers of two not below max|w| of w's
+ * catalogue and max|g|), formed from 30-bit integers and FP32 remainders, within
+ * one such unit of the exact product; a point's integers are added exactly
+ * over tiles of up to 32 points (the lanes' points) or over up to 127 tiles (the
+ * block's), and those sums, like the products of the rechecked pairs, in FP64.
+ * So every gradient is within n 2^-49 max|w| max|g| (plus the rounding of the
+ * FP64 additions) of the exact sum of its n products.  Catalogues
  * without weights count as unit weights.  Where the count falls back to the
  * all-FP64 kernel (FP32 windows too wide), so does the adjoint, which then
  * sums in FP64.  A non-finite g entry fails with FCFCG_ERR_ARG.
