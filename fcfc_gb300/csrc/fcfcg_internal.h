@@ -182,7 +182,8 @@ typedef struct {
   uint32_t *queue;
   unsigned long long *qcount;  /* fill: 64 bits, so it cannot wrap */
   uint32_t qcap;
-  unsigned long long *stats;   /* [0] candidates [1] in-range [2] recheck
+  unsigned long long *stats;   /* [0] candidates (pairs of the fours of A
+                                  tested against a block) [1] in-range [2] recheck
                                   [3] inline rechecks [4] blocks */
   int hist_smem;               /* histogram in shared memory */
   /* unweighted shared histogram: pairs a CTA adds between hand-overs to

@@ -1393,7 +1393,9 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
               }
             }
           }
-          cand += (uint32_t) (T.m * n);
+          /* the fours taken, the last one of fewer points perhaps */
+          const int na = 4 * __popc(T.gm);
+          cand += (uint32_t) ((T.gm >> ((T.m - 1) >> 2) ? na - (-T.m & 3) : na) * n);
           if constexpr (F64) {
             tile_pairs64<GEOM, WT, ADJ>(L, T, (TileWarp64 *) S, h, nq, n_in);
           } else {
