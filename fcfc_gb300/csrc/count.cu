@@ -70,7 +70,7 @@ __global__ void k_gwd_fold(double *gwd, long ntot, int copies) {
 /* ------------------------------------------------------------------------ */
 
 extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
-    int precision, int nsm, fcfcg_occ *occ) {
+    int precision, int nsm, fcfcg_occ *occ, uint64_t *nl) {
   int bin = L->bintype;
   if (bin == FCFCG_BIN_ISO && L->tlin) bin = BIN_ISOLIN;
   if (bin == FCFCG_BIN_SMU && L->tlin) bin = BIN_SMULIN;
@@ -108,10 +108,13 @@ extern "C" int fcfcg_k_count(void *stream, const fcfcg_launch *L,
     occ->next = (i + 1) % FCFCG_OCC;
   }
   f<<<nsm * per_sm, threads, smem, (cudaStream_t) stream>>>(*L);
+  ++*nl;
   const int copies = fcfcg_gwd_copies(L->ntot);
-  if (f64 && L->withwt && !L->adjoint && copies > 1)
+  if (f64 && L->withwt && !L->adjoint && copies > 1) {
     k_gwd_fold<<<(unsigned) ((L->ntot + 127) / 128), 128, 0,
                  (cudaStream_t) stream>>>(L->gwd, L->ntot, copies);
+    ++*nl;
+  }
   return (int) cudaGetLastError();
 }
 
@@ -129,8 +132,9 @@ extern "C" size_t fcfcg_k_tile32_hist(int hwords, int withwt) {
 
 #define RECHECK_CTAS 4
 extern "C" int fcfcg_k_recheck(void *stream, const fcfcg_launch *L,
-    uint32_t nq_bound) {
+    uint32_t nq_bound, uint64_t *nl) {
   if (!nq_bound) return 0;
+  ++*nl;
   /* (a queue is mostly short, or empty: more blocks than fit at once cost a
    * launch more than they gain a long one) */
   unsigned blocks = (nq_bound + 255) / 256;

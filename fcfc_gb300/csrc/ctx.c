@@ -927,8 +927,7 @@ static int slot_sort(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   const fcfcg_sort b = slot_buffers(c, s);
   CKK(fcfcg_k_grid(c->stream, n, s->x, s->y, s->z, survey ? s->s : NULL,
                    s->w, s->has_w, s->wexp, g->n, g->cw, g->lo,
-                   fcfcg_grid_curve_bits(nc, n), &b));
-  c->launches += n ? 5 : 3;
+                   fcfcg_grid_curve_bits(nc, n), &b, &c->launches));
   return FCFCG_OK;
 }
 
@@ -1545,13 +1544,11 @@ static int count_launch(fcfcg_ctx *c, const count_plan *P, int sort_a,
                        sizeof(double) * b->ntot * fcfcg_gwd_copies(b->ntot),
                        c->stream));
   if (timed) CK(cudaEventRecord(c->ev[2], c->stream));
-  CKK(fcfcg_k_count(c->stream, L, P->prec, c->nsm, &c->occ));
-  c->launches += 1;
+  CKK(fcfcg_k_count(c->stream, L, P->prec, c->nsm, &c->occ, &c->launches));
   if (timed) CK(cudaEventRecord(c->ev[3], c->stream));
   if (P->prec == FCFCG_PREC_FP32_RECHECK) {
     /* sized for a full queue; the kernel reads the fill on the device */
-    CKK(fcfcg_k_recheck(c->stream, L, (uint32_t) c->qcap));
-    c->launches += 1;
+    CKK(fcfcg_k_recheck(c->stream, L, (uint32_t) c->qcap, &c->launches));
   }
   if (timed) CK(cudaEventRecord(c->ev[4], c->stream));
   CK(cudaMemcpyAsync(res, c->d_res,
@@ -2523,8 +2520,7 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   const fcfcg_sort sbuf = slot_buffers(c, S);
   BCKK(fcfcg_k_grid_batch(c->stream, (const fcfcg_prep_cat *) c->d_pcat, na,
                           ntile, cells, N, c->d_mbase, sb, S->x, S->y, S->z,
-                          withwt ? S->w : NULL, withwt, &sbuf));
-  c->launches += 5;
+                          withwt ? S->w : NULL, withwt, &sbuf, &c->launches));
   /* 6. per-catalogue histograms and the catalogue table */
   const size_t per = (size_t) b->ntot * (withwt ? 2 : 1);
   BGROW(c->d_bout, c->d_bout_cap, sizeof(unsigned long long) * per * na);
@@ -2573,11 +2569,9 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   BCK(cudaMemsetAsync(c->d_res, 0, sizeof(unsigned long long) * RES_HDR,
                       c->stream));
   BCK(cudaEventRecord(c->ev[2], c->stream));
-  BCKK(fcfcg_k_count(c->stream, &L, prec, c->nsm, &c->occ));
-  c->launches += 1;
+  BCKK(fcfcg_k_count(c->stream, &L, prec, c->nsm, &c->occ, &c->launches));
   BCK(cudaEventRecord(c->ev[3], c->stream));
-  BCKK(fcfcg_k_recheck(c->stream, &L, (uint32_t) c->qcap));
-  c->launches += 1;
+  BCKK(fcfcg_k_recheck(c->stream, &L, (uint32_t) c->qcap, &c->launches));
   BCK(cudaEventRecord(c->ev[4], c->stream));
   /* 9. results */
   {

@@ -246,12 +246,12 @@ typedef struct {
 /* Sort into the grid: cells in order, within a cell runs along a Hilbert
  * curve of its sub-cells, within a run blocks of 32 (prep.cu:k_runs).
  * cstart[0..nc]: the cells' first sorted points; bstart: their first blocks;
- * blk, bcell: see fcfcg_dcat. */
+ * blk, bcell: see fcfcg_dcat.  *nl counts the launches (and below). */
 size_t fcfcg_max_blocks(size_t n, size_t ncell);
 int fcfcg_k_grid(void *stream, size_t n, const double *x, const double *y,
     const double *z, const double *s, const double *w, int has_w, int wexp,
     const int ncell[3], const double cw[3], const double lo[3], int sb,
-    const fcfcg_sort *S);
+    const fcfcg_sort *S, uint64_t *nl);
 /* One catalogue of a batch for the preparation kernels: its inputs (device
  * or GPU-readable host memory), its place o in the batch slot, its first
  * tile (tiles of fcfcg_batch_tile() points, numbered across the batch) and,
@@ -281,12 +281,10 @@ int fcfcg_k_prep_batch(void *stream, const fcfcg_prep_cat *d_cat, int ncat,
 int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat, int ncat,
     uint32_t ntile, size_t ncell, size_t n, const uint32_t *mbase, int sb,
     const double *x, const double *y, const double *z, const double *w,
-    int has_w, const fcfcg_sort *S);
+    int has_w, const fcfcg_sort *S, uint64_t *nl);
 /* out[sid[p]] = in[p] for p < n (sorted order back to input order). */
 int fcfcg_k_unsort(void *stream, size_t n, const uint32_t *sid,
     const double *in, double *out);
-int fcfcg_scan(void *stream, const uint32_t *in, size_t n, uint32_t *out,
-    uint32_t *tmp);
 /* Shared memory of the tile kernel: its tables, and besides them and its
  * histogram (kind: 0 unweighted, 1 weighted, 2 adjoint, 3 all-FP64). */
 size_t fcfcg_k_tile32_tab(const fcfcg_launch *L);
@@ -302,7 +300,7 @@ typedef struct {
   int per_sm[FCFCG_OCC], next;
 } fcfcg_occ;
 int fcfcg_k_count(void *stream, const fcfcg_launch *L, int precision,
-    int nsm, fcfcg_occ *occ);
+    int nsm, fcfcg_occ *occ, uint64_t *nl);
 /* Bits of the coarse cells (dim, cells of 1 / inv_cell from lo) that hold
  * an object, and their number (count). */
 int fcfcg_k_occupancy(void *stream, size_t n, const double *x,
@@ -311,8 +309,8 @@ int fcfcg_k_occupancy(void *stream, size_t n, const double *x,
     unsigned long long *count);
 /* FP64 recheck of the queued pairs; the kernels read the queue length on
  * the device, nq_bound (>= it) only sizes the grid. */
-int fcfcg_k_recheck(void *stream, const fcfcg_launch *L, uint32_t nq_bound);
-int fcfcg_k_flush_count(void *stream, const fcfcg_launch *L);
+int fcfcg_k_recheck(void *stream, const fcfcg_launch *L, uint32_t nq_bound,
+    uint64_t *nl);
 size_t fcfcg_scan_tmp_len(size_t n);
 const char *fcfcg_cuda_errstr(int code);
 

@@ -290,16 +290,17 @@ extern "C" size_t fcfcg_scan_tmp_len(size_t n) {
 /* out[0..n] = exclusive scan of in[0..n-1], out[n] = total; sb, cstart and
  * bstart as k_scan_apply.  One launch up to 8 tiles, where each block adds
  * up the items before its own; two up to 4096, where each adds up the tiles'
- * sums (16 KB from L2); else three. */
+ * sums (16 KB from L2); else three.  *nl counts them. */
 static int scan_u32(cudaStream_t s, const uint32_t *in, size_t n,
-    uint32_t *out, uint32_t *tmp, int sb = 0, uint32_t *cstart = NULL,
-    uint32_t *bstart = NULL) {
+    uint32_t *out, uint32_t *tmp, uint64_t *nl, int sb = 0,
+    uint32_t *cstart = NULL, uint32_t *bstart = NULL) {
   size_t ntile = (n + SCAN_TILE - 1) / SCAN_TILE;
   const int sums = ntile <= 8 ? 0 : (ntile <= 4096 ? 1 : 2);
   if (sums) k_scan_tiles<<<(unsigned) ntile, SCAN_THREADS, 0, s>>>(in, n, tmp);
   if (sums == 2) k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(tmp, ntile);
   k_scan_apply<<<(unsigned) (ntile ? ntile : 1), SCAN_THREADS, 0, s>>>(
       in, n, tmp, sums, out, sb, cstart, bstart);
+  *nl += (uint64_t) sums + 1;
   return (int) cudaGetLastError();
 }
 
@@ -817,22 +818,23 @@ extern "C" size_t fcfcg_max_blocks(size_t n, size_t ncell) {
 /* Fine counts (in cfill) to cell starts, keys and the block numbering. */
 static int sort_rest(cudaStream_t st, size_t nc, size_t n, int sb,
     uint32_t *cfill, uint32_t *fstart, uint32_t *scan_tmp, uint32_t *cstart,
-    uint32_t *bstart) {
+    uint32_t *bstart, uint64_t *nl) {
   const int gaps = gaps_ok(n, nc);
-  int r = scan_u32(st, cfill, nc << sb, fstart, scan_tmp, sb, cstart,
+  int r = scan_u32(st, cfill, nc << sb, fstart, scan_tmp, nl, sb, cstart,
                    gaps ? bstart : NULL);
   if (r || gaps) return r;
   cudaError_t e;
   k_block_count<<<grid_for(nc, PREP_THREADS), PREP_THREADS, 0, st>>>(
       cstart, (uint32_t) nc, cfill);
   if ((e = cudaGetLastError())) return (int) e;
-  return scan_u32(st, cfill, nc, bstart, scan_tmp);
+  ++*nl;
+  return scan_u32(st, cfill, nc, bstart, scan_tmp, nl);
 }
 
 extern "C" int fcfcg_k_grid(void *stream, size_t n, const double *x,
     const double *y, const double *z, const double *s, const double *w,
     int has_w, int wexp, const int ncell[3], const double cw[3],
-    const double lo[3], int sb, const fcfcg_sort *S) {
+    const double lo[3], int sb, const fcfcg_sort *S, uint64_t *nl) {
   cudaStream_t st = (cudaStream_t) stream;
   const size_t nc = (size_t) ncell[0] * ncell[1] * ncell[2];
   cudaError_t e = cudaMemsetAsync(S->cfill, 0, sizeof(uint32_t) * (nc << sb), st);
@@ -841,14 +843,16 @@ extern "C" int fcfcg_k_grid(void *stream, size_t n, const double *x,
     k_cell<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0, st>>>(
         n, x, y, z, fine_grid(ncell, cw, lo, sb), S->cell_of, S->rank, S->cfill);
     if ((e = cudaGetLastError())) return (int) e;
+    ++*nl;
   }
   int r = sort_rest(st, nc, n, sb, S->cfill, S->fstart, S->scan_tmp, S->cstart,
-                    S->bstart);
+                    S->bstart, nl);
   if (r) return r;
   if (n) {
     k_keys<<<grid_for(n, PREP_THREADS), PREP_THREADS, 0, st>>>(
         n, x, y, z, S->cell_of, S->rank, S->fstart, (float4 *) S->key);
     if ((e = cudaGetLastError())) return (int) e;
+    ++*nl;
   }
   RunArgs A;
   memset(&A, 0, sizeof A);
@@ -880,12 +884,8 @@ extern "C" int fcfcg_k_grid(void *stream, size_t n, const double *x,
   A.blk = (float4 *) S->blk;
   A.bcell = (uint2 *) S->bcell;
   launch_runs(&A, n, st);
+  ++*nl;
   return (int) cudaGetLastError();
-}
-
-extern "C" int fcfcg_scan(void *stream, const uint32_t *in, size_t n,
-    uint32_t *out, uint32_t *tmp) {
-  return scan_u32((cudaStream_t) stream, in, n, out, tmp);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_keys_batch(
 extern "C" int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat,
     int ncat, uint32_t ntile, size_t ncell, size_t n, const uint32_t *mbase,
     int sb, const double *x, const double *y, const double *z,
-    const double *w, int has_w, const fcfcg_sort *S) {
+    const double *w, int has_w, const fcfcg_sort *S, uint64_t *nl) {
   if (!ncat || !ntile) return 0;
   cudaStream_t st = (cudaStream_t) stream;
   cudaError_t e = cudaMemsetAsync(S->cfill, 0,
@@ -1045,12 +1045,14 @@ extern "C" int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat,
   k_cell_batch<<<ntile, PREP_THREADS, 0, st>>>(d_cat, ncat, sb, x, y, z,
                                                S->cell_of, S->rank, S->cfill);
   if ((e = cudaGetLastError())) return (int) e;
+  ++*nl;
   int r = sort_rest(st, ncell, n, sb, S->cfill, S->fstart, S->scan_tmp,
-                    S->cstart, S->bstart);
+                    S->cstart, S->bstart, nl);
   if (r) return r;
   k_keys_batch<<<ntile, PREP_THREADS, 0, st>>>(d_cat, ncat, x, y, z,
       S->cell_of, S->rank, S->fstart, (float4 *) S->key);
   if ((e = cudaGetLastError())) return (int) e;
+  ++*nl;
   RunArgs A;
   memset(&A, 0, sizeof A);
   A.cstart = S->cstart;
@@ -1075,6 +1077,7 @@ extern "C" int fcfcg_k_grid_batch(void *stream, const fcfcg_prep_cat *d_cat,
   A.blk = (float4 *) S->blk;
   A.bcell = (uint2 *) S->bcell;
   launch_runs(&A, n, st);
+  ++*nl;
   return (int) cudaGetLastError();
 }
 

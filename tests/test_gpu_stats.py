@@ -1,4 +1,5 @@
-"""Statistics of a count: the pairs whose separation was evaluated."""
+"""Statistics of a count: the pairs whose separation was evaluated, and the
+kernels launched."""
 import numpy as np
 import pytest
 
@@ -25,3 +26,28 @@ def test_candidates_are_the_pairs_evaluated(precision):
         assert list(st["ncell"]) == [12, 12, 12]
         assert st["candidates"] == want, (x, st["candidates"])
         assert st["in_range"] <= want
+
+
+def test_launches_are_those_made():
+    """The sort of a small catalogue (cells, one scan, keys, runs) or of one with
+    more counters than a scan's eight tiles (two), the count, its recheck
+    (none without a queue) and the fold of FP64 sums."""
+    import fcfc_gb300 as fg
+    pc = fg.PairCounter("box", fg.BIN_ISO, box=200.0, smin=0, smax=20, ds=2)
+    rng = np.random.default_rng(1)
+
+    def launches(call):
+        before = pc.stats()["launches"]
+        call()
+        return pc.stats()["launches"] - before
+    pc.load(0, rng.random((3000, 3)) * 200.0)
+    pc.count_pairs(0)
+    assert launches(lambda: pc.count_pairs(0)) == 2
+    pc.set_queue_capacity(0)
+    assert launches(lambda: pc.count_pairs(0)) == 1
+    assert launches(lambda: pc.count_pairs(0, weighted=True,
+                                           precision=fg.PREC_FP64)) == 2
+    pc.load(1, rng.random((3000, 3)) * 200.0)
+    assert launches(lambda: pc.count_pairs(1)) == 1 + 4 + 1     # load, sort
+    pc.load(1, rng.random((100000, 3)) * 200.0)
+    assert launches(lambda: pc.count_pairs(1)) == 1 + 5 + 1
