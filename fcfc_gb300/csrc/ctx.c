@@ -856,23 +856,39 @@ static void slot_mark(slot_t *s, const grid_t *g) {
   s->grid_valid = 1;
 }
 
-/* Buffers for sorting slot s into grid g (host side; may allocate). */
-static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
-  const size_t nc = (size_t) g->n[0] * g->n[1] * g->n[2];
-  const size_t n = s->n, m = n ? n : 1;
+/* Free the n device buffers of a list and forget them. */
+static void drop(void ***p, size_t n) {
+  for (size_t i = 0; i < n; i++) {
+    if (*p[i]) cudaFree(*p[i]);
+    *p[i] = NULL;
+  }
+}
+#define DROP(...)                                                           \
+  do {                                                                      \
+    void **p_[] = {__VA_ARGS__};                                            \
+    drop(p_, sizeof p_ / sizeof p_[0]);                                     \
+  } while (0)
+
+/* The arrays of a sorted copy of slot s: m points, nc cells, mb blocks (host
+ * side; may allocate).  A set that has to grow is dropped first, with its
+ * capacity and the record of the copy, so that after an allocation that fails
+ * nothing freed is left to be used and the slot does not pass for sorted. */
+static int slot_arrays(fcfcg_ctx *c, slot_t *s, size_t m, size_t nc,
+    size_t mb) {
   if (s->scap < m) {
     c->bufgen++;
-    void *p[] = {s->l4, s->wq, s->sx, s->sy, s->sz, s->ss, s->sw, s->sid,
-                 s->cell_of};
-    for (size_t i = 0; i < sizeof p / sizeof p[0]; i++)
-      if (p[i]) cudaFree(p[i]);
-    s->l4 = NULL;
+    s->grid_valid = 0;
+    s->scap = 0;
+    DROP((void **) &s->l4, (void **) &s->wq, (void **) &s->sx,
+         (void **) &s->sy, (void **) &s->sz, (void **) &s->ss,
+         (void **) &s->sw, (void **) &s->sid, (void **) &s->cell_of);
     CK(cudaMalloc((void **) &s->l4, sizeof(float) * 4 * m));
     CK(cudaMalloc((void **) &s->wq, sizeof(int) * 2 * m));
     CK(cudaMalloc((void **) &s->sx, sizeof(double) * m));
     CK(cudaMalloc((void **) &s->sy, sizeof(double) * m));
     CK(cudaMalloc((void **) &s->sz, sizeof(double) * m));
-    CK(cudaMalloc((void **) &s->ss, sizeof(double) * m));
+    CK(cudaMalloc((void **) &s->ss, sizeof(double) *
+                  (c->bins.geometry == FCFCG_GEOM_SURVEY ? m : 1)));
     CK(cudaMalloc((void **) &s->sw, sizeof(double) * m));
     CK(cudaMalloc((void **) &s->sid, sizeof(uint32_t) * m));
     CK(cudaMalloc((void **) &s->cell_of, sizeof(uint32_t) * m));
@@ -880,25 +896,31 @@ static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
   }
   if (s->ccap < nc + 1) {
     c->bufgen++;
-    if (s->cstart) cudaFree(s->cstart);
-    if (s->bstart) cudaFree(s->bstart);
-    s->cstart = s->bstart = NULL;
+    s->grid_valid = 0;
+    s->ccap = 0;
+    DROP((void **) &s->cstart, (void **) &s->bstart);
     CK(cudaMalloc((void **) &s->cstart, sizeof(uint32_t) * (nc + 1)));
     CK(cudaMalloc((void **) &s->bstart, sizeof(uint32_t) * (nc + 1)));
     s->ccap = nc + 1;
   }
-  const size_t mb = fcfcg_max_blocks(n, nc);
   if (s->blkcap < mb) {
     c->bufgen++;
-    if (s->blk) cudaFree(s->blk);
-    if (s->bcell) cudaFree(s->bcell);
-    s->blk = NULL;
-    s->bcell = NULL;
+    s->grid_valid = 0;
     s->blkcap = 0;
+    DROP((void **) &s->blk, (void **) &s->bcell);
     CK(cudaMalloc((void **) &s->blk, sizeof(float) * 8 * mb));
     CK(cudaMalloc((void **) &s->bcell, sizeof(uint32_t) * 2 * mb));
     s->blkcap = mb;
   }
+  return FCFCG_OK;
+}
+
+/* Buffers for sorting slot s into grid g (host side; may allocate). */
+static int slot_reserve(fcfcg_ctx *c, slot_t *s, const grid_t *g) {
+  const size_t nc = (size_t) g->n[0] * g->n[1] * g->n[2];
+  const size_t n = s->n, m = n ? n : 1;
+  const int rc = slot_arrays(c, s, m, nc, fcfcg_max_blocks(n, nc));
+  if (rc) return rc;
   const size_t nf = nc << fcfcg_grid_curve_bits(nc, n);
   GROW(c->cfill, c->cfill_cap, sizeof(uint32_t) * (nf + 1));
   GROW(c->fstart, c->fstart_cap, sizeof(uint32_t) * (nf + 1));
@@ -2446,60 +2468,10 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   }
   /* 5. cell sort of every catalogue into the shared sorted arrays */
   const size_t m = N;
-  if (S->scap < m) {
-    void *pp[] = {S->l4, S->wq, S->sx, S->sy, S->sz, S->ss, S->sw, S->sid,
-                  S->cell_of};
-    for (size_t i = 0; i < sizeof pp / sizeof pp[0]; i++)
-      if (pp[i]) cudaFree(pp[i]);
-    S->l4 = NULL;
-    S->scap = 0;
-    cudaError_t e = cudaMalloc((void **) &S->l4, sizeof(float) * 4 * m);
-    if (!e) e = cudaMalloc((void **) &S->wq, sizeof(int) * 2 * m);
-    if (!e) e = cudaMalloc((void **) &S->sx, sizeof(double) * m);
-    if (!e) e = cudaMalloc((void **) &S->sy, sizeof(double) * m);
-    if (!e) e = cudaMalloc((void **) &S->sz, sizeof(double) * m);
-    if (!e) e = cudaMalloc((void **) &S->ss, sizeof(double) * 1);
-    if (!e) e = cudaMalloc((void **) &S->sw, sizeof(double) * m);
-    if (!e) e = cudaMalloc((void **) &S->sid, sizeof(uint32_t) * m);
-    if (!e) e = cudaMalloc((void **) &S->cell_of, sizeof(uint32_t) * m);
-    if (e) {
-      free(wexp);
-      free(hbase);
-      BCK(e);
-    }
-    S->scap = m;
-  }
-  if (S->ccap < cells + 1) {
-    if (S->cstart) cudaFree(S->cstart);
-    if (S->bstart) cudaFree(S->bstart);
-    S->cstart = S->bstart = NULL;
-    S->ccap = 0;
-    cudaError_t e = cudaMalloc((void **) &S->cstart,
-                               sizeof(uint32_t) * (cells + 1));
-    if (!e) e = cudaMalloc((void **) &S->bstart,
-                           sizeof(uint32_t) * (cells + 1));
-    if (e) {
-      free(wexp);
-      free(hbase);
-      BCK(e);
-    }
-    S->ccap = cells + 1;
-  }
-  const size_t mb = fcfcg_max_blocks(N, cells);
-  if (S->blkcap < mb) {
-    if (S->blk) cudaFree(S->blk);
-    if (S->bcell) cudaFree(S->bcell);
-    S->blk = NULL;
-    S->bcell = NULL;
-    S->blkcap = 0;
-    cudaError_t e = cudaMalloc((void **) &S->blk, sizeof(float) * 8 * mb);
-    if (!e) e = cudaMalloc((void **) &S->bcell, sizeof(uint32_t) * 2 * mb);
-    if (e) {
-      free(wexp);
-      free(hbase);
-      BCK(e);
-    }
-    S->blkcap = mb;
+  if ((rc = slot_arrays(c, S, m, cells, fcfcg_max_blocks(N, cells)))) {
+    free(wexp);
+    free(hbase);
+    goto out;
   }
   /* fine counters: cells x sub-cells (the points of a cell grouped by
    * sub-cell in the sorted arrays) */
