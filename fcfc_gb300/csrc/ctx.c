@@ -747,7 +747,15 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
   g->k = k;
   const double f = (tile && widen && k == 1)
                        ? cell_widen(density, g->reach) : 1;
-  const double maxcells = 16.0 * 1024 * 1024;
+  /* no more cells than points where the cells may be wider than the reach: each
+   * costs the sort 0.1 ns, and a cell of less than a point saves no tile (1e5
+   * points in 250^3 cells 1880 us, in 46^3 252; 1e6 in 250^3 3850, in 100^3
+   * 1190).  32768 cost nothing. */
+  double maxcells = 16.0 * 1024 * 1024;
+  if (tile && widen && k == 1) {
+    const double n = (double) (A->n > B->n ? A->n : B->n);
+    maxcells = fmin(maxcells, fmax(32768.0, n));
+  }
   double scale = 1;
   for (;;) {
     double tot = 1;

@@ -353,7 +353,8 @@ int fcfcg_stats_get(const fcfcg_ctx *ctx, fcfcg_stats *out);
  * cell per maximum separation, or wider cells, up to 4 times, where they would
  * hold fewer than 256 objects of the first catalogue, its density counted in
  * the volume it occupies -- for a survey estimated at load time, not its
- * bounding box). */
+ * bounding box -- and at most as many as the larger catalogue has objects, or
+ * 32768). */
 int fcfcg_set_cells_per_smax(fcfcg_ctx *ctx, int k);
 
 /* Accepted and reported (256, 512, 1024; 0, the default, is reported as
