@@ -745,8 +745,14 @@ static int grid_setup(fcfcg_ctx *c, grid_t *g, const slot_t *A,
                           : pick_k(density, r3,
                                    box ? 24.0 : (spi ? 30.0 : 130.0)));
   g->k = k;
-  const double f = (tile && widen && k == 1)
-                       ? cell_widen(density, g->reach) : 1;
+  /* cells for the first catalogue's blocks, but where the other one is far
+   * denser, between the two: as wide as a few sparse points ask for, a block
+   * spans a cell that holds much of the dense side (300 x 1e6 points in a box
+   * 1745 -> 420 us, 1e4 x 1e6 755 -> 668; at a ratio of 10 up to 5 % slower) */
+  double wd = density;
+  if (box && (double) B->n > 32.0 * (double) A->n)
+    wd = sqrt((double) A->n * (double) B->n) / vol;
+  const double f = (tile && widen && k == 1) ? cell_widen(wd, g->reach) : 1;
   /* no more cells than points where the cells may be wider than the reach: each
    * costs the sort 0.1 ns, and a cell of less than a point saves no tile (1e5
    * points in 250^3 cells 1880 us, in 46^3 252; 1e6 in 250^3 3850, in 100^3

@@ -36,3 +36,20 @@ def test_sparse_catalogues(geom, n):
     st = pc.stats()
     assert np.prod(st["ncell"]) <= max(32768, n)
     np.testing.assert_array_equal(pc.count_pairs(0), ob.count(x, mode=1))
+
+
+def test_sparse_against_dense():
+    """300 points against 1e5: cells for a density between the two (2 per side;
+    the 300 alone would get one of the box), in either order of the catalogues."""
+    import fcfc_gb300 as fg
+    rng = np.random.default_rng(8)
+    a, b = rng.random((300, 3)) * 400.0, rng.random((100000, 3)) * 400.0
+    pc = fg.PairCounter("box", fg.BIN_SMU, box=400.0, smin=0, smax=100, ds=5,
+                        nmu=10)
+    want = fo.Bins(False, 1, smin=0, ds=5, ns=20, nmu=10, box=400.0).count(
+        a, b, mode=1)
+    pc.load(0, a)
+    pc.load(1, b)
+    np.testing.assert_array_equal(pc.count_pairs(0, 1), want)
+    assert list(pc.stats()["ncell"]) == [2, 2, 2]
+    np.testing.assert_array_equal(pc.count_pairs(1, 0), want)
