@@ -287,14 +287,20 @@ __device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
 }
 
 /* Weighted sums in shared memory: two 32-bit words per bin (the high words
- * hwords + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed;
- * the carries out of both are read from the returned values: out of lo into
- * hi, and out of hi, where an add overflows its 32 bits, 2^64 of the overflow's
- * sign into the global 128-bit accumulator.  Every overflow is seen by the one
- * add that makes it, whatever the others do, and hi is never changed behind
- * their backs: moving a part out at a limit instead lost sums of mixed signs,
- * of which a warp's 32 adds to one word step over the limit several times
- * before the first move takes effect. */
+ * hwords + 32 words behind), value = hi 2^32 + lo, lo unsigned and hi signed.
+ * The carry out of lo is read from the returned value.  An add that finds hi
+ * beyond +-2^30 takes all of hi by an exchange and adds it to the global 128-bit
+ * accumulator: whatever the other threads do meanwhile, what is in the word is
+ * counted once, and the adds under way (two of each of 256 threads, of 2^19 + 1
+ * at most) do not carry it to 2^31.  Of a thread's two words the larger is taken;
+ * the other, if beyond too, by the next add that finds it so: to rise a step (of
+ * 2^19) further unseen it has to meet a larger one that is then cleared, which
+ * doubles with each step.
+ * (Moving 2^30 out at each step over the limit lost sums of mixed signs, of which
+ * a warp's 32 adds to one word step over it several times before the first move
+ * takes effect.  Carrying hi's own overflow took the sum too: weighted (s, mu) of
+ * 2e6 points 23.4 ms a pass, 22.7 so; survey (s, mu) 311.7 and 300.7; exchanging
+ * both words 22.3 and 305.4.) */
 __device__ __forceinline__ uint32_t add_lo(uint32_t addr, uint32_t v) {
   uint32_t old;
   asm volatile("atom.shared.add.u32 %0, [%1], %2;"
@@ -307,18 +313,15 @@ __device__ __forceinline__ int add_hi(uint32_t addr, int v) {
                : "=r"(old) : "r"(addr), "r"(v));
   return old;
 }
-/* An add of h that took hi from o to n overflowed iff o and h are of one sign
- * and n is of the other. */
-__device__ __forceinline__ int hi_wraps(int o, int n, int h) {
-  return (o ^ n) & (h ^ n);
-}
-__device__ __forceinline__ void hi_carry(const fcfcg_launch &L, uint32_t mock,
-    uint32_t addr, uint32_t hb, int o, int n, int h) {
-  if (hi_wraps(o, n, h) >= 0) return;
+#define HI_LIMIT 0x40000000u
+__device__ __forceinline__ void hi_out(const fcfcg_launch &L, uint32_t mock,
+    uint32_t addr, uint32_t ah, uint32_t hb) {
+  int v;
+  asm volatile("atom.shared.exch.b32 %0, [%1], 0;" : "=r"(v) : "r"(ah));
   const int b = tile_gbin(L, (addr - hb) >> (2 + L.hlog));
   if (b >= 0)
-    atomicAdd((L.mocks ? L.mocks[mock].gwt : L.gwt) + 2 * b + 1,
-              h < 0 ? ~0ull : 1ull);
+    add128((L.mocks ? L.mocks[mock].gwt : L.gwt) + 2 * b,
+           (long long) v * (1ll << 32));
 }
 /* Two weighted pairs: their atomics overlap. */
 __device__ __forceinline__ void tile_add_w2(const fcfcg_launch &L,
@@ -329,11 +332,10 @@ __device__ __forceinline__ void tile_add_w2(const fcfcg_launch &L,
   const int h0 = (int) (v0 >> 32) + ((l0 + (uint32_t) v0) < l0 ? 1 : 0),
             h1 = (int) (v1 >> 32) + ((l1 + (uint32_t) v1) < l1 ? 1 : 0);
   const int o0 = add_hi(a0 + ho, h0), o1 = add_hi(a1 + ho, h1);
-  const int n0 = (int) ((uint32_t) o0 + (uint32_t) h0),
-            n1 = (int) ((uint32_t) o1 + (uint32_t) h1);
-  if ((hi_wraps(o0, n0, h0) | hi_wraps(o1, n1, h1)) < 0 && L.hist_smem) {
-    hi_carry(L, mock, a0, hb, o0, n0, h0);
-    hi_carry(L, mock, a1, hb, o1, n1, h1);
+  if ((int) (((uint32_t) o0 + HI_LIMIT) | ((uint32_t) o1 + HI_LIMIT)) < 0 &&
+      L.hist_smem) {
+    const uint32_t a = abs(o1) > abs(o0) ? a1 : a0;
+    hi_out(L, mock, a, a + ho, hb);
   }
 }
 
