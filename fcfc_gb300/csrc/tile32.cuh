@@ -992,6 +992,13 @@ __device__ __noinline__ void tile_handover(const fcfcg_launch &L,
   }
 }
 
+/* Add the lanes' n to a counter of the warp's (their sum may exceed 32 bits). */
+__device__ __forceinline__ void warp_count(unsigned long long *cnt, uint32_t n) {
+  const uint32_t lo = __reduce_add_sync(FULLMASK, n & 0xffffu),
+                 hi = __reduce_add_sync(FULLMASK, n >> 16);
+  if ((threadIdx.x & 31) == 0) *cnt += ((unsigned long long) hi << 16) + lo;
+}
+
 /* The catalogue a CTA of a batched launch is working on (shared memory). */
 struct TileMock {
   int nc[3];
@@ -1226,6 +1233,10 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
     __syncwarp();
     uint32_t seq = 0, seqt = 0;
     int ntile = 0;
+    /* this lane's pairs tested and in range, added up at the end of the item (at
+     * each group of blocks: (s, mu) weighted +0.4 %, survey +0.9 %; at most 1024
+     * per group, and 2^22 groups hold all points that there can be) */
+    uint32_t cand = 0, n_in = 0;
     for (int t0 = 0; t0 < L.nsten; t0 += 32) {
       /* 32 stencil entries, one per lane: the neighbour cell's blocks */
       uint32_t nb = 0, b0 = 0, ecode = 0;
@@ -1355,12 +1366,25 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             near = groups != 0u;
           }
         }
-        uint32_t todo = __ballot_sync(FULLMASK, near), cand = 0, n_in = 0;
+        uint32_t todo = __ballot_sync(FULLMASK, near);
+        if (npt > 1) {
+          /* by single tiles: this part's */
+          near &= ((seqt + (uint32_t) __popc(todo & ((1u << lane) - 1u))) &
+                   (npt - 1u)) == pt;
+          seqt += (uint32_t) __popc(todo);
+          todo = __ballot_sync(FULLMASK, near);
+        }
         if (ADJ && !F64) ntile += __popc(todo);
+        added += 1024u * (uint32_t) __popc(todo);
+        /* the pairs tested, of this lane's block: the fours taken, the last one
+         * of fewer points perhaps */
+        if (near) {
+          const int na = 4 * __popc(groups);
+          cand += (uint32_t) ((groups >> ((T.m - 1) >> 2) ? na - (-T.m & 3) : na) * bcnt);
+        }
         while (todo) {
           const int j = __ffs(todo) - 1;
           todo &= todo - 1u;
-          if (npt > 1 && (seqt++ & (npt - 1u)) != pt) continue;
           const uint32_t f = __shfl_sync(FULLMASK, bfirst, j);
           const int n = __shfl_sync(FULLMASK, bcnt, j);
           T.gm = __shfl_sync(FULLMASK, groups, j);
@@ -1405,9 +1429,6 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
               }
             }
           }
-          /* the fours taken, the last one of fewer points perhaps */
-          const int na = 4 * __popc(T.gm);
-          cand += (uint32_t) ((T.gm >> ((T.m - 1) >> 2) ? na - (-T.m & 3) : na) * n);
           if constexpr (F64) {
             tile_pairs64<GEOM, WT, ADJ>(L, T, (TileWarp64 *) S, h, nq, n_in);
           } else {
@@ -1444,21 +1465,17 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
             ntile = 0;
           }
         }
-        if (lane == 0) S->t.cnt[0] += cand;
-        added += cand;
         if (!WT && !ADJ && added > lim && L.hist_smem) {
           /* a warp that may have added its share of what a 32-bit bin holds
            * hands the CTA's bins over */
           tile_handover<WT>(L, h, T.mock, lane, 32, &S->t);
           added = 0;
         }
-        if (WT || (F64 && !L.hist_smem)) {
-          n_in = __reduce_add_sync(FULLMASK, n_in);
-          if (lane == 0) S->t.cnt[1] += n_in;
-        }
        }
       }
     }
+    warp_count(&S->t.cnt[0], cand);
+    if (WT || (F64 && !L.hist_smem)) warp_count(&S->t.cnt[1], n_in);
     if (ADJ && F64) {
       double &ga = ((TileWarp64 *) S)->ga[lane];
       __syncwarp();
