@@ -495,56 +495,71 @@ __device__ __forceinline__ LinConst lin_const(const fcfcg_launch &L) {
 /*
  * Without a shared histogram: the pairs of a tile (mask: this lane's) into
  * the global one, by FP32 where the windows allow; the others are returned.
+ * Two points of A at a time, the same for all lanes, whose bins then lie close
+ * together, and additions that return nothing (1e5 points, 8e4 bins: 3.66 ms
+ * with a point per lane at a time, 3.57 so, 2.67 with red in place of the
+ * generic atomic).
  */
 template <int GEOM, int BIN, int WT>
 __device__ __noinline__ uint32_t tile_global(const fcfcg_launch &L,
     const Tile T, TileWarpW *S, uint32_t mask, const EdgeTab ES,
     const EdgeTab EP) {
   const fcfcg_mock *M = L.mocks ? L.mocks + T.mock : NULL;
+  unsigned long long *out = WT ? (M ? M->gwt : L.gwt) : (M ? M->gcnt : L.gcnt);
+  const LinConst C = lin_const(L);
+  const f2 nbx = dup2(-T.bx), nby = dup2(-T.by), nbz = dup2(-T.bz);
   uint32_t n_in = 0;
-  uint32_t left = mask;
+  const uint32_t mine = mask;
   mask = 0;
-  while (left) {
-    const int i = __ffs(left) - 1;
-    left &= left - 1u;
-    const float *a = (const float *) S->t.p[i >> 2] + (i & 3);
-    const float dx = __fadd_rn(a[0], -T.bx), dy = __fadd_rn(a[4], -T.by),
-                dz = __fadd_rn(a[8], -T.bz);
-    float s2 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
-    if (!IS_SPI(BIN) || GEOM == FCFCG_GEOM_SURVEY) s2 = __fmaf_rn(dz, dz, s2);
-    float dm = 0.f, mm = 0.f;
+  /* two points of A at a time, the same for all lanes */
+  for (uint32_t left = __reduce_or_sync(FULLMASK, mine); left;) {
+    const int i0 = (__ffs((int) left) - 1) & ~1;
+    left &= ~(3u << i0);
+    const ulonglong2 *P = S->t.p[i0 >> 2];
+    const f2 dx = add2(i0 & 2 ? P[0].y : P[0].x, nbx),
+             dy = add2(i0 & 2 ? P[1].y : P[1].x, nby),
+             dz = add2(i0 & 2 ? P[2].y : P[2].x, nbz);
+    f2 s2 = fma2(dy, dy, mul2(dx, dx)), dm = 0, mm = 0;
+    if (!IS_SPI(BIN) || GEOM == FCFCG_GEOM_SURVEY) s2 = fma2(dz, dz, s2);
     if (GEOM == FCFCG_GEOM_SURVEY) {
-      const float mx = __fadd_rn(T.vx, dx), my = __fadd_rn(T.vy, dy),
-                  mz = __fadd_rn(T.vz, dz);
-      dm = __fmaf_rn(dz, mz, __fmaf_rn(dy, my, __fmul_rn(dx, mx)));
-      mm = __fmaf_rn(mz, mz, __fmaf_rn(my, my, __fmul_rn(mx, mx)));
+      const f2 mx = add2(dup2(T.vx), dx), my = add2(dup2(T.vy), dy),
+               mz = add2(dup2(T.vz), dz);
+      dm = fma2(dz, mz, fma2(dy, my, mul2(dx, mx)));
+      mm = fma2(mz, mz, fma2(my, my, mul2(mx, mx)));
     }
-    const PairBin p = pair_bin<GEOM, BIN>(lin_const(L), ES, EP, dup2(s2),
-                                          dup2(dz), dup2(dm), dup2(mm));
-    bool plain = (fabsf(unpack2(p.f).x) < unpack2(p.h).x) &
-                 (fabsf(unpack2(p.g).x) < unpack2(p.k).x);
-    if (GEOM == FCFCG_GEOM_SURVEY && !IS_ISO(BIN)) plain &= mm >= L.m2min;
-    /* (next to the observer pi's error is not bounded: rechecked) */
-    if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && mm >= L.m2min &&
-        !(p.pi.x < L.p_lim))
-      continue;
-    int b = -1;
-    if (plain) {
-      const int s = (int) (__float_as_uint(unpack2(p.col).x) - TMAGIC_BITS) -
+    const PairBin p = pair_bin<GEOM, BIN>(C, ES, EP, s2, dz, dm, mm);
+    const float2 f = unpack2(p.f), fh = unpack2(p.h), g = unpack2(p.g),
+                 gk = unpack2(p.k), mm2 = unpack2(mm), col = unpack2(p.col),
+                 nq = unpack2(p.nq);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int i = i0 + e;
+      if (!(mine >> i & 1u)) continue;
+      const float m = e ? mm2.y : mm2.x;
+      bool plain = (fabsf(e ? f.y : f.x) < (e ? fh.y : fh.x)) &
+                   (fabsf(e ? g.y : g.x) < (e ? gk.y : gk.x));
+      if (GEOM == FCFCG_GEOM_SURVEY && !IS_ISO(BIN)) plain &= m >= L.m2min;
+      /* (next to the observer pi's error is not bounded: rechecked) */
+      if (GEOM == FCFCG_GEOM_SURVEY && IS_SPI(BIN) && m >= L.m2min &&
+          !((e ? p.pi.y : p.pi.x) < L.p_lim))
+        continue;
+      if (!plain) {
+        mask |= 1u << i;
+        continue;
+      }
+      const int s = (int) (__float_as_uint(e ? col.y : col.x) - TMAGIC_BITS) -
                     L.hcol0,
-                q = (int) -unpack2(p.nq).x - L.hrow0;
-      if (s >= 0 && s < L.ns && q >= 0 && q < L.hrows) b = s + q * L.ns;
-    }
-    if (!plain) {
-      mask |= 1u << i;
-    } else if (b >= 0) {
+                q = (int) -(e ? nq.y : nq.x) - L.hrow0;
+      if (s < 0 || s >= L.ns || q < 0 || q >= L.hrows) continue;
+      const int bin = s + q * L.ns;
       n_in++;
       if (WT) {
         const float4 wa = S->aw[i];
-        add128((M ? M->gwt : L.gwt) + 2 * b,
+        add128(out + 2 * bin,
                fix_prod(__float_as_int(wa.x), wa.y, wa.z, T.wi, T.wr, T.wf));
       } else {
-        atomicAdd((M ? M->gcnt : L.gcnt) + b, 1ull);
+        asm volatile("red.global.add.u64 [%0], 1;"
+                     :: "l"(__cvta_generic_to_global(out + bin)) : "memory");
       }
     }
   }
