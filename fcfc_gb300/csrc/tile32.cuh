@@ -570,43 +570,70 @@ __device__ __noinline__ uint32_t tile_global(const fcfcg_launch &L,
   return mask;
 }
 
+/* A pair by the FP64 formula where the queue is full: is it in range? */
+template <int WT, int ADJ>
+__device__ __forceinline__ uint32_t rest_bin(const fcfcg_launch &L, uint32_t a,
+    uint32_t b, uint32_t c) {
+  const fcfcg_mock *M = L.mocks ? L.mocks + (c >> 6) : NULL;
+  const int bin = ref_bin_pair(L, a, b, c & 63u, M ? M->box : L.box);
+  if (bin < 0) return 0u;
+  if (ADJ) adj_pair(L, a, b, bin);
+  else if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, b));
+  else atomicAdd((M ? M->gcnt : L.gcnt) + bin, 1ull);
+  return 1u;
+}
+
 /*
- * The collected pairs to the FP64 recheck queue -- the warp reserves their
- * places with one atomic -- and those beyond the queue's capacity are binned
- * here by the FP64 formula.  Every pair counts in the queue's 64-bit fill
- * counter, queued or not, so the counter cannot wrap and hand out slots twice.
+ * The collected pairs, and those of a tile that are left (bit i of rest: this
+ * lane's point and A's i), to the FP64 recheck queue -- the warp reserves their
+ * places with one atomic, whose answer it waits for: where the observer is
+ * inside a survey tiles leave hundreds of pairs each (3e4 points around it,
+ * (s, mu): 0.69 ms 32 at a time, 0.31 so).  Those beyond the queue's capacity
+ * are binned here by the FP64 formula.  Every pair counts in the queue's 64-bit
+ * fill counter, queued or not, so the counter cannot wrap and hand out slots
+ * twice.
  */
 template <int WT, int ADJ>
-__device__ __noinline__ void rest_flush(const fcfcg_launch &L, TileWarp *t) {
+__device__ __noinline__ void rest_flush(const fcfcg_launch &L, TileWarp *t,
+    uint32_t rest, uint32_t first, uint32_t bj, uint32_t code) {
   const int lane = threadIdx.x & 31;
   __syncwarp();
-  const uint32_t n = t->nrest;
-  unsigned long long slot = 0;
-  if (lane == 0 && n) slot = atomicAdd(L.qcount, (unsigned long long) n);
-  slot = __shfl_sync(FULLMASK, slot, 0) + (unsigned long long) lane;
-  const bool mine = (uint32_t) lane < n, full = mine && slot >= L.qcap;
-  if (mine) {
-    const uint32_t a = t->ra[lane], b = t->rb[lane], c = t->rc[lane];
-    if (!full) ((uint4 *) L.queue)[slot] = make_uint4(a, b, c & 63u, c >> 6);
+  const uint32_t n = t->nrest, own = (uint32_t) __popc(rest);
+  uint32_t upto = own;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(FULLMASK, upto, o);
+    if (lane >= o) upto += v;
   }
-  uint32_t n_in = 0;
-  if (full) {
+  const uint32_t total = n + __shfl_sync(FULLMASK, upto, 31);
+  unsigned long long slot = 0;
+  if (lane == 0 && total) slot = atomicAdd(L.qcount, (unsigned long long) total);
+  slot = __shfl_sync(FULLMASK, slot, 0);
+  uint32_t n_in = 0, n_inl = 0;
+  if ((uint32_t) lane < n) {
     const uint32_t a = t->ra[lane], b = t->rb[lane], c = t->rc[lane];
-    const fcfcg_mock *M = L.mocks ? L.mocks + (c >> 6) : NULL;
-    const int bin = ref_bin_pair(L, a, b, c & 63u, M ? M->box : L.box);
-    if (bin >= 0) {
-      n_in = 1;
-      if (ADJ) adj_pair(L, a, b, bin);
-      else if (WT) add128((M ? M->gwt : L.gwt) + 2 * bin, fix_prod_pair(L, a, b));
-      else atomicAdd((M ? M->gcnt : L.gcnt) + bin, 1ull);
+    if (slot + lane < L.qcap) {
+      ((uint4 *) L.queue)[slot + lane] = make_uint4(a, b, c & 63u, c >> 6);
+    } else {
+      n_inl++;
+      n_in += rest_bin<WT, ADJ>(L, a, b, c);
+    }
+  }
+  for (slot += n + upto - own; rest; slot++) {
+    const uint32_t a = first + (uint32_t) (__ffs((int) rest) - 1);
+    rest &= rest - 1u;
+    if (slot < L.qcap) {
+      ((uint4 *) L.queue)[slot] = make_uint4(a, bj, code & 63u, code >> 6);
+    } else {
+      n_inl++;
+      n_in += rest_bin<WT, ADJ>(L, a, bj, code);
     }
   }
   __syncwarp();
   n_in = __reduce_add_sync(FULLMASK, n_in);
-  const uint32_t n_inl = (uint32_t) __popc(__ballot_sync(FULLMASK, full));
+  n_inl = __reduce_add_sync(FULLMASK, n_inl);
   if (lane == 0) {
     t->cnt[1] += n_in;
-    t->cnt[2] += n;
+    t->cnt[2] += total;
     t->cnt[3] += n_inl;
     t->nrest = 0;
   }
@@ -623,7 +650,10 @@ __device__ __forceinline__ void tile_rest(const fcfcg_launch &L, TileWarp *t,
   uint32_t bal;
   while ((bal = __ballot_sync(FULLMASK, rest != 0u)) != 0u) {
     const uint32_t n = (uint32_t) __popc(bal);
-    if (t->nrest + n > 32u) rest_flush<WT, ADJ>(L, t);
+    if (t->nrest + n > 32u) {
+      rest_flush<WT, ADJ>(L, t, rest, first, bj, code);
+      break;
+    }
     const uint32_t at = t->nrest + (uint32_t) __popc(bal & below);
     if (rest) {
       t->ra[at] = first + (uint32_t) (__ffs((int) rest) - 1);
@@ -1460,10 +1490,10 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
               if (!ADJ && !L.hist_smem)
                 rest = tile_global<GEOM, BIN, WT>(L, T, S, rest, ES, EP);
               /* (in place where the loop has many values to keep: the call
-               * saves them, 0.9 % of a weighted (s, mu) count; the others
-               * gain 2 % by the registers) */
+               * saves them, 0.9 % of a weighted (s, mu) count; the others gain
+               * 2 % by the registers, survey (s_perp, pi) 1.6 %) */
               const uint32_t code = T.code | T.mock << 6;
-              if (WT && (SURVEY || !IS_SPI(BIN)))
+              if (WT && !IS_SPI(BIN))
                 tile_rest<WT, ADJ>(L, &S->t, rest, T.first, T.bj, code);
               else
                 tile_rest_call<WT, ADJ>(L, &S->t, rest, T.first, T.bj, code);
@@ -1513,7 +1543,7 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
     if (L.hist_smem)
       tile_handover<WT, F64>(L, h, 0, threadIdx.x, CT32_THREADS, &S->t);
   }
-  if (!F64) rest_flush<WT, ADJ>(L, &S->t);
+  if (!F64) rest_flush<WT, ADJ>(L, &S->t, 0u, 0u, 0u, 0u);
   __syncwarp();
   if (lane < 4) atomicAdd(L.stats + lane, S->t.cnt[lane]);
 }

@@ -73,3 +73,39 @@ def test_single_pairs_across_the_observer(length):
         pc.load(1, y)
         np.testing.assert_array_equal(pc.count_pairs(0, 1),
                                       ob.count(x, y, mode=1))
+
+
+@pytest.mark.parametrize("bintype", [1, 2])
+@pytest.mark.parametrize("cap", [0, 37, 5000, None])
+def test_tiles_of_rechecks(bintype, cap):
+    """Catalogues around the observer, whose tiles leave hundreds of pairs each to
+    the recheck queue: with room for all, some or none."""
+    import fcfc_gb300 as fg
+    kw, ok = dict(smin=0, smax=40, ds=4), dict(smin=0, ds=4, ns=10)
+    if bintype == 1:
+        kw["nmu"] = ok["nmu"] = 12
+    else:
+        kw.update(pmin=0, pmax=30, dpi=2)
+        ok.update(pmin=0, dpi=2, np_=15)
+    pc, ob = fg.PairCounter("survey", bintype, **kw), fo.Bins(True, bintype, **ok)
+    rng = np.random.default_rng(7)
+    a, b = 20.0 * rng.normal(size=(1500, 3)), 20.0 * rng.normal(size=(700, 3))
+    w = rng.integers(1, 4, len(a)).astype(float)
+    if cap is not None:
+        pc.set_queue_capacity(cap)
+    pc.load(0, a, w)
+    pc.load(1, b)
+    for other in (None, 1):
+        y = None if other is None else b
+        np.testing.assert_array_equal(pc.count_pairs(0, other), ob.count(a, y, mode=1))
+        st = pc.stats()
+        assert st["in_range"] == ob.count(a, y, mode=1).sum()
+        assert st["rechecked"] > st["in_range"] // 2
+        assert st["recheck_inline"] == (0 if cap is None else st["rechecked"] - cap)
+        # (integer weights: exact sums)
+        np.testing.assert_array_equal(pc.count_pairs(0, other, weighted=True),
+                                      ob.count(a, y, wa=w, mode=1))
+    g = rng.integers(-3, 4, pc.ntot).astype(float)
+    got, want = pc.adjoint(0, 1, g), ob.adjoint(a, g, b=b, wa=w)
+    for x, y in zip(got, want):
+        np.testing.assert_array_equal(x, y)
