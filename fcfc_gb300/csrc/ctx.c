@@ -1447,7 +1447,10 @@ typedef struct {
  * points of the neighbour side; nsten cells each).  Where 16 parts make less
  * than 2 items per warp (16 with f64, whose tiles are long), up to 8 times as
  * many by single tiles (tshift of the log; survey graph of 1.4e4 x 6.9e4
- * points: 1.11 -> 1.06 ms).  A batch, whose CTAs wait for
+ * points: 1.11 -> 1.06 ms).  Places left unused, of which sparse catalogues have
+ * as many as cells, cost an item each: no more parts than make 8 items per warp
+ * (16 with f64) with them (1e3 points of a survey in 2.9e3 cells, f64: 128 parts
+ * 250 us, 32 parts 76).  A batch, whose CTAs wait for
  * their last warp at the end of every run of items: all blocks, 16 items per
  * warp (48 mocks of 2e4 to 6e4 points: 6.81 ms; 7.08 with 8, 7.16 with 64,
  * 6.94 with the last ones in parts).
@@ -1457,11 +1460,16 @@ static void tile_parts(size_t na, size_t nb, size_t ncell, int nsten, int nsm,
   const double warps = 32.0 * nsm, want = batch ? 16 : 8;
   double blocks = (double) na / 32 + 0.5 * (double) (na < ncell ? na : ncell);
   if (!batch && blocks > 2 * warps) blocks = 2 * warps;
+  /* places dealt, with those left unused */
+  const double places = fmin((double) fcfcg_max_blocks(na, ncell),
+                             batch ? 1e18 : 2 * warps);
   const double groups = nsten * ceil((double) nb / 32 / 32 / (double) ncell);
   int p = 0, t = 0;
-  while (p < 4 && blocks * (double) (1 << p) <
-                      (groups >= 7.0 * (1 << p) ? want : 4) * warps) p++;
+  while (p < 4 && places * (double) (1 << p) < want * warps &&
+         blocks * (double) (1 << p) <
+             (groups >= 7.0 * (1 << p) ? want : 4) * warps) p++;
   while (p == 4 && t < 3 &&
+         places * (double) (1 << (p + t)) < (f64 ? 16 : 8) * warps &&
          blocks * (double) (1 << (p + t)) < (f64 ? 16 : 2) * warps) t++;
   L->pshift = p + t;
   L->tshift = t;
