@@ -277,17 +277,28 @@ int fcfcg_axis_ftab(fcfcg_axis *a, int allow_log) {
 }
 
 /*
- * Edge table: cells a fixed fraction of an octave wide (16 to 4096 per
- * octave), each with the one edge that lies in it or within half its width
- * of it, as a float, and the column below that edge (0 below the first edge,
- * k + 1 in bin k).  A value of the cell has no other edge within half a
- * cell, so with a window below that the bin and its certainty follow from
- * the one comparison.  A cell with several edges near holds a NaN, which
- * every comparison fails: ambiguous.  The cells run from below the lowest
- * positive edge to above top; the finest spacing that leaves no NaN cell is
- * not exceeded, nor ETAB_MAX cells.
+ * Edge tables: cells a fixed fraction of an octave wide (16 to 4096 per
+ * octave), each with the one edge that lies in it or within a margin (a
+ * fraction of its width) of it, as a float, and the column below that edge (0
+ * below the first edge, k + 1 in bin k).  A value of the cell has no other edge
+ * within the margin, so with a window below that the bin and its certainty
+ * follow from the one comparison.  A cell with several edges near holds a NaN,
+ * which every comparison fails: ambiguous.  The cells run from below the lowest
+ * positive edge to above top.
+ *
+ * The general table: margins of half a cell, the coarsest cells that leave no
+ * NaN, or the finest that ETAB_MAX hold.  Where that leaves NaN, as with hundreds
+ * of bins, finer ones: margins of a half and of an eighth, for s and s_perp up
+ * to ETAB_BIG cells, cut off at the low end where there would be more still; for
+ * each margin the one with the smallest share of the range (in s^2, s_perp^2,
+ * pi) ambiguous, a big table (which leaves an SM fewer CTAs) counted as a
+ * twentieth of it.  A count takes the one that its windows leave the least
+ * ambiguous (ctx.c:etab_use).  With the general table alone most pairs of such
+ * bins went to the recheck: 5e4 points, 3000 log bins 6.48 ms a pass, 0.52 so;
+ * 500 linear s_perp bins 0.87, 0.27.
  */
 #define ETAB_MAX 4096
+#define ETAB_BIG 12288
 static float etab_value(long c, int lg) {
   const uint32_t u = (uint32_t) c << lg;
   float f;
@@ -301,55 +312,94 @@ static long etab_cell(double v, int lg) {
   return (long) (u >> lg);
 }
 
+/* Edges in cell i or within mg of its width of it (2: or more); *k: the edges
+ * below that, from those below an earlier cell on. */
+static int etab_near(const double *e, int n, long i, int lg, double mg,
+    int *k) {
+  const double x0 = etab_value(i, lg), x1 = etab_value(i + 1, lg);
+  const double w = mg * (x1 - x0);
+  while (*k <= n && e[*k] < x0 - w) (*k)++;
+  int near = 0;
+  while (near < 2 && *k + near <= n && e[*k + near] <= x1 + w) near++;
+  return near;
+}
+
+/* The cells of a table: all, or the highest cap; 0 if that leaves more than a
+ * fifth of the range out. */
+static int etab_cells(const double *e, int n, double first, double top, int lg,
+    double mg, long cap, fcfcg_etab *E) {
+  const long hi = etab_cell(top * 1.05, lg) + 2;
+  memset(E, 0, sizeof *E);
+  E->off = etab_cell(first * 0.8, lg) - 1;
+  E->lg = lg;
+  E->margin = mg;
+  if (cap && hi - E->off > cap) {
+    E->off = hi - cap;
+    E->cut = 1;
+    E->amb = etab_value(E->off, lg) / top;
+    if (E->amb > 0.2) return 0;
+  }
+  E->n = (int) (hi - E->off);
+  int k = 0;
+  for (int c = 0; c < E->n; c++)
+    if (etab_near(e, n, E->off + c, lg, mg, &k) > 1)
+      E->amb += (etab_value(E->off + c + 1, lg) - etab_value(E->off + c, lg)) / top;
+  return 1;
+}
+
+static int etab_fill(const double *e, int n, fcfcg_etab *E) {
+  float *t = E->t = malloc(sizeof(float) * 2 * (E->n + 2));
+  if (!t) return FCFCG_ERR_MEMORY;
+  int k = 0;
+  for (int c = 0; c < E->n; c++) {
+    const int near = etab_near(e, n, E->off + c, E->lg, E->margin, &k);
+    t[2 * c] = near == 1 ? (float) e[k] : (near ? NAN : INFINITY);
+    t[2 * c + 1] = 12582912.f + (float) k;   /* k edges below: column k */
+  }
+  /* values below the cells: none of the edges is near, or (where the windows
+   * exceed the cells, or edges are below them) ambiguous */
+  t += 2 * E->n;
+  t[0] = INFINITY;
+  t[1] = 12582912.f + (e[0] > 0 ? 0.f : 1.f);
+  t[2] = NAN;
+  t[3] = 12582912.f;
+  return FCFCG_OK;
+}
+
 int fcfcg_axis_etab(fcfcg_axis *a, double top, int root) {
   const int n = a->nbin;
   double *e = malloc(sizeof(double) * (n + 1));
   if (!e) return FCFCG_ERR_MEMORY;
   for (int k = 0; k <= n; k++) e[k] = root ? sqrt(a->edge[k]) : a->edge[k];
   const double first = e[0] > 0 ? e[0] : e[1];
-  free(a->etab);
-  a->etab = NULL;
-  for (int lg = 23 - 4; lg >= 23 - 12; lg--) {
-    const long lo = etab_cell(first * 0.8, lg) - 1,
-               hi = etab_cell(top * 1.05, lg) + 2;
-    const long m = hi - lo;
-    if (a->etab && m > ETAB_MAX) break;
-    float *t = malloc(sizeof(float) * 2 * (m + 2));
-    if (!t) {
-      free(e);
-      return FCFCG_ERR_MEMORY;
-    }
-    int multi = 0, k = 0;      /* k: the first edge above the cell's margin */
-    for (long c = 0; c < m; c++) {
-      const double x0 = etab_value(lo + c, lg), x1 = etab_value(lo + c + 1, lg);
-      const double w = 0.5 * (x1 - x0);
-      while (k <= n && e[k] < x0 - w) k++;
-      int near = 0;
-      while (k + near <= n && e[k + near] <= x1 + w) near++;
-      float edge = INFINITY;
-      if (near == 1) edge = (float) e[k];
-      if (near > 1) {
-        edge = NAN;
-        multi = 1;
-      }
-      t[2 * c] = edge;
-      t[2 * c + 1] = 12582912.f + (float) k;   /* k edges below: column k */
-    }
-    /* values below the cells: none of the edges is near, or (where the
-     * windows exceed the cells) ambiguous */
-    t[2 * m] = INFINITY;
-    t[2 * m + 1] = 12582912.f + (e[0] > 0 ? 0.f : 1.f);
-    t[2 * m + 2] = NAN;
-    t[2 * m + 3] = 12582912.f;
-    free(a->etab);
-    a->etab = t;
-    a->netab = (int) m;
-    a->elg = lg;
-    a->eoff = lo;
-    if (!multi) break;
+  for (int i = 0; i < FCFCG_NETAB; i++) {
+    free(a->etab[i].t);
+    memset(a->etab + i, 0, sizeof *a->etab);
   }
+  fcfcg_etab E, *G = a->etab;
+  for (int lg = 23 - 4; lg >= 23 - 12 && !(G->n && G->amb == 0); lg--) {
+    etab_cells(e, n, first, top, lg, 0.5, 0, &E);
+    if (G->n && E.n > ETAB_MAX) break;
+    *G = E;
+  }
+  for (int i = 1; i < FCFCG_NETAB && G->amb > 0; i++) {
+    double cost = 0.9 * G->amb;       /* (a finer one has to be worth it) */
+    for (int c = 0; c < (root ? 1 : 2); c++)
+      for (int lg = 23 - 4; lg >= 23 - 12; lg--) {
+        if (!etab_cells(e, n, first, top, lg, i == 1 ? 0.5 : 0.125,
+                        c ? ETAB_BIG : ETAB_MAX, &E)) break;
+        const double v = E.amb + (E.n > ETAB_MAX ? 0.05 : 0);
+        if (v < cost) {
+          cost = v;
+          a->etab[i] = E;
+        }
+      }
+  }
+  int rc = FCFCG_OK;
+  for (int i = 0; i < FCFCG_NETAB && !rc; i++)
+    if (a->etab[i].n) rc = etab_fill(e, n, a->etab + i);
   free(e);
-  return FCFCG_OK;
+  return rc;
 }
 
 /* allow_log: the kernels can use a bit-pattern FP32 table for this axis
@@ -376,7 +426,7 @@ static void axis_free(fcfcg_axis *a) {
   free(a->rtab);
   free(a->ftab);
   free(a->fedge);
-  free(a->etab);
+  for (int i = 0; i < FCFCG_NETAB; i++) free(a->etab[i].t);
   memset(a, 0, sizeof *a);
 }
 

@@ -58,7 +58,8 @@ struct fcfcg_ctx {
   size_t rank_cap, key_cap;
   uint16_t *d_rs, *d_rp;
   double *d_s2edge, *d_pedge;
-  float *d_se, *d_pe;             /* edge tables of the tile kernel */
+  /* edge tables of the tile kernel */
+  float *d_se[FCFCG_NETAB], *d_pe[FCFCG_NETAB];
   int *d_sten;                    /* the stencil's entries, displacements */
   int sten_up;                    /* entries there (h_sten holds them) */
   int *h_sten;                    /* pinned: what was copied there */
@@ -215,7 +216,8 @@ void fcfcg_destroy(fcfcg_ctx *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (int i = 0; i <= FCFCG_MAX_SLOT; i++) slot_free(c->slot + i);
     void *p[] = {c->cfill, c->fstart, c->rank, c->key, c->scan_tmp,
-                 c->d_se, c->d_pe, c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
+                 c->d_se[0], c->d_se[1], c->d_se[2], c->d_pe[0], c->d_pe[1],
+                 c->d_pe[2], c->d_rs, c->d_rp, c->d_s2edge, c->d_pedge,
                  c->d_sten, c->d_res,
                  c->d_bbox, c->d_wd, c->d_gtab, c->d_queue, c->d_cnvt,
                  c->d_mock, c->d_mbase, c->d_bout, c->d_bstat, c->d_grad,
@@ -281,13 +283,17 @@ int fcfcg_create(const fcfcg_binning *cfg, int device, fcfcg_ctx **out) {
   rc = upload(c, (void **) &c->d_s2edge, b->s.edge,
               sizeof(double) * (b->s.nbin + 1));
   if (rc) return rc;
-  rc = upload(c, (void **) &c->d_se, b->s.etab,
-              sizeof(float) * 2 * (b->s.netab + 2));
-  if (rc) return rc;
+  for (int i = 0; i < FCFCG_NETAB; i++)
+    if (b->s.etab[i].n &&
+        (rc = upload(c, (void **) &c->d_se[i], b->s.etab[i].t,
+                     sizeof(float) * 2 * (b->s.etab[i].n + 2))))
+      return rc;
   if (b->bintype == FCFCG_BIN_SPI) {
-    rc = upload(c, (void **) &c->d_pe, b->p.etab,
-                sizeof(float) * 2 * (b->p.netab + 2));
-    if (rc) return rc;
+    for (int i = 0; i < FCFCG_NETAB; i++)
+      if (b->p.etab[i].n &&
+          (rc = upload(c, (void **) &c->d_pe[i], b->p.etab[i].t,
+                       sizeof(float) * 2 * (b->p.etab[i].n + 2))))
+        return rc;
     rc = upload(c, (void **) &c->d_rp, b->p.rtab, sizeof(uint16_t) * b->p.nrtab);
     if (rc) return rc;
     rc = upload(c, (void **) &c->d_pedge, b->p.edge,
@@ -991,28 +997,39 @@ static int even_edges(const fcfcg_axis *x, int root, double *a, double *d) {
   return 1;
 }
 
-/* The cells of an axis' edge table in use, given the window at a value (w0 +
- * w1 v): from *skip on, where it is below 0.45 of a cell; *last: the entry
- * for the values below.  0 if the windows fit nowhere useful. */
+/* The edge table of an axis and its cells in use, given the window at a value
+ * (w0 + w1 v): from *skip on, where it is below 0.9 of the margin; *last: the
+ * entry for the values below.  Of the tables that the windows fit the one with
+ * the least of the range ambiguous: its number, or -1 if they fit none. */
 static int etab_use(const fcfcg_axis *x, double w0, double w1, double vmax,
     int *n, int *lg, int *off, int *skip, int *last) {
-  int c0 = 0;
-  double v0 = 0;
-  for (long c = x->netab - 1; c >= 0; c--) {
-    const double x0 = ftab_cell_value(x->eoff + c, x->elg),
-                 x1 = ftab_cell_value(x->eoff + c + 1, x->elg);
-    if (!(w0 + w1 * x1 < 0.45 * (x1 - x0))) {
-      c0 = (int) c + 1;
-      v0 = x1;
-      break;
+  int use = -1;
+  double least = INFINITY;
+  for (int i = 0; i < FCFCG_NETAB; i++) {
+    const fcfcg_etab *E = x->etab + i;
+    if (!E->n) continue;
+    int c0 = 0;
+    double v0 = 0;
+    for (long c = E->n - 1; c >= 0; c--) {
+      const double x0 = ftab_cell_value(E->off + c, E->lg),
+                   x1 = ftab_cell_value(E->off + c + 1, E->lg);
+      if (!(w0 + w1 * x1 < 0.9 * E->margin * (x1 - x0))) {
+        c0 = (int) c + 1;
+        v0 = x1;
+        break;
+      }
     }
+    const double amb = E->amb + v0 / vmax;
+    if (!(v0 <= 0.25 * vmax) || !(amb < least)) continue;
+    least = amb;
+    use = i;
+    *skip = c0;
+    *n = E->n - c0 + 1;
+    *lg = E->lg;
+    *off = (int) E->off + c0;
+    *last = E->n + (c0 || E->cut ? 1 : 0);
   }
-  *skip = c0;
-  *n = x->netab - c0 + 1;
-  *lg = x->elg;
-  *off = (int) x->eoff + c0;
-  *last = x->netab + (c0 ? 1 : 0);
-  return v0 <= 0.25 * vmax;
+  return use;
 }
 
 /*
@@ -1118,11 +1135,11 @@ static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
       rows = b->np + 2;
       L->hrow0 = 1;
       L->tl_hp = nextafterf((float) Wv, INFINITY);
-      if (b->p.nbin > FCFCG_FTAB_MAXBIN ||
-          !etab_use(&b->p, Wv, 0, pmax, &L->npe, &L->pe_lg, &L->pe_off,
-                    &L->pe_skip, &L->pe_last))
-        return -1;
-      L->pe = c->d_pe;
+      const int use = b->p.nbin > FCFCG_FTAB_MAXBIN ? -1
+          : etab_use(&b->p, Wv, 0, pmax, &L->npe, &L->pe_lg, &L->pe_off,
+                     &L->pe_skip, &L->pe_last);
+      if (use < 0) return -1;
+      L->pe = c->d_pe[use];
     }
     L->p_lim = (float) (pmax + TIGHT * Wv);
     if (!b->p.min0) L->tl_plo = (float) (pmin - TIGHT * Wv);
@@ -1164,11 +1181,11 @@ static int tile_bounds(const fcfcg_ctx *c, double dc, double K1, double K0a,
     const double Em = 1.01 * ((double) L->tl_ea * r2 + (double) L->tl_eb);
     const double w1 = (spi && !box) ? 0 : (double) L->tl_ea,
                  w0 = (spi && !box) ? Em : (double) L->tl_eb;
-    if (b->s.nbin > FCFCG_FTAB_MAXBIN || !(Em < 0.02 * b->s.vmax) ||
-        !etab_use(&b->s, w0, w1, b->s.vmax, &L->nse, &L->se_lg, &L->se_off,
-                  &L->se_skip, &L->se_last))
-      return -1;
-    L->se = c->d_se;
+    const int use = b->s.nbin > FCFCG_FTAB_MAXBIN || !(Em < 0.02 * b->s.vmax)
+        ? -1 : etab_use(&b->s, w0, w1, b->s.vmax, &L->nse, &L->se_lg,
+                        &L->se_off, &L->se_skip, &L->se_last);
+    if (use < 0) return -1;
+    L->se = c->d_se[use];
     L->hcols = b->ns + 2;
     L->hcol0 = 1;
     /* (a survey's window of s_perp^2 is at least its constant part) */

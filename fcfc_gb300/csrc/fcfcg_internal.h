@@ -27,6 +27,19 @@ extern "C" {
 #define FCFCG_FTAB_MAXBIN 4094    /* largest bin index an FP32 table holds */
 #define FCFCG_FTAB_MAXLEN 4096    /* cells of an FP32 table */
 
+/* An edge table (host): n cells of the value's FP32 bits >> lg, from cell off
+ * on, (edge, 1.5 2^23 + column) each, then two entries for the values below: no
+ * edge near, and ambiguous.  For windows below margin of a cell; cut: there are
+ * edges below the cells; amb: the ambiguous share of the range.  No table: n =
+ * 0. */
+#define FCFCG_NETAB 3
+typedef struct {
+  float *t;
+  int n, lg, cut;
+  long off;
+  double margin, amb;
+} fcfcg_etab;
+
 /*
  * One binned quantity (s^2, s_perp^2, pi or pi^2), as FCFC looks it up:
  * reference table rtab over (int) v - roff with FCFC's integer / hybrid
@@ -47,12 +60,10 @@ typedef struct {
   float *fedge;          /* nbin + 1 edges rounded to FP32 (host) */
   double vmin, vmax;     /* edge[0], edge[nbin] */
   int min0;              /* edge[0] == 0: no lower range check (smin0) */
-  /* edge table of the tile kernel (host): netab cells of the value's FP32
-   * bits >> elg, from cell eoff on, (edge, 1.5 2^23 + column) each, then two
-   * entries for the values below: no edge near, and ambiguous */
-  float *etab;
-  int netab, elg;
-  long eoff;
+  /* edge tables of the tile kernel: the general one and, where edges are too
+   * close for it, finer ones with margins of a half and an eighth of a cell
+   * (bins.c:fcfcg_axis_etab) */
+  fcfcg_etab etab[FCFCG_NETAB];
 } fcfcg_axis;
 
 typedef struct {
@@ -74,7 +85,7 @@ void fcfcg_bins_release(fcfcg_bins *b);
 /* Build the FP32 window table of an axis (ftab / foff / nftab); allow_log:
  * a bit-pattern table may replace a uniform one with multi-edge cells. */
 int fcfcg_axis_ftab(fcfcg_axis *a, int allow_log);
-/* Build the tile kernel's edge table of an axis for values up to top;
+/* Build the tile kernel's edge tables of an axis for values up to top;
  * root: of the square roots of the edges (pi of a survey). */
 int fcfcg_axis_etab(fcfcg_axis *a, double top, int root);
 /* Accessors of the opaque context used by the post-processing code. */
