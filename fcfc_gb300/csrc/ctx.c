@@ -1377,7 +1377,6 @@ static void launch_bins(const fcfcg_ctx *c, fcfcg_launch *L) {
   L->rpoff = b->p.roff;
   L->nrs = b->s.nrtab;
   L->nrp = b->p.nrtab;
-  L->tabtype = b->s.tabtype;
   L->s2edge = c->d_s2edge;
   L->pedge = c->d_pedge;
   L->s2min = b->s.vmin;
@@ -1560,7 +1559,6 @@ static int count_plan_make(fcfcg_ctx *c, slot_t *A, slot_t *B, int isauto,
     L->lo[d] = g->lo[d];
     L->box[d] = b->box[d];
     L->cwf[d] = (float) g->cw[d];
-    L->lof[d] = (float) g->lo[d];
   }
   L->nsten = P->nsten;
   L->tzero = -1;
@@ -2560,7 +2558,6 @@ int fcfcg_count_batch(fcfcg_ctx *c, fcfcg_job *jobs, int njobs, int withwt,
   launch_cat(&L.B, S);
   launch_bins(c, &L);
   L.mocks = (const fcfcg_mock *) c->d_mock;
-  L.nmock = na;
   L.mbase = c->d_mbase;
   hist_shape(&L, fcfcg_k_tile32_tab(&L) + fcfcg_k_tile32_stage(withwt), 0);
   L.nblk_dev = S->bstart + cells;

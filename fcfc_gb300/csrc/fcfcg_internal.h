@@ -17,8 +17,9 @@ extern "C" {
 #define FCFCG_MAX_SLOT 8
 #define FCFCG_MAX_STENCIL 4096
 #define FCFCG_FIX_F 51            /* fractional bits of a weight product */
-/* FP32 edge-window tables: one uint16 per cell of width w = 2^-shift units
- * of the binned quantity; cell i covers [i w, (i + 1) w). */
+/* FP32 edge-window tables (of which only the cells per octave are used, for
+ * fcfcg_bins_info): one uint16 per cell of width w = 2^-shift units of the
+ * binned quantity; cell i covers [i w, (i + 1) w). */
 #define FCFCG_FTAB_BIN_MASK 0x0FFFu /* bin at the cell start, or "out" */
 #define FCFCG_FTAB_LO 0x1000u     /* an edge lies in [i w - w/2, i w] */
 #define FCFCG_FTAB_HI 0x2000u     /* an edge lies in [(i+1) w, (i+1) w + w/2] */
@@ -109,7 +110,8 @@ typedef struct {
    * a batch) per block */
   const float *blk;
   const uint32_t *bstart, *bcell;
-  int wexp;              /* weights scaled by 2^-wexp */
+  int wexp;              /* weights scaled by 2^-wexp (for a count graph, which
+                            compares its plans, as the sort's scale is captured) */
 } fcfcg_dcat;
 
 /* One catalogue of a batch (periodic boxes; all share the bins and the
@@ -127,7 +129,7 @@ typedef struct {
   int geometry, bintype, isauto, withwt;
   int ncell[3];
   double cw[3], lo[3], box[3];
-  float cwf[3], lof[3];
+  float cwf[3];
   /* stencil: nsten entries of int4 (ox, oy, oz, 0) and float4 (-o * cw) */
   int nsten;
   const int *sten;
@@ -135,7 +137,7 @@ typedef struct {
   uint32_t *item_head;
   /* tile kernel: the number of A blocks (device), log2 of the parts a
    * block's tiles are dealt to, slack of the block box distance, and for a
-   * batch the catalogues' first cells (nmock + 1) */
+   * batch the catalogues' first cells (their number + 1) */
   const uint32_t *nblk_dev;
   int pshift, tshift;
   uint32_t nsplit;       /* the blocks dealt in parts, the last ones */
@@ -179,7 +181,6 @@ typedef struct {
   /* FP64 reference binning */
   const uint16_t *rs, *rp;
   long rsoff, rpoff, nrs, nrp;
-  int tabtype;
   const double *s2edge, *pedge;
   double s2min, s2max, pmin, pmax;
   int smin0, pmin0;
@@ -202,7 +203,6 @@ typedef struct {
   unsigned long long hs_limit;
   /* batch of catalogues (NULL: one catalogue pair) */
   const fcfcg_mock *mocks;
-  int nmock;
   /* adjoint of the weighted counts: gadj[ntot] in, FP64 gradients per
    * sorted point out (dA, dB; the same array for auto counts) */
   int adjoint;

@@ -60,9 +60,12 @@ extern "C" {
 #define FCFCG_GEOM_BOX    0
 #define FCFCG_GEOM_SURVEY 1
 
-/* Precision of the separation arithmetic. */
+/* Precision of the separation arithmetic.  FP64: every pair that can be in range
+ * is binned in FP64; which pairs cannot is decided by FP32 distances with a bound
+ * on their error, and a mu bin is taken from an FP32 root where that is certain.
+ * The counts are those of the FP64 formula either way. */
 #define FCFCG_PREC_FP32_RECHECK 0  /* FP32 separations, FP64 recheck near edges */
-#define FCFCG_PREC_FP64         1  /* every pair in FP64 */
+#define FCFCG_PREC_FP64         1  /* every pair in range in FP64 */
 
 /* Lookup-table kinds (FCFC_LOOKUP_TYPE_*). */
 #define FCFCG_TAB_INT    0
@@ -102,9 +105,10 @@ typedef struct {
   double rescale;        /* coordinate rescale factor */
   double box_rescaled[3];
   int64_t nstab, nptab;  /* lookup-table lengths */
-  int ftab_cells_per_octave;  /* the FP32 s (or s_perp) window table: cells
-                                 per octave of a bit-pattern table (log bins
-                                 in a box), 0 for a uniform table */
+  int ftab_cells_per_octave;  /* an FP32 s (or s_perp) window table's cells
+                                 per octave where it goes by bit patterns (log
+                                 bins in a box), 0 for a uniform table (the
+                                 counting kernels have tables of their own) */
 } fcfcg_bins_info;
 
 /* Counters of the last fcfcg_count() call. */
@@ -120,7 +124,8 @@ typedef struct {
   int cells_per_smax;    /* grid refinement used */
   int ncell[3];
   int nstencil;
-  uint64_t nchunks;
+  uint64_t nchunks;      /* blocks of up to 32 points of the first catalogue,
+                            with the places left unused */
   int precision_used;    /* FCFCG_PREC_*: FP32 windows too wide fall to FP64 */
   uint64_t launches;     /* kernels launched by this context since creation */
   int warp_queue;        /* as fcfcg_set_warp_queue (FP32 counts) */
@@ -374,9 +379,11 @@ int fcfcg_set_queue_capacity(fcfcg_ctx *ctx, size_t cap);
 /* Unweighted counts in the FP32 kernel: a CTA's shared-memory bins are 32
  * bits wide and take their adds unchecked, so the CTA hands them to the
  * global 64-bit counters before the pairs it may have added since the last
- * hand-over (a tile of m by t points adds at most m t) could pass this
- * threshold.  1..2^32 - 1, or 0 (default) for 2^32 - 1.  The counts do not
- * depend on it; meant for tests of that path. */
+ * hand-over (1024 for each tile visited) could pass this threshold.  1..2^32 -
+ * 1, or 0 (default) for 2^32 - 1.  The CTA's 8 warps look after every group of
+ * up to 32 tiles: a threshold below 8 x 2^16 is taken as a hand-over after each
+ * group, with up to 2^18 pairs in between.  The counts do not depend on it;
+ * meant for tests of that path. */
 int fcfcg_set_hist_handover(fcfcg_ctx *ctx, unsigned long long pairs);
 
 /*
