@@ -1719,7 +1719,7 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
     }
     if (P.prec == FCFCG_PREC_FP32_RECHECK) {
       /* the cotangent is scaled by 2^-gexp to at most 1, as the weights are:
-       * a term's unit is 2^-51 of the scales' product */
+       * a term's unit is 2^-52 of the scales' product */
       int gexp = 0;
       if (gmax > 0) {
         gexp = (int) ceil(log2(gmax));
@@ -1732,8 +1732,8 @@ static int count_impl(fcfcg_ctx *c, int sa, int sb, int isauto, int withwt,
         return FCFCG_ERR_ARG;
       }
       if (S > 1000) gexp += S - 1000;   /* units stay above 2^-1001 */
-      L->gunitA = ldexp(1.0, B->wexp + gexp - 51);
-      L->gunitB = ldexp(1.0, A->wexp + gexp - 51);
+      L->gunitA = ldexp(1.0, B->wexp + gexp - 52);
+      L->gunitB = ldexp(1.0, A->wexp + gexp - 52);
       gtab_exp = gexp;
     }
   }

@@ -234,25 +234,26 @@ __device__ __forceinline__ long long tile_prod(int ia, float ra, float fa,
 
 /*
  * Adjoint: the product of a weight and a cotangent entry, both scaled to at
- * most 1, in units of 2^-51: the integer parts (round(x 2^30)) multiply
- * exactly, the cross terms with the remainders (weight's: ra, scaled by 2^-30;
- * entry's: rb), at most 2^-30 in sum, are rounded to half units by the 1.5 2^23
- * trick (at most 2^22 of them), the product of the remainders (2^-11 of a unit)
- * is left out, and the sum is rounded to units once.  Within 1/2 + 1/4 unit and
- * the cross terms' FP32 roundings (the two remainders', the two factors', the
- * product's and the sum's: at most 7/32 unit) of the exact product: 0.97;
- * over 4e7 products the worst was 0.90 (with the cross terms rounded to whole
- * units 1.14).  An FP64 multiply-add per product kept the FP64 pipe the bound
- * (32 cycles of an SM per pair of a warp; GB300 has 2 FP64 lanes per SM), at
- * an error of up to 1.
+ * most 1, in units of 2^-52: the integer parts (round(x 2^30)) multiply exactly
+ * and are rounded by a shift, the cross terms with the remainders (weight's: ra,
+ * scaled by 2^-30; entry's: rb), at most 2^-30 in sum, by the 1.5 2^23 trick (at
+ * most 2^22 of them), and the product of the remainders (2^-10 of a unit) is left
+ * out.  Within 1/2 + 1/2 unit and the cross terms' FP32 roundings (the two
+ * remainders', the two factors', the product's and the sum's: at most 7/16
+ * unit): 1.44; over 4e7 products the worst was 1.29, and the mean 0, also for
+ * weights of 1, whose products have no low bits: with the sum of both rounded
+ * once to whole units, the cross terms' halves all go up (0.14 units a product,
+ * 10 times the error of a gradient of 5e5 terms).  An FP64 multiply-add per
+ * product kept the FP64 pipe the bound (32 cycles of an SM per pair of a warp;
+ * GB300 has 2 FP64 lanes per SM), at an error of up to 2 of these units.
  */
 __device__ __forceinline__ long long adj_prod(int ia, float ra, float fa,
     int ib, float rb, float ib_f) {
   const float c = __fmaf_rn(fa, rb, __fmul_rn(ra, ib_f));
   const float t = __fmaf_rn(c, 4503599627370496.0f /* 2^52 */, TMAGIC);
   const long long p = (long long) ia * (long long) ib +
-      (256ll - ((long long) TMAGIC_BITS << 8));
-  return (p + (long long) __float_as_int(t) * 256ll) >> 9;
+      (128ll - ((long long) TMAGIC_BITS << 8));
+  return (p + (long long) __float_as_int(t) * 256ll) >> 8;
 }
 
 __device__ __forceinline__ long long shfl_xor64(long long v, int o) {
@@ -278,9 +279,14 @@ __device__ __forceinline__ void adj_flush(const fcfcg_launch &L, TileWarpA *S,
     uint32_t first, int m) {
   const int lane = threadIdx.x & 31;
   __syncwarp();
-  long long v = 0;
-  for (int i = 0; i < 8; i++) v += S->ga[lane >> 2][(lane & 3) + 4 * i];
-  if (lane < m && v) atomicAdd(L.dA + first + lane, (double) v * L.gunitA);
+  /* (two sums: all eight words can pass 2^63) */
+  long long v = 0, u = 0;
+  for (int i = 0; i < 4; i++) {
+    v += S->ga[lane >> 2][(lane & 3) + 4 * i];
+    u += S->ga[lane >> 2][(lane & 3) + 16 + 4 * i];
+  }
+  if (lane < m && (v || u))
+    atomicAdd(L.dA + first + lane, ((double) v + (double) u) * L.gunitA);
   __syncwarp();
   for (int i = 0; i < 8; i++) S->ga[i][lane] = 0;
   __syncwarp();
@@ -1501,10 +1507,10 @@ k_tile32(const __grid_constant__ fcfcg_launch L) {
           }
         }
         if (ADJ && !F64) {
-          /* a term is at most 2^51 (2^51 itself for a weight and an entry of
-           * 1), a tile adds 32 of them to a point's eight words, whose sum
-           * adj_flush forms in 64 bits: out after at most 95 + 32
-           * tiles, 127 x 32 x 2^51 < 2^63 */
+          /* a term is at most 2^52 (2^52 itself for a weight and an entry of
+           * 1), a tile adds 32 of them to a point's eight words, which
+           * adj_flush adds up four at a time in 64 bits: out after at most 95 +
+           * 32 tiles, 127 x 16 x 2^52 < 2^63 */
           if (ntile > 127 - 32) {
             adj_flush(L, (TileWarpA *) S, T.first, T.m);
             ntile = 0;

@@ -338,9 +338,9 @@ void fcfcg_graph_destroy(fcfcg_graph *graph);
  * be NULL).  For auto counts every unordered pair feeds both of its points.
  * The pair bins are recomputed, exactly as the count bins them (FP32 windows
  * with the FP64 recheck).  Each product w_j g[b] is taken as an integer
- * multiple of 2^-51 of the scales (the powers of two not below max|w| of w's
+ * multiple of 2^-52 of the scales (the powers of two not below max|w| of w's
  * catalogue and max|g|), formed from 30-bit integers and FP32 remainders, within
- * one such unit of the exact product; a point's integers are added exactly
+ * 1.5 such units of the exact product; a point's integers are added exactly
  * over tiles of up to 32 points (the lanes' points) or over up to 127 tiles (the
  * block's), and those sums, like the products of the rechecked pairs, in FP64.
  * So every gradient is within n 2^-49 max|w| max|g| (plus the rounding of the
