@@ -1356,7 +1356,6 @@ static void launch_cat(fcfcg_dcat *D, const slot_t *S) {
   D->s = S->ss;
   D->w = S->sw;
   D->id = S->sid;
-  D->cstart = S->cstart;
   D->blk = S->blk;
   D->bstart = S->bstart;
   D->bcell = S->bcell;

@@ -103,7 +103,6 @@ typedef struct {
                             of the remainder, w scaled to |w| <= 1 */
   const double *x, *y, *z, *s, *w;   /* rescaled FP64, |x|^2, weight */
   const uint32_t *id;    /* input index */
-  const uint32_t *cstart;/* ncell + 1 */
   /* blocks of at most 32 points of a cell: two float4 each, (box centre,
    * bits of the first sorted index) and (half extents, bits of the count; 0
    * for a place left unused); bstart: the cells' first blocks (ncell + 1); bcell: (cell, catalogue of

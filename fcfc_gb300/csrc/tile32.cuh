@@ -32,15 +32,14 @@
  * so integer counts equal the FP64 build.
  *
  * What bounds it: instruction issue and the FMA pipe (unweighted (s, mu)
- * mocks: issue slots 81 % used, FMA pipe 52 %, ALU 57 %; weighted: 74 %, with
- * 64 % of the shared wavefronts).  1.35 warp instructions per in-range pair
- * (weighted 2.55, survey 3.4): 8 per pair slot for the distance test (1.7
- * slots per in-range pair) and 22 (54) for binning the slots whose step is not
- * empty.  A kernel that tested candidates first, queued them and binned them
+ * mocks: issue slots 80 % used, FMA pipe 51 %, ALU 57 %; weighted: 75 %, with
+ * 65 % of the shared wavefronts).  1.32 warp instructions per in-range pair
+ * (weighted 2.52, survey 3.33), with 1.44 (1.44, 1.76) pairs tested for each in
+ * range.  A kernel that tested candidates first, queued them and binned them
  * compacted took 2.8 (3.9, 4.8).  A pass before and after: (s, mu) box of 2e6
- * points weighted 33.6 -> 22.8 ms, (s_perp, pi) with log bins 6.4 -> 3.6, log
- * s bins of 4e5 points 3.9 -> 1.3, 256 mocks 631 -> 332, survey (s, mu) of 4e5
- * + 4e6 433 -> 308.
+ * points weighted 33.6 -> 22.4 ms, (s_perp, pi) with log bins 6.4 -> 3.6, log
+ * s bins of 4e5 points 3.9 -> 1.3, 256 mocks 631 -> 329, survey (s, mu) of 4e5
+ * + 4e6 433 -> 299.
  *
  * Histograms live in shared memory (u32 counts, or int64 fixed-point weight
  * products) and are merged into global 64/128-bit integer accumulators, so
@@ -938,7 +937,7 @@ __device__ __forceinline__ void bin64(const fcfcg_launch &L, TileWarp64 *S,
  * Bound by the FP64 pipe (2 lanes per SM and clock): 8 operations per pair
  * for the separation, and few others since the mu bin is taken from FP32
  * where that is certain (ref_mu).  Weighted (s, mu) count of a box of 3e4
- * points, 2.6e7 pairs: 15.0 -> 2.0 ms against a kernel that took every pair
+ * points, 2.6e7 pairs: 15.0 -> 1.7 ms against a kernel that took every pair
  * of the neighbouring cells, with an FP64 division each.
  */
 template <int GEOM, int WT, int ADJ>
